@@ -9,7 +9,7 @@
 // rule (Old/lib/thermodynamics.cpp:51-69, state.cpp:190-201) in FP32.
 #include <math.h>
 
-#include "nmmc_kernels.cuh"
+#include "nmmc_quad.cuh"
 
 namespace nmmc {
 
@@ -226,11 +226,10 @@ __device__ __forceinline__ void meas_block_rows(const float* acc, double* __rest
 // One quad (row `row`, first compact site h0) of one chain; the row's x offset of this colour
 // (x = 2h + xp) comes from (y + z + colour) per thread. With MEAS the quad's final spins are
 // summed into macc (see k_heis_half_q4); `active` false computes without storing or summing.
-template <int DIM, bool PERIODIC, int DK, int SPT, int MEAS>
+template <int DIM, bool PERIODIC, int DK, int MEAS>
 __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ spins, const float4* __restrict__ bh,
                                         const unsigned long long* __restrict__ sweep, unsigned sweep_off, int chain,
-                                        int colour, int row, int h0, bool active, float* macc, float esign) {
-    using VT = typename SiteVec<SPT>::T;
+                                        int colour, int row, int h0, bool active, f2* macc, float esign) {
     int y, z;
     if (DIM == 3) {
         z = (m.ly_shift >= 0) ? (row >> m.ly_shift) : (row / m.ly);
@@ -241,25 +240,30 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
     }
     const int xp = (y + z + colour) & 1;   // x = 2h + xp
     const size_t P = (size_t)m.nhalf_pad;
-    float* own = spins + ((size_t)chain * 2 + colour) * 3 * P;
-    const float* oth = spins + ((size_t)chain * 2 + (colour ^ 1)) * 3 * P;
-    const int rb = row * m.hx + h0;
+    float* own[3];
+    const float* oth[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        own[c] = spins + (((size_t)chain * 2 + colour) * 3 + c) * P;
+        oth[c] = spins + (((size_t)chain * 2 + (colour ^ 1)) * 3 + c) * P;
+    }
+    const uint32_t rb = (uint32_t)(row * m.hx + h0);
 
-    VT s[3], same[3], yp[3], ym[3], zp[3], zm[3];
-    const VT vz = {};
+    F2x2 s[3], same[3], yp[3], ym[3], zp[3], zm[3];
     float ex[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        s[c] = *reinterpret_cast<const VT*>(own + c * P + rb);
-        same[c] = __ldg(reinterpret_cast<const VT*>(oth + c * P + rb));
+        s[c] = ld_quad_rw(own[c], rb);
+        same[c] = ld_quad(oth[c], rb);
     }
-    // x-neighbour outside the quad: h0-1 (xp = 0) or h0+4 (xp = 1)
-    int hx_out = xp ? h0 + SPT : h0 - 1;
+    // x-neighbour outside the quad: h0-1 (xp = 0) or h0+4 (xp = 1); 0 past an open edge (the
+    // rows hold whole quads, so the other x-neighbours of the quad's sites are always inside)
+    int hx_out = xp ? h0 + 4 : h0 - 1;
     bool ex_ok = true;
     if (PERIODIC) hx_out = (hx_out < 0) ? m.hx - 1 : (hx_out >= m.hx ? 0 : hx_out);
     else ex_ok = hx_out >= 0 && hx_out < m.hx;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) ex[c] = ex_ok ? __ldg(oth + c * P + row * m.hx + hx_out) : 0.0f;
+    for (int c = 0; c < 3; ++c) ex[c] = ex_ok ? __ldg(oth[c] + (uint32_t)(row * m.hx + hx_out)) : 0.0f;
     // +-y rows
     {
         int yu = y + 1, yd = y - 1;
@@ -271,11 +275,11 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
             okU = yu < m.edge;
             okD = yd >= 0;
         }
-        const int ru = (z * m.ly + yu) * m.hx + h0, rd = (z * m.ly + yd) * m.hx + h0;
+        const uint32_t ru = (uint32_t)((z * m.ly + yu) * m.hx + h0), rd = (uint32_t)((z * m.ly + yd) * m.hx + h0);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            yp[c] = okU ? __ldg(reinterpret_cast<const VT*>(oth + c * P + ru)) : vz;
-            ym[c] = okD ? __ldg(reinterpret_cast<const VT*>(oth + c * P + rd)) : vz;
+            yp[c] = okU ? ld_quad(oth[c], ru) : zero_quad();
+            ym[c] = okD ? ld_quad(oth[c], rd) : zero_quad();
         }
     }
     if (DIM == 3) {
@@ -288,67 +292,58 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
             okU = zu < m.lz;
             okD = zd >= 0;
         }
-        const int ru = (zu * m.ly + y) * m.hx + h0, rd = (zd * m.ly + y) * m.hx + h0;
+        const uint32_t ru = (uint32_t)((zu * m.ly + y) * m.hx + h0), rd = (uint32_t)((zd * m.ly + y) * m.hx + h0);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            zp[c] = okU ? __ldg(reinterpret_cast<const VT*>(oth + c * P + ru)) : vz;
-            zm[c] = okD ? __ldg(reinterpret_cast<const VT*>(oth + c * P + rd)) : vz;
+            zp[c] = okU ? ld_quad(oth[c], ru) : zero_quad();
+            zm[c] = okD ? ld_quad(oth[c], rd) : zero_quad();
         }
     }
     const float4 p = bh[chain];
     const unsigned long long sw = sweep[chain] + sweep_off;
-    const uint32_t boxrow = (uint32_t)(m.edge * (y + m.edge * z));
-    constexpr int ND = 2 * DIM;
+    const uint32_t box = (uint32_t)(m.edge * (y + m.edge * z) + 2 * h0 + xp);
+    nmmc_u4 r0 = sweep_draw<true>(m, box, sw, (uint32_t)chain);
+    nmmc_u4 r1 = sweep_draw<true>(m, box + 2, sw, (uint32_t)chain);
+    F2x2 sh[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sh[c] = shifted_quad(same[c], ex[c], xp != 0);
+    f2 h[2][3], d[2][3];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        h[j][0] = pk(p.y, p.y);
+        h[j][1] = pk(p.z, p.z);
+        h[j][2] = pk(p.w, p.w);
+        d[j][0] = d[j][1] = d[j][2] = f2{0ull};
+    }
+    quad_axis_x<DK, MEAS != 0>(m, same, sh, xp != 0, h, d);
+    quad_axis<DK, 1, MEAS != 0>(m, yp, ym, h, d);
+    if (DIM == 3) quad_axis<DK, 2, MEAS != 0>(m, zp, zm, h, d);
     bool any = false;
-    nmmc_u4 rnext = sweep_draw<true>(m, boxrow + (uint32_t)(2 * h0 + xp), sw, (uint32_t)chain);
-    float out[3][SPT];
 #pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-        float nx[ND], ny[ND], nz[ND];
-        float* nn[3] = {nx, ny, nz};
+    for (int j = 0; j < 2; ++j) {
+        f2 v[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            // the neighbour of site h0+k at compact h0+k (same) and at h0+k-1 or h0+k+1 (shifted)
-            float sm = vel(same[c], k);
-            float sh = xp ? (k < SPT - 1 ? vel(same[c], k + 1) : ex[c]) : (k > 0 ? vel(same[c], k - 1) : ex[c]);
-            float plusx = xp ? sh : sm, minusx = xp ? sm : sh;
-            if (!PERIODIC) {
-                // open x boundary: the site at x = edge-1 has no +x neighbour, x = 0 no -x
-                const int x = 2 * (h0 + k) + xp;
-                if (x + 1 >= m.edge) plusx = 0.0f;
-                if (x == 0) minusx = 0.0f;
-            }
-            nn[c][0] = plusx;
-            nn[c][1] = minusx;
-            nn[c][2] = vel(yp[c], k);
-            nn[c][3] = vel(ym[c], k);
-            if (DIM == 3) {
-                nn[c][4] = vel(zp[c], k);
-                nn[c][5] = vel(zm[c], k);
-            }
+        for (int c = 0; c < 3; ++c) v[c] = j ? s[c].b : s[c].a;
+        const nmmc_u4 q0 = r0, q1 = r1;
+        if (j == 0) {   // the next pair's words are drawn while this pair's tests wait
+            r0 = sweep_draw<true>(m, box + 4, sw, (uint32_t)chain);
+            r1 = sweep_draw<true>(m, box + 6, sw, (uint32_t)chain);
         }
-        const float sx = vel(s[0], k), sy = vel(s[1], k), sz = vel(s[2], k);
-        float tx, ty, tz;
-        const nmmc_u4 r = rnext;
-        if (k < SPT - 1) rnext = sweep_draw<true>(m, boxrow + (uint32_t)(2 * (h0 + k + 1) + xp), sw, (uint32_t)chain);
-        float hx, hy, hz;
-        heis_field<ND, DK>(m, nx, ny, nz, p, hx, hy, hz);
-        const bool acc = heis_try(hx, hy, hz, sx, sy, sz, p, r, tx, ty, tz);
-        out[0][k] = acc ? tx : sx;
-        out[1][k] = acc ? ty : sy;
-        out[2][k] = acc ? tz : sz;
-        any |= acc;
+        any |= pair_try(h[j], v, p.x, q0, q1);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) (j ? s[c].b : s[c].a) = v[c];
         if (MEAS && active) {
-            float dx, dy, dz;
-            heis_dmi_part<ND, DK>(m, nx, ny, nz, dx, dy, dz);
-            const float fx = fmaf(esign, dx, hx - p.y), fy = fmaf(esign, dy, hy - p.z), fz = fmaf(esign, dz, hz - p.w);
-            macc[0] = fmaf(out[0][k], fx, fmaf(out[1][k], fy, fmaf(out[2][k], fz, macc[0])));
+            // the energy's field: the sweep's without H, its DMI part with the energy's sign
+            const f2 es = pk(esign, esign);
+            const f2 fx = fma2(es, d[j][0], sub2(h[j][0], pk(p.y, p.y)));
+            const f2 fy = fma2(es, d[j][1], sub2(h[j][1], pk(p.z, p.z)));
+            const f2 fz = fma2(es, d[j][2], sub2(h[j][2], pk(p.w, p.w)));
+            macc[0] = fma2(v[0], fx, fma2(v[1], fy, fma2(v[2], fz, macc[0])));
         }
     }
     if (any && active) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-            *reinterpret_cast<VT*>(own + c * P + rb) = make_vec(out[c]);
+        for (int c = 0; c < 3; ++c) st_quad(own[c], rb, s[c]);
     }
     if (MEAS && active) {
         // this quad's new colour-1 spins (M of colour 1); the colour-0 sites at the quad's
@@ -356,13 +351,9 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
         // (every colour-0 site is in exactly one colour-1 quad's same-row vector): M of colour
         // 0, which is submag(0), and sub4mag, whose sites are all of colour 0
 #pragma unroll
-        for (int k = 0; k < SPT; ++k) {
-            macc[1] += out[0][k];
-            macc[2] += out[1][k];
-            macc[3] += out[2][k];
-            macc[4] += vel(same[0], k);
-            macc[5] += vel(same[1], k);
-            macc[6] += vel(same[2], k);
+        for (int c = 0; c < 3; ++c) {
+            macc[1 + c] = add2(macc[1 + c], add2(s[c].a, s[c].b));
+            macc[4 + c] = add2(macc[4 + c], add2(same[c].a, same[c].b));
         }
         // sub4mag's sites (x+y, y-x+e4 and z all = 0 or all = 2 mod 4 with C's signed %,
         // e4 = edge - edge % 4) lie in the planes z = 0, 2 mod 4; x+y >= 0, and a negative
@@ -371,13 +362,15 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
         if ((zz & 1) == 0) {
             const int e4 = m.edge - m.edge % 4;
 #pragma unroll
-            for (int k = 0; k < SPT; ++k) {
+            for (int k = 0; k < 4; ++k) {
                 const int x = 2 * (h0 + k) + (xp ^ 1);
                 const int possum = x + y, posdiff = y - x + e4;
                 if ((possum & 3) == zz && (posdiff & 3) == zz && (posdiff >= 0 || zz == 0)) {
-                    macc[7] += vel(same[0], k);
-                    macc[8] += vel(same[1], k);
-                    macc[9] += vel(same[2], k);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const f2 t = k < 2 ? same[c].a : same[c].b;
+                        macc[7 + c] = add2(macc[7 + c], pk((k & 1) ? hi(t) : lo(t), 0.0f));
+                    }
                 }
             }
         }
@@ -402,34 +395,33 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
 // colour's rows and the other colour's same rows, 3 components each (192 lines of 128 B for
 // 256 quads of 4 sites). By the time that block runs, its first loads hit L2 instead of
 // waiting on DRAM; the prefetch changes no value.
-template <int DIM, bool PERIODIC, int DK, int MINB, int SPT = 4, int MEAS = 0>
+template <int DIM, bool PERIODIC, int DK, int MINB, int MEAS = 0>
 __global__ void __launch_bounds__(256, MINB)
 k_heis_half_q4(const DevModel m, float* __restrict__ spins, const float4* __restrict__ bh,
                const unsigned long long* __restrict__ sweep, const int* __restrict__ chains,
                int colour, unsigned sweep_off, int qpt, double* __restrict__ mpart, float esign, int pf,
                int nchain_list) {
     const int chain = chains[blockIdx.y];
-    const int qpr = m.hx / SPT;
+    const int qpr = m.hx / 4;
     const int nquads = qpr * m.ly * m.lz;
-    if (MEAS == 0 && pf > 0 && SPT == 4 && threadIdx.x < 192) {
-        const long tgt = (long)blockIdx.y * gridDim.x + blockIdx.x + pf;
-        const int ty = (int)(tgt / gridDim.x), tx = (int)(tgt - (long)ty * gridDim.x);
-        const int q0 = tx * 256;
-        if (ty < nchain_list && q0 < nquads) {
-            const int sel = threadIdx.x / 96, c = (threadIdx.x % 96) >> 5, line = threadIdx.x & 31;
-            const size_t P = (size_t)m.nhalf_pad;
-            const int tch = chains[ty];
-            const float* base = spins + (((size_t)tch * 2 + (colour ^ sel)) * 3 + c) * P + (size_t)q0 * SPT;
-            const size_t end_off = (size_t)nquads * SPT;   // the plane's last site
-            if ((size_t)q0 * SPT + (size_t)line * 32 < end_off)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)line * 32));
+    if (MEAS == 0 && pf > 0 && threadIdx.x < 192) {   // warps 0-5: (colour, component), one line a lane
+        unsigned tx = blockIdx.x + (unsigned)pf, ty = blockIdx.y;
+        if (tx >= gridDim.x) {
+            const unsigned k = tx / gridDim.x;
+            ty += k;
+            tx -= k * gridDim.x;
+        }
+        const uint32_t at = tx * 1024u + (threadIdx.x & 31) * 32u;   // floats into the plane
+        if (ty < (unsigned)nchain_list && at < (uint32_t)nquads * 4u) {
+            const int w = threadIdx.x >> 5, sel = w >= 3, c = w - 3 * sel;
+            const float* base = spins + (((size_t)chains[ty] * 2 + (colour ^ sel)) * 3 + c) * (size_t)m.nhalf_pad;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(base + at));
         }
     }
-    const int qshift = (m.qpr_shift >= 0) ? m.qpr_shift + (SPT == 2 ? 1 : 0) : -1;   // log2(hx / SPT)
     constexpr int NV = MEAS ? 10 : 1;
-    float macc[NV];
+    f2 macc[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) macc[v] = 0.0f;
+    for (int v = 0; v < NV; ++v) macc[v] = f2{0ull};
     const int stride = gridDim.x * blockDim.x;
     const int nit = (MEAS == 0) ? 1 : qpt;
     for (int i = 0; i < nit; ++i) {
@@ -440,14 +432,17 @@ k_heis_half_q4(const DevModel m, float* __restrict__ spins, const float4* __rest
         const bool active = t0 < nquads;
         if (MEAS == 0 && !active) return;
         const int q = active ? t0 : nquads - 1;
-        const int row = (qshift >= 0) ? (q >> qshift) : (q / qpr);
-        const int h0 = (q - row * qpr) * SPT;
-        q4_quad<DIM, PERIODIC, DK, SPT, MEAS>(m, spins, bh, sweep, sweep_off, chain, colour, row, h0,
-                                              MEAS == 0 || active, macc, esign);
+        const int row = (m.qpr_shift >= 0) ? (q >> m.qpr_shift) : (q / qpr);
+        const int h0 = (q - row * qpr) * 4;
+        q4_quad<DIM, PERIODIC, DK, MEAS>(m, spins, bh, sweep, sweep_off, chain, colour, row, h0,
+                                         MEAS == 0 || active, macc, esign);
     }
     if (MEAS != 0) {
-        macc[0] *= 2.0f;   // the energy's pair sum counts every bond twice (exact)
-        meas_block_rows<NV>(macc, mpart + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * NV);
+        float sums[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) sums[v] = lo(macc[v]) + hi(macc[v]);
+        sums[0] *= 2.0f;   // the energy's pair sum counts every bond twice (exact)
+        meas_block_rows<NV>(sums, mpart + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * NV);
     }
 }
 
@@ -944,7 +939,7 @@ static void heis_q4_meas_launch(Ctx& c, const int* d_chains, int n, int colour, 
     const int nb = q4_meas_blocks(c);
     dim3 grid(nb, n);
     const float esign = c.dmi_sign ? 0.0f : -2.0f;
-    k_heis_half_q4<DIM, PERIODIC, DK, 2, 4, 1><<<grid, 256, 0, c.stream>>>(
+    k_heis_half_q4<DIM, PERIODIC, DK, 2, 1><<<grid, 256, 0, c.stream>>>(
         c.m, sp, c.d_bh, c.d_sweep, d_chains, colour, off, kMeasQpt, c.d_mrows, esign, 0, n);
 }
 

@@ -7,6 +7,51 @@
 namespace nmmc {
 
 constexpr float kPi = 3.14159265358979f;
+constexpr float kLn2 = 0.693147180559945f;
+
+// Packed pairs of FP32 values: one instruction for two IEEE operations (round to nearest).
+struct f2 { unsigned long long v; };
+__device__ __forceinline__ f2 pk(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float lo(f2 a) { return __uint_as_float((uint32_t)a.v); }
+__device__ __forceinline__ float hi(f2 a) { return __uint_as_float((uint32_t)(a.v >> 32)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+// Approximations for arguments that are never subnormal (the .ftz forms need no code for
+// subnormal inputs): 1 / sqrt(x) and log2(x). The uniforms are at least 2^-24 and the
+// proposal's 1 - z^2 at least 2^-22.
+__device__ __forceinline__ float rsqrt_norm(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float log2_norm(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
 // Compact index, in the other colour's plane, of the neighbour of (x,y,z) in direction k
 // (+x,-x,+y,-y,+z,-z), or -1 when the neighbour falls off an open boundary.

@@ -47,6 +47,11 @@ NMMC_HD nmmc_u4 nmmc_philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
     return nmmc_u4{c0, c1, c2, c3};
 }
 
+#if defined(__CUDACC__)
+// 1 + k 2^-23 with k the top 23 bits of r: the exponent field of 1.0 shifted in above them.
+__device__ __forceinline__ float nmmc_u12f(uint32_t r) { return __uint_as_float(__funnelshift_r(r, 0x7fu, 9)); }
+#endif
+
 // Uniform float in (0,1) from the top 23 bits: (k + 1/2) 2^-23, exact in FP32. On the device
 // it is built from bits: (1 + k 2^-23) - (1 - 2^-24) is exact (Sterbenz) and equals the same value.
 NMMC_HD float nmmc_u01f(uint32_t r) {
