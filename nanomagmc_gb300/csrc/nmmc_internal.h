@@ -81,10 +81,18 @@ struct ResidentTables {
     // sweeps of every site, so that the resident kernel's updates skip the generator.
     bool hbm_faster = false;      // the autotuner timed the HBM path faster: the automatic path takes it
     bool stencil = false;         // sweeps run on the stencil resident kernel (nmmc_stencil.cu)
+    bool large_tuned = false;     // a lattice too large for the record kernel: path chosen (stencil or HBM)
     bool predraw = false;         // the shape in use launches the drawn-ahead variant
     int* d_site_chain = nullptr;  // per site: its chain
     uint4* d_draws = nullptr;     // [sweep of the launch][site] Philox words
     int draw_sweeps = 0;          // sweeps d_draws holds (longer calls are split)
+};
+
+// Shape of a stencil resident launch (nmmc_stencil.cu): CTAs per chain (0: not covered), threads
+// and dynamic shared memory of a CTA.
+struct StencilShape {
+    int C = 0, threads = 0, np = 2;   // np: pairs of sites per thread item (1 or 2)
+    size_t smem = 0;
 };
 
 struct TimedCall {
@@ -129,7 +137,7 @@ struct Ctx {
     bool wave_no_memory = false;        // the second array could not be allocated: half-sweeps only
     int wave_per_sm[8] = {};            // resident CTAs per SM of each wavefront kernel (0: not queried)
     int pf_per_sm[16] = {};             // the same for each prefetching half-sweep kernel
-    size_t stencil_smem[16] = {};       // dynamic shared memory set for each stencil resident kernel
+    std::map<int, StencilShape> st_shapes;   // stencil kernel: shape by the number of chains of a call
     uint8_t* d_mask = nullptr;          // split-colour mask planes (nullptr: unmasked)
     // masked lattices: per chain and colour, the compact indices of the filled sites in
     // increasing order (segment (chain * 2 + colour) of nhalf entries) and their counts, so
@@ -274,8 +282,7 @@ int launch_pf_half(Ctx& c, const int* d_chains, int n, int colour, unsigned off)
 long long global_sweep_launches(Ctx& c, int nsweeps, bool fused);
 
 // ---- stencil resident kernel (nmmc_stencil.cu) ----
-size_t stencil_chain_bytes(const Ctx& c);   // 0: the lattice is not covered
-int stencil_slots(const Ctx& c, int n);     // chains per CTA for a call on n chains (0: none fits)
+StencilShape stencil_shape(const Ctx& c, int n);   // of a call on n chains; C = 0: not covered
 int launch_stencil_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure, int accumulate);
 
 // ---- resident kernel (nmmc_resident.cu) ----

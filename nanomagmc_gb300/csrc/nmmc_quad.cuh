@@ -99,27 +99,37 @@ __device__ __forceinline__ void axis_terms(const DevModel& m, const f2 (&P)[3], 
     }
 }
 
-// Field (and DMI part) of a quad for one axis; x uses the same-row and shifted neighbours.
+// Field (and DMI part) of a pair or a quad for one axis; x uses the same-row and shifted neighbours.
 template <int DK, bool EF>
-__device__ __forceinline__ void quad_axis_x(const DevModel& m, const F2x2 (&same)[3], const F2x2 (&sh)[3], bool xp,
-                                            f2 (&h)[2][3], f2 (&d)[2][3]) {
+__device__ __forceinline__ void pair_axis_x(const DevModel& m, const f2 (&same)[3], const f2 (&sh)[3], bool xp,
+                                            f2 (&h)[3], f2 (&d)[3]) {
     // xp = 1: +x is the shifted neighbour. The +-pair kinds fold the order into a sign.
     const float flip = 1.0f - 2.0f * (float)!xp;   // (sh - same) = flip * (s+ - s-)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    if (DK == kDmiPairs || DK == kDmiAxial) {
+        axis_terms<DK, 0, EF>(m, sh, same, flip, h, d);
+    } else {
         f2 P[3], M[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const f2 a = j ? sh[c].b : sh[c].a, b = j ? same[c].b : same[c].a;
-            if (DK == kDmiPairs || DK == kDmiAxial) {
-                P[c] = a;
-                M[c] = b;
-            } else {
-                P[c].v = xp ? a.v : b.v;
-                M[c].v = xp ? b.v : a.v;
-            }
+            P[c].v = xp ? sh[c].v : same[c].v;
+            M[c].v = xp ? same[c].v : sh[c].v;
         }
-        axis_terms<DK, 0, EF>(m, P, M, flip, h[j], d[j]);
+        axis_terms<DK, 0, EF>(m, P, M, flip, h, d);
+    }
+}
+
+template <int DK, bool EF>
+__device__ __forceinline__ void quad_axis_x(const DevModel& m, const F2x2 (&same)[3], const F2x2 (&sh)[3], bool xp,
+                                            f2 (&h)[2][3], f2 (&d)[2][3]) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        f2 a[3], b[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            a[c] = j ? same[c].b : same[c].a;
+            b[c] = j ? sh[c].b : sh[c].a;
+        }
+        pair_axis_x<DK, EF>(m, a, b, xp, h[j], d[j]);
     }
 }
 
@@ -138,32 +148,45 @@ __device__ __forceinline__ void quad_axis(const DevModel& m, const F2x2 (&up)[3]
     }
 }
 
-// Proposals and Metropolis tests of a pair of sites (heis_try for each half): s becomes the new
-// spins; true when either site accepted.
-__device__ __forceinline__ bool pair_try(const f2 (&h)[3], f2 (&s)[3], float beta, const nmmc_u4& r0,
-                                         const nmmc_u4& r1) {
+// A pair of proposals (sphere_proposal) and the logarithms of their acceptance uniforms.
+struct PairProp { f2 t[3], lu; };
+
+__device__ __forceinline__ PairProp pair_propose(const nmmc_u4& r0, const nmmc_u4& r1) {
     const f2 c = pk(-0.99999994f, -0.99999994f), two = pk(2.0f, 2.0f), mone = pk(-1.0f, -1.0f);
     const f2 u0 = add2(pk(nmmc_u12f(r0.x), nmmc_u12f(r1.x)), c);
     const f2 u1 = add2(pk(nmmc_u12f(r0.y), nmmc_u12f(r1.y)), c);
     const f2 u2 = add2(pk(nmmc_u12f(r0.z), nmmc_u12f(r1.z)), c);
-    const f2 tz = fma2(two, u0, mone);
+    PairProp p;
+    p.t[2] = fma2(two, u0, mone);
     const f2 phi = mul2(fma2(two, u1, mone), pk(kPi, kPi));
     float sp0, cp0, sp1, cp1;
     __sincosf(lo(phi), &sp0, &cp0);
     __sincosf(hi(phi), &sp1, &cp1);
-    const f2 w = pk(fmaf(-lo(tz), lo(tz), 1.0f), fmaf(-hi(tz), hi(tz), 1.0f));
-    const f2 rxy = mul2(w, pk(rsqrt_norm(lo(w)), rsqrt_norm(hi(w))));
-    const f2 tx = mul2(rxy, pk(cp0, cp1)), ty = mul2(rxy, pk(sp0, sp1));
-    const f2 lu = mul2(pk(log2_norm(lo(u2)), log2_norm(hi(u2))), pk(kLn2, kLn2));
-    const f2 dx = sub2(s[0], tx), dy = sub2(s[1], ty), dz = sub2(s[2], tz);
+    const float z0 = lo(p.t[2]), z1 = hi(p.t[2]);
+    const float w0 = fmaf(-z0, z0, 1.0f), w1 = fmaf(-z1, z1, 1.0f);
+    const f2 rxy = mul2(pk(w0, w1), pk(rsqrt_norm(w0), rsqrt_norm(w1)));
+    p.t[0] = mul2(rxy, pk(cp0, cp1));
+    p.t[1] = mul2(rxy, pk(sp0, sp1));
+    p.lu = mul2(pk(log2_norm(lo(u2)), log2_norm(hi(u2))), pk(kLn2, kLn2));
+    return p;
+}
+
+// Metropolis tests of a pair of sites (heis_accept for each half): s becomes the new spins; true
+// when either site accepted.
+__device__ __forceinline__ bool pair_accept(const f2 (&h)[3], f2 (&s)[3], float beta, const PairProp& p) {
+    const f2 dx = sub2(s[0], p.t[0]), dy = sub2(s[1], p.t[1]), dz = sub2(s[2], p.t[2]);
     const f2 dE = fma2(h[2], dz, fma2(h[1], dy, mul2(h[0], dx)));
     const f2 q = mul2(dE, pk(-beta, -beta));
-    const bool a0 = (lo(dE) <= 0.0f) || (lo(q) > lo(lu));
-    const bool a1 = (hi(dE) <= 0.0f) || (hi(q) > hi(lu));
-    s[0] = pk(a0 ? lo(tx) : lo(s[0]), a1 ? hi(tx) : hi(s[0]));
-    s[1] = pk(a0 ? lo(ty) : lo(s[1]), a1 ? hi(ty) : hi(s[1]));
-    s[2] = pk(a0 ? lo(tz) : lo(s[2]), a1 ? hi(tz) : hi(s[2]));
+    const bool a0 = (lo(dE) <= 0.0f) || (lo(q) > lo(p.lu));
+    const bool a1 = (hi(dE) <= 0.0f) || (hi(q) > hi(p.lu));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s[c] = pk(a0 ? lo(p.t[c]) : lo(s[c]), a1 ? hi(p.t[c]) : hi(s[c]));
     return a0 | a1;
+}
+
+__device__ __forceinline__ bool pair_try(const f2 (&h)[3], f2 (&s)[3], float beta, const nmmc_u4& r0,
+                                         const nmmc_u4& r1) {
+    return pair_accept(h, s, beta, pair_propose(r0, r1));
 }
 
 }  // namespace nmmc

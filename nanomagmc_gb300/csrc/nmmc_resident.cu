@@ -436,6 +436,7 @@ void free_tables(ResidentTables& r) {
     r.d_slot_red = r.d_slot_black = nullptr;
     r.built = false;
     r.stencil = false;
+    r.large_tuned = false;
     r.hbm_faster = false;
     r.tables_bins = 0;
 }
@@ -583,13 +584,16 @@ bool predraw_fits(const Ctx& c) {
            dyn_smem(c, true) <= smem_budget(c);
 }
 
+// Shared-memory limit of this context's kernels, raised to what the path may use on this device
+// and not only to what this context needs: the limit belongs to the kernel, so that a second
+// context with smaller bins would lower it for the first one.
 int set_attr(Ctx& c) {
     for (bool pre : {false, true}) {
-        if (pre && !predraw_fits(c)) continue;
+        if (pre && c.dim != 2) continue;
         for (bool fused : {false, true}) {
             if (fused && c.dim == 3) continue;
             int rc = cuda_check(cudaFuncSetAttribute(kernel_for(c, fused, pre), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)dyn_smem(c, pre)),
+                                                     (int)smem_budget(c)),
                                 "cudaFuncSetAttribute(k_resident)");
             if (rc) return rc;
         }
@@ -702,8 +706,10 @@ std::string config_key(const Ctx& c) {
     mix((uint64_t)c.m.has_dmi);
     for (int v : c.num) mix((uint64_t)v);
     mix((uint64_t)c.m.dmi_kind);
-    mix(6);   // table and kernel format (5: the path choice, stencil kernel included, is part of the entry;
-              // 6: 16 bytes of shared memory per Heisenberg site)
+    // table and kernel format (5: the path choice, stencil kernel included, is part of the entry;
+    // 6: 16 bytes of shared memory per Heisenberg site; 7: the stencil kernel on clusters, for the
+    // lattices it covers)
+    mix(c.ising || c.masked || c.m.general ? 6 : 7);
     std::string g = c.gpu_name;
     for (char& ch : g)
         if (ch == ' ') ch = '_';
@@ -737,6 +743,87 @@ void cache_store(const std::string& key, int nbins, int threads, int pre, int hb
     if (f) f << key << " " << nbins << " " << threads << " " << pre << " " << hbm << "\n";
 }
 
+// Spins and sweep counters put aside while candidates run on the live chains.
+struct TuningSnapshot {
+    DeviceScratch ds;
+    void* spins = nullptr;
+    unsigned long long* sweep = nullptr;
+    int take(Ctx& c) {
+        NMMC_CUDA(ds.alloc(&spins, c.spins_bytes));
+        NMMC_CUDA(ds.alloc(&sweep, sizeof(unsigned long long) * c.nchains));
+        NMMC_CUDA(cudaMemcpyAsync(spins, c.d_spins, c.spins_bytes, cudaMemcpyDeviceToDevice, c.stream));
+        NMMC_CUDA(cudaMemcpyAsync(sweep, c.d_sweep, sizeof(unsigned long long) * c.nchains, cudaMemcpyDeviceToDevice,
+                                  c.stream));
+        return upload_params(c);
+    }
+    int restore(Ctx& c) {
+        NMMC_CUDA(cudaMemcpyAsync(c.d_spins, spins, c.spins_bytes, cudaMemcpyDeviceToDevice, c.stream));
+        NMMC_CUDA(cudaMemcpyAsync(c.d_sweep, sweep, sizeof(unsigned long long) * c.nchains, cudaMemcpyDeviceToDevice,
+                                  c.stream));
+        return cuda_check(cudaStreamSynchronize(c.stream), "autotuning");
+    }
+};
+
+// Device time of the best of three 8-sweep runs of step(nsweeps) after a warm-up (1e30: failed).
+template <class Step>
+float best_of_three(Ctx& c, Step step) {
+    float best = 1e30f;
+    if (step(1) != NMMC_OK) {
+        cudaGetLastError();
+        return best;
+    }
+    cudaEvent_t ea, eb;
+    cudaEventCreate(&ea);
+    cudaEventCreate(&eb);
+    for (int rep = 0; rep < 3; ++rep) {
+        cudaEventRecord(ea, c.stream);
+        const bool ok = step(8) == NMMC_OK;
+        cudaEventRecord(eb, c.stream);
+        float t = 0;
+        if (!ok || cudaEventSynchronize(eb) != cudaSuccess || cudaEventElapsedTime(&t, ea, eb) != cudaSuccess ||
+            cudaGetLastError() != cudaSuccess) {
+            best = 1e30f;
+            break;
+        }
+        best = std::min(best, t);
+    }
+    cudaEventDestroy(ea);
+    cudaEventDestroy(eb);
+    return best;
+}
+
+// Lattices too large for the record kernel, on the automatic path: the stencil kernel on
+// clusters against the HBM path, by the same timing (and the same cache: no bins, the path).
+// Small batches gain most (8 chains of 30^3 take 11 us per sweep in launches alone); the
+// streaming path keeps lattices that fit no cluster and batches that fill the GPU many times.
+int tune_large(Ctx& c) {
+    if (c.res.large_tuned) return NMMC_OK;
+    c.res.stencil = false;
+    c.res.large_tuned = true;
+    if (c.res_stencil == 1 || stencil_shape(c, c.nchains).C < 1) return NMMC_OK;
+    if (c.res_stencil == 2) {
+        c.res.stencil = true;
+        return NMMC_OK;
+    }
+    const std::string key = config_key(c);
+    int cb = 0, ct = 0, cp = 0, ch = 0;
+    if (cache_lookup(key, cb, ct, cp, ch)) {
+        c.res.stencil = ch == 2;
+        return NMMC_OK;
+    }
+    TuningSnapshot snap;
+    int rc = snap.take(c);
+    if (rc) return rc;
+    const bool fused = !c.measure_fp64;
+    const float th = best_of_three(c, [&](int k) { return hbm_tuning_step(c, k, fused); });
+    const float ts = best_of_three(c, [&](int k) { return launch_stencil_sweeps(c, c.d_all, c.nchains, k, fused, 0); });
+    cudaGetLastError();
+    if ((rc = snap.restore(c))) return rc;
+    c.res.stencil = ts < th;
+    cache_store(key, 0, 0, 0, c.res.stencil ? 2 : 1);
+    return NMMC_OK;
+}
+
 }  // namespace
 
 void resident_free(Ctx& c) { free_tables(c.res); }
@@ -752,9 +839,9 @@ int resident_prepare(Ctx& c) {
     for (int v : c.num) maxn = std::max(maxn, v);
     // general interaction tables use the multi-colour gather sweep
     c.res.eligible = maxn > 0 && maxn <= cap_sites && !c.m.general;
-    if (!c.res.eligible) return NMMC_OK;
-    // the stencil kernel covers unmasked 2-D Heisenberg lattices that fit one chain per CTA
-    const bool stencil_ok = c.res_stencil != 1 && stencil_slots(c, c.nchains) > 0;
+    // the stencil kernel covers unmasked Heisenberg lattices that fit a cluster
+    if (!c.res.eligible) return c.sweep_path == 0 ? tune_large(c) : NMMC_OK;
+    const bool stencil_ok = c.res_stencil != 1 && stencil_shape(c, c.nchains).C > 0;
 
     std::vector<int> load(c.num.begin(), c.num.end());
     auto tables_for = [&](int nbins) -> int {
@@ -830,16 +917,9 @@ int resident_prepare(Ctx& c) {
     // time each candidate on the live chains, with the variant the sampling loop launches
     // (2-D: sweeps + observables); spins and counters are restored afterwards
     const bool fused = c.dim == 2 && !c.measure_fp64;
-    DeviceScratch ds;
-    void* snap = nullptr;
-    unsigned long long* snap_sw = nullptr;
-    NMMC_CUDA(ds.alloc(&snap, c.spins_bytes));
-    NMMC_CUDA(ds.alloc(&snap_sw, sizeof(unsigned long long) * c.nchains));
-    NMMC_CUDA(cudaMemcpyAsync(snap, c.d_spins, c.spins_bytes, cudaMemcpyDeviceToDevice, c.stream));
-    NMMC_CUDA(cudaMemcpyAsync(snap_sw, c.d_sweep, sizeof(unsigned long long) * c.nchains,
-                              cudaMemcpyDeviceToDevice, c.stream));
+    TuningSnapshot snap;
     NMMC_CUDA(cudaMemsetAsync(c.d_active, 1, c.nchains, c.stream));
-    int rc = upload_params(c);
+    int rc = snap.take(c);
     if (rc) return rc;
     cudaEvent_t ea, eb;
     cudaEventCreate(&ea);
@@ -882,37 +962,16 @@ int resident_prepare(Ctx& c) {
     // observables on the streaming kernels (at few large lattices a resident kernel occupies
     // few SMs: 16 chains of 128^2 sweep in 8.6 us there against 16.6 us resident)
     bool hbm = false;
-    if (automatic && c.sweep_path == 0 && best_b > 0 && hbm_tuning_step(c, 1, fused) == NMMC_OK) {
-        float ms = 1e30f;
-        bool ok = true;
-        for (int rep = 0; rep < 3 && ok; ++rep) {
-            cudaEventRecord(ea, c.stream);
-            ok = hbm_tuning_step(c, 8, fused) == NMMC_OK;
-            cudaEventRecord(eb, c.stream);
-            float t = 0;
-            ok = ok && cudaEventSynchronize(eb) == cudaSuccess && cudaEventElapsedTime(&t, ea, eb) == cudaSuccess &&
-                 cudaGetLastError() == cudaSuccess;
-            ms = std::min(ms, t);
-        }
-        hbm = ok && ms < best;
+    if (automatic && c.sweep_path == 0 && best_b > 0) {
+        const float ms = best_of_three(c, [&](int k) { return hbm_tuning_step(c, k, fused); });
+        hbm = ms < best;
         if (hbm) best = ms;
     }
     // the stencil kernel: timed on the automatic choice, taken without timing when forced
     bool stencil = c.res_stencil == 2 && stencil_ok;
-    if (c.res_stencil == 0 && stencil_ok && best_b > 0 &&
-        launch_stencil_sweeps(c, c.d_all, c.nchains, 1, fused, 0) == NMMC_OK) {
-        float ms = 1e30f;
-        bool ok = true;
-        for (int rep = 0; rep < 3 && ok; ++rep) {
-            cudaEventRecord(ea, c.stream);
-            ok = launch_stencil_sweeps(c, c.d_all, c.nchains, 8, fused, 0) == NMMC_OK;
-            cudaEventRecord(eb, c.stream);
-            float t = 0;
-            ok = ok && cudaEventSynchronize(eb) == cudaSuccess && cudaEventElapsedTime(&t, ea, eb) == cudaSuccess &&
-                 cudaGetLastError() == cudaSuccess;
-            ms = std::min(ms, t);
-        }
-        if (ok && ms < best) {
+    if (c.res_stencil == 0 && stencil_ok && best_b > 0) {
+        const float ms = best_of_three(c, [&](int k) { return launch_stencil_sweeps(c, c.d_all, c.nchains, k, fused, 0); });
+        if (ms < best) {
             stencil = true;
             hbm = false;
         }
@@ -920,10 +979,7 @@ int resident_prepare(Ctx& c) {
     cudaGetLastError();
     cudaEventDestroy(ea);
     cudaEventDestroy(eb);
-    NMMC_CUDA(cudaMemcpyAsync(c.d_spins, snap, c.spins_bytes, cudaMemcpyDeviceToDevice, c.stream));
-    NMMC_CUDA(cudaMemcpyAsync(c.d_sweep, snap_sw, sizeof(unsigned long long) * c.nchains, cudaMemcpyDeviceToDevice,
-                              c.stream));
-    NMMC_CUDA(cudaStreamSynchronize(c.stream));
+    if ((rc = snap.restore(c))) return rc;
     c.active_all = true;   // every chain marked active above
     if (best_b == 0) {
         c.res.eligible = false;
@@ -937,7 +993,9 @@ int resident_prepare(Ctx& c) {
 }
 
 bool resident_chosen(const Ctx& c) {
-    return c.res.eligible && !(c.sweep_path == 0 && c.res.hbm_faster);
+    if (!c.res.eligible)   // the options that pick a streaming variant keep the streaming path
+        return c.sweep_path == 0 && c.res.large_tuned && c.res.stencil && c.half_kernel == 0 && !c.wave;
+    return !(c.sweep_path == 0 && c.res.hbm_faster);
 }
 
 __global__ void k_mark_active(uint8_t* active, int* pos, const int* chains, int n) {
@@ -949,6 +1007,7 @@ __global__ void k_mark_active(uint8_t* active, int* pos, const int* chains, int 
 }
 
 bool resident_can_measure(const Ctx& c) {
+    if (c.res.stencil && resident_chosen(c)) return !c.measure_fp64;
     // one z-slice, FP32 observables, and whole warps for the per-slot reductions
     return c.res.built && c.res.eligible && c.dim == 2 && !c.measure_fp64 && c.res.threads >= 32 &&
            c.res.threads % 32 == 0;

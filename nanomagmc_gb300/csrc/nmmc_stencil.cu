@@ -1,352 +1,750 @@
-// Shared-memory resident sweeps of unmasked 2-D Heisenberg lattices in their stencil layout.
+// Shared-memory resident sweeps of unmasked Heisenberg lattices in their stencil layout, one
+// chain per thread-block cluster.
 //
-// The general resident kernel (nmmc_resident.cu) keeps only filled sites and gives each one a
-// record of neighbour indices, so that Weibull particles of any size pack densely; a site then
-// costs a record decode and twelve scalar shared-memory gathers per update. An unmasked
-// lattice needs neither: here each CTA holds S whole chains in the split-colour layout of HBM
-// (per chain and colour three planes of ly rows of hx sites) and updates four consecutive
-// same-colour sites per thread item with 16-byte shared-memory loads of the own row and of the
-// other colour's rows y-1, y, y+1, exactly as the four-site HBM half-sweep does from HBM. The
-// per-site arithmetic, the draw order and the Philox counters are those of the HBM kernel
-// (and of the record kernel), so every path gives the same chain bit for bit. With MEASURE the
-// observables of each chain are computed from the spins still in shared memory after the last
-// sweep (the terms of the streaming measurement kernel, summed in FP32 per thread and warp and
-// in FP64 across warps) and written with the accumulators.
+// The record kernel (nmmc_resident.cu) keeps only filled sites and gives each one a record of
+// neighbour indices, so that Weibull particles of any size pack densely. An unmasked lattice
+// needs no records: a cluster of C CTAs (1 to 16) holds one chain, cut into slabs of whole rows
+// (2-D) or whole planes (3-D), and every thread updates four consecutive same-colour sites of a
+// row with the packed arithmetic of nmmc_quad.cuh. Each CTA also keeps a copy of the row or
+// plane below and above its slab; a thread that accepts a move in a boundary row stores it into
+// the neighbour CTA's copy through distributed shared memory, and one cluster barrier per
+// half-sweep orders the colours. The spins leave shared memory once per call.
+//
+// What bounds it: with many chains (C = 1, several CTAs per SM) instruction issue, as the
+// streaming half-sweep; with few chains the latency of one update chain plus the barrier, so
+// the next half-sweep's draws and proposals are computed between the barrier's arrive and wait.
+// The streaming path pays a launch of about 4.8 us per half-sweep there.
+//
+// Layout in shared memory: [colour][slab unit, with the two copies][row][quad][component][4]
+// floats. The three components of a quad lie 16 bytes apart, so a neighbour row costs one
+// address; 48-byte steps between the lanes of a 16-byte access hit different banks. Rows that
+// are not a multiple of four sites per colour end in a quad with padding: on periodic lattices
+// the first padding element repeats the row's first site, which makes it the +x neighbour of the
+// last one. Open edges read zeros (empty copies, padding and one zero quad), which add nothing.
+//
+// The per-site arithmetic, the draws and their counters are those of the streaming kernels, so
+// every path gives the same chain bit for bit. With MEASURE the observables are computed from
+// the spins still in shared memory after the last sweep: FP32 per thread and warp, FP64 across
+// warps and CTAs in a fixed order, finished by one warp per chain.
 #include <algorithm>
 
-#include "nmmc_kernels.cuh"
+#include "nmmc_quad.cuh"
 
 namespace nmmc {
 
 namespace {
 
-constexpr int kStThreads = 768;
-constexpr int kStMaxSlots = 32;
+constexpr int kStThreads = 768;     // 80 registers: 24 warps per SM in one, two or three CTAs
+constexpr int kStMaxCluster = 16;
+constexpr int kQuadBytes = 48;
 
-__device__ __forceinline__ float stv(const float4& v, int k) {
-    return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w));
+// n / d for n, d < 65536 by one multiplication (mul = ceil(2^32 / d); d = 1 has mul = 0).
+struct FastDiv { uint32_t mul; int d; };
+__device__ __forceinline__ int fdiv(int n, const FastDiv& f) { return f.mul ? (int)__umulhi((uint32_t)n, f.mul) : n; }
+
+struct StencilArgs {
+    float* spins;
+    const float4* bh;
+    unsigned long long* sweep;
+    const int* chains;
+    int nsweeps;
+    int C;                   // CTAs per chain
+    int NU, R, U;            // slab units of the lattice, rows per unit, largest slab
+    int qpr, ipr;            // quads and thread items per row (rounded up)
+    FastDiv div_ipr, div_pairs, div_rows, div_cols, div_planes;   // items, rows per unit; load columns, rows per plane
+    const double* Hd;
+    double* obs;
+    double* q;               // nullptr: not wanted
+    double* acc;
+    int nslices, accumulate;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The address of this CTA's shared-memory location in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void peer_st(uint32_t a, f2 v) {
+    asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v.v) : "memory");
+}
+__device__ __forceinline__ void peer_st(uint32_t a, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void peer_st(uint32_t a, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
-// Loads of one quad from shared memory: own spins, the other colour's same row, the
-// x-neighbour outside the quad and rows y +- 1 (zero where missing on an open lattice).
-template <bool PERIODIC>
-__device__ __forceinline__ void st_load(const DevModel& m, const float* own, const float* oth, int NH, int y,
-                                        int h0, int xp, float4 (&s)[3], float4 (&same)[3], float (&ex)[3],
-                                        float4 (&yp)[3], float4 (&ym)[3]) {
-    const int hx = m.hx, ly = m.ly;
-    const int rb = y * hx + h0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        s[c] = *reinterpret_cast<const float4*>(own + c * NH + rb);
-        same[c] = *reinterpret_cast<const float4*>(oth + c * NH + rb);
-    }
-    int ho = xp ? h0 + 4 : h0 - 1;
-    bool ok = true;
-    if (PERIODIC) ho = (ho < 0) ? hx - 1 : (ho >= hx ? 0 : ho);
-    else ok = ho >= 0 && ho < hx;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) ex[c] = ok ? oth[c * NH + y * hx + ho] : 0.0f;
-    int yu = y + 1, yd = y - 1;
-    bool oU = true, oD = true;
-    if (PERIODIC) {
-        yu = (yu == ly) ? 0 : yu;
-        yd = (yd < 0) ? ly - 1 : yd;
-    } else {
-        oU = yu < ly;
-        oD = yd >= 0;
-    }
-    const float4 vz = {};
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        yp[c] = oU ? *reinterpret_cast<const float4*>(oth + c * NH + yu * hx + h0) : vz;
-        ym[c] = oD ? *reinterpret_cast<const float4*>(oth + c * NH + yd * hx + h0) : vz;
-    }
+__device__ __forceinline__ F2x2 lds_quad(const char* p, int c) {
+    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p + 16 * c);
+    return F2x2{{t.x}, {t.y}};
 }
-
-// The four sites' neighbours in stencil order (+x, -x, +y, -y) for component c.
-template <bool PERIODIC>
-__device__ __forceinline__ void st_nb(const DevModel& m, const float4& same, float ex, const float4& yp,
-                                      const float4& ym, int k, int h0, int xp, float (&nb)[4]) {
-    const float sm = stv(same, k);
-    const float sh = xp ? (k < 3 ? stv(same, k + 1) : ex) : (k > 0 ? stv(same, k - 1) : ex);
-    float plusx = xp ? sh : sm, minusx = xp ? sm : sh;
-    if (!PERIODIC) {
-        const int x = 2 * (h0 + k) + xp;
-        if (x + 1 >= m.edge) plusx = 0.0f;
-        if (x == 0) minusx = 0.0f;
-    }
-    nb[0] = plusx;
-    nb[1] = minusx;
-    nb[2] = stv(yp, k);
-    nb[3] = stv(ym, k);
-}
-
 }  // namespace
 
-template <int DK, bool PERIODIC, bool MEASURE>
-__global__ void __launch_bounds__(kStThreads, 1)
-k_resident_stencil(const DevModel m, float* __restrict__ spins, const float4* __restrict__ bh,
-                   unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int n, int S,
-                   int nsweeps, const double* __restrict__ Hd, double* __restrict__ obs, double* __restrict__ qout,
-                   double* __restrict__ acc, int accumulate) {
-    extern __shared__ __align__(16) float st_sm[];
-    __shared__ float4 sp[kStMaxSlots];
-    __shared__ unsigned long long ssw[kStMaxSlots];
-    __shared__ int sch[kStMaxSlots];
+// One item is NP pairs of sites: a quad (NP = 2) where the chains fill the GPU, a pair (NP = 1)
+// where they leave it short of warps.
+template <int DIM, int DK, int NP, bool MEASURE>
+__global__ void __launch_bounds__(kStThreads, 1) k_resident_stencil(const DevModel m, const StencilArgs g) {
+    extern __shared__ __align__(16) char st_sm[];
     __shared__ float wred[kStThreads / 32][kNP];
-    const int NH = m.nhalf;                 // sites per colour plane (hx * ly)
-    const size_t P = (size_t)m.nhalf_pad;
-    const int hx = m.hx, qpr = hx >> 2, Q = qpr * m.ly;
-    const int c0 = blockIdx.x * S;
-    const int ns = min(S, n - c0);
-    if (ns <= 0) return;
+    __shared__ double cred[kStMaxCluster][kNP];   // rank 0: the CTAs' totals
+    const int C = g.C, rank = C > 1 ? (int)cluster_rank() : 0;
+    const int ci = blockIdx.x / C, chain = g.chains[ci];
     const int tid = threadIdx.x;
-    for (int t = tid; t < ns; t += blockDim.x) {
-        const int ch = chains[c0 + t];
-        sch[t] = ch;
-        sp[t] = bh[ch];
-        ssw[t] = sweep[ch];
-    }
+    const bool per = m.periodic;
+    const int hx = m.hx, qpr = g.qpr, ipr = g.ipr, R = g.R, NU = g.NU;
+    const int u0 = rank * NU / C, nu = (rank + 1) * NU / C - u0;
+    const int rowb = qpr * kQuadBytes, unitb = R * rowb, colb = (g.U + 2) * unitb;
+    char* const zero = st_sm;                       // one quad of zeros
+    char* const base = st_sm + kQuadBytes;          // colour 0, then colour 1
+    // the slabs below and above: their CTA and where in its copies this slab's edge units go
+    const int lo_rank = rank > 0 ? rank - 1 : C - 1, hi_rank = rank + 1 < C ? rank + 1 : 0;
+    const bool has_lo = per || rank > 0, has_hi = per || rank + 1 < C;
+    const int lo_slot = (lo_rank + 1) * NU / C - lo_rank * NU / C + 1;   // past its last unit
+    const size_t P = (size_t)m.nhalf_pad;
+    float* const gsp = g.spins + (size_t)chain * 6 * P;
+
+    for (int i = tid; i < (kQuadBytes + 2 * colb) / 16; i += blockDim.x)
+        reinterpret_cast<float4*>(st_sm)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    const int nv = NH >> 2;                 // float4 per plane
-    for (int i = tid; i < ns * 6 * nv; i += blockDim.x) {
-        const int sl = i / (6 * nv), r = i - sl * 6 * nv, pl = r / nv, j = r - pl * nv;
-        reinterpret_cast<float4*>(st_sm)[(size_t)(sl * 6 + pl) * nv + j] =
-            __ldg(reinterpret_cast<const float4*>(spins + ((size_t)sch[sl] * 6 + pl) * P) + j);
-    }
-    __syncthreads();
-    const int qshift = m.qpr_shift;         // log2(hx / 4) or -1
-    const int Qs = (Q & (Q - 1)) == 0 ? __ffs(Q) - 1 : -1;   // log2(Q) or -1
-    for (int sw = 0; sw < nsweeps; ++sw) {
-        for (int colour = 0; colour < 2; ++colour) {
-            for (int it = tid; it < ns * Q; it += blockDim.x) {
-                const int sl = Qs >= 0 ? (it >> Qs) : (it / Q), r = it - sl * Q;
-                const int y = qshift >= 0 ? (r >> qshift) : (r / qpr);
-                const int h0 = (r - y * qpr) * 4;
-                const int xp = (y + colour) & 1;
-                float* own = st_sm + (size_t)(sl * 6 + colour * 3) * NH;
-                const float* oth = st_sm + (size_t)(sl * 6 + (colour ^ 1) * 3) * NH;
-                float4 s[3], same[3], yp[3], ym[3];
-                float ex[3];
-                st_load<PERIODIC>(m, own, oth, NH, y, h0, xp, s, same, ex, yp, ym);
-                const int chain = sch[sl];
-                const float4 p = sp[sl];
-                const unsigned long long swc = ssw[sl] + (unsigned)sw;
-                const uint32_t boxrow = (uint32_t)(m.edge * y);
-                nmmc_u4 rnext = sweep_draw<true>(m, boxrow + (uint32_t)(2 * h0 + xp), swc, (uint32_t)chain);
-                float out[3][4];
-                bool any = false;
+    // units u0 - 1 .. u0 + nu: the slab and its two copies, several loads in flight per thread
+    const bool whole = (hx & 3) == 0;
+    const int ncol = whole ? qpr : hx + 1;   // float4 columns, or sites and the padding repeat
+    {
+        const int nrow = (nu + 2) * R, total = 6 * nrow * ncol;
+        constexpr int B = 6;
+        for (int i0 = tid; i0 < total; i0 += B * blockDim.x) {
+            float4 v[B];
+            char* dst[B];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    float nx[4], ny[4], nz[4];
-                    st_nb<PERIODIC>(m, same[0], ex[0], yp[0], ym[0], k, h0, xp, nx);
-                    st_nb<PERIODIC>(m, same[1], ex[1], yp[1], ym[1], k, h0, xp, ny);
-                    st_nb<PERIODIC>(m, same[2], ex[2], yp[2], ym[2], k, h0, xp, nz);
-                    const float sx = stv(s[0], k), sy = stv(s[1], k), sz = stv(s[2], k);
-                    const nmmc_u4 rr = rnext;
-                    if (k < 3)
-                        rnext = sweep_draw<true>(m, boxrow + (uint32_t)(2 * (h0 + k + 1) + xp), swc, (uint32_t)chain);
-                    float hxf, hyf, hzf, tx, ty, tz;
-                    heis_field<4, DK>(m, nx, ny, nz, p, hxf, hyf, hzf);
-                    const bool a = heis_try(hxf, hyf, hzf, sx, sy, sz, p, rr, tx, ty, tz);
-                    out[0][k] = a ? tx : sx;
-                    out[1][k] = a ? ty : sy;
-                    out[2][k] = a ? tz : sz;
-                    any |= a;
+            for (int b = 0; b < B; ++b) {
+                const int i = i0 + b * blockDim.x;
+                dst[b] = nullptr;
+                if (i >= total) continue;
+                const int pr = fdiv(i, g.div_cols), h = i - pr * ncol;
+                const int pu = fdiv(pr, g.div_rows), y = pr - pu * R;   // (plane, unit), row
+                const int pl = nu == g.U ? fdiv(pu, g.div_planes) : pu / (nu + 2);   // 3 colour + component
+                const int ul = pu - pl * (nu + 2);
+                int u = u0 - 1 + ul;
+                if (u < 0 || u >= NU) {
+                    if (!per) continue;
+                    u = u < 0 ? u + NU : u - NU;
                 }
-                if (any) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c)
-                        *reinterpret_cast<float4*>(own + c * NH + y * hx + h0) =
-                            make_float4(out[c][0], out[c][1], out[c][2], out[c][3]);
+                const int k = pl >= 3 ? 1 : 0;
+                const float* src = gsp + pl * P + (size_t)(u * R + y) * hx;
+                char* d = base + k * colb + (ul * R + y) * rowb + (pl - 3 * k) * 16;
+                if (whole) {
+                    v[b] = __ldg(reinterpret_cast<const float4*>(src) + h);
+                    dst[b] = d + h * kQuadBytes;
+                } else if (h < hx || per) {
+                    v[b].x = __ldg(src + (h < hx ? h : 0));
+                    dst[b] = d + (h >> 2) * kQuadBytes + 4 * (h & 3);
                 }
             }
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                if (!dst[b]) continue;
+                if (whole) *reinterpret_cast<float4*>(dst[b]) = v[b];
+                else *reinterpret_cast<float*>(dst[b]) = v[b].x;
+            }
+        }
+    }
+    if (C > 1) {
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
+
+    const float4 p = g.bh[chain];
+    const unsigned long long sw0 = g.sweep[chain];
+    const int items = nu * R * ipr;
+
+    // item `it` of the slab: its row r (unit r / R), row y of the unit, plane z, first site h0
+    auto decode = [&](int it, int& r, int& h0, int& y, int& z) {
+        r = fdiv(it, g.div_ipr);
+        h0 = (it - r * ipr) * 2 * NP;
+        if (DIM == 3) {
+            const int ul = fdiv(r, g.div_rows);
+            y = r - ul * R;
+            z = u0 + ul;
+        } else {
+            y = u0 + r;
+            z = 0;
+        }
+    };
+    auto propose = [&](int colour, int h0, int y, int z, unsigned long long sw, PairProp (&pp)[NP]) {
+        const int xp = (y + z + colour) & 1;
+        const uint32_t box = (uint32_t)(m.edge * (y + m.edge * z) + 2 * h0 + xp);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            const nmmc_u4 ra = sweep_draw<true>(m, box + 4 * j, sw, (uint32_t)chain);
+            const nmmc_u4 rb = sweep_draw<true>(m, box + 4 * j + 2, sw, (uint32_t)chain);
+            pp[j] = pair_propose(ra, rb);
+        }
+    };
+    // sites: a row's bytes are [quad][component][4 sites]
+    auto site_at = [&](int h) { return (h >> 2) * kQuadBytes + (h & 3) * 4; };
+    // the item's sites in the rows y -+ 1 (2-D: the units -+ 1, copies included)
+    auto up_row = [&](const char* q, int y) -> const char* {
+        if (DIM == 2) return q + unitb;
+        return y + 1 < R ? q + rowb : (per ? q - (R - 1) * rowb : zero);
+    };
+    auto dn_row = [&](const char* q, int y) -> const char* {
+        if (DIM == 2) return q - unitb;
+        return y > 0 ? q - rowb : (per ? q + (R - 1) * rowb : zero);
+    };
+    // the x-neighbour outside the item whose first site h0 lies at q, in the row at `row`: site
+    // h0 - 1 (xp = 0) or h0 + 2 NP. In a padded row the padding repeat stands for site hx.
+    const int last = site_at(hx - 1);
+    auto ex_site = [&](const char* row, const char* q, int h0, int xp) -> const char* {
+        if (xp) {
+            if (h0 + 2 * NP >= hx && (whole || NP == 2)) return per && whole ? row : zero;
+            return NP == 2 ? q + kQuadBytes : q + ((h0 & 2) ? kQuadBytes - 8 : 8);
+        }
+        if (h0 == 0) return per ? row + last : zero;
+        return NP == 2 || !(h0 & 2) ? q - kQuadBytes + 12 : q - 4;
+    };
+    auto lds_pair = [&](const char* q, int j, int c) -> f2 {
+        return f2{*reinterpret_cast<const unsigned long long*>(q + 16 * c + 8 * j)};
+    };
+
+    PairProp pp[NP];
+    int r1 = 0, h1 = 0, y1 = 0, z1 = 0;   // this thread's first item: the same in every half-sweep
+    const bool mine = tid < items;
+    // with pairs (few warps) the first item's proposals are ready before the barrier; with quads the
+    // registers are worth more (420 chains of 64^2: 9.8 -> 9.5 us per sweep without)
+    constexpr bool ahead = NP == 1;
+    if (mine) {
+        decode(tid, r1, h1, y1, z1);
+        if (ahead && g.nsweeps > 0) propose(0, h1, y1, z1, sw0, pp);
+    }
+    for (int hs = 0; hs < 2 * g.nsweeps; ++hs) {
+        const int colour = hs & 1;
+        const unsigned long long sw = sw0 + (unsigned)(hs >> 1);
+        char* const cown = base + colour * colb + unitb;          // unit 1: the slab's first
+        const char* const coth = base + (colour ^ 1) * colb + unitb;
+        int r = r1, h0 = h1, y = y1, z = z1;
+        for (int it = tid; it < items; it += blockDim.x) {
+            if (it != tid) decode(it, r, h0, y, z);
+            if (it != tid || !ahead) propose(colour, h0, y, z, sw, pp);
+            const int xp = (y + z + colour) & 1;
+            const int at = site_at(h0);
+            char* const own = cown + r * rowb + at;
+            const char* const orow = coth + r * rowb;
+            const char* const oth = orow + at;
+            const char* const yu = up_row(oth, y);
+            const char* const yd = dn_row(oth, y);
+            const char* const exq = ex_site(orow, oth, h0, xp);
+            f2 s[NP][3], h[NP][3], d[3];
+            {
+                f2 same[NP][3], sh[NP][3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const float ex = *reinterpret_cast<const float*>(exq + 16 * c);
+                    if (NP == 2) {
+                        const F2x2 t = lds_quad(own, c), o = lds_quad(oth, c), q = shifted_quad(o, ex, xp != 0);
+                        s[0][c] = t.a;
+                        s[NP - 1][c] = t.b;
+                        same[0][c] = o.a;
+                        same[NP - 1][c] = o.b;
+                        sh[0][c] = q.a;
+                        sh[NP - 1][c] = q.b;
+                    } else {
+                        s[0][c] = lds_pair(own, 0, c);
+                        const f2 o = lds_pair(oth, 0, c);
+                        same[0][c] = o;
+                        sh[0][c] = pk(xp ? hi(o) : ex, xp ? ex : lo(o));
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < NP; ++j) {
+                    h[j][0] = pk(p.y, p.y);
+                    h[j][1] = pk(p.z, p.z);
+                    h[j][2] = pk(p.w, p.w);
+                    pair_axis_x<DK, false>(m, same[j], sh[j], xp != 0, h[j], d);
+                }
+            }
+#pragma unroll
+            for (int ax = 1; ax < DIM; ++ax) {
+                const char* const ua = ax == 1 ? yu : oth + unitb;
+                const char* const da = ax == 1 ? yd : oth - unitb;
+                f2 a[NP][3], b[NP][3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    if (NP == 2) {
+                        const F2x2 t = lds_quad(ua, c), u = lds_quad(da, c);
+                        a[0][c] = t.a;
+                        a[NP - 1][c] = t.b;
+                        b[0][c] = u.a;
+                        b[NP - 1][c] = u.b;
+                    } else {
+                        a[0][c] = lds_pair(ua, 0, c);
+                        b[0][c] = lds_pair(da, 0, c);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < NP; ++j) {
+                    if (ax == 1) axis_terms<DK, 1, false>(m, a[j], b[j], 1.0f, h[j], d);
+                    else axis_terms<DK, 2, false>(m, a[j], b[j], 1.0f, h[j], d);
+                }
+            }
+            bool any = false;
+#pragma unroll
+            for (int j = 0; j < NP; ++j) any |= pair_accept(h[j], s[j], p.x, pp[j]);
+            if (any) {
+                const int ul = DIM == 3 ? z - u0 : r;
+                const bool to_lo = ul == 0 && has_lo, to_hi = ul == nu - 1 && has_hi;
+                const int row_in_unit = DIM == 3 ? y * rowb : 0;
+                char* const lo_row = base + colour * colb + lo_slot * unitb + row_in_unit;   // in CTA lo_rank
+                char* const hi_row = base + colour * colb + row_in_unit;                     // in CTA hi_rank
+                const int n = hx - h0;   // sites of the row from this item on
+                const bool full = n >= 2 * NP;
+                if (full) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        if (NP == 2)
+                            *reinterpret_cast<ulonglong2*>(own + 16 * c) = make_ulonglong2(s[0][c].v, s[NP - 1][c].v);
+                        else
+                            *reinterpret_cast<unsigned long long*>(own + 16 * c) = s[0][c].v;
+                    }
+                    if (to_lo) {
+                        const uint32_t a = peer_addr(lo_row + at, lo_rank);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+#pragma unroll
+                            for (int j = 0; j < NP; ++j) peer_st(a + 16 * c + 8 * j, s[j][c]);
+                    }
+                    if (to_hi) {
+                        const uint32_t a = peer_addr(hi_row + at, hi_rank);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+#pragma unroll
+                            for (int j = 0; j < NP; ++j) peer_st(a + 16 * c + 8 * j, s[j][c]);
+                    }
+                }
+                if (!whole && (!full || (h0 == 0 && per))) {
+                    // a part-filled item stores its sites one by one; a row's first item also the
+                    // padding repeat of its first site
+                    const uint32_t la = peer_addr(lo_row, lo_rank), ha = peer_addr(hi_row, hi_rank);
+                    const int pad = site_at(hx);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+                        for (int k = 0; k < 2 * NP - 1; ++k) {
+                            if (full || k >= n) continue;
+                            const float v = (k & 1) ? hi(s[k >> 1][c]) : lo(s[k >> 1][c]);
+                            *reinterpret_cast<float*>(own + 16 * c + 4 * k) = v;
+                            if (to_lo) peer_st(la + at + 16 * c + 4 * k, v);
+                            if (to_hi) peer_st(ha + at + 16 * c + 4 * k, v);
+                        }
+                        if (h0 == 0 && per) {
+                            *reinterpret_cast<float*>(own + pad + 16 * c) = lo(s[0][c]);
+                            if (to_lo) peer_st(la + pad + 16 * c, lo(s[0][c]));
+                            if (to_hi) peer_st(ha + pad + 16 * c, lo(s[0][c]));
+                        }
+                    }
+                }
+            }
+        }
+        // the next half-sweep's draws and proposals do not depend on spins: computed while the
+        // other CTAs arrive
+        const int nh = hs + 1;
+        const bool more = mine && nh < 2 * g.nsweeps;
+        if (C > 1) {
+            cluster_arrive();
+            if (more) propose(nh & 1, h1, y1, z1, sw0 + (unsigned)(nh >> 1), pp);
+            cluster_wait();
+        } else {
+            if (more && ahead) propose(nh & 1, h1, y1, z1, sw0 + (unsigned)(nh >> 1), pp);
             __syncthreads();
         }
     }
     if constexpr (MEASURE) {
-        // per chain: the streaming measurement kernel's per-site terms (Old/lib/thermodynamics.cpp:
-        // 71-221) over both colours, FP32 per thread and warp, FP64 across warps in warp order
+        // the streaming measurement kernel's per-site terms (Old/lib/thermodynamics.cpp:71-221)
+        // over both colours of the slab; the angles are summed per plane in 3-D (a slice's charge)
         const int lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-        const bool pq = PERIODIC && m.periodic_q;
+        const bool pq = per && m.periodic_q;
         const int e4 = m.edge - m.edge % 4;
-        for (int sl = 0; sl < ns; ++sl) {
-            float a[kNP];
+        // items of two sites (few registers), 32 items of one plane to a warp at a time
+        const int pairs = (hx + 1) >> 1;
+        const int grows = DIM == 3 ? R : nu * R, gitems = grows * pairs, ngroup = DIM == 3 ? nu : 1;
+        const int chunks = (2 * gitems + 31) >> 5;
+        float* const qpart = reinterpret_cast<float*>(base + 2 * colb);   // [plane][warp] angle sums
+        for (int k = tid; k < ngroup * nw; k += blockDim.x) qpart[k] = 0.0f;
+        float a[kNP];
 #pragma unroll
-            for (int k = 0; k < kNP; ++k) a[k] = 0.0f;
-            for (int it = tid; it < 2 * Q; it += blockDim.x) {
-                const int colour = it & 1, r = it >> 1;
-                const int y = qshift >= 0 ? (r >> qshift) : (r / qpr);
-                const int h0 = (r - y * qpr) * 4;
-                const int xp = (y + colour) & 1;
-                const float* own = st_sm + (size_t)(sl * 6 + colour * 3) * NH;
-                const float* oth = st_sm + (size_t)(sl * 6 + (colour ^ 1) * 3) * NH;
-                float4 s[3], same[3], yp[3], ym[3];
-                float ex[3];
-                st_load<PERIODIC>(m, own, oth, NH, y, h0, xp, s, same, ex, yp, ym);
-                const bool qyu = (y + 1 < m.edge || pq) && (PERIODIC || y + 1 < m.ly);
-                const bool qyd = (y >= 1 || pq);
+        for (int k = 0; k < kNP; ++k) a[k] = 0.0f;
+        __syncthreads();
+        for (int ch = warp; ch < ngroup * chunks; ch += nw) {
+            const int gr = ch / chunks, i2 = (ch - gr * chunks) * 32 + lane;
+            a[10] = 0.0f;
+            if (i2 < 2 * gitems) {
+                const int colour = i2 >= gitems, it = i2 - colour * gitems;
+                const int rg = fdiv(it, g.div_pairs), h0 = (it - rg * pairs) * 2;
+                const int r = gr * grows + rg;
+                const int y = DIM == 3 ? rg : u0 + rg, z = DIM == 3 ? u0 + gr : 0;
+                const int xp = (y + z + colour) & 1, at = site_at(h0);
+                const char* const own = base + colour * colb + unitb + r * rowb + at;
+                const char* const orow = base + (colour ^ 1) * colb + unitb + r * rowb;
+                const char* const oth = orow + at;
+                const char* const yu = up_row(oth, y);
+                const char* const yd = dn_row(oth, y);
+                // the x-neighbour outside the pair
+                int he = xp ? h0 + 2 : h0 - 1;
+                if (he < 0) he = per ? hx - 1 : -1;
+                else if (he >= hx) he = whole ? (per ? 0 : -1) : (he == hx ? hx : -1);
+                const char* const exq = he < 0 ? zero : orow + site_at(he);
+                float sv[3][2], n[3][2 * DIM][2];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
+                for (int c = 0; c < 3; ++c) {
+                    auto two = [&](const char* q, float (&o)[2]) {
+                        const float2 t = *reinterpret_cast<const float2*>(q + 16 * c);
+                        o[0] = t.x;
+                        o[1] = t.y;
+                    };
+                    float same[2];
+                    two(own, sv[c]);
+                    two(oth, same);
+                    const float ex = *reinterpret_cast<const float*>(exq + 16 * c);
+                    const float sh[2] = {xp ? same[1] : ex, xp ? ex : same[0]};
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        n[c][0][k] = xp ? sh[k] : same[k];
+                        n[c][1][k] = xp ? same[k] : sh[k];
+                    }
+                    two(yu, n[c][2]);
+                    two(yd, n[c][3]);
+                    if (DIM == 3) {
+                        two(oth + unitb, n[c][2 * DIM - 2]);
+                        two(oth - unitb, n[c][2 * DIM - 1]);
+                    }
+                }
+                const bool qyu = y + 1 < m.edge || pq, qyd = y >= 1 || pq;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    if (h0 + k >= hx) continue;
                     const int x = 2 * (h0 + k) + xp;
-                    float n0[4], n1[4], n2[4];
-                    st_nb<PERIODIC>(m, same[0], ex[0], yp[0], ym[0], k, h0, xp, n0);
-                    st_nb<PERIODIC>(m, same[1], ex[1], yp[1], ym[1], k, h0, xp, n1);
-                    st_nb<PERIODIC>(m, same[2], ex[2], yp[2], ym[2], k, h0, xp, n2);
-                    const float s0 = stv(s[0], k), s1 = stv(s[1], k), s2 = stv(s[2], k);
-                    float f0 = 0.f, f1 = 0.f, f2 = 0.f;
-                    if (DK <= kDmiGeneral) {
+                    const float s0 = sv[0][k], s1 = sv[1][k], s2 = sv[2][k];
+                    float f0 = 0.f, f1 = 0.f, f2v = 0.f;
 #pragma unroll
-                        for (int d = 0; d < 4; ++d) {
-                            const float J = m.J[d];
-                            f0 = fmaf(J, n0[d], f0);
-                            f1 = fmaf(J, n1[d], f1);
-                            f2 = fmaf(J, n2[d], f2);
+                    for (int ax = 0; ax < DIM; ++ax) {
+                        const int kp = 2 * ax, km = 2 * ax + 1;
+                        const float a0 = n[0][kp][k], a1 = n[1][kp][k], a2 = n[2][kp][k];
+                        const float b0 = n[0][km][k], b1 = n[1][km][k], b2 = n[2][km][k];
+                        if (DK <= kDmiGeneral) {
+                            f0 = fmaf(m.J[km], b0, fmaf(m.J[kp], a0, f0));
+                            f1 = fmaf(m.J[km], b1, fmaf(m.J[kp], a1, f1));
+                            f2v = fmaf(m.J[km], b2, fmaf(m.J[kp], a2, f2v));
                             if (DK == kDmiGeneral) {
-                                f0 = fmaf(m.De[d][1], n2[d], fmaf(-m.De[d][2], n1[d], f0));
-                                f1 = fmaf(m.De[d][2], n0[d], fmaf(-m.De[d][0], n2[d], f1));
-                                f2 = fmaf(m.De[d][0], n1[d], fmaf(-m.De[d][1], n0[d], f2));
+                                f0 = fmaf(m.De[kp][1], a2, fmaf(-m.De[kp][2], a1, f0));
+                                f1 = fmaf(m.De[kp][2], a0, fmaf(-m.De[kp][0], a2, f1));
+                                f2v = fmaf(m.De[kp][0], a1, fmaf(-m.De[kp][1], a0, f2v));
+                                f0 = fmaf(m.De[km][1], b2, fmaf(-m.De[km][2], b1, f0));
+                                f1 = fmaf(m.De[km][2], b0, fmaf(-m.De[km][0], b2, f1));
+                                f2v = fmaf(m.De[km][0], b1, fmaf(-m.De[km][1], b0, f2v));
                             }
-                        }
-                    } else {
-#pragma unroll
-                        for (int ax = 0; ax < 2; ++ax) {
-                            const int kp = 2 * ax, km = 2 * ax + 1;
-                            const float J = m.J[kp];
-                            f0 = fmaf(J, n0[kp] + n0[km], f0);
-                            f1 = fmaf(J, n1[kp] + n1[km], f1);
-                            f2 = fmaf(J, n2[kp] + n2[km], f2);
-                            const float d0 = n0[kp] - n0[km], d1 = n1[kp] - n1[km], d2 = n2[kp] - n2[km];
-                            if (DK == kDmiPairs) {
-                                f0 = fmaf(m.De[kp][1], d2, fmaf(-m.De[kp][2], d1, f0));
-                                f1 = fmaf(m.De[kp][2], d0, fmaf(-m.De[kp][0], d2, f1));
-                                f2 = fmaf(m.De[kp][0], d1, fmaf(-m.De[kp][1], d0, f2));
-                            } else {
-                                const float D = m.De[kp][ax];
-                                if (ax == 0) {
-                                    f1 = fmaf(-D, d2, f1);
-                                    f2 = fmaf(D, d1, f2);
-                                } else {
-                                    f0 = fmaf(D, d2, f0);
-                                    f2 = fmaf(-D, d0, f2);
-                                }
+                        } else {   // +-axis pairs: J (n+ + n-) + De(+a) x (n+ - n-)
+                            const float J = m.J[kp], D0 = m.De[kp][0], D1 = m.De[kp][1], D2 = m.De[kp][2];
+                            const float d0 = a0 - b0, d1 = a1 - b1, d2 = a2 - b2;
+                            f0 = fmaf(J, a0 + b0, f0);
+                            f1 = fmaf(J, a1 + b1, f1);
+                            f2v = fmaf(J, a2 + b2, f2v);
+                            if (DK == kDmiPairs || ax != 0) {
+                                f0 = fmaf(D1, d2, fmaf(-D2, d1, f0));
+                            }
+                            if (DK == kDmiPairs || ax != 1) {
+                                f1 = fmaf(D2, d0, fmaf(-D0, d2, f1));
+                            }
+                            if (DK == kDmiPairs || ax != 2) {
+                                f2v = fmaf(D0, d1, fmaf(-D1, d0, f2v));
                             }
                         }
                     }
-                    a[0] = fmaf(s0, f0, fmaf(s1, f1, fmaf(s2, f2, a[0])));
+                    a[0] = fmaf(s0, f0, fmaf(s1, f1, fmaf(s2, f2v, a[0])));
                     a[1] += s0;
                     a[2] += s1;
                     a[3] += s2;
-                    if (colour == 0) {
+                    if (colour == 0) {   // subM(0): (sum of coordinates) % 2 == 0
                         a[4] += s0;
                         a[5] += s1;
                         a[6] += s2;
                     }
-                    const int possum = x + y, posdiff = -x + y + e4;
-                    if (possum % 4 == 0 && posdiff % 4 == 0) {
+                    const int possum = x + y, posdiff = y - x + e4;   // C truncating remainders
+                    const int z4 = z & 3;
+                    if ((z4 & 1) == 0 && (possum & 3) == z4 && posdiff % 4 == z4) {
                         a[7] += s0;
                         a[8] += s1;
                         a[9] += s2;
                     }
-                    const bool qxm = (x >= 1 || pq), qxp = (x + 1 < m.edge || pq);
-                    if (qxm && qyu) a[10] += solid_angle_f(s0, s1, s2, n0[1], n1[1], n2[1], n0[2], n1[2], n2[2]);
-                    if (qxp && qyd) a[10] += solid_angle_f(s0, s1, s2, n0[0], n1[0], n2[0], n0[3], n1[3], n2[3]);
+                    const bool qxm = x >= 1 || pq, qxp = x + 1 < m.edge || pq;
+                    if (qxm && qyu)
+                        a[10] += solid_angle_f(s0, s1, s2, n[0][1][k], n[1][1][k], n[2][1][k], n[0][2][k],
+                                               n[1][2][k], n[2][2][k]);
+                    if (qxp && qyd)
+                        a[10] += solid_angle_f(s0, s1, s2, n[0][0][k], n[1][0][k], n[2][0][k], n[0][3][k],
+                                               n[1][3][k], n[2][3][k]);
                 }
             }
+            float v = a[10];
 #pragma unroll
-            for (int k = 0; k < kNP; ++k) {
-                float v = a[k];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) qpart[gr * nw + warp] += v;   // this warp's own slot
+        }
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                if (lane == 0) wred[warp][k] = v;
+        for (int k = 0; k < kNP - 1; ++k) {
+            float v = a[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) wred[warp][k] = v;
+        }
+        __syncthreads();
+        // a lane per plane: its angles over the warps, the slice's charge in 3-D
+        if (warp == 0) {
+            double qsum = 0.0;
+            for (int gr = lane; gr < ngroup; gr += 32) {
+                double t = 0.0;
+                for (int w = 0; w < nw; ++w) t += (double)qpart[gr * nw + w];
+                qsum += t;
+                if (DIM == 3 && g.q) g.q[(size_t)ci * g.nslices + u0 + gr] = t / (2 * M_PI);
             }
-            __syncthreads();
-            if (warp == 0) {
-                double v = 0.0;
-                if (lane < kNP)
-                    for (int w = 0; w < nw; ++w) v += (double)wred[w][lane];
-                const int ch = sch[sl], ci = c0 + sl;
-                const double qv = __shfl_sync(0xffffffffu, v, 10) / (2 * M_PI);
-                if (qout && lane == 0) qout[ci] = qv;
-                finalize_chain_warp(v, lane, Hd + 3 * (size_t)ch, qv, obs + (size_t)ci * NMMC_OBS_N,
-                                    acc + (size_t)ch * NMMC_ACC_N, accumulate);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) qsum += __shfl_down_sync(0xffffffffu, qsum, o);
+            qsum = __shfl_sync(0xffffffffu, qsum, 0);
+            double v = 0.0;
+            if (lane < kNP - 1)
+                for (int w = 0; w < nw; ++w) v += (double)wred[w][lane];
+            if (lane == kNP - 1) v = qsum;
+            if (lane < kNP) {
+                if (rank == 0) cred[0][lane] = v;
+                else peer_st(peer_addr(&cred[rank][lane], 0), v);
             }
+        }
+        if (C > 1) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
             __syncthreads();
         }
+        if (rank == 0 && warp == 0) {
+            double v = 0.0;
+            if (lane < kNP)
+                for (int k = 0; k < C; ++k) v += cred[k][lane];
+            const double qv = __shfl_sync(0xffffffffu, v, kNP - 1) / (2 * M_PI);
+            if (DIM == 2 && g.q && lane == 0) g.q[ci] = qv;
+            finalize_chain_warp(v, lane, g.Hd + 3 * (size_t)chain, qv, g.obs + (size_t)ci * NMMC_OBS_N,
+                                g.acc + (size_t)chain * NMMC_ACC_N, g.accumulate);
+        }
     }
-    for (int i = tid; i < ns * 6 * nv; i += blockDim.x) {
-        const int sl = i / (6 * nv), r = i - sl * 6 * nv, pl = r / nv, j = r - pl * nv;
-        reinterpret_cast<float4*>(spins + ((size_t)sch[sl] * 6 + pl) * P)[j] =
-            reinterpret_cast<const float4*>(st_sm)[(size_t)(sl * 6 + pl) * nv + j];
+    // the slab back to HBM, without its copies
+    {
+        const int n4 = whole ? qpr : hx, nrow = nu * R, total = 6 * nrow * n4;
+#pragma unroll 4
+        for (int i = tid; i < total; i += blockDim.x) {
+            const int pr = i / n4, h = i - pr * n4;
+            const int pl = pr / nrow, r = pr - pl * nrow;
+            const int k = pl >= 3 ? 1 : 0;
+            float* dst = gsp + pl * P + (size_t)(u0 * R + r) * hx;
+            const char* src = base + k * colb + unitb + r * rowb + (pl - 3 * k) * 16;
+            if (whole)
+                reinterpret_cast<float4*>(dst)[h] = *reinterpret_cast<const float4*>(src + h * kQuadBytes);
+            else
+                dst[h] = *reinterpret_cast<const float*>(src + site_at(h));
+        }
     }
-    for (int t = tid; t < ns; t += blockDim.x) sweep[sch[t]] += (unsigned long long)nsweeps;
+    if (rank == 0 && tid == 0) g.sweep[chain] = sw0 + (unsigned long long)g.nsweeps;
 }
 
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
-// Bytes of one chain in shared memory (6 planes of hx * ly floats), or 0 when the lattice is not
-// covered: unmasked 2-D Heisenberg lattices with rows of a multiple of 4 sites per colour and
-// the checkerboard's axis tables.
-size_t stencil_chain_bytes(const Ctx& c) {
-    if (c.ising || c.masked || c.m.general || c.dim != 2 || (c.m.hx % 4) != 0) return 0;
-    return (size_t)6 * c.m.nhalf * sizeof(float);
-}
+namespace {
 
-// Chains per CTA for a call on n chains: spread over the SMs, as many as the shared memory
-// holds (0: not even one).
-int stencil_slots(const Ctx& c, int n) {
-    const size_t cb = stencil_chain_bytes(c);
-    if (cb == 0 || n <= 0) return 0;
-    const size_t static_bytes = kStMaxSlots * (sizeof(float4) + sizeof(unsigned long long) + sizeof(int)) +
-                                (kStThreads / 32) * kNP * sizeof(float) + 64;
-    if (c.smem_optin <= static_bytes) return 0;
-    const int fit = (int)std::min<size_t>(kStMaxSlots, (c.smem_optin - static_bytes) / cb);
-    if (fit < 1) return 0;
-    const int spread = (n + c.sm_count - 1) / c.sm_count;
-    return std::min(fit, std::max(1, spread));
-}
+using StencilFn = void (*)(const DevModel, const StencilArgs);
 
-template <int DK, bool PERIODIC, bool MEASURE>
-static int stencil_launch_t(Ctx& c, const int* d_chains, int n, int nsweeps, int accumulate) {
-    const int S = stencil_slots(c, n);
-    if (S < 1) return set_error(NMMC_ERR_UNSUPPORTED, "lattice does not fit the stencil resident kernel");
-    const size_t smem = (size_t)S * stencil_chain_bytes(c);
-    auto kern = k_resident_stencil<DK, PERIODIC, MEASURE>;
-    size_t& set = c.stencil_smem[DK * 4 + (PERIODIC ? 2 : 0) + (MEASURE ? 1 : 0)];
-    if (set < smem) {   // raised once per kernel and context to the largest size launched
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return cuda_check(e, "stencil kernel shared memory");
-        set = smem;
+template <int DIM, int NP, bool MEASURE>
+StencilFn stencil_kernel_dk(int dk) {
+    switch (dk) {
+        case kDmiNone: return k_resident_stencil<DIM, kDmiNone, NP, MEASURE>;
+        case kDmiGeneral: return k_resident_stencil<DIM, kDmiGeneral, NP, MEASURE>;
+        case kDmiPairs: return k_resident_stencil<DIM, kDmiPairs, NP, MEASURE>;
+        default: return k_resident_stencil<DIM, kDmiAxial, NP, MEASURE>;
     }
-    const int grid = (n + S - 1) / S;
-    // a width that gives every thread the same number of quads per half-sweep
-    const int items = S * (c.m.hx / 4) * c.m.ly;
-    const int per = (items + kStThreads - 1) / kStThreads;
-    const int threads = std::max(32, ((items + per - 1) / per + 31) / 32 * 32);
-    kern<<<grid, threads, smem, c.stream>>>(c.m, (float*)c.d_spins, c.d_bh, c.d_sweep, d_chains, n, S, nsweeps,
-                                            c.d_Hd, c.d_obs, c.d_q, c.d_acc, accumulate);
-    return cuda_check(cudaGetLastError(), "k_resident_stencil");
 }
 
-template <bool PERIODIC, bool MEASURE>
-static int stencil_launch_d(Ctx& c, const int* d_chains, int n, int nsweeps, int accumulate) {
-    switch (c.m.dmi_kind) {
-        case kDmiNone: return stencil_launch_t<kDmiNone, PERIODIC, MEASURE>(c, d_chains, n, nsweeps, accumulate);
-        case kDmiGeneral: return stencil_launch_t<kDmiGeneral, PERIODIC, MEASURE>(c, d_chains, n, nsweeps, accumulate);
-        case kDmiPairs: return stencil_launch_t<kDmiPairs, PERIODIC, MEASURE>(c, d_chains, n, nsweeps, accumulate);
-        default: return stencil_launch_t<kDmiAxial, PERIODIC, MEASURE>(c, d_chains, n, nsweeps, accumulate);
+template <int DIM, bool MEASURE>
+StencilFn stencil_kernel_np(int dk, int np) {
+    return np == 1 ? stencil_kernel_dk<DIM, 1, MEASURE>(dk) : stencil_kernel_dk<DIM, 2, MEASURE>(dk);
+}
+
+StencilFn stencil_kernel(const Ctx& c, int np, bool measure) {
+    const int dk = c.m.dmi_kind;
+    if (c.dim == 3) return measure ? stencil_kernel_np<3, true>(dk, np) : stencil_kernel_np<3, false>(dk, np);
+    return measure ? stencil_kernel_np<2, true>(dk, np) : stencil_kernel_np<2, false>(dk, np);
+}
+
+FastDiv fast_div(int d) { return FastDiv{d <= 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d), d}; }
+
+int units_of(const Ctx& c) { return c.dim == 3 ? c.m.lz : c.m.ly; }
+int rows_of(const Ctx& c) { return c.dim == 3 ? c.m.ly : 1; }
+int quads_per_row(const Ctx& c) { return (c.m.hx + 3) / 4; }
+
+// Dynamic shared memory of a CTA with 1/C of a chain.
+size_t stencil_bytes(const Ctx& c, int C) {
+    const size_t U = (units_of(c) + C - 1) / C;
+    return kQuadBytes + 2 * (U + 2) * (size_t)rows_of(c) * quads_per_row(c) * kQuadBytes +
+           (c.dim == 3 ? U : 1) * (kStThreads / 32) * sizeof(float);   // with the planes' angle sums
+}
+
+size_t stencil_budget(const Ctx& c) {
+    const size_t fixed = sizeof(float) * (kStThreads / 32) * kNP + sizeof(double) * kStMaxCluster * kNP + 64;
+    return c.smem_optin > fixed ? c.smem_optin - fixed : 0;
+}
+
+cudaLaunchConfig_t stencil_config(int n, const StencilShape& s, cudaStream_t stream, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)n * s.C);
+    cfg.blockDim = dim3(s.threads);
+    cfg.dynamicSmemBytes = s.smem;
+    cfg.stream = stream;
+    if (s.C > 1) {
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = s.C;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
     }
+    return cfg;
+}
+
+// Both limits are raised to this device's maximum, the same value in every context: a kernel's
+// attributes belong to the process, so a context that set only what it needs would lower them
+// for the others.
+int stencil_attrs(const Ctx& c) {
+    for (int v = 0; v < 4; ++v) {
+        const void* k = (const void*)stencil_kernel(c, 1 + (v & 1), v >= 2);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stencil_budget(c));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return cuda_check(e, "stencil kernel attributes");
+    }
+    return NMMC_OK;
+}
+
+// Items of a CTA's largest slab with np pairs per item.
+int stencil_items(const Ctx& c, int C, int np) {
+    const int U = (units_of(c) + C - 1) / C;
+    return U * rows_of(c) * ((c.m.hx + 2 * np - 1) / (2 * np));
+}
+
+// Item size and threads of a CTA. 768 threads per SM (the register file at 80 each) are shared by
+// the CTAs that run on one; quads, unless pairs still leave every thread at most one item.
+void stencil_width(const Ctx& c, int n, StencilShape& s) {
+    const size_t fit = std::max<size_t>(1, (c.smem_optin + 1024) / (s.smem + 4096));
+    const int share = (int)std::min<size_t>(std::min(fit, (size_t)3), (size_t)((long)n * s.C + c.sm_count - 1) / c.sm_count);
+    const int most = kStThreads / std::max(1, share) / 32 * 32;
+    s.np = stencil_items(c, s.C, 1) <= most ? 1 : 2;
+    const int items = stencil_items(c, s.C, s.np), each = (items + most - 1) / most;
+    s.threads = std::max(32, ((items + each - 1) / each + 31) / 32 * 32);
+}
+
+// Clusters of C CTAs that run at the same time (0: none fits).
+int active_clusters(const Ctx& c, const StencilShape& s) {
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t cfg = stencil_config(1, s, c.stream, &at);
+    int k = 0;
+    const void* f = (const void*)stencil_kernel(c, s.np, true);   // the variant with the larger footprint
+    cudaError_t e;
+    if (s.C > 1) {
+        e = cudaOccupancyMaxActiveClusters(&k, f, &cfg);
+    } else {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, f, s.threads, s.smem);
+        k *= c.sm_count;
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return k;
+}
+
+}  // namespace
+
+// The shape of a call on n chains (C = 0: the lattice is not covered, or does not fit). The time
+// of a half-sweep is close to 1000 cycles (update latency and barrier) plus 2.2 cycles for every
+// site that the CTAs sharing an SM update, once per wave of clusters that run together; C is the
+// smallest cluster with the least of that. Measured per sweep, model against time at 1.92 GHz:
+// 16 chains of 128^2 C = 16 3.4 / 3.3 us, C = 8 (two waves) 6.8 / 5.0; 8 of 30^3 C = 10 4.3 / 4.6,
+// C = 8 5.4 / 6.1, C = 16 (two waves) 5.4 / 6.9; 420 of 64^2 C = 1 15 / 9.6, C = 2 26 / 9.9 (two
+// waves overlap there, but do not win).
+StencilShape stencil_shape(const Ctx& c, int n) {
+    StencilShape best;
+    if (c.ising || c.masked || c.m.general || n <= 0 || stencil_attrs(c) != NMMC_OK) return best;
+    double best_cost = 0;
+    for (int C = 1; C <= kStMaxCluster && C <= units_of(c); ++C) {
+        StencilShape s;
+        s.C = C;
+        s.smem = stencil_bytes(c, C);
+        if (s.smem > stencil_budget(c) || s.smem / 4 > 65535) continue;   // 65535: FastDiv's range
+        stencil_width(c, n, s);
+        auto cost_of = [&](int active) {
+            const int waves = (n + active - 1) / active, at_once = std::min(n, active);
+            const int per_sm = (int)(((long)at_once * C + c.sm_count - 1) / c.sm_count);
+            return waves * (1000.0 + 2.2 * per_sm * stencil_items(c, C, s.np) * 2 * s.np);
+        };
+        if (best.C && cost_of(n) >= 0.99 * best_cost) continue;   // not even with every cluster running
+        const int active = active_clusters(c, s);
+        if (active < 1) continue;
+        const double cost = cost_of(active);
+        if (!best.C || cost < 0.99 * best_cost) {
+            best = s;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 // nsweeps sweeps of the listed chains (d_chains, n entries, each chain at most once) and, with
 // measure, their observables in list order and (accumulate) their accumulators.
 int launch_stencil_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure, int accumulate) {
     if (n <= 0) return NMMC_OK;
-    if (c.periodic) return measure ? stencil_launch_d<true, true>(c, d_chains, n, nsweeps, accumulate)
-                                   : stencil_launch_d<true, false>(c, d_chains, n, nsweeps, accumulate);
-    return measure ? stencil_launch_d<false, true>(c, d_chains, n, nsweeps, accumulate)
-                   : stencil_launch_d<false, false>(c, d_chains, n, nsweeps, accumulate);
+    auto known = c.st_shapes.find(n);
+    if (known == c.st_shapes.end()) known = c.st_shapes.emplace(n, stencil_shape(c, n)).first;
+    const StencilShape& s = known->second;
+    if (s.C < 1) return set_error(NMMC_ERR_UNSUPPORTED, "lattice does not fit the stencil resident kernel");
+    StencilArgs g{};
+    g.spins = (float*)c.d_spins;
+    g.bh = c.d_bh;
+    g.sweep = c.d_sweep;
+    g.chains = d_chains;
+    g.nsweeps = nsweeps;
+    g.C = s.C;
+    g.NU = units_of(c);
+    g.R = rows_of(c);
+    g.U = (g.NU + s.C - 1) / s.C;
+    g.qpr = quads_per_row(c);
+    g.ipr = (c.m.hx + 2 * s.np - 1) / (2 * s.np);
+    g.div_ipr = fast_div(g.ipr);
+    g.div_pairs = fast_div((c.m.hx + 1) / 2);
+    g.div_rows = fast_div(g.R);
+    g.div_cols = fast_div(c.m.hx % 4 ? c.m.hx + 1 : g.qpr);
+    g.div_planes = fast_div(g.U + 2);
+    g.Hd = c.d_Hd;
+    g.obs = c.d_obs;
+    g.q = c.d_q;
+    g.acc = c.d_acc;
+    g.nslices = c.nslices;
+    g.accumulate = accumulate;
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t cfg = stencil_config(n, s, c.stream, &at);
+    return cuda_check(cudaLaunchKernelEx(&cfg, stencil_kernel(c, s.np, measure), (const DevModel)c.m, (const StencilArgs)g),
+                      "k_resident_stencil");
 }
 
 }  // namespace nmmc

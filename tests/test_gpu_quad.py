@@ -44,3 +44,36 @@ def test_quad_half_sweep_identical(shape, edge, periodic, kind, sign):
     a = chains(shape, edge, periodic, kind, OPT_SWEEP_PATH=1, OPT_DMI_SIGN=sign, OPT_HALF_KERNEL=0)
     b = chains(shape, edge, periodic, kind, OPT_SWEEP_PATH=1, OPT_DMI_SIGN=sign, OPT_HALF_KERNEL=1)
     assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 3, 40])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("shape,edge,periodic", [("s", 2, True), ("s", 6, False), ("s", 10, True), ("s", 64, True),
+                                                 ("s", 130, True), ("c", 4, True), ("c", 6, False), ("c", 10, True),
+                                                 ("c", 30, True), ("c", 32, False)])
+def test_cluster_stencil_identical(shape, edge, periodic, kind, n):
+    """One chain per cluster of 1 to 16 CTAs: chains and observables against the streaming path."""
+    dim = 3 if shape == "c" else 2
+    opt = make_options(shape, edge=edge, periodic=periodic, J=1.0, D=0.0 if kind == "none" else 1.0)
+    res = []
+    for path, stencil in ((0, 2), (1, 0)):
+        s = Sampler(opt, table(dim, kind), T=np.linspace(0.4, 1.3, n), H=np.linspace(0.3, -0.2, n), seed=5)
+        s.option(L.OPT_SWEEP_PATH, path)
+        s.option(L.OPT_RESIDENT_STENCIL, stencil)
+        s.sweep(3)
+        s.sweep(2, [n - 1])
+        o, q = s.sweep_measure(2, accumulate=True)
+        h, hq = s.sample(1, 2, np.arange(n)[::-1], with_q=True)
+        res.append((np.stack([s.get_spins(k) for k in range(n)]), np.concatenate([o[None], h]),
+                    np.concatenate([q[None], hq]), s.accumulators()))
+        s.close()
+    (sa, oa, qa, aa), (sb, ob, qb, ab) = res
+    assert np.array_equal(sa, sb)
+    # FP32 terms in another order: 2^-24 per term of at most 4 (energy) or 1, pi per angle
+    N = edge ** dim
+    tol = np.full(14, 2.0 ** -20 * N)
+    tol[13] = 2.0 ** -20 * N
+    assert np.all(np.abs(oa - ob) <= tol)
+    assert np.all(np.abs(qa - qb) <= 2.0 ** -20 * edge ** 2 + 1e-6)
+    assert np.array_equal(aa[:, 0], ab[:, 0])
