@@ -52,7 +52,7 @@ int upload_params(Ctx& c) {
                               cudaMemcpyHostToDevice, c.stream));
     NMMC_CUDA(cudaEventRecord(c.ev_params, c.stream));
     c.params_dirty = false;
-    return NMMC_OK;
+    return launch_ising_table(c);
 }
 
 // A list that names every chain in order is the all-chains call: no list upload, and the
@@ -213,6 +213,7 @@ static void destroy_ctx(Ctx* c) {
     cudaFree(c->d_cspins);
     cudaFree(c->d_ctab);
     cudaFree(c->d_bh);   // d_Hd lives in the same block
+    cudaFree(c->d_itab);
     cudaFree(c->d_sweep);
     cudaFree(c->d_all);
     cudaFree(c->d_list);
@@ -548,6 +549,7 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
     // (beta, H) float4 per chain, then H in FP64 (3 per chain): one block, one upload
     NMMC_TRY(cudaMalloc(&c->d_bh, (sizeof(float4) + 3 * sizeof(double)) * nchains));
     c->d_Hd = reinterpret_cast<double*>(c->d_bh + nchains);
+    if (ising_table_bytes(*c)) NMMC_TRY(cudaMalloc(&c->d_itab, ising_table_bytes(*c)));
     NMMC_TRY(cudaMalloc(&c->d_sweep, sizeof(unsigned long long) * nchains));
     NMMC_TRY(cudaMemset(c->d_sweep, 0, sizeof(unsigned long long) * nchains));
     NMMC_TRY(cudaMalloc(&c->d_all, sizeof(int) * nchains));

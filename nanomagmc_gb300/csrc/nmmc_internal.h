@@ -162,6 +162,7 @@ struct Ctx {
     bool ctab_built = false;
     bool ctab_packed = true;
     float4* d_bh = nullptr;             // per chain (beta, H0, H1, H2) in FP32
+    uint32_t* d_itab = nullptr;         // Ising word kernels: per chain 128 acceptance limits (nmmc_ising.cu)
     double* d_Hd = nullptr;             // per chain H in FP64 (3 doubles) for the energy
     unsigned long long* d_sweep = nullptr;  // per chain sweep counter
     int* d_all = nullptr;               // 0..nchains-1
@@ -270,6 +271,13 @@ int launch_add_av(Ctx& c);   // adds the av chains' spins to their sums (no-op w
 int launch_delta_e(Ctx& c, int chain, const int32_t* d_sites, const float* d_trial, int n, double* d_out);
 int launch_replay(Ctx& c, int chain, const nmmc_event* d_ev, size_t n, uint8_t* d_acc, long long* d_first);
 int launch_advance(Ctx& c, const int* d_chains, int n, int nsweeps);
+
+// ---- Ising words (nmmc_ising.cu) ----
+bool ising_words_ok(const Ctx& c);             // the lattice is covered
+size_t ising_table_bytes(const Ctx& c);
+int launch_ising_table(Ctx& c);                // acceptance limits from the uploaded (beta, H)
+void launch_ising_words(Ctx& c, const int* d_chains, int n, int colour, unsigned off);
+void launch_measure_ising(Ctx& c, dim3 grid, const int* d_chains, int rows, int nblk_slice, double* partial);
 
 // ---- wavefront sweeps (nmmc_wave.cu) ----
 // Tile rows of the wavefront sweep on this lattice (0: the lattice is not covered).

@@ -1058,6 +1058,7 @@ static HalfFn pick_half(const Ctx& c) {
         if (c.dim == 3) return per ? pick_heis_q4<3, true>(dk) : pick_heis_q4<3, false>(dk);
         return per ? pick_heis_q4<2, true>(dk) : pick_heis_q4<2, false>(dk);
     }
+    if (ising_words_ok(c) && c.half_kernel != 1) return launch_ising_words;
     if (c.ising) {
         if (c.dim == 3) {
             if (per) return msk ? ising_launch<3, true, true> : ising_launch<3, true, false>;
@@ -2154,6 +2155,8 @@ static int measure_with(Ctx& c, const int* d_chains, int n, double* partial, dou
         dim3 grid(nblk, n);
         const float* sp = (const float*)c.d_spins;
         measure_q4_launch(c, grid, sp, d_chains, rows, nblk_slice, partial);
+    } else if (ising_words_ok(c) && c.half_kernel != 1) {   // integer sums: exact in both modes
+        launch_measure_ising(c, dim3(nblk, n), d_chains, rows, nblk_slice, partial);
     } else if (c.ising) {
         if (c.dim == 3) c.masked ? measure_launch<3, true, true>(c, d_chains, n, rows, nblk_slice, fp64, partial)
                                  : measure_launch<3, true, false>(c, d_chains, n, rows, nblk_slice, fp64, partial);
