@@ -196,8 +196,11 @@ int sweep_measure_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, 
             return accumulate ? launch_add_av(c) : NMMC_OK;
         }
         if ((rc = run_sweeps(c, d_chains, h_chains, n, nsweeps, res, false, 0, allow_timing))) return rc;
+        c.class_fresh = c.m.general != 0;
     }
-    if ((rc = launch_measure(c, d_chains, n, accumulate))) return rc;
+    rc = launch_measure(c, d_chains, n, accumulate);
+    c.class_fresh = false;
+    if (rc) return rc;
     return accumulate ? launch_add_av(c) : NMMC_OK;
 }
 
@@ -226,6 +229,7 @@ static void destroy_ctx(Ctx* c) {
     if (c->ev_list) cudaEventDestroy(c->ev_list);
     cudaFree(c->d_av);
     cudaFree(c->d_av_list);
+    cudaFree(c->d_class);
     cudaFree(c->d_goff);
     cudaFree(c->d_gjs);
     cudaFree(c->d_gje);
@@ -465,6 +469,7 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
         while ((1 << k) < v) ++k;
         return k;
     };
+    c->h_goff = goff;
     m.qpr_shift = (m.hx % 4 == 0) ? log2_or(m.hx / 4) : -1;
     m.ly_shift = log2_or(m.ly);
     m.key0 = (uint32_t)seed;
@@ -767,6 +772,7 @@ int nmmc_sample(nmmc_ctx* c, const int* chains, int n, int nsweeps, int nsamples
     // the HBM path's compact tables: no allocation or table upload inside the capture
     if (!(c->sweep_path != 1 && resident_chosen(*c))) {
         if ((rc = compact_prepare(*c))) return rc;
+        class_ready(*c);  // the class planes of a general table
         wave_ready(*c);   // the wavefront sweeps' second array (when enabled), not inside the capture
     }
     if ((rc = measure_prepare(*c, n))) return rc;

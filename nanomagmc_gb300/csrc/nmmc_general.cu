@@ -8,6 +8,17 @@
 //
 // The Philox draw of a site is the one the checkerboard kernels use (box index, sweep
 // counter, chain), so only the order of the classes differs from them.
+//
+// Unmasked Heisenberg lattices are swept in class planes: per chain and class its sites in row
+// order, one float4 (x, y, z, 0) each, gathered from the box layout by each call and written back.
+// The neighbours of a class through one record are all of one other class, so a warp's gather
+// through a record is one contiguous 16-byte load per lane; in the box layout it was three
+// scalar loads at a stride of half the period with its own wrap and plane arithmetic. A class of
+// 20 chains of 64^3, 18 records: 1360 -> 773 instructions per update, 34.6 -> 23.6 us (issue 61 %
+// busy, DRAM 44 %: every launch reads the whole lattices, 84 MB). Tables of more than 36 records
+// and other lattices keep the box layout (k_colour_sweep).
+#include <algorithm>
+
 #include "nmmc_kernels.cuh"
 
 namespace nmmc {
@@ -155,6 +166,375 @@ k_colour_sweep(const DevModel m, void* __restrict__ spins_v, const uint8_t* __re
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// Class planes of unmasked Heisenberg lattices
+// ------------------------------------------------------------------------------------------
+// Cells of a class: kind 1 (x + b y + c z mod q) every row's x = r, r + q, ...; kind 2 (product)
+// every axis' residue cx, cx + p, .... Each class has room for the longest; cells whose site
+// would lie outside the box are never used. Divisions are by multiplication: n / d =
+// __umulhi(n, ceil(2^32 / d)) for n * d < 2^32 and d > 1.
+struct Div32 { uint32_t mul; int d; };
+struct ClassShape {
+    int kx, ky, kz, cells;
+    int step;                // q (kind 1) or p (kind 2)
+    Div32 by_step, by_kx, by_ky;
+    size_t chain;            // float4 of a chain: every class, and one zero cell past them
+};
+
+__device__ __forceinline__ unsigned div32(unsigned n, const Div32& d) { return d.mul ? __umulhi(n, d.mul) : n; }
+
+static Div32 make_div(int d) { return Div32{d <= 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d), d}; }
+
+static ClassShape class_shape(const Ctx& c) {
+    ClassShape s;
+    s.step = c.m.col_kind == 1 ? c.m.col_q : c.m.col_p;
+    s.kx = (c.edge + s.step - 1) / s.step;
+    s.ky = c.m.col_kind == 1 ? c.m.ly : s.kx;
+    s.kz = c.dim == 2 ? 1 : (c.m.col_kind == 1 ? c.m.lz : s.kx);
+    s.cells = s.kx * s.ky * s.kz;
+    s.by_step = make_div(s.step);
+    s.by_kx = make_div(s.kx);
+    s.by_ky = make_div(s.ky);
+    s.chain = (size_t)s.cells * c.m.col_q + 1;
+    return s;
+}
+
+// Site of cell t of class `cls`; false where the cell has none.
+template <int DIM>
+__device__ __forceinline__ bool class_site(const DevModel& m, const ClassShape& s, int cls, int t, int& x, int& y,
+                                           int& z) {
+    const int row = div32(t, s.by_kx), k = t - row * s.kx;
+    const int jz = DIM == 3 ? div32(row, s.by_ky) : 0, jy = row - jz * s.ky;
+    if (m.col_kind == 1) {
+        y = jy;
+        z = jz;
+        const int q = m.col_q;   // x = cls - b y - c z (mod q)
+        const unsigned w = (unsigned)(m.col_b * y + m.col_c * z);
+        int r = cls - (int)(w - div32(w, s.by_step) * q);
+        r += r < 0 ? q : 0;
+        x = r + k * q;
+    } else {
+        const int p = m.col_p;
+        x = cls % p + k * p;
+        y = (cls / p) % p + jy * p;
+        z = DIM == 3 ? cls / (p * p) + jz * p : 0;
+    }
+    return jz < s.kz && x < m.edge && y < m.ly && z < m.lz;
+}
+
+// A table in the form the class kernels take, as a kernel parameter: a neighbour's index in the
+// chain's class planes is base (its class, the same for every site of a class) + the term of its
+// row (one of `na` distinct (oy, oz)) + the term of its column (one of `nb` distinct ox). A thread
+// computes its site's na + nb terms once and keeps them in its own column of shared memory.
+constexpr int kClassBatch = 9, kClassRecs = 4 * kClassBatch, kClassRows = 16, kClassCols = 8;
+struct ClassTable {
+    int n, na, nb;                 // n: records, padded to whole batches with records of J = D = 0
+    int2 row[kClassRows];          // distinct (oy, oz), wrapped into [0, edge) on periodic lattices
+    int col[kClassCols];           // distinct ox
+    int2 at[kClassRecs];           // per record: its row and its column term (offsets into the slots)
+    float4 j[kClassRecs];          // J, D
+};
+struct ClassBase { int b[kClassRecs]; };   // per record: first cell of the neighbours' class
+constexpr int kNoCell = -(1 << 30);        // a term that makes the index negative: past an open edge
+
+// The site's terms into its column of `slots` ([slot][256]; the last slot holds 0, for padding).
+template <int DIM, bool PERIODIC>
+__device__ __forceinline__ void class_terms(const DevModel& m, const ClassShape& s, const ClassTable& t, int x, int y,
+                                            int z, int* slots) {
+    const unsigned e = m.edge;
+    const bool lin = m.col_kind == 1;
+#pragma unroll 3
+    for (int i = 0; i < t.na; ++i) {
+        unsigned qy = y + t.row[i].x, qz = DIM == 3 ? z + t.row[i].y : 0;
+        bool ok = true;
+        if (PERIODIC) {   // offsets are in [0, edge): one subtraction wraps, and underflows where it must not
+            qy = min(qy, qy - e);
+            if (DIM == 3) qz = min(qz, qz - e);
+        } else {
+            ok = qy < e && (DIM == 2 || qz < e);
+        }
+        if (!lin) {
+            qy = div32(qy, s.by_step);
+            if (DIM == 3) qz = div32(qz, s.by_step);
+        }
+        slots[i * 256] = ok ? (int)((qz * s.ky + qy) * s.kx) : kNoCell;
+    }
+#pragma unroll 3
+    for (int i = 0; i < t.nb; ++i) {
+        unsigned qx = x + t.col[i];
+        if (PERIODIC) qx = min(qx, qx - e);
+        slots[(t.na + i) * 256] = PERIODIC || qx < e ? (int)div32(qx, s.by_step) : kNoCell;
+    }
+    slots[(t.na + t.nb) * 256] = 0;
+}
+
+// Adds the records' terms to the field in file order, the loads of a batch before its terms.
+// SWEEP: s_j x Ds (the sweep's convention), else De x s_j (the energy's). Products of a zero J or D
+// change nothing; neighbours past an open edge read the zero cell.
+template <bool PERIODIC, bool SWEEP>
+__device__ __forceinline__ void class_field(const ClassTable& t, const ClassBase& base, const float4* __restrict__ plane,
+                                            int zero, const int* slots, float& hx, float& hy, float& hz) {
+    constexpr int B = kClassBatch;
+#pragma unroll
+    for (int r0 = 0; r0 < kClassRecs; r0 += B) {
+        if (r0 >= t.n) break;
+        float4 v[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const int2 at = t.at[r0 + u];
+            int i = base.b[r0 + u] + slots[at.x] + slots[at.y];
+            if (!PERIODIC) i = i < 0 ? zero : i;
+            v[u] = __ldg(plane + i);
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const float4 j = t.j[r0 + u];
+            const float sx = v[u].x, sy = v[u].y, sz = v[u].z;
+            hx = fmaf(j.x, sx, hx);
+            hy = fmaf(j.x, sy, hy);
+            hz = fmaf(j.x, sz, hz);
+            if (SWEEP) {
+                hx = fmaf(sy, j.w, fmaf(-sz, j.z, hx));
+                hy = fmaf(sz, j.y, fmaf(-sx, j.w, hy));
+                hz = fmaf(sx, j.z, fmaf(-sy, j.y, hz));
+            } else {
+                hx = fmaf(j.z, sz, fmaf(-j.w, sy, hx));
+                hy = fmaf(j.w, sx, fmaf(-j.y, sz, hy));
+                hz = fmaf(j.y, sy, fmaf(-j.z, sx, hz));
+            }
+        }
+    }
+}
+
+// One colour class of every listed chain, in its class planes.
+template <int DIM, bool PERIODIC>
+__global__ void __launch_bounds__(256, 4)
+k_class_sweep(const __grid_constant__ DevModel m, const ClassShape s, const __grid_constant__ ClassTable t,
+              const __grid_constant__ ClassBase base, float4* __restrict__ planes, const float4* __restrict__ bh,
+              const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour, unsigned off) {
+    extern __shared__ int cl_slots[];
+    const int chain = chains[blockIdx.y];
+    const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+    int x, y, z;
+    if (cell >= s.cells || !class_site<DIM>(m, s, colour, cell, x, y, z)) return;
+    int* const slots = cl_slots + threadIdx.x;
+    class_terms<DIM, PERIODIC>(m, s, t, x, y, z, slots);
+    float4* const plane = planes + (size_t)chain * s.chain;
+    float4* const own = plane + (size_t)colour * s.cells + cell;
+    const float4 p = bh[chain];
+    const uint32_t box = (uint32_t)(x + m.edge * (y + m.edge * z));
+    const nmmc_u4 r = sweep_draw<true>(m, box, sweep[chain] + off, (uint32_t)chain);
+    float hx = p.y, hy = p.z, hz = p.w;
+    class_field<PERIODIC, true>(t, base, plane, (int)s.chain - 1, slots, hx, hy, hz);
+    const float4 v = *own;
+    float tx, ty, tz;
+    if (heis_try(hx, hy, hz, v.x, v.y, v.z, p, r, tx, ty, tz)) *own = make_float4(tx, ty, tz, 0.0f);
+}
+
+// Between the box layout and the class planes of the listed chains.
+template <int DIM>
+__global__ void __launch_bounds__(256)
+k_class_copy(const DevModel m, const ClassShape s, float4* __restrict__ planes, float* __restrict__ spins,
+             const int* __restrict__ chains, int to_class) {
+    const int chain = chains[blockIdx.y];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m.col_q * s.cells) return;
+    const int cls = i / s.cells;
+    int x, y, z;
+    if (!class_site<DIM>(m, s, cls, i - cls * s.cells, x, y, z)) return;
+    const size_t P = (size_t)m.nhalf_pad;
+    float* b = spins + ((size_t)chain * 2 + ((x + y + z) & 1)) * 3 * P + plane_index(m, x, y, z);
+    float4* q = planes + (size_t)chain * s.chain + i;
+    if (to_class) {
+        *q = make_float4(b[0], b[P], b[2 * P], 0.0f);
+    } else {
+        const float4 v = *q;
+        b[0] = v.x;
+        b[P] = v.y;
+        b[2 * P] = v.z;
+    }
+}
+
+// The table's energy term over the class planes: block b of a chain takes an equal run of class
+// `cls`'s cells and adds its sum to slot 0 of the measurement's block b (as k_energy_general; FP32
+// terms, FP64 across warps). One launch per class: the launches of a stream follow one another.
+template <int DIM, bool PERIODIC>
+__global__ void __launch_bounds__(256, 4)
+k_class_energy(const __grid_constant__ DevModel m, const ClassShape s, const __grid_constant__ ClassTable t,
+               const __grid_constant__ ClassBase base, const float4* __restrict__ planes, const int* __restrict__ chains,
+               int cls, int nblk, float scale, double* __restrict__ partial) {
+    extern __shared__ int cl_slots[];
+    __shared__ float red[8];
+    const int chain = chains[blockIdx.y];
+    const float4* const plane = planes + (size_t)chain * s.chain;
+    int* const slots = cl_slots + threadIdx.x;
+    float acc = 0.0f;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.cells; i += gridDim.x * blockDim.x) {
+        int x, y, z;
+        if (!class_site<DIM>(m, s, cls, i, x, y, z)) continue;
+        class_terms<DIM, PERIODIC>(m, s, t, x, y, z, slots);
+        const float4 v = __ldg(plane + (size_t)cls * s.cells + i);
+        float fx = 0.0f, fy = 0.0f, fz = 0.0f;
+        class_field<PERIODIC, false>(t, base, plane, (int)s.chain - 1, slots, fx, fy, fz);
+        acc += fmaf(v.x, fx, fmaf(v.y, fy, v.z * fz));
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) red[warp] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double tot = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += (double)red[w];
+        partial[((size_t)blockIdx.y * nblk + blockIdx.x) * kNP] += scale * tot;
+    }
+}
+
+// The records a class kernel takes, in file order: all but those that land on the site itself. The
+// energy of a table of +-o pairs (J(o) = J(-o), D(o) = -D(-o)) counts every bond from both ends with
+// the same value, so the first record of each pair stands for both (class_energy_scale 2).
+static bool class_paired(const Ctx& c, size_t r, size_t q) {
+    const int4 a = c.h_goff[r], b = c.h_goff[q];
+    const int e = c.edge;
+    auto opposite = [&](int u, int v) { return c.periodic ? (u + v) % e == 0 : u + v == 0; };
+    const float4 ja = c.h_gje[r], jb = c.h_gje[q];
+    return opposite(a.x, b.x) && opposite(a.y, b.y) && opposite(a.z, b.z) && ja.x == jb.x && ja.y == -jb.y &&
+           ja.z == -jb.z && ja.w == -jb.w;
+}
+
+static bool class_halves(const Ctx& c, std::vector<size_t>& first) {
+    const size_t n = c.h_goff.size();
+    std::vector<char> used(n, 0);
+    first.clear();
+    for (size_t r = 0; r < n; ++r) {
+        if (used[r] || c.h_goff[r].w) continue;
+        size_t q = r + 1;
+        while (q < n && (used[q] || !class_paired(c, r, q))) ++q;
+        if (q == n) return false;
+        used[q] = 1;
+        first.push_back(r);
+    }
+    return true;
+}
+
+static std::vector<size_t> class_records(const Ctx& c, bool sweep) {
+    std::vector<size_t> recs;
+    if (!sweep && c.h_goff.size() <= 2 * kClassRecs && class_halves(c, recs)) return recs;
+    recs.clear();
+    for (size_t r = 0; r < c.h_goff.size(); ++r)
+        if (!c.h_goff[r].w) recs.push_back(r);
+    return recs;
+}
+
+static float class_energy_scale(const Ctx& c) {
+    std::vector<size_t> recs;
+    return c.h_goff.size() <= 2 * kClassRecs && class_halves(c, recs) ? 2.0f : 1.0f;
+}
+
+// The class form of the context's records (js: in the wanted DMI convention); false where it has
+// more records, rows or columns than the kernels take.
+static bool class_table(const Ctx& c, bool sweep, ClassTable& t) {
+    t.n = 0;
+    t.na = t.nb = 0;
+    for (size_t r : class_records(c, sweep)) {
+        const int4 o = c.h_goff[r];
+        if (t.n == kClassRecs) return false;
+        int a = 0, b = 0;
+        while (a < t.na && (t.row[a].x != o.y || t.row[a].y != o.z)) ++a;
+        if (a == t.na) {
+            if (t.na == kClassRows) return false;
+            t.row[t.na++] = make_int2(o.y, o.z);
+        }
+        while (b < t.nb && t.col[b] != o.x) ++b;
+        if (b == t.nb) {
+            if (t.nb == kClassCols) return false;
+            t.col[t.nb++] = o.x;
+        }
+        const float4 e = c.h_gje[r];
+        t.j[t.n] = sweep && c.dmi_sign ? make_float4(e.x, -e.y, -e.z, -e.w) : e;
+        t.at[t.n++] = make_int2(a, b);
+    }
+    for (int r = 0; r < t.n; ++r) t.at[r] = make_int2(t.at[r].x * 256, (t.na + t.at[r].y) * 256);
+    while (t.n % kClassBatch) {   // padding: the zero cell, by the zero slot
+        t.at[t.n] = make_int2((t.na + t.nb) * 256, (t.na + t.nb) * 256);
+        t.j[t.n++] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    return true;
+}
+
+static ClassBase class_base(const Ctx& c, const ClassShape& s, bool sweep, int cls) {
+    ClassBase base{};
+    const int q = c.m.col_q, p = c.m.col_p;
+    int n = 0;
+    for (size_t r : class_records(c, sweep)) {
+        const int4 o = c.h_goff[r];
+        int k;
+        if (c.m.col_kind == 1) {
+            k = (int)(((cls + o.x + (long)c.m.col_b * o.y + (long)c.m.col_c * o.z) % q + q) % q);
+        } else {
+            auto mod = [&](int v) { return (v % p + p) % p; };
+            k = mod(cls % p + o.x) + p * mod((cls / p) % p + o.y) + (c.dim == 3 ? p * p * mod(cls / (p * p) + o.z) : 0);
+        }
+        base.b[n++] = k * s.cells;
+    }
+    while (n < kClassRecs) base.b[n++] = (int)s.chain - 1;
+    return base;
+}
+
+static bool use_class(const Ctx& c) {
+    if (!c.m.general || c.masked || c.ising || c.class_no_memory || c.half_kernel == 1) return false;
+    const ClassShape s = class_shape(c);
+    ClassTable t;
+    // indices below the no-cell marker; the division by multiplication
+    return (long long)s.cells * c.m.col_q < (1LL << 29) && (long long)s.cells * s.kx < (1LL << 32) &&
+           (long long)(s.ky * s.kz) * s.ky < (1LL << 32) && (long long)(c.m.col_q + 1) * 2 * c.edge * s.step < (1LL << 32) &&
+           class_table(c, true, t);
+}
+
+// The class planes, allocated at the first sweep; without the memory the sweeps stay in the box.
+bool class_ready(Ctx& c) {
+    if (!use_class(c)) return false;
+    if (c.d_class) return true;
+    const ClassShape s = class_shape(c);
+    if (cudaMalloc(&c.d_class, (size_t)c.nchains * s.chain * sizeof(float4)) != cudaSuccess ||
+        cudaMemsetAsync(c.d_class, 0, (size_t)c.nchains * s.chain * sizeof(float4), c.stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(c.d_class);
+        c.d_class = nullptr;
+        c.class_no_memory = true;
+        return false;
+    }
+    return true;
+}
+
+static int class_copy(Ctx& c, const int* d_chains, int n, bool to_class) {
+    const ClassShape s = class_shape(c);
+    const dim3 grid((c.m.col_q * s.cells + 255) / 256, n);
+    if (c.dim == 3) k_class_copy<3><<<grid, 256, 0, c.stream>>>(c.m, s, c.d_class, (float*)c.d_spins, d_chains, to_class);
+    else k_class_copy<2><<<grid, 256, 0, c.stream>>>(c.m, s, c.d_class, (float*)c.d_spins, d_chains, to_class);
+    return cuda_check(cudaGetLastError(), "k_class_copy");
+}
+
+static int class_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps) {
+    const ClassShape s = class_shape(c);
+    if (int rc = class_copy(c, d_chains, n, true)) return rc;
+    const dim3 grid((s.cells + 255) / 256, n);
+    auto kern = c.dim == 3 ? (c.periodic ? k_class_sweep<3, true> : k_class_sweep<3, false>)
+                           : (c.periodic ? k_class_sweep<2, true> : k_class_sweep<2, false>);
+    ClassTable t;
+    class_table(c, true, t);
+    std::vector<ClassBase> base;
+    for (int colour = 0; colour < c.m.col_q; ++colour) base.push_back(class_base(c, s, true, colour));
+    const size_t smem = (size_t)(t.na + t.nb + 1) * 256 * sizeof(int);   // at most 25 KB
+    for (int k = 0; k < nsweeps; ++k)
+        for (int colour = 0; colour < c.m.col_q; ++colour)
+            kern<<<grid, 256, smem, c.stream>>>(c.m, s, t, base[colour], c.d_class, c.d_bh, c.d_sweep, d_chains, colour,
+                                                (unsigned)k);
+    if (int rc = cuda_check(cudaGetLastError(), "k_class_sweep")) return rc;
+    if (int rc = class_copy(c, d_chains, n, false)) return rc;
+    return launch_advance(c, d_chains, n, nsweeps);
+}
+
 // Threads per chain for one colour class (the largest class).
 static int colour_threads(const Ctx& c) {
     const DevModel& m = c.m;
@@ -179,6 +559,7 @@ static ColourFn pick_colour_pm(const Ctx& c) {
 }
 
 int launch_colour_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps) {
+    if (class_ready(c)) return class_sweeps(c, d_chains, n, nsweeps);
     ColourFn f = (c.dim == 3) ? (c.periodic ? pick_colour_pm<3, true>(c) : pick_colour_pm<3, false>(c))
                               : (c.periodic ? pick_colour_pm<2, true>(c) : pick_colour_pm<2, false>(c));
     for (int s = 0; s < nsweeps; ++s)
@@ -308,6 +689,22 @@ static void energy_pm(Ctx& c, const int* d, int n, int rows, int nbs, int nbt, d
 
 int launch_energy_general(Ctx& c, const int* d_chains, int n, int rows, int nblk_slice, int nblk_total,
                           double* partial) {
+    if (!c.measure_fp64 && use_class(c) && c.d_class) {
+        // a sample step's sweeps have left the listed chains' class planes current
+        if (!c.class_fresh)
+            if (int rc = class_copy(c, d_chains, n, true)) return rc;
+        auto kern = c.dim == 3 ? (c.periodic ? k_class_energy<3, true> : k_class_energy<3, false>)
+                               : (c.periodic ? k_class_energy<2, true> : k_class_energy<2, false>);
+        const ClassShape s = class_shape(c);
+        ClassTable t;
+        class_table(c, false, t);
+        const size_t smem = (size_t)(t.na + t.nb + 1) * 256 * sizeof(int);
+        const int blocks = std::min(nblk_total, (s.cells + 255) / 256);
+        for (int cls = 0; cls < c.m.col_q; ++cls)
+            kern<<<dim3(blocks, n), 256, smem, c.stream>>>(c.m, s, t, class_base(c, s, false, cls), c.d_class, d_chains, cls,
+                                                          nblk_total, class_energy_scale(c), partial);
+        return cuda_check(cudaGetLastError(), "k_class_energy");
+    }
     if (c.dim == 3) {
         if (c.periodic) energy_pm<3, true>(c, d_chains, n, rows, nblk_slice, nblk_total, partial);
         else energy_pm<3, false>(c, d_chains, n, rows, nblk_slice, nblk_total, partial);

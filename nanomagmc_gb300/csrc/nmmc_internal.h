@@ -107,6 +107,7 @@ struct Ctx {
     ReplayModel* d_rm = nullptr;        // device copy for the replay kernel
     Colouring col;                      // colour classes of the sweep (kind 0: checkerboard)
     std::vector<float4> h_gje;          // general records, energy convention (host copy)
+    std::vector<int4> h_goff;           // their offsets, as on the device
     int4* d_goff = nullptr;             // general records on the device (DevModel g_*)
     float4* d_gjs = nullptr;
     float4* d_gje = nullptr;
@@ -161,6 +162,10 @@ struct Ctx {
     int4* d_ctab = nullptr;
     bool ctab_built = false;
     bool ctab_packed = true;
+    // general tables, unmasked Heisenberg: the class planes (nmmc_general.cu)
+    float4* d_class = nullptr;
+    bool class_no_memory = false;
+    bool class_fresh = false;           // within one sample step: the planes hold what its sweeps left
     float4* d_bh = nullptr;             // per chain (beta, H0, H1, H2) in FP32
     uint32_t* d_itab = nullptr;         // Ising word kernels: per chain 128 acceptance limits (nmmc_ising.cu)
     double* d_Hd = nullptr;             // per chain H in FP64 (3 doubles) for the energy
@@ -250,6 +255,7 @@ int launch_colour_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps);
 int launch_energy_general(Ctx& c, const int* d_chains, int n, int rows, int nblk_slice, int nblk_total,
                           double* partial);
 int launch_delta_e_general(Ctx& c, int chain, const int32_t* d_sites, const float* d_trial, int n, double* d_out);
+bool class_ready(Ctx& c);     // class planes in use (allocated at the first call)
 int upload_general(Ctx& c);   // (re)writes the device records from h_gje and the DMI sign
 
 // ---- kernels (nmmc_kernels.cu) ----

@@ -2151,7 +2151,7 @@ static int measure_with(Ctx& c, const int* d_chains, int n, double* partial, dou
     if (measure_by_compact(c)) {
         int rc = measure_compact_launch(c, d_chains, n, nblk, nblk_slice, partial);
         if (rc) return rc;
-    } else if (!c.ising && !c.masked && !fp64 && (c.m.hx % 4) == 0 && c.half_kernel != 1 && !c.m.general) {
+    } else if (!c.ising && !c.masked && !fp64 && (c.m.hx % 4) == 0 && c.half_kernel != 1) {   // (general: J = 0 here)
         dim3 grid(nblk, n);
         const float* sp = (const float*)c.d_spins;
         measure_q4_launch(c, grid, sp, d_chains, rows, nblk_slice, partial);
