@@ -92,16 +92,16 @@ static int set_list(Ctx& c, const int* chains, int n, const int** d_out) {
     return NMMC_OK;
 }
 
-static bool use_resident(Ctx& c, int* rc) {
+static bool use_resident(Ctx& c, const int* d_chains, int n, int* rc) {
     *rc = NMMC_OK;
     if (c.sweep_path == 1) return false;
-    *rc = resident_prepare(c);
+    *rc = resident_prepare(c, d_chains, n);
     if (*rc) return false;
     if (c.sweep_path == 2 && !c.res.eligible) {
         *rc = set_error(NMMC_ERR_UNSUPPORTED, "lattice does not fit the shared-memory resident path");
         return false;
     }
-    return resident_chosen(c);
+    return resident_chosen(c, n);
 }
 
 long long count_sites(const Ctx& c, const int* h_chains, int n) {
@@ -168,7 +168,7 @@ int sweep_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, int nswe
     if (nsweeps <= 0 || n == 0) return NMMC_OK;
     int rc = upload_params(c);
     if (rc) return rc;
-    bool res = use_resident(c, &rc);
+    bool res = use_resident(c, d_chains, n, &rc);
     if (rc) return rc;
     return run_sweeps(c, d_chains, h_chains, n, nsweeps, res, false, 0, allow_timing);
 }
@@ -182,9 +182,9 @@ int sweep_measure_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, 
     int rc = upload_params(c);
     if (rc) return rc;
     if (nsweeps > 0) {
-        bool res = use_resident(c, &rc);
+        bool res = use_resident(c, d_chains, n, &rc);
         if (rc) return rc;
-        if (res && resident_can_measure(c)) {
+        if (res && resident_can_measure(c, n)) {
             if ((rc = run_sweeps(c, d_chains, h_chains, n, nsweeps, true, true, accumulate, allow_timing))) return rc;
             return accumulate ? launch_add_av(c) : NMMC_OK;
         }
@@ -766,15 +766,6 @@ int nmmc_sample(nmmc_ctx* c, const int* chains, int n, int nsweeps, int nsamples
     if (nsamples == 0 || n == 0) return NMMC_OK;
     int rc = upload_params(*c);
     if (rc) return rc;
-    if (c->sweep_path != 1) {
-        if ((rc = resident_prepare(*c))) return rc;
-    }
-    // the HBM path's compact tables: no allocation or table upload inside the capture
-    if (!(c->sweep_path != 1 && resident_chosen(*c))) {
-        if ((rc = compact_prepare(*c))) return rc;
-        class_ready(*c);  // the class planes of a general table
-        wave_ready(*c);   // the wavefront sweeps' second array (when enabled), not inside the capture
-    }
     if ((rc = measure_prepare(*c, n))) return rc;
     // history buffers on the device, one D2H at the end
     DeviceScratch ds;
@@ -784,12 +775,22 @@ int nmmc_sample(nmmc_ctx* c, const int* chains, int n, int nsweeps, int nsamples
     if (q) NMMC_CUDA(ds.alloc(&d_qhist, sizeof(double) * c->nslices * n * (size_t)nsamples));
     NMMC_CUDA(ds.alloc(&d_l, sizeof(int) * n));
     NMMC_CUDA(cudaMemcpy(d_l, list.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+    const bool all = all_if_identity(*c, list.data(), n) == nullptr;   // every chain, in order
+    const int* list_dev = all ? c->d_all : d_l;
+    if (c->sweep_path != 1) {
+        if ((rc = resident_prepare(*c, list_dev, n))) return rc;
+    }
+    // the HBM path's compact tables: no allocation or table upload inside the capture
+    if (!(c->sweep_path != 1 && resident_chosen(*c, n))) {
+        if ((rc = compact_prepare(*c))) return rc;
+        class_ready(*c);  // the class planes of a general table
+        wave_ready(*c);   // the wavefront sweeps' second array (when enabled), not inside the capture
+    }
     // one graph: nsweeps sweeps + measure (accumulating), as nmmc_sweep_measure
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     NMMC_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    const bool all = all_if_identity(*c, list.data(), n) == nullptr;   // every chain, in order
-    rc = sweep_measure_impl(*c, all ? c->d_all : d_l, all ? nullptr : list.data(), n, nsweeps, 1, false);
+    rc = sweep_measure_impl(*c, list_dev, all ? nullptr : list.data(), n, nsweeps, 1, false);
     cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
     if (rc || ce != cudaSuccess) {
         if (g) cudaGraphDestroy(g);

@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(256)
 k_colour_sweep(const DevModel m, void* __restrict__ spins_v, const uint8_t* __restrict__ mask,
                const float4* __restrict__ bh, const unsigned long long* __restrict__ sweep,
                const int* __restrict__ chains, int colour, unsigned off) {
+    seq_begin();
     const int chain = chains[blockIdx.y];
     int x, y, z;
     if (!colour_site<DIM>(m, colour, blockIdx.x * blockDim.x + threadIdx.x, x, y, z)) return;
@@ -284,7 +285,7 @@ __device__ __forceinline__ void class_field(const ClassTable& t, const ClassBase
             const int2 at = t.at[r0 + u];
             int i = base.b[r0 + u] + slots[at.x] + slots[at.y];
             if (!PERIODIC) i = i < 0 ? zero : i;
-            v[u] = __ldg(plane + i);
+            v[u] = plane[i];
         }
 #pragma unroll
         for (int u = 0; u < B; ++u) {
@@ -313,12 +314,14 @@ k_class_sweep(const __grid_constant__ DevModel m, const ClassShape s, const __gr
               const __grid_constant__ ClassBase base, float4* __restrict__ planes, const float4* __restrict__ bh,
               const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour, unsigned off) {
     extern __shared__ int cl_slots[];
-    const int chain = chains[blockIdx.y];
     const int cell = blockIdx.x * blockDim.x + threadIdx.x;
     int x, y, z;
-    if (cell >= s.cells || !class_site<DIM>(m, s, colour, cell, x, y, z)) return;
+    const bool mine = cell < s.cells && class_site<DIM>(m, s, colour, cell, x, y, z);
     int* const slots = cl_slots + threadIdx.x;
-    class_terms<DIM, PERIODIC>(m, s, t, x, y, z, slots);
+    if (mine) class_terms<DIM, PERIODIC>(m, s, t, x, y, z, slots);   // before the wait: parameters only
+    seq_begin();
+    if (!mine) return;
+    const int chain = chains[blockIdx.y];
     float4* const plane = planes + (size_t)chain * s.chain;
     float4* const own = plane + (size_t)colour * s.cells + cell;
     const float4 p = bh[chain];
@@ -336,6 +339,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 k_class_copy(const DevModel m, const ClassShape s, float4* __restrict__ planes, float* __restrict__ spins,
              const int* __restrict__ chains, int to_class) {
+    seq_begin();
     const int chain = chains[blockIdx.y];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.col_q * s.cells) return;
@@ -363,6 +367,7 @@ __global__ void __launch_bounds__(256, 4)
 k_class_energy(const __grid_constant__ DevModel m, const ClassShape s, const __grid_constant__ ClassTable t,
                const __grid_constant__ ClassBase base, const float4* __restrict__ planes, const int* __restrict__ chains,
                int cls, int nblk, float scale, double* __restrict__ partial) {
+    seq_begin();
     extern __shared__ int cl_slots[];
     __shared__ float red[8];
     const int chain = chains[blockIdx.y];
@@ -373,7 +378,7 @@ k_class_energy(const __grid_constant__ DevModel m, const ClassShape s, const __g
         int x, y, z;
         if (!class_site<DIM>(m, s, cls, i, x, y, z)) continue;
         class_terms<DIM, PERIODIC>(m, s, t, x, y, z, slots);
-        const float4 v = __ldg(plane + (size_t)cls * s.cells + i);
+        const float4 v = plane[(size_t)cls * s.cells + i];
         float fx = 0.0f, fy = 0.0f, fz = 0.0f;
         class_field<PERIODIC, false>(t, base, plane, (int)s.chain - 1, slots, fx, fy, fz);
         acc += fmaf(v.x, fx, fmaf(v.y, fy, v.z * fz));
@@ -510,8 +515,8 @@ bool class_ready(Ctx& c) {
 static int class_copy(Ctx& c, const int* d_chains, int n, bool to_class) {
     const ClassShape s = class_shape(c);
     const dim3 grid((c.m.col_q * s.cells + 255) / 256, n);
-    if (c.dim == 3) k_class_copy<3><<<grid, 256, 0, c.stream>>>(c.m, s, c.d_class, (float*)c.d_spins, d_chains, to_class);
-    else k_class_copy<2><<<grid, 256, 0, c.stream>>>(c.m, s, c.d_class, (float*)c.d_spins, d_chains, to_class);
+    if (c.dim == 3) launch_seq(c, k_class_copy<3>, grid, 256, 0, c.m, s, c.d_class, (float*)c.d_spins, d_chains, to_class);
+    else launch_seq(c, k_class_copy<2>, grid, 256, 0, c.m, s, c.d_class, (float*)c.d_spins, d_chains, to_class);
     return cuda_check(cudaGetLastError(), "k_class_copy");
 }
 
@@ -528,7 +533,7 @@ static int class_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps) {
     const size_t smem = (size_t)(t.na + t.nb + 1) * 256 * sizeof(int);   // at most 25 KB
     for (int k = 0; k < nsweeps; ++k)
         for (int colour = 0; colour < c.m.col_q; ++colour)
-            kern<<<grid, 256, smem, c.stream>>>(c.m, s, t, base[colour], c.d_class, c.d_bh, c.d_sweep, d_chains, colour,
+            launch_seq(c, kern, grid, 256, smem, c.m, s, t, base[colour], c.d_class, c.d_bh, c.d_sweep, d_chains, colour,
                                                 (unsigned)k);
     if (int rc = cuda_check(cudaGetLastError(), "k_class_sweep")) return rc;
     if (int rc = class_copy(c, d_chains, n, false)) return rc;
@@ -546,7 +551,7 @@ static int colour_threads(const Ctx& c) {
 template <int DIM, bool PERIODIC, bool MASKED, bool ISING>
 static void colour_launch(Ctx& c, const int* d_chains, int n, int colour, unsigned off) {
     dim3 grid((colour_threads(c) + 255) / 256, n);
-    k_colour_sweep<DIM, PERIODIC, MASKED, ISING><<<grid, 256, 0, c.stream>>>(
+    launch_seq(c, k_colour_sweep<DIM, PERIODIC, MASKED, ISING>, grid, 256, 0,
         c.m, c.d_spins, c.d_mask, c.d_bh, c.d_sweep, d_chains, colour, off);
 }
 
@@ -701,7 +706,7 @@ int launch_energy_general(Ctx& c, const int* d_chains, int n, int rows, int nblk
         const size_t smem = (size_t)(t.na + t.nb + 1) * 256 * sizeof(int);
         const int blocks = std::min(nblk_total, (s.cells + 255) / 256);
         for (int cls = 0; cls < c.m.col_q; ++cls)
-            kern<<<dim3(blocks, n), 256, smem, c.stream>>>(c.m, s, t, class_base(c, s, false, cls), c.d_class, d_chains, cls,
+            launch_seq(c, kern, dim3(blocks, n), 256, smem, c.m, s, t, class_base(c, s, false, cls), c.d_class, d_chains, cls,
                                                           nblk_total, class_energy_scale(c), partial);
         return cuda_check(cudaGetLastError(), "k_class_energy");
     }

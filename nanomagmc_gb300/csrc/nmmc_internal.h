@@ -81,7 +81,9 @@ struct ResidentTables {
     // sweeps of every site, so that the resident kernel's updates skip the generator.
     bool hbm_faster = false;      // the autotuner timed the HBM path faster: the automatic path takes it
     bool stencil = false;         // sweeps run on the stencil resident kernel (nmmc_stencil.cu)
-    bool large_tuned = false;     // a lattice too large for the record kernel: path chosen (stencil or HBM)
+    // lattices too large for the record kernel: by the number of chains of a call, whether the
+    // stencil kernel takes it (else the HBM path)
+    std::map<int, bool> large_stencil;
     bool predraw = false;         // the shape in use launches the drawn-ahead variant
     int* d_site_chain = nullptr;  // per site: its chain
     uint4* d_draws = nullptr;     // [sweep of the launch][site] Philox words
@@ -244,6 +246,25 @@ struct DeviceScratch {
         for (void* q : ptrs) cudaFree(q);
     }
 };
+// Launch on the context's stream that may begin while the previous kernel of the stream drains
+// (programmatic stream serialisation). Only for kernels that start with seq_begin()
+// (nmmc_kernels.cuh), which waits for that kernel's completion before the first read or write.
+// Half-sweeps follow one another 20 to 160 times per call; a plain launch leaves 2-3 us between
+// them (24 Ising chains of 64^3: 13.9 us kernels, 18 us apart).
+template <class... P, class... A>
+void launch_seq(Ctx& c, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // errors: the caller's cudaGetLastError
+}
 #define NMMC_CUDA(call)                                         \
     do {                                                        \
         cudaError_t _e = (call);                                \
@@ -265,9 +286,9 @@ int launch_global_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool f
 bool hbm_fused_measure_ok(const Ctx& c);
 int launch_measure_fused_tail(Ctx& c, const int* d_chains, int n, int accumulate);
 int launch_measure(Ctx& c, const int* d_chains, int n, int accumulate);
-// nsweeps HBM-path sweeps of every chain and, with `measure`, the observables as
+// nsweeps HBM-path sweeps of the listed chains and, with `measure`, the observables as
 // nmmc_sweep_measure takes them on that path (the autotuner's HBM candidate)
-int hbm_tuning_step(Ctx& c, int nsweeps, bool measure);
+int hbm_tuning_step(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure);
 int measure_prepare(Ctx& c, int n);
 size_t measure_partials_per_chain(const Ctx& c);   // partial-sum doubles one chain's measurement uses
 int launch_measure_into(Ctx& c, const int* d_chains, int n, double* scratch, size_t scratch_doubles,
@@ -300,15 +321,15 @@ StencilShape stencil_shape(const Ctx& c, int n);   // of a call on n chains; C =
 int launch_stencil_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure, int accumulate);
 
 // ---- resident kernel (nmmc_resident.cu) ----
-int resident_prepare(Ctx& c);
+int resident_prepare(Ctx& c, const int* d_chains, int n);   // for a call on these n chains
 // all: the list is every chain in order. measure: after the sweeps, compute the listed
 // chains' observables in the same launch (2-D lattices; see resident_can_measure).
 int launch_resident_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool all, bool measure,
                            int accumulate);
-bool resident_can_measure(const Ctx& c);
+bool resident_can_measure(const Ctx& c, int n);
 // The sweeps of this context run on the resident path (after resident_prepare): the option,
 // eligibility, and on the automatic path the autotuner's choice between the two paths.
-bool resident_chosen(const Ctx& c);
+bool resident_chosen(const Ctx& c, int n);
 void resident_free(Ctx& c);
 // Compact form of masked Heisenberg lattices on the HBM path: allocates and builds the tables
 // of every chain when the sweeps will use it (a no-op otherwise or when built); and rebuilds

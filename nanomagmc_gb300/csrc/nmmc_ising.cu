@@ -29,13 +29,13 @@ template <int W>
 __device__ __forceinline__ Words<W> ld_words(const int8_t* p) {
     Words<W> r;
     if (W == 4) {
-        const uint4 t = __ldg(reinterpret_cast<const uint4*>(p));
+        const uint4 t = *reinterpret_cast<const uint4*>(p);
         r.w[0] = t.x;
         r.w[W > 1 ? 1 : 0] = t.y;
         r.w[W > 2 ? 2 : 0] = t.z;
         r.w[W > 3 ? 3 : 0] = t.w;
     } else {
-        r.w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+        r.w[0] = *reinterpret_cast<const uint32_t*>(p);
     }
     return r;
 }
@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(256)
 k_ising_words(const DevModel m, int8_t* __restrict__ spins, const float4* __restrict__ bh,
               const unsigned long long* __restrict__ sweep, const int* __restrict__ chains,
               const uint32_t* __restrict__ tab, int colour, unsigned sweep_off) {
+    seq_begin();
     constexpr int ND = 2 * DIM;
     __shared__ uint32_t st[2 << ND];
     const int chain = chains[blockIdx.y];
@@ -120,7 +121,7 @@ k_ising_words(const DevModel m, int8_t* __restrict__ spins, const float4* __rest
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
                 const int j = nb_compact<false>(m, 2 * (h0 + k) + xp, y, z, d);
-                n[d] = j >= 0 ? (float)__ldg(oth + j) : 0.0f;
+                n[d] = j >= 0 ? (float)oth[j] : 0.0f;
             }
             const nmmc_u4 r = sweep_draw<true>(m, box + 2 * k, sw, (uint32_t)chain);
             float t;
@@ -135,7 +136,7 @@ k_ising_words(const DevModel m, int8_t* __restrict__ spins, const float4* __rest
         zp = ld_words<W>(oth + (zu * m.ly + y) * m.hx + h0);
         zm = ld_words<W>(oth + (zd * m.ly + y) * m.hx + h0);
     }
-    const uint32_t ex = (uint8_t)__ldg(oth + hrow + ho);
+    const uint32_t ex = (uint8_t)oth[hrow + ho];
     Words<W> out = s;
     uint32_t changed = 0;
 #pragma unroll
@@ -273,7 +274,7 @@ int launch_ising_table(Ctx& c) {
 template <int DIM, bool PERIODIC, int W>
 static void ising_words_launch_w(Ctx& c, const int* d_chains, int n, int colour, unsigned off) {
     const int items = c.m.hx / (4 * W) * c.m.ly * c.m.lz;
-    k_ising_words<DIM, PERIODIC, W><<<dim3((items + 255) / 256, n), 256, 0, c.stream>>>(
+    launch_seq(c, k_ising_words<DIM, PERIODIC, W>, dim3((items + 255) / 256, n), 256, 0,
         c.m, (int8_t*)c.d_spins, c.d_bh, c.d_sweep, d_chains, c.d_itab, colour, off);
 }
 

@@ -22,6 +22,7 @@ k_heis_half(const DevModel m, float* __restrict__ spins, const uint32_t* __restr
             const int* __restrict__ fill_n, const float4* __restrict__ bh,
             const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour,
             unsigned sweep_off) {
+    seq_begin();
     const int chain = chains[blockIdx.y];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (MASKED) {   // thread j: the chain's j-th filled site of this colour
@@ -43,9 +44,9 @@ k_heis_half(const DevModel m, float* __restrict__ spins, const uint32_t* __restr
     for (int k = 0; k < ND; ++k) {
         int j = nb_compact<PERIODIC>(m, x, y, z, k);
         if (PERIODIC || j >= 0) {
-            nx[k] = __ldg(oth + j);
-            ny[k] = __ldg(oth + P + j);
-            nz[k] = __ldg(oth + 2 * P + j);
+            nx[k] = oth[j];
+            ny[k] = oth[P + j];
+            nz[k] = oth[2 * P + j];
         } else {
             nx[k] = ny[k] = nz[k] = 0.0f;
         }
@@ -68,6 +69,7 @@ k_ising_half(const DevModel m, int8_t* __restrict__ spins, const uint32_t* __res
              const int* __restrict__ fill_n, const float4* __restrict__ bh,
              const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour,
              unsigned sweep_off) {
+    seq_begin();
     const int chain = chains[blockIdx.y];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (MASKED) {   // thread j: the chain's j-th filled site of this colour
@@ -88,7 +90,7 @@ k_ising_half(const DevModel m, int8_t* __restrict__ spins, const uint32_t* __res
 #pragma unroll
     for (int k = 0; k < ND; ++k) {
         int j = nb_compact<PERIODIC>(m, x, y, z, k);
-        n[k] = (PERIODIC || j >= 0) ? (float)__ldg(oth + j) : 0.0f;
+        n[k] = (PERIODIC || j >= 0) ? (float)oth[j] : 0.0f;
     }
     const float4 p = bh[chain];
     const uint32_t box = (uint32_t)(x + m.edge * (y + m.edge * z));
@@ -133,6 +135,7 @@ k_heis_compact(const DevModel m, float4* __restrict__ cs, const int4* __restrict
                const int* __restrict__ fill_n, const float4* __restrict__ bh,
                const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour,
                unsigned sweep_off) {
+    seq_begin();
     const int chain = chains[blockIdx.y];
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int seg = chain * 2 + colour;
@@ -148,7 +151,7 @@ k_heis_compact(const DevModel m, float4* __restrict__ cs, const int4* __restrict
 #pragma unroll
     for (int k = 0; k < ND; ++k) {   // one 16-byte load per neighbour (x, y, z, 0)
         const int q = nbi[k];
-        const float4 v = q >= 0 ? __ldg(oth + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 v = q >= 0 ? oth[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         nx[k] = v.x;
         ny[k] = v.y;
         nz[k] = v.z;
@@ -167,6 +170,7 @@ __global__ void __launch_bounds__(256)
 k_compact_copy(float4* __restrict__ cs, float* __restrict__ spins, const uint32_t* __restrict__ fill,
                const int* __restrict__ fill_n, const int* __restrict__ chains, int nhalf, size_t P,
                int to_compact) {
+    seq_begin();
     const int chain = chains[blockIdx.y >> 1];
     const int seg = chain * 2 + (int)(blockIdx.y & 1);
     const int n = fill_n[seg];
@@ -253,7 +257,7 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
     float ex[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        s[c] = ld_quad_rw(own[c], rb);
+        s[c] = ld_quad(own[c], rb);
         same[c] = ld_quad(oth[c], rb);
     }
     // x-neighbour outside the quad: h0-1 (xp = 0) or h0+4 (xp = 1); 0 past an open edge (the
@@ -263,7 +267,7 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
     if (PERIODIC) hx_out = (hx_out < 0) ? m.hx - 1 : (hx_out >= m.hx ? 0 : hx_out);
     else ex_ok = hx_out >= 0 && hx_out < m.hx;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) ex[c] = ex_ok ? __ldg(oth[c] + (uint32_t)(row * m.hx + hx_out)) : 0.0f;
+    for (int c = 0; c < 3; ++c) ex[c] = ex_ok ? oth[c][(uint32_t)(row * m.hx + hx_out)] : 0.0f;
     // +-y rows
     {
         int yu = y + 1, yd = y - 1;
@@ -401,6 +405,7 @@ k_heis_half_q4(const DevModel m, float* __restrict__ spins, const float4* __rest
                const unsigned long long* __restrict__ sweep, const int* __restrict__ chains,
                int colour, unsigned sweep_off, int qpt, double* __restrict__ mpart, float esign, int pf,
                int nchain_list) {
+    seq_begin();
     const int chain = chains[blockIdx.y];
     const int qpr = m.hx / 4;
     const int nquads = qpr * m.ly * m.lz;
@@ -896,6 +901,7 @@ k_heis_half_ws(const DevModel m, float* __restrict__ spins, const float4* __rest
 }
 
 __global__ void k_advance(unsigned long long* sweep, const int* chains, int n, int nsweeps) {
+    seq_begin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) sweep[chains[i]] += (unsigned long long)nsweeps;
 }
@@ -904,7 +910,7 @@ template <int DIM, bool PERIODIC, bool MASKED, int DK>
 static void heis_launch(Ctx& c, const int* d_chains, int n, int colour, unsigned off) {
     dim3 grid(((MASKED ? c.fill_max : c.m.nhalf) + 255) / 256, n);
     if (grid.x == 0) return;   // no filled site in any chain
-    k_heis_half<DIM, PERIODIC, MASKED, DK><<<grid, 256, 0, c.stream>>>(
+    launch_seq(c, k_heis_half<DIM, PERIODIC, MASKED, DK>, grid, 256, 0,
         c.m, (float*)c.d_spins, c.d_fill, c.d_fill_n, c.d_bh, c.d_sweep, d_chains, colour, off);
 }
 
@@ -924,10 +930,10 @@ static void heis_q4_launch(Ctx& c, const int* d_chains, int n, int colour, unsig
     // L2 prefetch distance in blocks: the option's waves of resident blocks ahead (0: off)
     const int pf = c.l2_prefetch > 0 ? c.l2_prefetch * c.sm_count * per_sm / 4 : 0;
     if (c.half_kernel == 2)   // register cap for 2 CTAs/SM (no spills)
-        k_heis_half_q4<DIM, PERIODIC, DK, 2><<<grid, 256, 0, c.stream>>>(
+        launch_seq(c, k_heis_half_q4<DIM, PERIODIC, DK, 2>, grid, 256, 0,
             c.m, sp, c.d_bh, c.d_sweep, d_chains, colour, off, 1, nullptr, 0.0f, pf, n);
     else                      // 3 CTAs/SM (80 registers, more warps in flight)
-        k_heis_half_q4<DIM, PERIODIC, DK, 3><<<grid, 256, 0, c.stream>>>(
+        launch_seq(c, k_heis_half_q4<DIM, PERIODIC, DK, 3>, grid, 256, 0,
             c.m, sp, c.d_bh, c.d_sweep, d_chains, colour, off, 1, nullptr, 0.0f, pf, n);
 }
 
@@ -939,7 +945,7 @@ static void heis_q4_meas_launch(Ctx& c, const int* d_chains, int n, int colour, 
     const int nb = q4_meas_blocks(c);
     dim3 grid(nb, n);
     const float esign = c.dmi_sign ? 0.0f : -2.0f;
-    k_heis_half_q4<DIM, PERIODIC, DK, 2, 1><<<grid, 256, 0, c.stream>>>(
+    launch_seq(c, k_heis_half_q4<DIM, PERIODIC, DK, 2, 1>, grid, 256, 0,
         c.m, sp, c.d_bh, c.d_sweep, d_chains, colour, off, kMeasQpt, c.d_mrows, esign, 0, n);
 }
 
@@ -1026,7 +1032,7 @@ template <int DIM, bool PERIODIC, bool MASKED>
 static void ising_launch(Ctx& c, const int* d_chains, int n, int colour, unsigned off) {
     dim3 grid(((MASKED ? c.fill_max : c.m.nhalf) + 255) / 256, n);
     if (grid.x == 0) return;   // no filled site in any chain
-    k_ising_half<DIM, PERIODIC, MASKED><<<grid, 256, 0, c.stream>>>(
+    launch_seq(c, k_ising_half<DIM, PERIODIC, MASKED>, grid, 256, 0,
         c.m, (int8_t*)c.d_spins, c.d_fill, c.d_fill_n, c.d_bh, c.d_sweep, d_chains, colour, off);
 }
 
@@ -1076,7 +1082,7 @@ static HalfFn pick_half(const Ctx& c) {
 }
 
 int launch_advance(Ctx& c, const int* d_chains, int n, int nsweeps) {
-    k_advance<<<(n + 127) / 128, 128, 0, c.stream>>>(c.d_sweep, d_chains, n, nsweeps);
+    launch_seq(c, k_advance, dim3((n + 127) / 128), 128, 0, c.d_sweep, d_chains, n, nsweeps);
     return cuda_check(cudaGetLastError(), "k_advance");
 }
 
@@ -1089,10 +1095,10 @@ static void heis_compact_launch(Ctx& c, const int* d_chains, int n, int colour, 
     dim3 grid((c.fill_max + 255) / 256, n);
     if (grid.x == 0) return;
     if (c.ctab_packed)
-        k_heis_compact<DIM, DK, true><<<grid, 256, 0, c.stream>>>(c.m, c.d_cspins, c.d_ctab, c.d_fill_n, c.d_bh,
+        launch_seq(c, k_heis_compact<DIM, DK, true>, grid, 256, 0, c.m, c.d_cspins, c.d_ctab, c.d_fill_n, c.d_bh,
                                                                    c.d_sweep, d_chains, colour, off);
     else
-        k_heis_compact<DIM, DK, false><<<grid, 256, 0, c.stream>>>(c.m, c.d_cspins, c.d_ctab, c.d_fill_n, c.d_bh,
+        launch_seq(c, k_heis_compact<DIM, DK, false>, grid, 256, 0, c.m, c.d_cspins, c.d_ctab, c.d_fill_n, c.d_bh,
                                                                     c.d_sweep, d_chains, colour, off);
 }
 
@@ -1111,7 +1117,7 @@ static int compact_copy(Ctx& c, const int* d_chains, int n, bool to_compact) {
     const int bx = std::min((c.fill_max + 255) / 256, 64);
     for (int c0 = 0; c0 < n; c0 += 32767) {   // grid.y = 2 x chains of this part
         const int part = std::min(32767, n - c0);
-        k_compact_copy<<<dim3(bx, 2 * part), 256, 0, c.stream>>>(c.d_cspins, (float*)c.d_spins, c.d_fill, c.d_fill_n,
+        launch_seq(c, k_compact_copy, dim3(bx, 2 * part), 256, 0, c.d_cspins, (float*)c.d_spins, c.d_fill, c.d_fill_n,
                                                                  d_chains + c0, c.m.nhalf, (size_t)c.m.nhalf_pad,
                                                                  to_compact ? 1 : 0);
     }
@@ -1868,6 +1874,7 @@ __global__ void k_measure_finalize(const int* __restrict__ chains, int nblk, int
                                    const double* __restrict__ Hd, double* __restrict__ obs,
                                    double* __restrict__ q, double* __restrict__ accum,
                                    int accumulate) {
+    seq_begin();
     const int ci = blockIdx.x;
     const int chain = chains[ci];
     const int lane = threadIdx.x;
@@ -1876,7 +1883,7 @@ __global__ void k_measure_finalize(const int* __restrict__ chains, int nblk, int
 #pragma unroll
     for (int k = 0; k < kNP - 1; ++k) {
         double v = 0;
-        for (int b = lane; b < nblk; b += 32) v += pp[(size_t)b * kNP + k];
+        for (int b = lane; b < nblk; b += 32) v += __ldcg(pp + (size_t)b * kNP + k);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         const double t = __shfl_sync(0xffffffffu, v, 0);
@@ -1886,7 +1893,7 @@ __global__ void k_measure_finalize(const int* __restrict__ chains, int nblk, int
     double qsum = 0;
     for (int zs = lane; zs < nslices; zs += 32) {
         double v = 0;
-        for (int b = 0; b < nblk_slice; ++b) v += pp[((size_t)zs * nblk_slice + b) * kNP + 10];
+        for (int b = 0; b < nblk_slice; ++b) v += __ldcg(pp + ((size_t)zs * nblk_slice + b) * kNP + 10);
         v = ising ? 0.0 : v / (2 * M_PI);
         if (q) q[(size_t)ci * nslices + zs] = v;
         qsum += v;
@@ -1909,6 +1916,7 @@ k_measure_finalize_fused(const int* __restrict__ chains, const double* __restric
                          const double* __restrict__ Hd,
                          double* __restrict__ obs, double* __restrict__ q, double* __restrict__ accum,
                          int accumulate) {
+    seq_begin();
     const int ci = blockIdx.x;
     const int chain = chains[ci];
     const double* B = rows + (size_t)ci * nrows * 10;
@@ -1918,12 +1926,13 @@ k_measure_finalize_fused(const int* __restrict__ chains, const double* __restric
     for (int k = 0; k < 10; ++k) t[k] = 0.0;
     for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
         const double* bb = B + (size_t)r * 10;   // 2 e, M of colour 1, M of colour 0, sub4M
-        t[0] += bb[0];
+        t[0] += __ldcg(bb);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            t[1 + c] += bb[4 + c] + bb[1 + c];
-            t[4 + c] += bb[4 + c];
-            t[7 + c] += bb[7 + c];
+            const double m1 = __ldcg(bb + 1 + c), m0 = __ldcg(bb + 4 + c);
+            t[1 + c] += m0 + m1;
+            t[4 + c] += m0;
+            t[7 + c] += __ldcg(bb + 7 + c);
         }
     }
     __shared__ double red[10][256];
@@ -1951,7 +1960,7 @@ k_measure_finalize_fused(const int* __restrict__ chains, const double* __restric
     double qsum = 0;
     for (int zs = lane; zs < nslices; zs += 32) {
         double v = 0;
-        for (int b = 0; b < nblk_slice; ++b) v += pp[((size_t)zs * nblk_slice + b) * kNP + 10];
+        for (int b = 0; b < nblk_slice; ++b) v += __ldcg(pp + ((size_t)zs * nblk_slice + b) * kNP + 10);
         v = v / (2 * M_PI);
         if (q) q[(size_t)ci * nslices + zs] = v;
         qsum += v;
@@ -2172,7 +2181,7 @@ static int measure_with(Ctx& c, const int* d_chains, int n, double* partial, dou
         int rc = launch_energy_general(c, d_chains, n, rows, nblk_slice, nblk, partial);
         if (rc) return rc;
     }
-    k_measure_finalize<<<n, 32, 0, c.stream>>>(d_chains, nblk, nblk_slice, c.m.lz, c.ising ? 1 : 0, partial,
+    launch_seq(c, k_measure_finalize, dim3(n), 32, 0, d_chains, nblk, nblk_slice, c.m.lz, c.ising ? 1 : 0, partial,
                                                c.d_Hd, obs, q, c.d_acc, accumulate);
     return cuda_check(cudaGetLastError(), "measure launch");
 }
@@ -2185,15 +2194,15 @@ int launch_measure(Ctx& c, const int* d_chains, int n, int accumulate) {
     return measure_with(c, d_chains, n, c.d_partial, c.d_obs, c.d_q, accumulate);
 }
 
-int hbm_tuning_step(Ctx& c, int nsweeps, bool measure) {
+int hbm_tuning_step(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure) {
     int rc;
     if (measure && hbm_fused_measure_ok(c)) {
-        if ((rc = measure_prepare(c, c.nchains))) return rc;
-        if ((rc = launch_global_sweeps(c, c.d_all, c.nchains, nsweeps, true))) return rc;
-        return launch_measure_fused_tail(c, c.d_all, c.nchains, 0);
+        if ((rc = measure_prepare(c, n))) return rc;
+        if ((rc = launch_global_sweeps(c, d_chains, n, nsweeps, true))) return rc;
+        return launch_measure_fused_tail(c, d_chains, n, 0);
     }
-    if ((rc = launch_global_sweeps(c, c.d_all, c.nchains, nsweeps, false))) return rc;
-    return measure ? launch_measure(c, c.d_all, c.nchains, 0) : NMMC_OK;
+    if ((rc = launch_global_sweeps(c, d_chains, n, nsweeps, false))) return rc;
+    return measure ? launch_measure(c, d_chains, n, 0) : NMMC_OK;
 }
 
 // After the fused last sweep of a sample step: the charge pass over every site's triangles and
@@ -2220,7 +2229,7 @@ int launch_measure_fused_tail(Ctx& c, const int* d_chains, int n, int accumulate
                 k_charge_rows<false><<<grid, 256, 0, c.stream>>>(c.m, sp, d_chains, nstrip, nseg, R, nblk_slice,
                                                                  c.d_partial);
             const int nb = q4_meas_blocks(c);
-            k_measure_finalize_fused<<<n, 256, 0, c.stream>>>(d_chains, c.d_partial, nblk, nblk_slice, c.m.lz,
+            launch_seq(c, k_measure_finalize_fused, dim3(n), 256, 0, d_chains, c.d_partial, nblk, nblk_slice, c.m.lz,
                                                               c.d_mrows, nb, c.d_Hd, c.d_obs, c.d_q, c.d_acc,
                                                               accumulate);
             return cuda_check(cudaGetLastError(), "fused measure launch");
@@ -2240,7 +2249,7 @@ int launch_measure_fused_tail(Ctx& c, const int* d_chains, int n, int accumulate
     else { if (c.periodic) NMMC_QP(2, true); else NMMC_QP(2, false); }
 #undef NMMC_QP
     const int nb = q4_meas_blocks(c);
-    k_measure_finalize_fused<<<n, 256, 0, c.stream>>>(d_chains, c.d_partial, ms.nblk, ms.nblk_slice, c.m.lz,
+    launch_seq(c, k_measure_finalize_fused, dim3(n), 256, 0, d_chains, c.d_partial, ms.nblk, ms.nblk_slice, c.m.lz,
                                                       c.d_mrows, nb, c.d_Hd, c.d_obs, c.d_q, c.d_acc, accumulate);
     return cuda_check(cudaGetLastError(), "fused measure launch");
 }

@@ -9,6 +9,17 @@ namespace nmmc {
 constexpr float kPi = 3.14159265358979f;
 constexpr float kLn2 = 0.693147180559945f;
 
+// First statement of a kernel launched by launch_seq: lets the next kernel's blocks move in as
+// soon as this one's are all running, then waits until the previous kernel is complete and its
+// writes are visible. Every thread of every block calls it before its first access to global
+// memory (a kernel that finished without waiting would let its successor overtake its
+// predecessor). Data that the previous kernel wrote is read with plain loads afterwards, not through
+// the read-only path.
+__device__ __forceinline__ void seq_begin() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Packed pairs of FP32 values: one instruction for two IEEE operations (round to nearest).
 struct f2 { unsigned long long v; };
 __device__ __forceinline__ f2 pk(float a, float b) {

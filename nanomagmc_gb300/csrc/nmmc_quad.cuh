@@ -20,11 +20,7 @@ struct F2x2 { f2 a, b; };
 // A quad at `off` floats past a plane's base (16-byte aligned). The base is the same for every
 // thread of a block and the offset 32 bits, so that an access needs one address register and
 // no 64-bit arithmetic of its own.
-__device__ __forceinline__ F2x2 ld_quad(const float* base, uint32_t off) {   // read-only data
-    const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(reinterpret_cast<const char*>(base) + off * 4u));
-    return F2x2{{t.x}, {t.y}};
-}
-__device__ __forceinline__ F2x2 ld_quad_rw(const float* base, uint32_t off) {   // data that this thread writes back
+__device__ __forceinline__ F2x2 ld_quad(const float* base, uint32_t off) {
     const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(reinterpret_cast<const char*>(base) + off * 4u);
     return F2x2{{t.x}, {t.y}};
 }

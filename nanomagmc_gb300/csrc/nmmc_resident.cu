@@ -436,7 +436,7 @@ void free_tables(ResidentTables& r) {
     r.d_slot_red = r.d_slot_black = nullptr;
     r.built = false;
     r.stencil = false;
-    r.large_tuned = false;
+    r.large_stencil.clear();
     r.hbm_faster = false;
     r.tables_bins = 0;
 }
@@ -793,34 +793,39 @@ float best_of_three(Ctx& c, Step step) {
 }
 
 // Lattices too large for the record kernel, on the automatic path: the stencil kernel on
-// clusters against the HBM path, by the same timing (and the same cache: no bins, the path).
-// Small batches gain most (8 chains of 30^3 take 11 us per sweep in launches alone); the
-// streaming path keeps lattices that fit no cluster and batches that fill the GPU many times.
-int tune_large(Ctx& c) {
-    if (c.res.large_tuned) return NMMC_OK;
-    c.res.stencil = false;
-    c.res.large_tuned = true;
-    if (c.res_stencil == 1 || stencil_shape(c, c.nchains).C < 1) return NMMC_OK;
-    if (c.res_stencil == 2) {
-        c.res.stencil = true;
+// clusters against the HBM path, by the same timing, for each number of chains that is swept
+// together (8 chains of 30^3 take 4.5 us per sweep against 10.6 in launches, 16 of them 8.9
+// against 11.0) and kept in the same cache. The streaming path keeps lattices that fit no cluster
+// and batches that fill the GPU many times.
+int tune_large(Ctx& c, const int* d_chains, int n) {
+    if (n <= 0 || c.res.large_stencil.count(n)) return NMMC_OK;
+    if (c.res_stencil == 1 || stencil_shape(c, n).C < 1) {
+        c.res.large_stencil[n] = false;
         return NMMC_OK;
     }
-    const std::string key = config_key(c);
+    if (c.res_stencil == 2) {
+        c.res.large_stencil[n] = true;
+        return NMMC_OK;
+    }
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    NMMC_CUDA(cudaStreamIsCapturing(c.stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return NMMC_OK;   // nothing is timed in a capture: the HBM path
+    const std::string key = config_key(c) + "/" + std::to_string(n);
     int cb = 0, ct = 0, cp = 0, ch = 0;
     if (cache_lookup(key, cb, ct, cp, ch)) {
-        c.res.stencil = ch == 2;
+        c.res.large_stencil[n] = ch == 2;
         return NMMC_OK;
     }
     TuningSnapshot snap;
     int rc = snap.take(c);
     if (rc) return rc;
     const bool fused = !c.measure_fp64;
-    const float th = best_of_three(c, [&](int k) { return hbm_tuning_step(c, k, fused); });
-    const float ts = best_of_three(c, [&](int k) { return launch_stencil_sweeps(c, c.d_all, c.nchains, k, fused, 0); });
+    const float th = best_of_three(c, [&](int k) { return hbm_tuning_step(c, d_chains, n, k, fused); });
+    const float ts = best_of_three(c, [&](int k) { return launch_stencil_sweeps(c, d_chains, n, k, fused, 0); });
     cudaGetLastError();
     if ((rc = snap.restore(c))) return rc;
-    c.res.stencil = ts < th;
-    cache_store(key, 0, 0, 0, c.res.stencil ? 2 : 1);
+    c.res.large_stencil[n] = ts < th;
+    cache_store(key, 0, 0, 0, ts < th ? 2 : 1);
     return NMMC_OK;
 }
 
@@ -828,10 +833,12 @@ int tune_large(Ctx& c) {
 
 void resident_free(Ctx& c) { free_tables(c.res); }
 
-int resident_launches(const Ctx& c, int nsweeps) { return c.res.stencil ? 1 : launches_for(c, nsweeps); }
+int resident_launches(const Ctx& c, int nsweeps) {
+    return c.res.stencil || !c.res.eligible ? 1 : launches_for(c, nsweeps);
+}
 
 // Decides eligibility and builds the tables (autotuned unless options fix the shape).
-int resident_prepare(Ctx& c) {
+int resident_prepare(Ctx& c, const int* d_chains, int n) {
     if (c.res.built) return NMMC_OK;
     const size_t budget = smem_budget(c);
     const int cap_sites = (int)std::min<size_t>(65534, budget / site_bytes(c) - 1);
@@ -840,7 +847,7 @@ int resident_prepare(Ctx& c) {
     // general interaction tables use the multi-colour gather sweep
     c.res.eligible = maxn > 0 && maxn <= cap_sites && !c.m.general;
     // the stencil kernel covers unmasked Heisenberg lattices that fit a cluster
-    if (!c.res.eligible) return c.sweep_path == 0 ? tune_large(c) : NMMC_OK;
+    if (!c.res.eligible) return c.sweep_path == 0 ? tune_large(c, d_chains, n) : NMMC_OK;
     const bool stencil_ok = c.res_stencil != 1 && stencil_shape(c, c.nchains).C > 0;
 
     std::vector<int> load(c.num.begin(), c.num.end());
@@ -963,7 +970,7 @@ int resident_prepare(Ctx& c) {
     // few SMs: 16 chains of 128^2 sweep in 8.6 us there against 16.6 us resident)
     bool hbm = false;
     if (automatic && c.sweep_path == 0 && best_b > 0) {
-        const float ms = best_of_three(c, [&](int k) { return hbm_tuning_step(c, k, fused); });
+        const float ms = best_of_three(c, [&](int k) { return hbm_tuning_step(c, c.d_all, c.nchains, k, fused); });
         hbm = ms < best;
         if (hbm) best = ms;
     }
@@ -992,9 +999,16 @@ int resident_prepare(Ctx& c) {
     return rc;
 }
 
-bool resident_chosen(const Ctx& c) {
+// The stencil kernel takes a call on n chains.
+static bool takes_stencil(const Ctx& c, int n) {
+    if (c.res.eligible) return c.res.stencil;
+    const auto it = c.res.large_stencil.find(n);
+    return it != c.res.large_stencil.end() && it->second;
+}
+
+bool resident_chosen(const Ctx& c, int n) {
     if (!c.res.eligible)   // the options that pick a streaming variant keep the streaming path
-        return c.sweep_path == 0 && c.res.large_tuned && c.res.stencil && c.half_kernel == 0 && !c.wave;
+        return c.sweep_path == 0 && takes_stencil(c, n) && c.half_kernel == 0 && !c.wave;
     return !(c.sweep_path == 0 && c.res.hbm_faster);
 }
 
@@ -1006,8 +1020,8 @@ __global__ void k_mark_active(uint8_t* active, int* pos, const int* chains, int 
     }
 }
 
-bool resident_can_measure(const Ctx& c) {
-    if (c.res.stencil && resident_chosen(c)) return !c.measure_fp64;
+bool resident_can_measure(const Ctx& c, int n) {
+    if (takes_stencil(c, n) && resident_chosen(c, n)) return !c.measure_fp64;
     // one z-slice, FP32 observables, and whole warps for the per-slot reductions
     return c.res.built && c.res.eligible && c.dim == 2 && !c.measure_fp64 && c.res.threads >= 32 &&
            c.res.threads % 32 == 0;
@@ -1015,8 +1029,8 @@ bool resident_can_measure(const Ctx& c) {
 
 int launch_resident_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool all, bool measure,
                            int accumulate) {
-    if (c.res.stencil) {   // whole chains from the list: no chain marks needed
-        if (measure && !resident_can_measure(c)) return set_error(NMMC_ERR_UNSUPPORTED, "fused measurement not available");
+    if (takes_stencil(c, n)) {   // whole chains from the list: no chain marks needed
+        if (measure && !resident_can_measure(c, n)) return set_error(NMMC_ERR_UNSUPPORTED, "fused measurement not available");
         return launch_stencil_sweeps(c, d_chains, n, nsweeps, measure, accumulate);
     }
     // Mark the chains of this call; the others keep their spins and counters. A direct call on
@@ -1034,7 +1048,7 @@ int launch_resident_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool
         c.active_all = false;
     }
     if (!measure) return do_launch(c, nsweeps, nullptr);
-    if (!resident_can_measure(c)) return set_error(NMMC_ERR_UNSUPPORTED, "fused measurement not available");
+    if (!resident_can_measure(c, n)) return set_error(NMMC_ERR_UNSUPPORTED, "fused measurement not available");
     FusedMeasure fm{c.d_obs, c.d_q, c.d_acc, c.d_Hd, direct_all ? nullptr : c.d_pos,
                     c.res.d_slot_red, c.res.d_slot_black, accumulate};
     return do_launch(c, nsweeps, &fm);
