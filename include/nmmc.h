@@ -271,7 +271,7 @@ int nmmc_fork(nmmc_ctx* ctx, int src_chain, int dst_chain);
  * nsweeps two-colour checkerboard sweeps. The first sweep call of a context (and the first
  * after an option that changes the resident shape) builds the path's tables on the device
  * (the resident kernel's site tables and autotuning, the compact form of masked lattices):
- * make it outside any stream capture (nmmc_sample prepares them before it captures). */
+ * make it outside any stream capture. */
 int nmmc_sweep(nmmc_ctx* ctx, const int* chains, int n, int nsweeps);
 
 /* magnetisation / energy / submag(0) / sub4mag / tcharge (Old/lib/state.cpp:205-246,
@@ -325,8 +325,8 @@ int nmmc_measure_static(nmmc_ctx* ctx, const int* d_chains, int n, double* d_obs
 int nmmc_sweep_measure(nmmc_ctx* ctx, const int* chains, int n, int nsweeps, double* obs, double* q,
                        int accumulate);
 
-/* nsamples x nmmc_sweep_measure(nsweeps, accumulate = 1), replayed as one CUDA graph per
- * sample, for the inner sampling loop of Old/lib/main.cpp:182-240.
+/* nsamples x nmmc_sweep_measure(nsweeps, accumulate = 1) without a host round trip between
+ * samples, for the inner sampling loop of Old/lib/main.cpp:182-240.
  * obs: nsamples x n x NMMC_OBS_N, q: nsamples x n x nslices (may be NULL). */
 int nmmc_sample(nmmc_ctx* ctx, const int* chains, int n, int nsweeps, int nsamples,
                 double* obs, double* q);

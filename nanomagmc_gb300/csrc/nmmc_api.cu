@@ -236,8 +236,7 @@ static void destroy_ctx(Ctx* c) {
     cudaFree(c->d_gjed);
     cudaFree(c->d_partial);
     cudaFree(c->d_mrows);
-    cudaFree(c->d_obs);
-    cudaFree(c->d_q);
+    cudaFreeHost(c->h_out);   // d_obs and d_q live there
     cudaFree(c->d_acc);
     cudaFree(c->d_replay);
     cudaFree(c->d_flag);
@@ -492,12 +491,18 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
     r.dmi_sign = 0;
 
     // shapes and site counts
-    c->mask.assign((size_t)nchains * box, 1);
+    if (c->masked) c->mask.assign((size_t)nchains * box, 1);   // unmasked: every box site is filled
     c->num.resize(nchains);
     c->snum.resize(nchains);
     c->s4num.resize(nchains);
     for (int i = 0; i < nchains; ++i) {
-        uint8_t* mk = &c->mask[(size_t)i * box];
+        if (!weib && i > 0) {   // the same full box
+            c->num[i] = c->num[0];
+            c->snum[i] = c->snum[0];
+            c->s4num[i] = c->s4num[0];
+            continue;
+        }
+        uint8_t* mk = weib ? &c->mask[(size_t)i * box] : nullptr;
         if (weib) {
             if (!(opt->beta_w > 0)) {
                 destroy_ctx(c);
@@ -505,7 +510,7 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
             }
             weibull_mask(dim, edge, chains[i].size, opt->beta_w, seed, (uint32_t)chains[i].lattice, mk);
         }
-        site_counts(dim, edge, weib ? mk : nullptr, &c->num[i], &c->snum[i], &c->s4num[i]);
+        site_counts(dim, edge, mk, &c->num[i], &c->snum[i], &c->s4num[i]);
     }
 
     // device
@@ -561,8 +566,14 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
     NMMC_TRY(cudaMalloc(&c->d_list, sizeof(int) * nchains));
     NMMC_TRY(cudaMalloc(&c->d_active, nchains));
     NMMC_TRY(cudaMalloc(&c->d_pos, sizeof(int) * nchains));
-    NMMC_TRY(cudaMalloc(&c->d_obs, sizeof(double) * NMMC_OBS_N * nchains));
-    NMMC_TRY(cudaMalloc(&c->d_q, sizeof(double) * c->nslices * nchains));
+    // the observables go straight to page-locked host memory: a few doubles per chain, written by
+    // the finishing kernel, cost less than the copy that would follow it. Room for several samples
+    // of nmmc_sample.
+    c->out_stride = (size_t)(NMMC_OBS_N + c->nslices) * nchains;
+    c->out_slots = std::max<size_t>(1, std::min<size_t>(64, (64u << 10) / (c->out_stride * sizeof(double))));
+    NMMC_TRY(cudaHostAlloc(&c->h_out, c->out_slots * c->out_stride * sizeof(double), cudaHostAllocDefault));
+    c->d_obs = c->h_out;
+    c->d_q = c->h_out + (size_t)NMMC_OBS_N * nchains;
     NMMC_TRY(cudaMalloc(&c->d_acc, sizeof(double) * NMMC_ACC_N * nchains));
     NMMC_TRY(cudaMemset(c->d_acc, 0, sizeof(double) * NMMC_ACC_N * nchains));
     NMMC_TRY(cudaMalloc(&c->d_flag, sizeof(int)));
@@ -726,10 +737,9 @@ int nmmc_measure(nmmc_ctx* c, const int* chains, int n, double* obs, double* q, 
     if ((rc = launch_measure(*c, d, n, accumulate))) return rc;
     if (accumulate && (rc = launch_add_av(*c))) return rc;
     if (!obs) return NMMC_OK;   // results stay on the device (accumulators), no synchronisation
-    NMMC_CUDA(cudaMemcpyAsync(obs, c->d_obs, sizeof(double) * NMMC_OBS_N * n, cudaMemcpyDeviceToHost, c->stream));
-    if (q)
-        NMMC_CUDA(cudaMemcpyAsync(q, c->d_q, sizeof(double) * c->nslices * n, cudaMemcpyDeviceToHost, c->stream));
     NMMC_CUDA(cudaStreamSynchronize(c->stream));
+    memcpy(obs, c->d_obs, sizeof(double) * NMMC_OBS_N * n);
+    if (q) memcpy(q, c->d_q, sizeof(double) * c->nslices * n);
     return NMMC_OK;
 }
 
@@ -745,71 +755,42 @@ int nmmc_sweep_measure(nmmc_ctx* c, const int* chains, int n, int nsweeps, doubl
     if ((rc = measure_prepare(*c, n))) return rc;
     if ((rc = sweep_measure_impl(*c, d, chains, n, nsweeps, accumulate, true))) return rc;
     if (!obs) return NMMC_OK;   // results stay on the device (accumulators), no synchronisation
-    NMMC_CUDA(cudaMemcpyAsync(obs, c->d_obs, sizeof(double) * NMMC_OBS_N * n, cudaMemcpyDeviceToHost, c->stream));
-    if (q)
-        NMMC_CUDA(cudaMemcpyAsync(q, c->d_q, sizeof(double) * c->nslices * n, cudaMemcpyDeviceToHost, c->stream));
     NMMC_CUDA(cudaStreamSynchronize(c->stream));
+    memcpy(obs, c->d_obs, sizeof(double) * NMMC_OBS_N * n);
+    if (q) memcpy(q, c->d_q, sizeof(double) * c->nslices * n);
     return NMMC_OK;
 }
 
 int nmmc_sample(nmmc_ctx* c, const int* chains, int n, int nsweeps, int nsamples, double* obs, double* q) {
     if (!c || !obs || nsamples < 0 || nsweeps < 0) return set_error(NMMC_ERR_ARG, "bad argument");
-    if (chains) {
-        if (int rc = check_list(*c, chains, n)) return rc;
-    }
-    std::vector<int> list;
-    if (chains) list.assign(chains, chains + n);
-    else {
-        n = c->nchains;
-        for (int i = 0; i < n; ++i) list.push_back(i);
-    }
-    if (nsamples == 0 || n == 0) return NMMC_OK;
-    int rc = upload_params(*c);
+    chains = all_if_identity(*c, chains, n);
+    const int* d = nullptr;
+    int rc = set_list(*c, chains, n, &d);
     if (rc) return rc;
+    if (!chains) n = c->nchains;
+    if (nsamples == 0 || n == 0) return NMMC_OK;
     if ((rc = measure_prepare(*c, n))) return rc;
-    // history buffers on the device, one D2H at the end
-    DeviceScratch ds;
-    double *d_hist = nullptr, *d_qhist = nullptr;
-    int* d_l = nullptr;
-    NMMC_CUDA(ds.alloc(&d_hist, sizeof(double) * NMMC_OBS_N * n * (size_t)nsamples));
-    if (q) NMMC_CUDA(ds.alloc(&d_qhist, sizeof(double) * c->nslices * n * (size_t)nsamples));
-    NMMC_CUDA(ds.alloc(&d_l, sizeof(int) * n));
-    NMMC_CUDA(cudaMemcpy(d_l, list.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    const bool all = all_if_identity(*c, list.data(), n) == nullptr;   // every chain, in order
-    const int* list_dev = all ? c->d_all : d_l;
-    if (c->sweep_path != 1) {
-        if ((rc = resident_prepare(*c, list_dev, n))) return rc;
+    // each sample's observables into their own slot of the page-locked results, the host reading
+    // them out once per out_slots samples
+    double *const obs0 = c->d_obs, *const q0 = c->d_q;
+    const size_t no = (size_t)NMMC_OBS_N * n, nq = (size_t)c->nslices * n;
+    for (int done = 0; done < nsamples && !rc;) {
+        const int k = (int)std::min<size_t>(c->out_slots, (size_t)(nsamples - done));
+        for (int s = 0; s < k && !rc; ++s) {
+            c->d_obs = obs0 + s * c->out_stride;
+            c->d_q = q0 + s * c->out_stride;
+            rc = sweep_measure_impl(*c, d, chains, n, nsweeps, 1, false);
+        }
+        const cudaError_t se = cudaStreamSynchronize(c->stream);
+        if (!rc) rc = cuda_check(se, "nmmc_sample");
+        for (int s = 0; s < k && !rc; ++s) {
+            memcpy(obs + no * (done + s), obs0 + s * c->out_stride, no * sizeof(double));
+            if (q) memcpy(q + nq * (done + s), q0 + s * c->out_stride, nq * sizeof(double));
+        }
+        done += k;
     }
-    // the HBM path's compact tables: no allocation or table upload inside the capture
-    if (!(c->sweep_path != 1 && resident_chosen(*c, n))) {
-        if ((rc = compact_prepare(*c))) return rc;
-        class_ready(*c);  // the class planes of a general table
-        wave_ready(*c);   // the wavefront sweeps' second array (when enabled), not inside the capture
-    }
-    // one graph: nsweeps sweeps + measure (accumulating), as nmmc_sweep_measure
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t ge = nullptr;
-    NMMC_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    rc = sweep_measure_impl(*c, list_dev, all ? nullptr : list.data(), n, nsweeps, 1, false);
-    cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
-    if (rc || ce != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        return rc ? rc : cuda_check(ce, "cudaStreamEndCapture");
-    }
-    ce = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
-    if (ce != cudaSuccess) return cuda_check(ce, "cudaGraphInstantiate");
-    const size_t ob = sizeof(double) * NMMC_OBS_N * n, qb = sizeof(double) * c->nslices * n;
-    for (int s = 0; s < nsamples && !rc; ++s) {
-        rc = cuda_check(cudaGraphLaunch(ge, c->stream), "cudaGraphLaunch");
-        if (!rc) rc = cuda_check(cudaMemcpyAsync((char*)d_hist + ob * s, c->d_obs, ob, cudaMemcpyDeviceToDevice, c->stream), "obs copy");
-        if (!rc && q) rc = cuda_check(cudaMemcpyAsync((char*)d_qhist + qb * s, c->d_q, qb, cudaMemcpyDeviceToDevice, c->stream), "q copy");
-    }
-    if (!rc) rc = cuda_check(cudaMemcpyAsync(obs, d_hist, ob * nsamples, cudaMemcpyDeviceToHost, c->stream), "obs D2H");
-    if (!rc && q) rc = cuda_check(cudaMemcpyAsync(q, d_qhist, qb * nsamples, cudaMemcpyDeviceToHost, c->stream), "q D2H");
-    cudaError_t se = cudaStreamSynchronize(c->stream);
-    if (!rc) rc = cuda_check(se, "nmmc_sample");
-    cudaGraphExecDestroy(ge);
+    c->d_obs = obs0;
+    c->d_q = q0;
     return rc;
 }
 
@@ -836,11 +817,20 @@ int nmmc_reset_accumulators(nmmc_ctx* c) {
 int nmmc_get_spins(nmmc_ctx* c, int chain, double* xyz, size_t n_sites) {
     if (!c || !xyz || chain < 0 || chain >= c->nchains) return set_error(NMMC_ERR_ARG, "bad argument");
     if (n_sites != (size_t)c->box_sites) return set_error(NMMC_ERR_ARG, "expected %lld sites", c->box_sites);
-    const size_t bytes = chain_elems(*c) * elem_bytes(*c);
-    std::vector<char> buf(bytes);
+    if (!c->d_replay && cudaMalloc(&c->d_replay, sizeof(double) * 3 * (size_t)c->box_sites) != cudaSuccess) {
+        cudaGetLastError();   // no room for the FP64 box: the planes are rearranged on the host
+        c->d_replay = nullptr;
+        const size_t bytes = chain_elems(*c) * elem_bytes(*c);
+        std::vector<char> buf(bytes);
+        NMMC_CUDA(cudaStreamSynchronize(c->stream));
+        NMMC_CUDA(cudaMemcpy(buf.data(), (char*)c->d_spins + chain * bytes, bytes, cudaMemcpyDeviceToHost));
+        planes_to_box(*c, buf.data(), xyz);
+        return NMMC_OK;
+    }
+    if (int rc = launch_to_fp64(*c, chain)) return rc;
+    NMMC_CUDA(cudaMemcpyAsync(xyz, c->d_replay, sizeof(double) * 3 * (size_t)c->box_sites, cudaMemcpyDeviceToHost,
+                              c->stream));
     NMMC_CUDA(cudaStreamSynchronize(c->stream));
-    NMMC_CUDA(cudaMemcpy(buf.data(), (char*)c->d_spins + chain * bytes, bytes, cudaMemcpyDeviceToHost));
-    planes_to_box(*c, buf.data(), xyz);
     return NMMC_OK;
 }
 
@@ -861,6 +851,11 @@ int nmmc_set_av_chains(nmmc_ctx* c, const int* chains, int n) {
         if (chains[i] < 0 || chains[i] >= c->nchains) return set_error(NMMC_ERR_ARG, "chain index out of range");
         for (int k = 0; k < i; ++k)
             if (chains[k] == chains[i]) return set_error(NMMC_ERR_ARG, "chain %d listed twice", chains[i]);
+    }
+    const bool same = (size_t)n == c->av_chains.size() && std::equal(chains, chains + n, c->av_chains.begin());
+    if (same && n) {   // the list is on the device: only the sums start again
+        NMMC_CUDA(cudaMemsetAsync(c->d_av, 0, sizeof(double) * 3 * (size_t)c->box_sites * n, c->stream));
+        return NMMC_OK;
     }
     NMMC_CUDA(cudaStreamSynchronize(c->stream));
     c->av_chains.assign(chains, chains + n);
@@ -886,16 +881,17 @@ int nmmc_get_av(nmmc_ctx* c, int chain, double* xyz, size_t n_sites) {
     size_t slot = 0;
     while (slot < c->av_chains.size() && c->av_chains[slot] != chain) ++slot;
     if (slot == c->av_chains.size()) return set_error(NMMC_ERR_ARG, "chain %d is not summed (nmmc_set_av_chains)", chain);
+    NMMC_CUDA(cudaMemcpyAsync(xyz, c->d_av + slot * 3 * (size_t)c->box_sites, sizeof(double) * 3 * (size_t)c->box_sites,
+                              cudaMemcpyDeviceToHost, c->stream));
     NMMC_CUDA(cudaStreamSynchronize(c->stream));
-    NMMC_CUDA(cudaMemcpy(xyz, c->d_av + slot * 3 * (size_t)c->box_sites, sizeof(double) * 3 * (size_t)c->box_sites,
-                         cudaMemcpyDeviceToHost));
     return NMMC_OK;
 }
 
 int nmmc_get_mask(nmmc_ctx* c, int chain, uint8_t* mask, size_t n_sites) {
     if (!c || !mask || chain < 0 || chain >= c->nchains) return set_error(NMMC_ERR_ARG, "bad argument");
     if (n_sites != (size_t)c->box_sites) return set_error(NMMC_ERR_ARG, "expected %lld sites", c->box_sites);
-    std::copy_n(&c->mask[(size_t)chain * c->box_sites], c->box_sites, mask);
+    if (c->masked) std::copy_n(&c->mask[(size_t)chain * c->box_sites], c->box_sites, mask);
+    else std::fill_n(mask, c->box_sites, (uint8_t)1);
     return NMMC_OK;
 }
 
@@ -905,7 +901,7 @@ int nmmc_delta_e(nmmc_ctx* c, int chain, const int32_t* sites, const double* tri
     if (n == 0) return NMMC_OK;
     for (int i = 0; i < n; ++i) {
         if (sites[i] < 0 || sites[i] >= c->box_sites) return set_error(NMMC_ERR_ARG, "site %d out of range", sites[i]);
-        if (!c->mask[(size_t)chain * c->box_sites + sites[i]]) return set_error(NMMC_ERR_ARG, "site %d is outside the particle", sites[i]);
+        if (c->masked && !c->mask[(size_t)chain * c->box_sites + sites[i]]) return set_error(NMMC_ERR_ARG, "site %d is outside the particle", sites[i]);
     }
     int rc = upload_params(*c);
     if (rc) return rc;
@@ -935,7 +931,7 @@ int nmmc_debug_replay(nmmc_ctx* c, int chain, const nmmc_event* ev, size_t n, ui
     for (size_t i = 0; i < n; ++i) {
         int s = ev[i].site_box;
         if (s < 0 || s >= c->box_sites) return set_error(NMMC_ERR_ARG, "event %zu: site %d out of range", i, s);
-        if (!c->mask[(size_t)chain * c->box_sites + s]) return set_error(NMMC_ERR_ARG, "event %zu: site %d outside the particle", i, s);
+        if (c->masked && !c->mask[(size_t)chain * c->box_sites + s]) return set_error(NMMC_ERR_ARG, "event %zu: site %d outside the particle", i, s);
         if (ev[i].u <= 0 && ev[i].accepted == 0) return set_error(NMMC_ERR_ARG, "event %zu: rejection without a uniform", i);
     }
     c->rm.dmi_sign = c->dmi_sign;

@@ -181,8 +181,12 @@ struct Ctx {
     size_t partial_cap = 0;             // doubles
     double* d_mrows = nullptr;          // block rows of the fused half-sweeps (nmmc_sweep_measure, HBM path)
     size_t mrows_cap = 0;               // doubles
-    double* d_obs = nullptr;            // nchains x NMMC_OBS_N
-    double* d_q = nullptr;              // nchains x nslices
+    // results of the current call, in page-locked host memory (h_out: out_slots slots of out_stride
+    // doubles, each nchains x NMMC_OBS_N, then nchains x nslices)
+    double* h_out = nullptr;
+    size_t out_stride = 0, out_slots = 1;
+    double* d_obs = nullptr;            // n x NMMC_OBS_N
+    double* d_q = nullptr;              // n x nslices
     double* d_acc = nullptr;            // nchains x NMMC_ACC_N
     double* d_replay = nullptr;         // FP64 working copy for the sequential replay
     int* d_flag = nullptr;              // device error word
@@ -294,6 +298,7 @@ size_t measure_partials_per_chain(const Ctx& c);   // partial-sum doubles one ch
 int launch_measure_into(Ctx& c, const int* d_chains, int n, double* scratch, size_t scratch_doubles,
                         double* obs, double* q);
 int launch_init_spins(Ctx& c);
+int launch_to_fp64(Ctx& c, int chain);   // the chain's spins in box order into d_replay
 int launch_add_av(Ctx& c);   // adds the av chains' spins to their sums (no-op without a list)
 int launch_delta_e(Ctx& c, int chain, const int32_t* d_sites, const float* d_trial, int n, double* d_out);
 int launch_replay(Ctx& c, int chain, const nmmc_event* d_ev, size_t n, uint8_t* d_acc, long long* d_first);

@@ -2438,6 +2438,11 @@ __global__ void k_replay(const DevModel m, const ReplayModel* __restrict__ rmp, 
     *first = fm;
 }
 
+int launch_to_fp64(Ctx& c, int chain) {
+    k_to_fp64<<<(unsigned)((c.box_sites + 255) / 256), 256, 0, c.stream>>>(c.m, c.d_spins, chain, c.d_replay);
+    return cuda_check(cudaGetLastError(), "k_to_fp64");
+}
+
 int launch_replay(Ctx& c, int chain, const nmmc_event* d_ev, size_t n, uint8_t* d_acc, long long* d_first) {
     long long nbox = c.box_sites;
     int g = (int)((nbox + 255) / 256);
