@@ -54,6 +54,7 @@ struct GenLayer {
     __nv_bfloat16* wt = nullptr;     // BF16 flipped transpose [9][cout][cin] (data gradient)
     uint8_t* wimg = nullptr;         // BF16 weights in the tensor-core B layout of k_gen_conv_tma
                                      // (kWimgBytes), staged by one bulk copy per CTA
+    uint8_t* wtimg = nullptr;        // hidden layers: wt as TF32 in that layout (2 kWimgBytes)
     float* gw = nullptr;
     float* gb = nullptr;
     float* mw = nullptr;
@@ -526,15 +527,16 @@ k_gen_conv_tc(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_b
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }
 
-// TMA-fed variant for L = 128 (the configured size): a tile is one image row (128 positions =
+// Bulk-copy-fed variant for L = 128 (the configured size): a tile is one image row (128 positions =
 // the 128 TMEM lanes). Its window is the three wrapped rows y-1, y, y+1, each staged as kCh
-// blocks (one per 16-byte channel chunk) of 130 slots (x = -1 .. 128) by one TMA box
-// [chunk elements, 130 x, 1 row, 1 chunk, 1 image] per block (a contiguous run of the chunk
-// plane), completing on one mbarrier: 3 kCh bulk copies per tile. TMA fills x = -1 and x = 128 with
-// zeros; the threads then copy x = 127 and x = 0 into those slots (periodic in x), fence them
-// to the async proxy, and thread 0 issues the 9 taps x kCh/2 MMAs, each tap a descriptor offset
-// (row block, and x shift of one slot). The next tile's copies are issued as soon as the MMAs
-// have committed, so they land while the epilogue drains the accumulator.
+// blocks (one per 16-byte channel chunk) of 130 slots (x = -1 .. 128). A row of a chunk plane is
+// 2048 contiguous bytes, so each block is one cp.async.bulk into slots 1 .. 128, completing on one
+// mbarrier: 3 kCh copies per tile. (As tensor-map boxes of 130 positions x 16 bytes the same
+// windows moved 16 bytes at a time: a hidden forward layer of 16 x 128^2 took 24.6 us and the TF32
+// data gradient 84 us.) The threads then copy x = 127 and x = 0 into slots 0 and 129 (periodic
+// in x), fence them to the async proxy, and thread 0 issues the 9 taps x kCh/2 MMAs, each tap a
+// descriptor offset (row block, and x shift of one slot). The next tile's copies are issued as
+// soon as the MMAs have committed, so they land while the epilogue drains the accumulator.
 namespace tma {
 constexpr int kSlots = 130;                   // x = -1 .. 128
 constexpr int kBlk = 2176;                    // bytes per (row, chunk) block: 130 x 16 B, 128-B aligned
@@ -546,8 +548,8 @@ template <int MODE, int ICH = tc::chunks<MODE>(), int KCH = ICH, int CO = tc::kC
 __host__ __device__ constexpr int smem_bytes() { return 9 * btap<MODE, KCH, CO>() + (R + 2) * KCH * kBlk + 1024; }
 }  // namespace tma
 
-// Every convolution of the generator at L = 128 with TMA-staged windows. ICH input chunks
-// (16 bytes of channels each) come in by TMA; the K of one tap is KCH chunks (KCH - ICH zero
+// Every convolution of the generator at L = 128 with bulk-copied windows. ICH input chunks
+// (16 bytes of channels each) come in by bulk copies; the K of one tap is KCH chunks (KCH - ICH zero
 // blocks when a layer's inputs do not fill an MMA's K: the first layer's 8 BF16 channels are
 // one chunk of the two of K = 16); N = CO output channels rounded up to 16.
 //   MODE 0: bias + ReLU, BF16 out (48 channels);  MODE 1: bias, FP32 out (48 channels);
@@ -557,11 +559,11 @@ __host__ __device__ constexpr int smem_bytes() { return 9 * btap<MODE, KCH, CO>(
 // MMAs of output row j read window rows j .. j+2 into accumulator j (R x the TMEM columns),
 // and one commit and one epilogue pass cover the R rows, so the per-tile latency of the copy,
 // the commit and the epilogue is paid once for R rows.
-// With wimg (the forward modes), the weights arrive by one bulk copy of their tensor-core image
-// (k_gen_wimage) instead of being rearranged by the threads.
+// With wimg the weights arrive by one bulk copy of their tensor-core image (k_gen_wimage, for the
+// data gradient k_gen_wimage32) instead of being rearranged by the threads.
 template <int MODE, int ICH, int KCH, int CO, int R>
 __global__ void __launch_bounds__(128, 2)
-k_gen_conv_tma(const __grid_constant__ CUtensorMap tmap, const __nv_bfloat16* __restrict__ w,
+k_gen_conv_tma(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_bfloat16* __restrict__ w,
                const uint8_t* __restrict__ wimg, const float* __restrict__ bias,
                const __nv_bfloat16* __restrict__ mask, void* __restrict__ out_v, int ntiles,
                int* __restrict__ flag) {
@@ -574,7 +576,7 @@ k_gen_conv_tma(const __grid_constant__ CUtensorMap tmap, const __nv_bfloat16* __
     constexpr int kCols = NN <= 32 ? 32 : 64;                // TMEM columns of one accumulator
     constexpr int kL = kM;                                   // lattice edge of this kernel
     constexpr int kTpi = kL / R;                             // tiles per image
-    constexpr uint32_t kTx = (R + 2u) * ICH * tma::kSlots * 16u;   // bytes per window (OOB fill included)
+    constexpr uint32_t kRowB = kL * 16u, kTx = (R + 2u) * ICH * kRowB;   // bytes per chunk row and per window
     static_assert(KCH % 2 == 0 && KCH >= ICH && NN <= 64 && (MODE != 3 || CO == 4) && (MODE == 3 || CO == kC) &&
                   (R == 1 || R == 2 || R == 4) && kL % R == 0, "convolution shape");
     extern __shared__ uint8_t tsm_raw[];
@@ -589,24 +591,24 @@ k_gen_conv_tma(const __grid_constant__ CUtensorMap tmap, const __nv_bfloat16* __
 
     const uint32_t aBase = gen_smem_u32(sA), bBase = gen_smem_u32(sB);
     const uint32_t mb = gen_smem_u32(&mbar), tb = gen_smem_u32(&tbar), wbr = gen_smem_u32(&wbar);
-    const bool use_img = MODE != 2 && wimg != nullptr;
-    // thread 0: the window of tile t (image t / kTpi, rows R (t % kTpi) ..): R + 2 rows x ICH chunk blocks
+    const bool use_img = wimg != nullptr;
+    // warp 0: the window of tile t (image t / kTpi, rows R (t % kTpi) ..): R + 2 rows x ICH chunk
+    // blocks, one copy per lane at a time
     auto issue_window = [&](int t) {
         const int img = t / kTpi, y = (t - img * kTpi) * R;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tb), "r"(kTx) : "memory");
-#pragma unroll
-        for (int r = 0; r < R + 2; ++r) {
+        if (lane == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tb), "r"(kTx) : "memory");
+        __syncwarp();
+        const char* src = reinterpret_cast<const char*>(in) + (size_t)img * ICH * kL * kRowB;
+        for (int i = lane; i < (R + 2) * ICH; i += 32) {
+            const int r = i / ICH, c = i - r * ICH;
             int yy = y + r - 1;
             yy += (yy < 0) ? kL : ((yy >= kL) ? -kL : 0);
-#pragma unroll
-            for (int c = 0; c < ICH; ++c) {
-                const uint32_t dst = aBase + (uint32_t)((r * KCH + c) * tma::kBlk);
-                asm volatile(
-                    "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-                    "%5, %6}], [%7];" ::"r"(dst),
-                    "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(-1), "r"(yy), "r"(c), "r"(img), "r"(tb)
-                    : "memory");
-            }
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                    aBase + (uint32_t)((r * KCH + c) * tma::kBlk + 16)),
+                "l"(src + ((size_t)c * kL + yy) * kRowB), "r"(kRowB), "r"(tb)
+                : "memory");
         }
     };
     const int first = blockIdx.x, stride = gridDim.x;
@@ -616,7 +618,6 @@ k_gen_conv_tma(const __grid_constant__ CUtensorMap tmap, const __nv_bfloat16* __
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tb) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbr) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (n > 0) issue_window(first);   // the first window lands while the weights are staged
         if (use_img && n > 0) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(wbr), "r"(9u * kBT) : "memory");
             asm volatile(
@@ -624,6 +625,10 @@ k_gen_conv_tma(const __grid_constant__ CUtensorMap tmap, const __nv_bfloat16* __
                 "l"(reinterpret_cast<uint64_t>(wimg)), "r"(9u * kBT), "r"(wbr)
                 : "memory");
         }
+    }
+    if (warp == 0) {
+        __syncwarp();   // the barriers are initialised
+        if (n > 0) issue_window(first);   // the first window lands while the weights are staged
     }
     if constexpr (KCH > ICH) {   // K-padding blocks: zero once, never written by TMA
         constexpr int kZ = KCH - ICH, kU = tma::kBlk / 16;
@@ -719,7 +724,7 @@ k_gen_conv_tma(const __grid_constant__ CUtensorMap tmap, const __nv_bfloat16* __
         }
         // the MMAs have read the window: the next tile's copies overlap this epilogue
         if (k + 1 < n) {
-            if (tid == 0) issue_window(t + stride);
+            if (warp == 0) issue_window(t + stride);
             window_pending = true;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1782,32 +1787,28 @@ int window_map(const typename tc::Traits<MODE>::TA* in, int L, int nimg, CUtenso
     return NMMC_OK;
 }
 
-// single-role TMA kernel (every mode and layer shape; the data gradient's TF32 window leaves
-// room for one stage). Forward layers take tiles of NMMC_GEN_OPT_TILE_ROWS output rows (default
-// 2), the TF32 data gradient one.
+// single-role kernel (every mode and layer shape) in tiles of NMMC_GEN_OPT_TILE_ROWS output rows
+// (default 2); the TF32 data gradient's window and weights leave room for one CTA per SM.
 template <int MODE, int ICH, int KCH, int CO, int R>
-int conv_tma_launch_r(nmmc_gen* g, const CUtensorMap& map, const __nv_bfloat16* w, const uint8_t* wimg,
+int conv_tma_launch_r(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w, const uint8_t* wimg,
                       const float* bias, const __nv_bfloat16* mask, void* out, int nimg) {
     const int smem = tma::smem_bytes<MODE, ICH, KCH, CO, R>();
     if (int rc = ensure_smem(g, (const void*)k_gen_conv_tma<MODE, ICH, KCH, CO, R>, smem, true)) return rc;
     const int per_sm = std::max(1, std::min(2, g->smem_per_sm / (smem + 2048)));
     const int ntiles = nimg * g->L / R;
     const int grid = std::min(ntiles, per_sm * g->sm_count);
-    k_gen_conv_tma<MODE, ICH, KCH, CO, R><<<grid, 128, smem, g->stream>>>(map, w, wimg, bias, mask, out, ntiles,
+    k_gen_conv_tma<MODE, ICH, KCH, CO, R><<<grid, 128, smem, g->stream>>>(in, w, wimg, bias, mask, out, ntiles,
                                                                           g->d_flag);
     return cuda_check(cudaGetLastError(), "k_gen_conv_tma");
 }
 
-// wimg: the layer's weight image (forward modes; nullptr: the threads rearrange w)
+// wimg: the layer's weight image (nullptr: the threads rearrange w)
 template <int MODE, int ICH = tc::chunks<MODE>(), int KCH = ICH, int CO = tc::kC>
 int conv_tma_launch(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w, const float* bias,
                     const __nv_bfloat16* mask, void* out, int nimg, const uint8_t* wimg = nullptr) {
-    alignas(64) CUtensorMap map;
-    if (int rc = window_map<MODE, ICH>(in, g->L, nimg, &map)) return rc;
-    if (MODE == 2 || !g->use_wimg) wimg = nullptr;
-    if constexpr (MODE != 2)
-        if (g->tile_rows == 2) return conv_tma_launch_r<MODE, ICH, KCH, CO, 2>(g, map, w, wimg, bias, mask, out, nimg);
-    return conv_tma_launch_r<MODE, ICH, KCH, CO, 1>(g, map, w, wimg, bias, mask, out, nimg);
+    if (!g->use_wimg) wimg = nullptr;
+    if (g->tile_rows == 2) return conv_tma_launch_r<MODE, ICH, KCH, CO, 2>(g, in, w, wimg, bias, mask, out, nimg);
+    return conv_tma_launch_r<MODE, ICH, KCH, CO, 1>(g, in, w, wimg, bias, mask, out, nimg);
 }
 
 // The first (8 -> 48, ReLU) and last (48 -> 4, linear) layers on the tensor cores when L = 128
@@ -1941,6 +1942,16 @@ __global__ void k_gen_wimage(const __nv_bfloat16* __restrict__ wb, int cin, int 
                                       (k % 8) * 2) = v;
 }
 
+// A hidden layer's flipped weights wt[tap][k][n] as TF32 in the same layout (chunks of 4 k).
+__global__ void k_gen_wimage32(const __nv_bfloat16* __restrict__ wt, uint8_t* __restrict__ img) {
+    constexpr int C = kGenC, kBT = (C / 8) * (C / 4) * tc::kCore;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 9 * C * C) return;
+    const int tap = i / (C * C), r = i - tap * C * C, k = r / C, nn = r - k * C;
+    *reinterpret_cast<float*>(img + tap * kBT + ((nn >> 3) * (C / 4) + k / 4) * tc::kCore + (nn & 7) * 16 + (k % 4) * 4) =
+        __bfloat162float(wt[i]);
+}
+
 int refresh_weights(nmmc_gen* g) {
     for (int l = 0; l < kGenLayers; ++l) {
         GenLayer& y = g->layer[l];
@@ -1955,6 +1966,8 @@ int refresh_weights(nmmc_gen* g) {
                                                                                                   y.wimg);
         else
             k_gen_wimage<6, tma::nmma(kGenC)><<<(9 * 48 * 48 + 255) / 256, 256, 0, g->stream>>>(y.wb, y.cin, y.cout, y.wimg);
+        if (l > 0 && l < kGenLayers - 1)
+            k_gen_wimage32<<<(9 * 48 * 48 + 255) / 256, 256, 0, g->stream>>>(y.wt, y.wtimg);
     }
     return cuda_check(cudaGetLastError(), "k_gen_cast");
 }
@@ -2026,7 +2039,7 @@ int backward(nmmc_gen* g, int nb) {
     for (int l = last - 1; l >= 1; --l) {
         if ((rc = wgrad_launch<kGenC, kGenC>(g, g->act[l], cur, y[l].gw, nb))) return rc;
         if ((rc = bgrad_launch(g, cur, npix, kGenC, y[l].gb))) return rc;
-        rc = g->use_tc ? conv_tc_launch<2>(g, cur, y[l].wt, nullptr, g->act[l], nxt, nb)
+        rc = g->use_tc ? conv_tc_launch<2>(g, cur, y[l].wt, nullptr, g->act[l], nxt, nb, y[l].wtimg)
                        : conv_launch<kGenC, kGenC, float, 2>(g, cur, y[l].wt, nullptr, g->act[l], kGenC, nxt, nb);
         if (rc) return rc;
         float* t = cur;
@@ -2047,6 +2060,7 @@ void free_gen(nmmc_gen* g) {
         cudaFree(y.wb);
         cudaFree(y.wt);
         cudaFree(y.wimg);
+        cudaFree(y.wtimg);
         cudaFree(y.gw);
         cudaFree(y.gb);
         cudaFree(y.mw);
@@ -2118,6 +2132,7 @@ int nmmc_gen_create(int L, int capacity, uint64_t seed, nmmc_gen** out) {
         NMMC_GTRY(cudaMalloc(&y.wb, n * sizeof(__nv_bfloat16)));
         NMMC_GTRY(cudaMalloc(&y.wt, n * sizeof(__nv_bfloat16)));
         NMMC_GTRY(cudaMalloc(&y.wimg, kWimgBytes));
+        NMMC_GTRY(cudaMalloc(&y.wtimg, 2 * kWimgBytes));
         NMMC_GTRY(cudaMalloc(&y.gw, n * sizeof(float)));
         NMMC_GTRY(cudaMalloc(&y.gb, y.cout * sizeof(float)));
         NMMC_GTRY(cudaMalloc(&y.mw, n * sizeof(float)));
