@@ -22,7 +22,7 @@
 #include <map>
 #include <vector>
 
-#include "nmmc_internal.h"
+#include "nmmc_kernels.cuh"
 
 namespace nmmc {
 
@@ -55,6 +55,7 @@ struct GenLayer {
     uint8_t* wimg = nullptr;         // BF16 weights in the tensor-core B layout of k_gen_conv_tma
                                      // (kWimgBytes), staged by one bulk copy per CTA
     uint8_t* wtimg = nullptr;        // hidden layers: wt as TF32 in that layout (2 kWimgBytes)
+    int kch = 0;                     // 16-byte chunks of K per tap in wimg
     float* gw = nullptr;
     float* gb = nullptr;
     float* mw = nullptr;
@@ -84,6 +85,7 @@ struct nmmc_gen {
     float* g0 = nullptr;             // gradient ping-pong [b][12][L][L][4] (chunk-planar)
     float* g1 = nullptr;
     float* gv = nullptr;             // [b][L][L][4]
+    float* grads = nullptr;          // every layer's gw and gb, in parameter order
     float* wpart = nullptr;          // weight-gradient partials
     size_t wpart_cap = 0;
     int* d_idx = nullptr;            // snapshot index per batch item
@@ -559,8 +561,8 @@ __host__ __device__ constexpr int smem_bytes() { return 9 * btap<MODE, KCH, CO>(
 // MMAs of output row j read window rows j .. j+2 into accumulator j (R x the TMEM columns),
 // and one commit and one epilogue pass cover the R rows, so the per-tile latency of the copy,
 // the commit and the epilogue is paid once for R rows.
-// With wimg the weights arrive by one bulk copy of their tensor-core image (k_gen_wimage, for the
-// data gradient k_gen_wimage32) instead of being rearranged by the threads.
+// With wimg the weights arrive by one bulk copy of their tensor-core image (k_gen_update) instead
+// of being rearranged by the threads.
 template <int MODE, int ICH, int KCH, int CO, int R>
 __global__ void __launch_bounds__(128, 2)
 k_gen_conv_tma(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_bfloat16* __restrict__ w,
@@ -1489,11 +1491,135 @@ k_gen_wgrad(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout
         }
 }
 
-__global__ void k_gen_sum_parts(const float* __restrict__ part, int nparts, int n, float* __restrict__ out) {
+// The same for the two edge layers (8 -> 48 and 48 -> 4), whose few channels left most threads of
+// that layout without work and one scalar load per multiply-add: kGroups groups of 54 threads
+// take every kGroups-th row of the tile, a thread one tap x 8 input channels x TC output channels
+// with 16-byte loads and packed multiply-adds. Rows of a pixel are padded by 4 floats so that the
+// staging's stores and the loads spread over the banks. 16 x 128^2: 136 -> 62 us and 54 -> 48 us.
+template <int CIN, int COUT>
+struct EdgeGrad {
+    static constexpr int TC = COUT < 8 ? COUT : 8;                 // output channels of a thread
+    static constexpr int CG = CIN / 8, OG = COUT / TC;             // channel groups
+    static constexpr int kThr = 9 * CG * OG, kGroups = 4, kThreads = kThr * kGroups;
+    static constexpr int SI = CIN + (CIN > 8 ? 4 : 0), SO = COUT + (COUT > 8 ? 4 : 0);   // floats per pixel
+    static constexpr int kTin = (kTile + 2) * (kTile + 2) * SI, kTdo = kTile * kTile * SO;
+    static constexpr int kRed = (kGroups - 1) * kThr * (8 * TC + 1);
+    static constexpr size_t smem = (kTin + kTdo > kRed ? kTin + kTdo : kRed) * sizeof(float);
+};
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(EdgeGrad<CIN, COUT>::kThreads, 2)
+k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout, float* __restrict__ part,
+                 int L, int images_per_cta, int nimg) {
+    using E = EdgeGrad<CIN, COUT>;
+    static_assert(CIN % 8 == 0 && COUT % 4 == 0, "16-byte staging");
+    extern __shared__ __align__(16) float gsm[];
+    constexpr int T2 = kTile + 2, TC = E::TC;
+    float* tin = gsm;                // [T2*T2][SI]
+    float* tdo = gsm + E::kTin;      // [kTile*kTile][SO]
+    const int tiles_x = L / kTile;
+    const int tile = blockIdx.x % (tiles_x * tiles_x);
+    const int igrp = blockIdx.x / (tiles_x * tiles_x);
+    const int ty0 = (tile / tiles_x) * kTile, tx0 = (tile % tiles_x) * kTile;
+    const int t = threadIdx.x, grp = t / E::kThr, tg = t - grp * E::kThr;
+    const int tap = tg / (E::CG * E::OG), rr = tg % (E::CG * E::OG), cg = rr / E::OG, og = rr % E::OG;
+    const int dy = tap / 3, dx = tap % 3;
+    f2 acc[8][TC / 2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < TC / 2; ++j) acc[i][j] = f2{0ull};
+    const size_t LL = (size_t)L * L;
+    for (int im = 0; im < images_per_cta; ++im) {
+        const int img = igrp * images_per_cta + im;
+        if (img >= nimg) break;
+        const size_t ibase = (size_t)img * LL;
+        const uint4* isrc = reinterpret_cast<const uint4*>(in + ibase * CIN);
+        const float4* gsrc = reinterpret_cast<const float4*>(dout + ibase * COUT);
+        __syncthreads();
+        // chunk planes of this image; pixel index fastest, so consecutive threads read consecutive pixels
+#pragma unroll 4
+        for (int i = t; i < T2 * T2 * (CIN / 8); i += E::kThreads) {
+            const int c8 = i / (T2 * T2), pix = i - c8 * T2 * T2, yy = pix / T2, xx = pix - yy * T2;
+            int gy = ty0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
+            gy += (gy < 0) ? L : ((gy >= L) ? -L : 0);
+            gx += (gx < 0) ? L : ((gx >= L) ? -L : 0);
+            const uint4 q = __ldg(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
+            float4* d = reinterpret_cast<float4*>(tin + pix * E::SI + c8 * 8);   // a BF16 is an FP32's top half
+            d[0] = make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xFFFF0000u),
+                               __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xFFFF0000u));
+            d[1] = make_float4(__uint_as_float(q.z << 16), __uint_as_float(q.z & 0xFFFF0000u),
+                               __uint_as_float(q.w << 16), __uint_as_float(q.w & 0xFFFF0000u));
+        }
+#pragma unroll 4
+        for (int i = t; i < kTile * kTile * (COUT / 4); i += E::kThreads) {
+            const int c4 = i / (kTile * kTile), pix = i - c4 * kTile * kTile, yy = pix / kTile, xx = pix - yy * kTile;
+            *reinterpret_cast<float4*>(tdo + pix * E::SO + c4 * 4) =
+                __ldg(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
+        }
+        __syncthreads();
+        for (int py = grp; py < kTile; py += E::kGroups) {
+            const float* xi = tin + ((py + dy) * T2 + dx) * E::SI + cg * 8;
+            const float* go = tdo + py * kTile * E::SO + og * TC;
+#pragma unroll 2
+            for (int px = 0; px < kTile; ++px, xi += E::SI, go += E::SO) {
+                const float4 x0 = *reinterpret_cast<const float4*>(xi), x1 = *reinterpret_cast<const float4*>(xi + 4);
+                const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+                f2 gv[TC / 2];
+#pragma unroll
+                for (int j = 0; j < TC / 4; ++j) {
+                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(go + 4 * j);
+                    gv[2 * j].v = q.x;
+                    gv[2 * j + 1].v = q.y;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < TC / 2; ++j) acc[i][j] = fma2(pk(xv[i], xv[i]), gv[j], acc[i][j]);
+            }
+        }
+    }
+    // the groups' sums in order, through shared memory (the tiles are done with)
+    __syncthreads();
+    if (grp > 0) {
+        float* o = gsm + (size_t)((grp - 1) * E::kThr + tg) * (8 * TC + 1);   // odd stride: no bank conflicts
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < TC / 2; ++j) {
+                o[i * TC + 2 * j] = lo(acc[i][j]);
+                o[i * TC + 2 * j + 1] = hi(acc[i][j]);
+            }
+    }
+    __syncthreads();
+    if (grp > 0) return;
+    float* dst = part + (size_t)blockIdx.x * 9 * CIN * COUT;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < TC; ++j) {
+            float v = (j & 1) ? hi(acc[i][j >> 1]) : lo(acc[i][j >> 1]);
+            for (int q = 1; q < E::kGroups; ++q) v += gsm[(size_t)((q - 1) * E::kThr + tg) * (8 * TC + 1) + i * TC + j];
+            dst[(tap * CIN + cg * 8 + i) * COUT + og * TC + j] = v;
+        }
+}
+
+// out[i] = the sum of nparts partials in order, the loads of 16 of them in flight at a time (one
+// at a time, each waited for the last: 13 us for 152 partials of 20736 weights, now 9.6 us).
+__global__ void __launch_bounds__(64)
+k_gen_sum_parts(const float* __restrict__ part, int nparts, int n, float* __restrict__ out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = 0.0f;
-    for (int p = 0; p < nparts; ++p) s += part[(size_t)p * n + i];
+    int p = 0;
+    for (; p + 16 <= nparts; p += 16) {
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = __ldg(part + (size_t)(p + k) * n + i);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s += v[k];
+    }
+    for (; p < nparts; ++p) s += part[(size_t)p * n + i];
     out[i] = s;
 }
 
@@ -1514,63 +1640,91 @@ k_gen_sum_parts_wide(const float* __restrict__ part, int nparts, int n, float* _
     if (t == 0) out[i] = red[0];
 }
 
-// Bias gradient, first stage: block b sums pixels [b*chunk, (b+1)*chunk) of the planar FP32
-// dout (4 channels per 16-byte vector) into part[b][co]. Threads = channel group g x pixel
-// lane; consecutive lanes read consecutive pixels of one group (coalesced 16-byte loads); the
-// lanes are then added in a fixed order. The partials are summed by k_gen_sum_parts_wide.
+// Bias gradient, first stage: a block sums kBgradRun consecutive pixels of one 4-channel plane of
+// one image of the planar FP32 dout (contiguous 16-byte loads, eight in flight per thread) into
+// part[image * segments + segment][co]; lanes and warps are added in a fixed order, the partials
+// by k_gen_sum_parts_wide. 31 -> 10.4 us for 16 x 128^2 x 48 (50 MB): a division per pixel and 21
+// lanes per channel group before.
+constexpr int kBgradRun = 2048;
 __global__ void __launch_bounds__(256)
-k_gen_bgrad_part(const float* __restrict__ dout, int npix, int LL, int cout, int chunk, float* __restrict__ part) {
-    const int G = cout / 4, lanes = blockDim.x / G;
-    const int t = threadIdx.x, g = t / lanes, pl = t - g * lanes;
-    const int p0 = blockIdx.x * chunk, p1 = min(p0 + chunk, npix);
+k_gen_bgrad_part(const float* __restrict__ dout, int LL, int cout, int nseg, float* __restrict__ part) {
+    const int seg = blockIdx.x, g = blockIdx.y, img = blockIdx.z, G = cout / 4;
+    const float4* src = reinterpret_cast<const float4*>(dout) + ((size_t)img * G + g) * LL;
+    const int p0 = seg * kBgradRun, p1 = min(p0 + kBgradRun, LL);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (g < G) {
-#pragma unroll 4
-        for (int p = p0 + pl; p < p1; p += lanes) {
-            const int img = p / LL, pp = p - img * LL;
-            const float4 v = __ldg(reinterpret_cast<const float4*>(dout) + ((size_t)img * G + g) * LL + pp);
-            s.x += v.x;
-            s.y += v.y;
-            s.z += v.z;
-            s.w += v.w;
-        }
+#pragma unroll 8
+    for (int p = p0 + threadIdx.x; p < p1; p += 256) {
+        const float4 v = __ldg(src + p);
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
     }
-    __shared__ float4 red[256];
-    red[t] = s;
+    __shared__ float red[8][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_down_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_down_sync(0xffffffffu, s.y, o);
+        s.z += __shfl_down_sync(0xffffffffu, s.z, o);
+        s.w += __shfl_down_sync(0xffffffffu, s.w, o);
+    }
+    if (lane == 0) {
+        red[warp][0] = s.x;
+        red[warp][1] = s.y;
+        red[warp][2] = s.z;
+        red[warp][3] = s.w;
+    }
     __syncthreads();
-    if (t < cout) {
-        const int gg = t / 4, e = t % 4;
+    if (threadIdx.x < 4) {
         float v = 0.0f;
-        for (int k = 0; k < lanes; ++k) {
-            const float4 r = red[gg * lanes + k];
-            v += e == 0 ? r.x : e == 1 ? r.y : e == 2 ? r.z : r.w;
-        }
-        part[(size_t)blockIdx.x * cout + t] = v;
+        for (int w = 0; w < 8; ++w) v += red[w][threadIdx.x];
+        part[((size_t)img * nseg + seg) * cout + 4 * g + threadIdx.x] = v;
     }
 }
 
-// BF16 copies of the weights: wb[tap][ci][co] and the flipped transpose wt[8-tap][co][ci].
-__global__ void k_gen_cast(const float* __restrict__ w, int cin, int cout, __nv_bfloat16* __restrict__ wb,
-                           __nv_bfloat16* __restrict__ wt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 9 * cin * cout) return;
-    const int tap = i / (cin * cout), r = i - tap * cin * cout, ci = r / cout, co = r - ci * cout;
-    const __nv_bfloat16 v = __float2bfloat16(w[i]);
-    wb[i] = v;
-    wt[((8 - tap) * cout + co) * cin + ci] = v;
-}
+// Weight update and every form of the weights that a pass reads, one launch for all layers (the
+// Adam steps, BF16 copies and operand images were 46 launches of about 3 us): thread i of layer
+// blockIdx.y steps weight i, then the biases (adam != 0), and writes wb[tap][ci][co], the flipped
+// transpose wt[8-tap][co][ci], and where the layer has them its images in the B-operand layout
+// k_gen_conv_tma uses in shared memory: per tap, NN/8 x KCH core matrices of 8 rows (n) x 16 bytes
+// (8 BF16 or 4 TF32 consecutive k); entries past cin and cout stay zero from the allocation.
+struct UpdateArgs {
+    GenLayer layer[kGenLayers];
+    float lr, b1, b2, c1, c2, eps;
+    int adam;
+};
 
-__global__ void k_gen_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                           float* __restrict__ v, int n, float lr, float b1, float b2, float c1, float c2,
-                           float eps) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__device__ __forceinline__ float adam_step(const UpdateArgs& u, float* p, const float* g, float* m, float* v, int i) {
     const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    const float mi = u.b1 * m[i] + (1.0f - u.b1) * gi;
+    const float vi = u.b2 * v[i] + (1.0f - u.b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] -= u.lr * (mi / u.c1) / (sqrtf(vi / u.c2) + u.eps);
+    return p[i];
+}
+
+__global__ void __launch_bounds__(128) k_gen_update(const __grid_constant__ UpdateArgs u) {
+    const GenLayer& y = u.layer[blockIdx.y];
+    const int cin = y.cin, cout = y.cout, n = 9 * cin * cout;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) {
+        if (u.adam && i < n + cout) adam_step(u, y.b, y.gb, y.mb, y.vb, i - n);
+        return;
+    }
+    const float w = u.adam ? adam_step(u, y.w, y.gw, y.mw, y.vw, i) : y.w[i];
+    const int tap = i / (cin * cout), r = i - tap * cin * cout, ci = r / cout, co = r - ci * cout;
+    const __nv_bfloat16 v = __float2bfloat16(w);
+    y.wb[i] = v;
+    y.wt[((8 - tap) * cout + co) * cin + ci] = v;
+    const int kch = y.kch, nn = (cout + 15) / 16 * 16;
+    *reinterpret_cast<__nv_bfloat16*>(y.wimg + tap * (nn / 8) * kch * 128 + ((co >> 3) * kch + ci / 8) * 128 + (co & 7) * 16 +
+                                      (ci % 8) * 2) = v;
+    if (y.wtimg)   // hidden layers: wt's k is co, its n is ci
+        *reinterpret_cast<float*>(y.wtimg + (8 - tap) * (kGenC / 8) * (kGenC / 4) * 128 +
+                                  ((ci >> 3) * (kGenC / 4) + co / 4) * 128 + (ci & 7) * 16 + (co % 4) * 4) =
+            __bfloat162float(v);
 }
 
 // Network input for a batch: y = normalise(sqrt(1 - s^2) x + s g) and the condition channels.
@@ -1633,9 +1787,10 @@ __global__ void k_gen_input(int mode, const __nv_bfloat16* __restrict__ snaps, c
     const float inv = n2 > 0.0f ? rsqrtf(n2) : 0.0f;
     __nv_bfloat16* a = act0 + ((size_t)item * L * L + p) * kGenCin0;
     for (int c = 0; c < 3; ++c) a[c] = __float2bfloat16(y[c] * inv);
-    a[3] = __float2bfloat16(cnd[3 * item] / 1.5f);
-    a[4] = __float2bfloat16(cnd[3 * item + 1]);
-    a[5] = __float2bfloat16(cnd[3 * item + 2] / 0.8f);
+    const float* cd = cnd + 3 * (size_t)(mode == 0 ? idx[item] : item);   // mode 0: the snapshot's own
+    a[3] = __float2bfloat16(cd[0] / 1.5f);
+    a[4] = __float2bfloat16(cd[1]);
+    a[5] = __float2bfloat16(cd[2] / 0.8f);
     a[6] = __float2bfloat16(s);
     a[7] = __float2bfloat16(0.0f);
     if (mode == 0 && target) {
@@ -1894,7 +2049,7 @@ int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, flo
         k_gen_wgrad_tc<2><<<nparts, wg::kThreads, wg::kSmem, g->stream>>>(in, dout, g->wpart, g->L, nkb, g->d_flag);
     else
         k_gen_wgrad_tc<1><<<nparts, wg::kThreads, wg::kSmem, g->stream>>>(in, dout, g->wpart, g->L, nkb, g->d_flag);
-    k_gen_sum_parts<<<(int)((n + 255) / 256), 256, 0, g->stream>>>(g->wpart, nparts, (int)n, gw);
+    k_gen_sum_parts<<<(int)((n + 63) / 64), 64, 0, g->stream>>>(g->wpart, nparts, (int)n, gw);
     return cuda_check(cudaGetLastError(), "k_gen_wgrad_tc");
 }
 
@@ -1908,68 +2063,41 @@ int wgrad_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float*
     const int nparts = tiles * groups;
     const size_t n = (size_t)9 * CIN * COUT;
     if ((size_t)nparts * n > g->wpart_cap) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
-    const size_t smem = (size_t)((kTile + 2) * (kTile + 2) * CIN + kTile * kTile * COUT) * sizeof(float);
-    if (int rc = ensure_smem(g, (const void*)k_gen_wgrad<CIN, COUT>, (int)smem, false)) return rc;
-    k_gen_wgrad<CIN, COUT><<<nparts, 432, smem, g->stream>>>(in, dout, g->wpart, g->L, per, nimg);
-    k_gen_sum_parts<<<(int)((n + 255) / 256), 256, 0, g->stream>>>(g->wpart, nparts, (int)n, gw);
+    if constexpr (CIN == kGenC && COUT == kGenC) {
+        const size_t smem = (size_t)((kTile + 2) * (kTile + 2) * CIN + kTile * kTile * COUT) * sizeof(float);
+        if (int rc = ensure_smem(g, (const void*)k_gen_wgrad<CIN, COUT>, (int)smem, false)) return rc;
+        k_gen_wgrad<CIN, COUT><<<nparts, 432, smem, g->stream>>>(in, dout, g->wpart, g->L, per, nimg);
+    } else {
+        using E = EdgeGrad<CIN, COUT>;
+        if (int rc = ensure_smem(g, (const void*)k_gen_wgrad_edge<CIN, COUT>, (int)E::smem, false)) return rc;
+        k_gen_wgrad_edge<CIN, COUT><<<nparts, E::kThreads, E::smem, g->stream>>>(in, dout, g->wpart, g->L, per, nimg);
+    }
+    k_gen_sum_parts<<<(int)((n + 63) / 64), 64, 0, g->stream>>>(g->wpart, nparts, (int)n, gw);
     return cuda_check(cudaGetLastError(), "k_gen_wgrad");
 }
 
 // Bias gradient gb[co] = sum over the batch's pixels of dout[p, co] (wpart as scratch).
-int bgrad_launch(nmmc_gen* g, const float* dout, int npix, int cout, float* gb) {
-    // about two blocks per SM, chunks a multiple of 64 pixels
-    const int per = (npix + 2 * std::max(1, g->sm_count) - 1) / (2 * std::max(1, g->sm_count));
-    const int chunk = std::max(64, (per + 63) / 64 * 64);
-    const int nblk = (npix + chunk - 1) / chunk;
+int bgrad_launch(nmmc_gen* g, const float* dout, int nimg, int cout, float* gb) {
+    const int LL = g->L * g->L, nseg = (LL + kBgradRun - 1) / kBgradRun;
     if (cout % 4 != 0 || cout > 256) return set_error(NMMC_ERR_ARG, "bias gradient: channels not a multiple of 4");
-    if ((size_t)nblk * cout > g->wpart_cap) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
-    k_gen_bgrad_part<<<nblk, 256, 0, g->stream>>>(dout, npix, g->L * g->L, cout, chunk, g->wpart);
-    k_gen_sum_parts_wide<<<cout, 128, 0, g->stream>>>(g->wpart, nblk, cout, gb);
+    if ((size_t)nimg * nseg * cout > g->wpart_cap) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
+    k_gen_bgrad_part<<<dim3(nseg, cout / 4, nimg), 256, 0, g->stream>>>(dout, LL, cout, nseg, g->wpart);
+    k_gen_sum_parts_wide<<<cout, 128, 0, g->stream>>>(g->wpart, nimg * nseg, cout, gb);
     return cuda_check(cudaGetLastError(), "k_gen_bgrad_part");
 }
 
-// One layer's BF16 weights wb[tap][k][n] in the B-operand layout k_gen_conv_tma uses in shared
-// memory: per tap, NN/8 x KCH core matrices of 8 rows (n) x 16 bytes (8 consecutive k), zeros past
-// cin and cout (KCH chunks of 8 inputs, NN outputs rounded up to 16).
-template <int KCH, int NN>
-__global__ void k_gen_wimage(const __nv_bfloat16* __restrict__ wb, int cin, int cout, uint8_t* __restrict__ img) {
-    constexpr int KK = KCH * 8, kBT = (NN / 8) * KCH * tc::kCore;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 9 * NN * KK) return;
-    const int tap = i / (NN * KK), r = i - tap * NN * KK, nn = r / KK, k = r - nn * KK;
-    const __nv_bfloat16 v = (nn < cout && k < cin) ? wb[(tap * cin + k) * cout + nn] : __float2bfloat16(0.0f);
-    *reinterpret_cast<__nv_bfloat16*>(img + tap * kBT + ((nn >> 3) * KCH + k / 8) * tc::kCore + (nn & 7) * 16 +
-                                      (k % 8) * 2) = v;
-}
-
-// A hidden layer's flipped weights wt[tap][k][n] as TF32 in the same layout (chunks of 4 k).
-__global__ void k_gen_wimage32(const __nv_bfloat16* __restrict__ wt, uint8_t* __restrict__ img) {
-    constexpr int C = kGenC, kBT = (C / 8) * (C / 4) * tc::kCore;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 9 * C * C) return;
-    const int tap = i / (C * C), r = i - tap * C * C, k = r / C, nn = r - k * C;
-    *reinterpret_cast<float*>(img + tap * kBT + ((nn >> 3) * (C / 4) + k / 4) * tc::kCore + (nn & 7) * 16 + (k % 4) * 4) =
-        __bfloat162float(wt[i]);
-}
-
-int refresh_weights(nmmc_gen* g) {
+// The weights' compute forms, after one Adam step where `step` says so.
+int update_weights(nmmc_gen* g, const UpdateArgs* step) {
+    UpdateArgs u{};
+    if (step) u = *step;
+    u.adam = step != nullptr;
+    int most = 0;
     for (int l = 0; l < kGenLayers; ++l) {
-        GenLayer& y = g->layer[l];
-        const int n = (int)y.nw();
-        k_gen_cast<<<(n + 255) / 256, 256, 0, g->stream>>>(y.w, y.cin, y.cout, y.wb, y.wt);
-        // the images of the TMA kernel's layer shapes: first 8 -> 48 (K of two chunks), hidden
-        // 48 -> 48, last 48 -> 4 (N = 16)
-        if (l == 0)
-            k_gen_wimage<2, tma::nmma(kGenC)><<<(9 * 48 * 16 + 255) / 256, 256, 0, g->stream>>>(y.wb, y.cin, y.cout, y.wimg);
-        else if (l == kGenLayers - 1)
-            k_gen_wimage<6, tma::nmma(kGenCout)><<<(9 * 16 * 48 + 255) / 256, 256, 0, g->stream>>>(y.wb, y.cin, y.cout,
-                                                                                                  y.wimg);
-        else
-            k_gen_wimage<6, tma::nmma(kGenC)><<<(9 * 48 * 48 + 255) / 256, 256, 0, g->stream>>>(y.wb, y.cin, y.cout, y.wimg);
-        if (l > 0 && l < kGenLayers - 1)
-            k_gen_wimage32<<<(9 * 48 * 48 + 255) / 256, 256, 0, g->stream>>>(y.wt, y.wtimg);
+        u.layer[l] = g->layer[l];
+        most = std::max(most, (int)g->layer[l].nw() + g->layer[l].cout);
     }
-    return cuda_check(cudaGetLastError(), "k_gen_cast");
+    k_gen_update<<<dim3((most + 127) / 128, kGenLayers), 128, 0, g->stream>>>(u);
+    return cuda_check(cudaGetLastError(), "k_gen_update");
 }
 
 int ensure_batch(nmmc_gen* g, int b) {
@@ -2027,18 +2155,17 @@ int forward(nmmc_gen* g, int nb) {
 int backward(nmmc_gen* g, int nb) {
     int rc;
     GenLayer* y = g->layer;
-    const int npix = nb * g->L * g->L;
     const int last = kGenLayers - 1;
     // last layer: weights and bias, then data gradient into g0 (masked by act[last] > 0)
     if ((rc = wgrad_launch<kGenC, kGenCout>(g, g->act[last], g->gv, y[last].gw, nb))) return rc;
-    if ((rc = bgrad_launch(g, g->gv, npix, kGenCout, y[last].gb))) return rc;
+    if ((rc = bgrad_launch(g, g->gv, nb, kGenCout, y[last].gb))) return rc;
     if ((rc = conv_launch<kGenCout, kGenC, float, 2>(g, g->gv, y[last].wt, nullptr, g->act[last], kGenC, g->g0, nb)))
         return rc;
     float* cur = g->g0;
     float* nxt = g->g1;
     for (int l = last - 1; l >= 1; --l) {
         if ((rc = wgrad_launch<kGenC, kGenC>(g, g->act[l], cur, y[l].gw, nb))) return rc;
-        if ((rc = bgrad_launch(g, cur, npix, kGenC, y[l].gb))) return rc;
+        if ((rc = bgrad_launch(g, cur, nb, kGenC, y[l].gb))) return rc;
         rc = g->use_tc ? conv_tc_launch<2>(g, cur, y[l].wt, nullptr, g->act[l], nxt, nb, y[l].wtimg)
                        : conv_launch<kGenC, kGenC, float, 2>(g, cur, y[l].wt, nullptr, g->act[l], kGenC, nxt, nb);
         if (rc) return rc;
@@ -2047,7 +2174,7 @@ int backward(nmmc_gen* g, int nb) {
         nxt = t;
     }
     if ((rc = wgrad_launch<kGenCin0, kGenC>(g, g->act[0], cur, y[0].gw, nb))) return rc;
-    if ((rc = bgrad_launch(g, cur, npix, kGenC, y[0].gb))) return rc;
+    if ((rc = bgrad_launch(g, cur, nb, kGenC, y[0].gb))) return rc;
     return cuda_check(cudaGetLastError(), "backward");
 }
 
@@ -2061,14 +2188,13 @@ void free_gen(nmmc_gen* g) {
         cudaFree(y.wt);
         cudaFree(y.wimg);
         cudaFree(y.wtimg);
-        cudaFree(y.gw);
-        cudaFree(y.gb);
         cudaFree(y.mw);
         cudaFree(y.vw);
         cudaFree(y.mb);
         cudaFree(y.vb);
         cudaFree(g->act[l]);
     }
+    cudaFree(g->grads);
     cudaFree(g->snaps);
     cudaFree(g->cond);
     cudaFree(g->vout);
@@ -2111,6 +2237,12 @@ int nmmc_gen_create(int L, int capacity, uint64_t seed, nmmc_gen** out) {
         }                                                \
     } while (0)
     NMMC_GTRY(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
+    for (int l = 0; l < kGenLayers; ++l) {
+        g->layer[l].cin = (l == 0) ? kGenCin0 : kGenC;
+        g->layer[l].cout = (l == kGenLayers - 1) ? kGenCout : kGenC;
+    }
+    NMMC_GTRY(cudaMalloc(&g->grads, (size_t)nmmc_gen_param_count(g) * sizeof(float)));
+    size_t goff = 0;
     // He-style initialisation from Philox (host)
     for (int l = 0; l < kGenLayers; ++l) {
         GenLayer& y = g->layer[l];
@@ -2131,10 +2263,13 @@ int nmmc_gen_create(int L, int capacity, uint64_t seed, nmmc_gen** out) {
         NMMC_GTRY(cudaMalloc(&y.b, y.cout * sizeof(float)));
         NMMC_GTRY(cudaMalloc(&y.wb, n * sizeof(__nv_bfloat16)));
         NMMC_GTRY(cudaMalloc(&y.wt, n * sizeof(__nv_bfloat16)));
+        y.kch = l == 0 ? 2 : kGenC / 8;   // the first layer's 8 channels are one chunk of the two of K = 16
         NMMC_GTRY(cudaMalloc(&y.wimg, kWimgBytes));
-        NMMC_GTRY(cudaMalloc(&y.wtimg, 2 * kWimgBytes));
-        NMMC_GTRY(cudaMalloc(&y.gw, n * sizeof(float)));
-        NMMC_GTRY(cudaMalloc(&y.gb, y.cout * sizeof(float)));
+        NMMC_GTRY(cudaMemset(y.wimg, 0, kWimgBytes));
+        if (l > 0 && l < kGenLayers - 1) NMMC_GTRY(cudaMalloc(&y.wtimg, 2 * kWimgBytes));
+        y.gw = g->grads + goff;
+        y.gb = y.gw + n;
+        goff += n + y.cout;
         NMMC_GTRY(cudaMalloc(&y.mw, n * sizeof(float)));
         NMMC_GTRY(cudaMalloc(&y.vw, n * sizeof(float)));
         NMMC_GTRY(cudaMalloc(&y.mb, y.cout * sizeof(float)));
@@ -2160,7 +2295,7 @@ int nmmc_gen_create(int L, int capacity, uint64_t seed, nmmc_gen** out) {
         NMMC_GTRY(cudaDeviceGetAttribute(&g->smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     }
 #undef NMMC_GTRY
-    int rc = refresh_weights(g);
+    int rc = update_weights(g, nullptr);
     if (!rc) rc = cuda_check(cudaStreamSynchronize(g->stream), "nmmc_gen_create");
     if (rc) {
         free_gen(g);
@@ -2208,7 +2343,7 @@ int nmmc_gen_set_params(nmmc_gen* g, const float* in, int n) {
         NMMC_CUDA(cudaMemcpy(y.b, in + o, y.cout * sizeof(float), cudaMemcpyHostToDevice));
         o += y.cout;
     }
-    return refresh_weights(g);
+    return update_weights(g, nullptr);
 }
 
 // Snapshots of 2-D Heisenberg chains of `ctx` (edge == generator L) with their (T, B, D).
@@ -2247,13 +2382,9 @@ int nmmc_gen_train_step(nmmc_gen* g, const int* idx, const float* sig, int nb, f
     if (rc) return rc;
     NMMC_CUDA(cudaMemcpyAsync(g->d_idx, idx, sizeof(int) * nb, cudaMemcpyHostToDevice, g->stream));
     NMMC_CUDA(cudaMemcpyAsync(g->d_sig, sig, sizeof(float) * nb, cudaMemcpyHostToDevice, g->stream));
-    // condition of each item from the dataset's table (device gather by a tiny copy loop)
-    for (int i = 0; i < nb; ++i)
-        NMMC_CUDA(cudaMemcpyAsync(g->d_cnd + 3 * i, g->cond + 3 * (size_t)idx[i], 3 * sizeof(float),
-                                  cudaMemcpyDeviceToDevice, g->stream));
     const int npix = g->L * g->L;
     dim3 gi((npix + 255) / 256, nb);
-    k_gen_input<<<gi, 256, 0, g->stream>>>(0, g->snaps, g->d_idx, nullptr, g->d_sig, g->d_cnd, g->L, (uint32_t)g->seed,
+    k_gen_input<<<gi, 256, 0, g->stream>>>(0, g->snaps, g->d_idx, nullptr, g->d_sig, g->cond, g->L, (uint32_t)g->seed,
                                            (uint32_t)(g->seed >> 32), g->draws, g->act[0], g->target, 1.0f);
     g->draws += (unsigned long long)nb;
     if ((rc = forward(g, nb))) return rc;
@@ -2265,13 +2396,14 @@ int nmmc_gen_train_step(nmmc_gen* g, const int* idx, const float* sig, int nb, f
         g->adam_t++;
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.0f - powf(b1, (float)g->adam_t), c2 = 1.0f - powf(b2, (float)g->adam_t);
-        for (int l = 0; l < kGenLayers; ++l) {
-            GenLayer& y = g->layer[l];
-            const int n = (int)y.nw();
-            k_gen_adam<<<(n + 255) / 256, 256, 0, g->stream>>>(y.w, y.gw, y.mw, y.vw, n, lr, b1, b2, c1, c2, 1e-8f);
-            k_gen_adam<<<1, 64, 0, g->stream>>>(y.b, y.gb, y.mb, y.vb, y.cout, lr, b1, b2, c1, c2, 1e-8f);
-        }
-        if ((rc = refresh_weights(g))) return rc;
+        UpdateArgs u{};
+        u.lr = lr;
+        u.b1 = b1;
+        u.b2 = b2;
+        u.c1 = c1;
+        u.c2 = c2;
+        u.eps = 1e-8f;
+        if ((rc = update_weights(g, &u))) return rc;
     }
     double l = 0;
     NMMC_CUDA(cudaMemcpyAsync(&l, g->d_loss, sizeof(double), cudaMemcpyDeviceToHost, g->stream));
@@ -2285,14 +2417,7 @@ int nmmc_gen_train_step(nmmc_gen* g, const int* idx, const float* sig, int nb, f
 int nmmc_gen_get_grads(nmmc_gen* g, float* out, int n) {
     if (!g || !out || n != nmmc_gen_param_count(g)) return set_error(NMMC_ERR_ARG, "bad parameter buffer");
     NMMC_CUDA(cudaStreamSynchronize(g->stream));
-    size_t o = 0;
-    for (int l = 0; l < kGenLayers; ++l) {
-        GenLayer& y = g->layer[l];
-        NMMC_CUDA(cudaMemcpy(out + o, y.gw, y.nw() * sizeof(float), cudaMemcpyDeviceToHost));
-        o += y.nw();
-        NMMC_CUDA(cudaMemcpy(out + o, y.gb, y.cout * sizeof(float), cudaMemcpyDeviceToHost));
-        o += y.cout;
-    }
+    NMMC_CUDA(cudaMemcpy(out, g->grads, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost));
     return NMMC_OK;
 }
 
