@@ -120,6 +120,7 @@ template <int CIN, int COUT, typename TIN, int EPI>
 __global__ void __launch_bounds__(256)
 k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
            const __nv_bfloat16* __restrict__ mask, int mask_c, void* __restrict__ out, int L) {
+    seq_begin();
     extern __shared__ float gsm[];
     constexpr int HALF = (COUT + 1) / 2;          // output channels per thread
     constexpr int T2 = kTile + 2;
@@ -132,7 +133,7 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
     static_assert((9 * CIN * COUT) % 8 == 0 && (CIN * sizeof(TIN)) % 16 == 0, "16-byte staging");
 #pragma unroll 4
     for (int i = threadIdx.x; i < 9 * CIN * COUT / 8; i += blockDim.x) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(w) + i);
+        const uint4 q = __ldcg(reinterpret_cast<const uint4*>(w) + i);
         const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
 #pragma unroll
         for (int k = 0; k < 8; ++k) wsm[8 * i + k] = __bfloat162float(e[k]);
@@ -146,7 +147,7 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
         int gy = ty0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
         gy += (gy < 0) ? L : ((gy >= L) ? -L : 0);
         gx += (gx < 0) ? L : ((gx >= L) ? -L : 0);
-        const uint4 q = __ldg(src + (size_t)v * LL + (size_t)gy * L + gx);
+        const uint4 q = __ldcg(src + (size_t)v * LL + (size_t)gy * L + gx);
         const TIN* e = reinterpret_cast<const TIN*>(&q);
 #pragma unroll
         for (int k = 0; k < EPV; ++k) tsm[((v * EPV + k) * T2 + yy) * T2 + xx] = (float)e[k];
@@ -155,13 +156,12 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
     const int pair = threadIdx.x & 127, half = threadIdx.x >> 7;
     const int px = pair & 15, py = pair >> 4;      // rows py and py + 8
     const int co0 = half * HALF;
-    float a0[HALF], a1[HALF];
+    static_assert(HALF % 2 == 0 && COUT == 2 * HALF, "channel pairs");
+    f2 a0[HALF / 2], a1[HALF / 2];   // channel pairs: packed multiply-adds
 #pragma unroll
-    for (int k = 0; k < HALF; ++k) {
-        const int co = co0 + k;
-        const float bv = (bias && co < COUT) ? bias[co] : 0.0f;
-        a0[k] = bv;
-        a1[k] = bv;
+    for (int k = 0; k < HALF / 2; ++k) {
+        a0[k] = bias ? pk(__ldcg(bias + co0 + 2 * k), __ldcg(bias + co0 + 2 * k + 1)) : f2{0ull};
+        a1[k] = a0[k];
     }
 #pragma unroll 1
     for (int tap = 0; tap < 9; ++tap) {
@@ -170,13 +170,13 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
         for (int ci = 0; ci < CIN; ++ci) {
             const float x0 = tsm[(ci * T2 + py + dy) * T2 + px + dx];
             const float x1 = tsm[(ci * T2 + py + 8 + dy) * T2 + px + dx];
+            const f2 p0 = pk(x0, x0), p1 = pk(x1, x1);
             const float* wr = wsm + (tap * CIN + ci) * COUT + co0;
 #pragma unroll
-            for (int k = 0; k < HALF; ++k) {
-                if (co0 + k < COUT) {
-                    a0[k] = fmaf(x0, wr[k], a0[k]);
-                    a1[k] = fmaf(x1, wr[k], a1[k]);
-                }
+            for (int k = 0; k < HALF / 2; ++k) {
+                const f2 wv{*reinterpret_cast<const unsigned long long*>(wr + 2 * k)};
+                a0[k] = fma2(p0, wv, a0[k]);
+                a1[k] = fma2(p1, wv, a1[k]);
             }
         }
     }
@@ -184,19 +184,38 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
     for (int r = 0; r < 2; ++r) {
         const int y = ty0 + py + 8 * r, x = tx0 + px;
         const size_t pp = (size_t)y * L + x;
-        const float* a = r ? a1 : a0;
+        float v[HALF];
+#pragma unroll
+        for (int k = 0; k < HALF / 2; ++k) {
+            v[2 * k] = lo(r ? a1[k] : a0[k]);
+            v[2 * k + 1] = hi(r ? a1[k] : a0[k]);
+        }
+        if constexpr (EPI == 2 && HALF % 8 == 0) {   // whole 16-byte chunks
+#pragma unroll
+            for (int c = 0; c < HALF / 8; ++c) {
+                const uint4 m4 = __ldcg(reinterpret_cast<const uint4*>(
+                    mask + pl_off<__nv_bfloat16>(mask_c, LL, img, pp, co0 + 8 * c)));
+                const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&m4);
+                float o[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) o[k] = __bfloat162float(mh[k]) > 0.0f ? v[8 * c + k] : 0.0f;
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    *reinterpret_cast<float4*>((float*)out + pl_off<float>(COUT, LL, img, pp, co0 + 8 * c + 4 * q)) =
+                        make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+            }
+            continue;
+        }
 #pragma unroll
         for (int k = 0; k < HALF; ++k) {
             const int co = co0 + k;
-            if (co >= COUT) continue;
-            float v = a[k];
             if (EPI == 0) {
-                ((__nv_bfloat16*)out)[pl_off<__nv_bfloat16>(COUT, LL, img, pp, co)] = __float2bfloat16(fmaxf(v, 0.0f));
+                ((__nv_bfloat16*)out)[pl_off<__nv_bfloat16>(COUT, LL, img, pp, co)] = __float2bfloat16(fmaxf(v[k], 0.0f));
             } else if (EPI == 1) {
-                ((float*)out)[pl_off<float>(COUT, LL, img, pp, co)] = v;
+                ((float*)out)[pl_off<float>(COUT, LL, img, pp, co)] = v[k];
             } else {
                 const float mk = __bfloat162float(mask[pl_off<__nv_bfloat16>(mask_c, LL, img, pp, co)]);
-                ((float*)out)[pl_off<float>(COUT, LL, img, pp, co)] = mk > 0.0f ? v : 0.0f;
+                ((float*)out)[pl_off<float>(COUT, LL, img, pp, co)] = mk > 0.0f ? v[k] : 0.0f;
             }
         }
     }
@@ -306,7 +325,7 @@ __device__ __forceinline__ void stage_weights(uint8_t* sB, const __nv_bfloat16* 
     constexpr int kC = tc::kC, kG = 9 * kC * kC / 8;
 #pragma unroll 7
     for (int g8 = tid; g8 < kG; g8 += nthr) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(w) + g8);
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(w) + g8);
         const int i = g8 * 8;
         const int tap = i / (kC * kC), r = i - tap * kC * kC, k = r / kC, n = r - k * kC;
         uint8_t* base = sB + tap * kBT + ((n >> 3) * kCh + k / kEpc) * tc::kCore + (k % kEpc) * (int)sizeof(TA);
@@ -346,10 +365,12 @@ __device__ __forceinline__ void conv_store(const float* v, const float* sbias, v
     } else {
         const uint4* mk = reinterpret_cast<const uint4*>(mask + img * LL * kC) + pp;
         float4* dst = reinterpret_cast<float4*>((float*)out_v + img * LL * kC) + pp;
+        uint4 m4[kC / 8];   // all loads before the first store, which they could not pass
+#pragma unroll
+        for (int c = 0; c < kC / 8; ++c) m4[c] = __ldcg(mk + (size_t)c * LL);
 #pragma unroll
         for (int c = 0; c < kC / 8; ++c) {
-            const uint4 m4 = __ldg(mk + (size_t)c * LL);
-            const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&m4);
+            const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&m4[c]);
             float o[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) o[k] = (__bfloat162float(mh[k]) > 0.0f) ? v[8 * c + k] : 0.0f;
@@ -384,6 +405,7 @@ __global__ void __launch_bounds__(128, 2)
 k_gen_conv_tc(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_bfloat16* __restrict__ w,
               const float* __restrict__ bias, const __nv_bfloat16* __restrict__ mask, void* __restrict__ out_v,
               int L, int tiles_per_img, int ntiles, int* __restrict__ flag) {
+    seq_begin();
     using namespace tc;
     using TA = typename Traits<MODE>::TA;
     constexpr int kCh = chunks<MODE>();
@@ -402,7 +424,7 @@ k_gen_conv_tc(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_b
 
     // weights w[tap][k][n] (k: input channel of this convolution) -> B_tap[n][k], K-major
     stage_weights<MODE>(sB, w, tid, blockDim.x);
-    if (tid < kC) sbias[tid] = (MODE == 2) ? 0.0f : bias[tid];
+    if (tid < kC) sbias[tid] = (MODE == 2) ? 0.0f : __ldcg(bias + tid);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gen_smem_u32(&tmem_slot)),
                      "r"(kTmemCols)
@@ -569,6 +591,7 @@ k_gen_conv_tma(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_
                const uint8_t* __restrict__ wimg, const float* __restrict__ bias,
                const __nv_bfloat16* __restrict__ mask, void* __restrict__ out_v, int ntiles,
                int* __restrict__ flag) {
+    seq_begin();
     using namespace tc;
     using TA = typename Traits<MODE>::TA;
     constexpr int kEpc = Traits<MODE>::kEpc;
@@ -649,12 +672,12 @@ k_gen_conv_tma(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_
 #pragma unroll 8
         for (int i = tid; i < 9 * NN * KK; i += blockDim.x) {
             const int tap = i / (NN * KK), r = i - tap * NN * KK, nn = r / KK, k = r - nn * KK;
-            const float v = (nn < CO && k < CI) ? __bfloat162float(__ldg(w + (tap * CI + k) * CO + nn)) : 0.0f;
+            const float v = (nn < CO && k < CI) ? __bfloat162float(__ldcg(w + (tap * CI + k) * CO + nn)) : 0.0f;
             *(TA*)(sB + tap * kBT + ((nn >> 3) * KCH + k / kEpc) * kCore + (nn & 7) * 16 + (k % kEpc) * (int)sizeof(TA)) =
                 (TA)v;
         }
     }
-    if (tid < NN) sbias[tid] = (MODE == 2 || tid >= CO) ? 0.0f : bias[tid];
+    if (tid < NN) sbias[tid] = (MODE == 2 || tid >= CO) ? 0.0f : __ldcg(bias + tid);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gen_smem_u32(&tmem_slot)),
                      "r"(R * kCols)
@@ -1214,6 +1237,7 @@ template <int KS>   // MMA K-steps (16 positions) per K-block: W = 16 KS
 __global__ void __launch_bounds__(wg::kThreads, 1)
 k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout, float* __restrict__ part,
                int L, int nkb, int* __restrict__ flag) {
+    seq_begin();
     using namespace wg;
     constexpr int kC = tc::kC, W = 16 * KS;
     extern __shared__ uint8_t wsm_raw[];
@@ -1415,6 +1439,7 @@ template <int CIN, int COUT>
 __global__ void __launch_bounds__(432)
 k_gen_wgrad(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout, float* __restrict__ part,
             int L, int images_per_cta, int nimg) {
+    seq_begin();
     extern __shared__ float gsm[];
     constexpr int T2 = kTile + 2;
     constexpr int CG = (CIN + 5) / 6, OG = (COUT + 7) / 8;
@@ -1450,7 +1475,7 @@ k_gen_wgrad(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout
             int gy = ty0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
             gy += (gy < 0) ? L : ((gy >= L) ? -L : 0);
             gx += (gx < 0) ? L : ((gx >= L) ? -L : 0);
-            const uint4 q = __ldg(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
+            const uint4 q = __ldcg(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
             const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
             float* d = tin + pix * CIN + c8 * 8;
 #pragma unroll
@@ -1460,7 +1485,7 @@ k_gen_wgrad(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout
         for (int i = threadIdx.x; i < kTile * kTile * (COUT / 4); i += blockDim.x) {
             const int c4 = i / (kTile * kTile), pix = i - c4 * kTile * kTile, yy = pix / kTile, xx = pix - yy * kTile;
             reinterpret_cast<float4*>(tdo + pix * COUT)[c4] =
-                __ldg(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
+                __ldcg(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
         }
         __syncthreads();
         if (active) {
@@ -1511,6 +1536,7 @@ template <int CIN, int COUT>
 __global__ void __launch_bounds__(EdgeGrad<CIN, COUT>::kThreads, 2)
 k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout, float* __restrict__ part,
                  int L, int images_per_cta, int nimg) {
+    seq_begin();
     using E = EdgeGrad<CIN, COUT>;
     static_assert(CIN % 8 == 0 && COUT % 4 == 0, "16-byte staging");
     extern __shared__ __align__(16) float gsm[];
@@ -1544,7 +1570,7 @@ k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__
             int gy = ty0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
             gy += (gy < 0) ? L : ((gy >= L) ? -L : 0);
             gx += (gx < 0) ? L : ((gx >= L) ? -L : 0);
-            const uint4 q = __ldg(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
+            const uint4 q = __ldcg(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
             float4* d = reinterpret_cast<float4*>(tin + pix * E::SI + c8 * 8);   // a BF16 is an FP32's top half
             d[0] = make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xFFFF0000u),
                                __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xFFFF0000u));
@@ -1555,7 +1581,7 @@ k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__
         for (int i = t; i < kTile * kTile * (COUT / 4); i += E::kThreads) {
             const int c4 = i / (kTile * kTile), pix = i - c4 * kTile * kTile, yy = pix / kTile, xx = pix - yy * kTile;
             *reinterpret_cast<float4*>(tdo + pix * E::SO + c4 * 4) =
-                __ldg(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
+                __ldcg(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
         }
         __syncthreads();
         for (int py = grp; py < kTile; py += E::kGroups) {
@@ -1608,6 +1634,7 @@ k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__
 // at a time, each waited for the last: 13 us for 152 partials of 20736 weights, now 9.6 us).
 __global__ void __launch_bounds__(64)
 k_gen_sum_parts(const float* __restrict__ part, int nparts, int n, float* __restrict__ out) {
+    seq_begin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = 0.0f;
@@ -1615,11 +1642,11 @@ k_gen_sum_parts(const float* __restrict__ part, int nparts, int n, float* __rest
     for (; p + 16 <= nparts; p += 16) {
         float v[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = __ldg(part + (size_t)(p + k) * n + i);
+        for (int k = 0; k < 16; ++k) v[k] = __ldcg(part + (size_t)(p + k) * n + i);
 #pragma unroll
         for (int k = 0; k < 16; ++k) s += v[k];
     }
-    for (; p < nparts; ++p) s += part[(size_t)p * n + i];
+    for (; p < nparts; ++p) s += __ldcg(part + (size_t)p * n + i);
     out[i] = s;
 }
 
@@ -1627,10 +1654,11 @@ k_gen_sum_parts(const float* __restrict__ part, int nparts, int n, float* __rest
 // t, t + 128, ..., then a fixed-order tree (the same result on every run).
 __global__ void __launch_bounds__(128)
 k_gen_sum_parts_wide(const float* __restrict__ part, int nparts, int n, float* __restrict__ out) {
+    seq_begin();
     __shared__ float red[128];
     const int i = blockIdx.x, t = threadIdx.x;
     float s = 0.0f;
-    for (int p = t; p < nparts; p += 128) s += part[(size_t)p * n + i];
+    for (int p = t; p < nparts; p += 128) s += __ldcg(part + (size_t)p * n + i);
     red[t] = s;
     __syncthreads();
     for (int h = 64; h > 0; h >>= 1) {
@@ -1648,13 +1676,14 @@ k_gen_sum_parts_wide(const float* __restrict__ part, int nparts, int n, float* _
 constexpr int kBgradRun = 2048;
 __global__ void __launch_bounds__(256)
 k_gen_bgrad_part(const float* __restrict__ dout, int LL, int cout, int nseg, float* __restrict__ part) {
+    seq_begin();
     const int seg = blockIdx.x, g = blockIdx.y, img = blockIdx.z, G = cout / 4;
     const float4* src = reinterpret_cast<const float4*>(dout) + ((size_t)img * G + g) * LL;
     const int p0 = seg * kBgradRun, p1 = min(p0 + kBgradRun, LL);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int p = p0 + threadIdx.x; p < p1; p += 256) {
-        const float4 v = __ldg(src + p);
+        const float4 v = __ldcg(src + p);
         s.x += v.x;
         s.y += v.y;
         s.z += v.z;
@@ -1706,6 +1735,7 @@ __device__ __forceinline__ float adam_step(const UpdateArgs& u, float* p, const 
 }
 
 __global__ void __launch_bounds__(128) k_gen_update(const __grid_constant__ UpdateArgs u) {
+    seq_begin();
     const GenLayer& y = u.layer[blockIdx.y];
     const int cin = y.cin, cout = y.cout, n = 9 * cin * cout;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1740,6 +1770,7 @@ __global__ void k_gen_input(int mode, const __nv_bfloat16* __restrict__ snaps, c
                             const float* __restrict__ cnd, int L, uint32_t k0, uint32_t k1,
                             unsigned long long draw0, __nv_bfloat16* __restrict__ act0,
                             float* __restrict__ target, float s_prev) {
+    seq_begin();
     const int item = blockIdx.y;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= L * L) return;
@@ -1748,8 +1779,10 @@ __global__ void k_gen_input(int mode, const __nv_bfloat16* __restrict__ snaps, c
         const __nv_bfloat16* s = snaps + ((size_t)idx[item] * L * L + p) * 3;
         for (int c = 0; c < 3; ++c) x[c] = __bfloat162float(s[c]);
     } else {
-        const float* s = cur + ((size_t)item * L * L + p) * kGenCout;
-        for (int c = 0; c < 3; ++c) x[c] = s[c];
+        const float4 e = __ldcg(reinterpret_cast<const float4*>(cur) + (size_t)item * L * L + p);
+        x[0] = e.x;
+        x[1] = e.y;
+        x[2] = e.z;
     }
     const float s = sig[item];
     const unsigned long long d = draw0 + (unsigned long long)item;
@@ -1804,13 +1837,16 @@ __global__ void k_gen_input(int mode, const __nv_bfloat16* __restrict__ snaps, c
 
 // Loss and its gradient through spin = v/|v|: loss += |s - x|^2 / npix_total;
 // dL/dv = (g - s (s.g)) / |v| with g = 2 (s - x) / npix_total.
-__global__ void k_gen_head(const float* __restrict__ v, const float* __restrict__ target, int npix, float scale,
-                           float* __restrict__ gv, double* __restrict__ loss) {
+__global__ void __launch_bounds__(256)
+k_gen_head(const float* __restrict__ v, const float* __restrict__ target, int npix, float scale,
+           float* __restrict__ gv, double* __restrict__ loss) {
+    seq_begin();
+    __shared__ float red[8];
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     float l = 0.0f;
     if (p < npix) {
-        const float* a = v + (size_t)p * kGenCout;
-        const float* x = target + (size_t)p * kGenCout;
+        const float4 a4 = __ldcg(reinterpret_cast<const float4*>(v) + p), x4 = __ldcg(reinterpret_cast<const float4*>(target) + p);
+        const float a[3] = {a4.x, a4.y, a4.z}, x[3] = {x4.x, x4.y, x4.z};
         const float n2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + 1e-12f;
         const float inv = rsqrtf(n2);
         float s[3], g[3], sg = 0.0f;
@@ -1821,26 +1857,29 @@ __global__ void k_gen_head(const float* __restrict__ v, const float* __restrict_
             g[c] = 2.0f * d * scale;
             sg += s[c] * g[c];
         }
-        float* o = gv + (size_t)p * kGenCout;
-        for (int c = 0; c < 3; ++c) o[c] = (g[c] - s[c] * sg) * inv;
-        o[3] = 0.0f;
+        reinterpret_cast<float4*>(gv)[p] =
+            make_float4((g[0] - s[0] * sg) * inv, (g[1] - s[1] * sg) * inv, (g[2] - s[2] * sg) * inv, 0.0f);
     }
+    // one FP64 addition per block of 256 pixels (one per warp took 15 us for 16 x 128^2)
     for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, (double)(l * scale));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += (double)(red[w] * scale);
+        atomicAdd(loss, t);
+    }
 }
 
 // Sampling: cur <- normalise(v) (the denoised estimate)
 __global__ void k_gen_normalise(const float* __restrict__ v, int npix, float* __restrict__ cur) {
+    seq_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npix) return;
-    const float* a = v + (size_t)p * kGenCout;
-    const float n2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(v) + p);
+    const float n2 = a.x * a.x + a.y * a.y + a.z * a.z;
     const float inv = n2 > 0.0f ? rsqrtf(n2) : 0.0f;
-    float* o = cur + (size_t)p * kGenCout;
-    o[0] = a[0] * inv;
-    o[1] = a[1] * inv;
-    o[2] = a[2] * inv;
-    o[3] = 0.0f;
+    reinterpret_cast<float4*>(cur)[p] = make_float4(a.x * inv, a.y * inv, a.z * inv, 0.0f);
 }
 
 // Sampler chain (split-colour FP32 planes, 2-D) <-> NHWC
@@ -1898,7 +1937,7 @@ int conv_launch(nmmc_gen* g, const TIN* in, const __nv_bfloat16* w, const float*
     const size_t smem = (size_t)(9 * CIN * COUT + CIN * (kTile + 2) * (kTile + 2)) * sizeof(float);
     if (int rc = ensure_smem(g, (const void*)k_gen_conv<CIN, COUT, TIN, EPI>, (int)smem, false)) return rc;
     dim3 grid(g->L / kTile, g->L / kTile, nimg);
-    k_gen_conv<CIN, COUT, TIN, EPI><<<grid, 256, smem, g->stream>>>(in, w, bias, mask, mask_c, out, g->L);
+    launch_seq(g->stream, k_gen_conv<CIN, COUT, TIN, EPI>, dim3(grid), 256, smem, in, w, bias, mask, mask_c, out, g->L);
     return cuda_check(cudaGetLastError(), "k_gen_conv");
 }
 
@@ -1952,7 +1991,7 @@ int conv_tma_launch_r(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, cons
     const int per_sm = std::max(1, std::min(2, g->smem_per_sm / (smem + 2048)));
     const int ntiles = nimg * g->L / R;
     const int grid = std::min(ntiles, per_sm * g->sm_count);
-    k_gen_conv_tma<MODE, ICH, KCH, CO, R><<<grid, 128, smem, g->stream>>>(in, w, wimg, bias, mask, out, ntiles,
+    launch_seq(g->stream, k_gen_conv_tma<MODE, ICH, KCH, CO, R>, dim3(grid), 128, smem, in, w, wimg, bias, mask, out, ntiles,
                                                                           g->d_flag);
     return cuda_check(cudaGetLastError(), "k_gen_conv_tma");
 }
@@ -2016,7 +2055,7 @@ int conv_tc_launch(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const _
     const int tiles_per_img = (g->L * (g->L + 2) + tc::kM - 1) / tc::kM;   // padded rows 1..L
     const int ntiles = nimg * tiles_per_img;
     const int grid = std::min(ntiles, per_sm * g->sm_count);
-    k_gen_conv_tc<MODE><<<grid, 128, smem, g->stream>>>(in, w, bias, mask, out, g->L, tiles_per_img, ntiles, g->d_flag);
+    launch_seq(g->stream, k_gen_conv_tc<MODE>, dim3(grid), 128, smem, in, w, bias, mask, out, g->L, tiles_per_img, ntiles, g->d_flag);
     return cuda_check(cudaGetLastError(), "k_gen_conv_tc");
 }
 
@@ -2042,14 +2081,14 @@ int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, flo
                    : W == 32 ? (const void*)k_gen_wgrad_tc<2> : (const void*)k_gen_wgrad_tc<1>;
     if (int rc = ensure_smem(g, fn, (int)wg::kSmem, true)) return rc;
     if (W == 64)
-        k_gen_wgrad_tc<4><<<nparts, wg::kThreads, wg::kSmem, g->stream>>>(in, dout, g->wpart, g->L, nkb, g->d_flag);
+        launch_seq(g->stream, k_gen_wgrad_tc<4>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
     else if (W == 48)
-        k_gen_wgrad_tc<3><<<nparts, wg::kThreads, wg::kSmem, g->stream>>>(in, dout, g->wpart, g->L, nkb, g->d_flag);
+        launch_seq(g->stream, k_gen_wgrad_tc<3>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
     else if (W == 32)
-        k_gen_wgrad_tc<2><<<nparts, wg::kThreads, wg::kSmem, g->stream>>>(in, dout, g->wpart, g->L, nkb, g->d_flag);
+        launch_seq(g->stream, k_gen_wgrad_tc<2>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
     else
-        k_gen_wgrad_tc<1><<<nparts, wg::kThreads, wg::kSmem, g->stream>>>(in, dout, g->wpart, g->L, nkb, g->d_flag);
-    k_gen_sum_parts<<<(int)((n + 63) / 64), 64, 0, g->stream>>>(g->wpart, nparts, (int)n, gw);
+        launch_seq(g->stream, k_gen_wgrad_tc<1>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
+    launch_seq(g->stream, k_gen_sum_parts, dim3((int)((n + 63) / 64)), 64, 0, g->wpart, nparts, (int)n, gw);
     return cuda_check(cudaGetLastError(), "k_gen_wgrad_tc");
 }
 
@@ -2066,13 +2105,13 @@ int wgrad_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float*
     if constexpr (CIN == kGenC && COUT == kGenC) {
         const size_t smem = (size_t)((kTile + 2) * (kTile + 2) * CIN + kTile * kTile * COUT) * sizeof(float);
         if (int rc = ensure_smem(g, (const void*)k_gen_wgrad<CIN, COUT>, (int)smem, false)) return rc;
-        k_gen_wgrad<CIN, COUT><<<nparts, 432, smem, g->stream>>>(in, dout, g->wpart, g->L, per, nimg);
+        launch_seq(g->stream, k_gen_wgrad<CIN, COUT>, dim3(nparts), 432, smem, in, dout, g->wpart, g->L, per, nimg);
     } else {
         using E = EdgeGrad<CIN, COUT>;
         if (int rc = ensure_smem(g, (const void*)k_gen_wgrad_edge<CIN, COUT>, (int)E::smem, false)) return rc;
-        k_gen_wgrad_edge<CIN, COUT><<<nparts, E::kThreads, E::smem, g->stream>>>(in, dout, g->wpart, g->L, per, nimg);
+        launch_seq(g->stream, k_gen_wgrad_edge<CIN, COUT>, dim3(nparts), E::kThreads, E::smem, in, dout, g->wpart, g->L, per, nimg);
     }
-    k_gen_sum_parts<<<(int)((n + 63) / 64), 64, 0, g->stream>>>(g->wpart, nparts, (int)n, gw);
+    launch_seq(g->stream, k_gen_sum_parts, dim3((int)((n + 63) / 64)), 64, 0, g->wpart, nparts, (int)n, gw);
     return cuda_check(cudaGetLastError(), "k_gen_wgrad");
 }
 
@@ -2081,8 +2120,8 @@ int bgrad_launch(nmmc_gen* g, const float* dout, int nimg, int cout, float* gb) 
     const int LL = g->L * g->L, nseg = (LL + kBgradRun - 1) / kBgradRun;
     if (cout % 4 != 0 || cout > 256) return set_error(NMMC_ERR_ARG, "bias gradient: channels not a multiple of 4");
     if ((size_t)nimg * nseg * cout > g->wpart_cap) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
-    k_gen_bgrad_part<<<dim3(nseg, cout / 4, nimg), 256, 0, g->stream>>>(dout, LL, cout, nseg, g->wpart);
-    k_gen_sum_parts_wide<<<cout, 128, 0, g->stream>>>(g->wpart, nimg * nseg, cout, gb);
+    launch_seq(g->stream, k_gen_bgrad_part, dim3(nseg, cout / 4, nimg), 256, 0, dout, LL, cout, nseg, g->wpart);
+    launch_seq(g->stream, k_gen_sum_parts_wide, dim3(cout), 128, 0, g->wpart, nimg * nseg, cout, gb);
     return cuda_check(cudaGetLastError(), "k_gen_bgrad_part");
 }
 
@@ -2096,7 +2135,7 @@ int update_weights(nmmc_gen* g, const UpdateArgs* step) {
         u.layer[l] = g->layer[l];
         most = std::max(most, (int)g->layer[l].nw() + g->layer[l].cout);
     }
-    k_gen_update<<<dim3((most + 127) / 128, kGenLayers), 128, 0, g->stream>>>(u);
+    launch_seq(g->stream, k_gen_update, dim3((most + 127) / 128, kGenLayers), 128, 0, u);
     return cuda_check(cudaGetLastError(), "k_gen_update");
 }
 
@@ -2384,13 +2423,13 @@ int nmmc_gen_train_step(nmmc_gen* g, const int* idx, const float* sig, int nb, f
     NMMC_CUDA(cudaMemcpyAsync(g->d_sig, sig, sizeof(float) * nb, cudaMemcpyHostToDevice, g->stream));
     const int npix = g->L * g->L;
     dim3 gi((npix + 255) / 256, nb);
-    k_gen_input<<<gi, 256, 0, g->stream>>>(0, g->snaps, g->d_idx, nullptr, g->d_sig, g->cond, g->L, (uint32_t)g->seed,
+    launch_seq(g->stream, k_gen_input, dim3(gi), 256, 0, 0, g->snaps, g->d_idx, nullptr, g->d_sig, g->cond, g->L, (uint32_t)g->seed,
                                            (uint32_t)(g->seed >> 32), g->draws, g->act[0], g->target, 1.0f);
     g->draws += (unsigned long long)nb;
     if ((rc = forward(g, nb))) return rc;
     NMMC_CUDA(cudaMemsetAsync(g->d_loss, 0, sizeof(double), g->stream));
     const int np = nb * npix;
-    k_gen_head<<<(np + 255) / 256, 256, 0, g->stream>>>(g->vout, g->target, np, 1.0f / (float)np, g->gv, g->d_loss);
+    launch_seq(g->stream, k_gen_head, dim3((np + 255) / 256), 256, 0, g->vout, g->target, np, 1.0f / (float)np, g->gv, g->d_loss);
     if ((rc = backward(g, nb))) return rc;
     if (lr > 0) {
         g->adam_t++;
@@ -2473,14 +2512,14 @@ int nmmc_gen_warm_start(nmmc_gen* g, nmmc_ctx* c, const int* chains, int n, cons
     float s_prev = 1.0f;
     for (int k = 0; k < steps; ++k) {
         const float s = sched(k);
-        k_gen_input<<<gi, 256, 0, g->stream>>>(reuse_noise == 2 ? 3 : (reuse_noise ? 2 : 1), nullptr, nullptr, cur,
+        launch_seq(g->stream, k_gen_input, dim3(gi), 256, 0, reuse_noise == 2 ? 3 : (reuse_noise ? 2 : 1), nullptr, nullptr, cur,
                                                d_sigs + (size_t)k * n, g->d_cnd, g->L,
                                                (uint32_t)g->seed, (uint32_t)(g->seed >> 32), g->draws, g->act[0],
                                                nullptr, k == 0 ? 1.0f : s_prev);
         s_prev = s;
         g->draws += (unsigned long long)n;
         if ((rc = forward(g, n))) return rc;
-        k_gen_normalise<<<(n * npix + 255) / 256, 256, 0, g->stream>>>(g->vout, n * npix, cur);
+        launch_seq(g->stream, k_gen_normalise, dim3((n * npix + 255) / 256), 256, 0, g->vout, n * npix, cur);
     }
     int* d_ch = nullptr;
     NMMC_CUDA(ds.alloc(&d_ch, sizeof(int) * n));

@@ -256,7 +256,7 @@ struct DeviceScratch {
 // Half-sweeps follow one another 20 to 160 times per call; a plain launch leaves 2-3 us between
 // them (24 Ising chains of 64^3: 13.9 us kernels, 18 us apart).
 template <class... P, class... A>
-void launch_seq(Ctx& c, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, A... args) {
+void launch_seq(cudaStream_t stream, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, A... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -264,10 +264,14 @@ void launch_seq(Ctx& c, void (*kernel)(P...), dim3 grid, unsigned block, size_t 
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = c.stream;
+    cfg.stream = stream;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // errors: the caller's cudaGetLastError
+}
+template <class... P, class... A>
+void launch_seq(Ctx& c, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, A... args) {
+    launch_seq(c.stream, kernel, grid, block, smem, args...);
 }
 #define NMMC_CUDA(call)                                         \
     do {                                                        \
