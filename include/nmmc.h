@@ -442,16 +442,15 @@ int nmmc_gen_gated_warm_start(nmmc_gen* gen, nmmc_ctx* ctx, const int* chains, i
 /* Generator options. NMMC_GEN_OPT_TENSOR_CORES: 1 (default) runs the six 48-channel hidden
  * convolutions on the tensor cores (tcgen05.mma, FP32 accumulation in tensor memory; forward
  * in BF16, data gradient in TF32, weight gradient with the FP32 output gradient as BF16 hi + lo
- * operands), with the input windows staged by TMA at L = 128 and by cp.async otherwise. 2: warp-specialised forward with cp.async-staged windows; 3: cp.async
- * staging at every L; 4: at L = 128 a warp-specialised forward (producer, MMA and epilogue
- * warps over a ring of TMA-staged windows); 0: the FP32 FMA pipes. The tensor-core variants
- * give identical results. */
+ * operands), at L = 128 with the input rows passing once through a ring of bulk-copied rows and
+ * by cp.async-staged windows otherwise. 2: warp-specialised forward with cp.async-staged windows;
+ * 3: cp.async staging at every L; 4: the same as 1; 0: the FP32 FMA pipes. The tensor-core
+ * variants give identical results. */
 #define NMMC_GEN_OPT_TENSOR_CORES 1
-/* NMMC_GEN_OPT_TILE_ROWS: output rows per tile of the TMA-staged forward convolutions at
- * L = 128, 2 (default: one window of four input rows, one commit and one epilogue pass per
- * two rows) or 1; the same results. */
+/* NMMC_GEN_OPT_TILE_ROWS: 1 or 2 (default), accepted for existing callers: the convolutions at
+ * L = 128 take one output row per tile in either case. */
 #define NMMC_GEN_OPT_TILE_ROWS 2
-/* NMMC_GEN_OPT_WEIGHT_IMAGE: 1 (default) the TMA-staged forward convolutions copy each layer's
+/* NMMC_GEN_OPT_WEIGHT_IMAGE: 1 (default) the convolutions at L = 128 copy each layer's
  * weights into shared memory as one bulk copy of an image in the tensor-core operand layout
  * (rebuilt whenever the weights change); 0 the threads rearrange the BF16 weights; the same
  * results. */

@@ -12,7 +12,6 @@
 // FP32; gradients, biases, master weights and the Adam moments are FP32.
 //
 // Layouts: activations NHWC [image][y][x][channel]; weights [tap = 3*(dy+1)+(dx+1)][cin][cout].
-#include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
 #include <stdio.h>
@@ -35,7 +34,7 @@ constexpr int kTile = 16;        // pixel tile edge of the convolution kernels
 
 // Activations and gradients are stored chunk-planar: C channels of element type T as
 // [image][C / epc][L*L pixels][epc], epc = 16 / sizeof(T) (8 BF16 or 4 FP32 channels per
-// 16-byte chunk), so that a chunk of consecutive pixels of a row is contiguous: one TMA box
+// 16-byte chunk), so that a chunk of consecutive pixels of a row is contiguous: one bulk copy
 // per (row, chunk) of a convolution window and coalesced stores. A tensor of a single chunk
 // (the 8-channel input, the 4-channel output and its gradient) is plain [pixel][C].
 template <typename T>
@@ -52,7 +51,7 @@ struct GenLayer {
     float* b = nullptr;              // [cout]
     __nv_bfloat16* wb = nullptr;     // BF16 compute copy [9][cin][cout]
     __nv_bfloat16* wt = nullptr;     // BF16 flipped transpose [9][cout][cin] (data gradient)
-    uint8_t* wimg = nullptr;         // BF16 weights in the tensor-core B layout of k_gen_conv_tma
+    uint8_t* wimg = nullptr;         // BF16 weights in the tensor-core B layout of k_gen_conv_row
                                      // (kWimgBytes), staged by one bulk copy per CTA
     uint8_t* wtimg = nullptr;        // hidden layers: wt as TF32 in that layout (2 kWimgBytes)
     int kch = 0;                     // 16-byte chunks of K per tap in wimg
@@ -95,11 +94,9 @@ struct nmmc_gen {
     int* d_flag = nullptr;           // device error word (4: a tensor-core wait gave up)
     int use_tc = 1;                  // hidden layers on tcgen05 (NMMC_GEN_OPT_TENSOR_CORES)
     int use_ws = 0;                  // warp-specialised tcgen05 kernel for the BF16 modes (opt-in)
-    int use_tma = 1;                 // L = 128: 1 TMA-staged single-role kernels, 2 TMA-staged
-                                     // warp-specialised forward, 0 cp.async staging
-    int tile_rows = 2;               // output rows per tile of the TMA forward kernels (1 or 2)
+    int use_rows = 1;                // L = 128: the row-ring kernels (0: cp.async staging)
     int schedule = 0;                // warm-start noise levels: 0 linear, 1 quadratic, 2 cosine
-    int use_wimg = 1;                // TMA forward kernels stage the weights by one bulk copy of
+    int use_wimg = 1;                // the row-ring kernels stage the weights by one bulk copy of
                                      // their image (0: the threads rearrange the BF16 weights)
     int sm_count = 0;
     int smem_per_sm = 0;             // shared memory per SM of the generator's device
@@ -274,6 +271,11 @@ __host__ __device__ constexpr uint32_t idesc() {
     return (1u << 4) | (Traits<MODE>::kFmt << 7) | (Traits<MODE>::kFmt << 10) | ((uint32_t)(N >> 3) << 17) |
            ((uint32_t)(kM >> 4) << 24);
 }
+// the same for a number of columns n known at run time
+template <int MODE>
+__device__ __forceinline__ uint32_t idesc_n(uint32_t n) {
+    return (1u << 4) | (Traits<MODE>::kFmt << 7) | (Traits<MODE>::kFmt << 10) | ((n >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
+}
 __host__ __device__ constexpr int window(int L) { return kM + 2 * (L + 3); }
 template <int MODE>
 __host__ __device__ constexpr int smem_bytes(int L) { return 9 * btap<MODE>() + chunks<MODE>() * window(L) * 16 + 1024; }
@@ -301,6 +303,29 @@ __device__ __forceinline__ bool gen_mbar_try_wait(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
+// Bounded wait for phase `parity` of `bar`; gives up (abort word and error flag `code` set) after
+// the limit or as soon as another role has given up.
+__device__ __forceinline__ bool gen_wait(uint32_t bar, uint32_t parity, volatile int* abort, int* flag, int code) {
+    for (unsigned it = 0; it < tc::kWaitLimit; ++it) {
+        if (gen_mbar_try_wait(bar, parity)) return true;
+        if (*abort) return false;
+    }
+    *abort = 1;
+    atomicExch(flag, code);
+    return false;
+}
+
+__device__ __forceinline__ void gen_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// an arrival on `bar` when the MMAs issued so far by this thread have completed
+__device__ __forceinline__ void gen_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 // 16 consecutive FP32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     uint32_t r[16];
@@ -314,11 +339,20 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 16 consecutive FP32 columns of this thread's TMEM lane <- 0 (before a wait::st)
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(
+            taddr),
+        "r"(0)
+        : "memory");
+}
+
 // Weights w[tap][k][n] (BF16, 16-byte aligned) -> B_tap[n][k] as K-major core matrices in
 // shared memory. One 16-byte load brings 8 consecutive n (48 is a multiple of 8) and the loop
 // is unrolled so that several loads are in flight per thread; element by element, the loads
 // would each wait for the previous store.
-template <int MODE>
+template <int MODE, bool ROWS = false>
 __device__ __forceinline__ void stage_weights(uint8_t* sB, const __nv_bfloat16* __restrict__ w, int tid, int nthr) {
     using TA = typename tc::Traits<MODE>::TA;
     constexpr int kEpc = tc::Traits<MODE>::kEpc, kCh = tc::chunks<MODE>(), kBT = tc::btap<MODE>();
@@ -328,20 +362,31 @@ __device__ __forceinline__ void stage_weights(uint8_t* sB, const __nv_bfloat16* 
         const uint4 v = __ldcg(reinterpret_cast<const uint4*>(w) + g8);
         const int i = g8 * 8;
         const int tap = i / (kC * kC), r = i - tap * kC * kC, k = r / kC, n = r - k * kC;
-        uint8_t* base = sB + tap * kBT + ((n >> 3) * kCh + k / kEpc) * tc::kCore + (k % kEpc) * (int)sizeof(TA);
+        uint8_t* base = sB + (ROWS ? tap % 3 * 3 + 2 - tap / 3 : tap) * kBT + ((n >> 3) * kCh + k / kEpc) * tc::kCore + (k % kEpc) * (int)sizeof(TA);
         const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
 #pragma unroll
         for (int q = 0; q < 8; ++q) *(TA*)(base + q * 16) = (TA)e[q];
     }
 }
 
+// The mask of one output position (MODE 2): all loads before the first store, which they could
+// not pass (one by one a data gradient of 16 x 128^2 took 85 us instead of 55).
+template <int MODE>
+__device__ __forceinline__ void load_mask(uint4* m4, const __nv_bfloat16* __restrict__ mask, size_t img, size_t pp, size_t LL) {
+    if (MODE == 2) {
+        const uint4* mk = reinterpret_cast<const uint4*>(mask + img * LL * tc::kC) + pp;
+#pragma unroll
+        for (int c = 0; c < tc::kC / 8; ++c) m4[c] = __ldcg(mk + (size_t)c * LL);
+    }
+}
+
 // Epilogue of one output position of a tensor-core convolution: v[48] FP32 accumulators of
 // pixel pp (y*L + x) of image img, written chunk-planar (16 bytes per chunk, consecutive
 // pixels of a warp contiguous). MODE 0: bias + ReLU, BF16. MODE 1: bias, FP32. MODE 2:
-// times (mask > 0) with the mask the layer's BF16 activation, FP32.
+// times (mask > 0) with the mask the layer's BF16 activation (m4, load_mask), FP32.
 template <int MODE>
 __device__ __forceinline__ void conv_store(const float* v, const float* sbias, void* out_v,
-                                           const __nv_bfloat16* __restrict__ mask, size_t img, size_t pp, size_t LL) {
+                                           const uint4* m4, size_t img, size_t pp, size_t LL) {
     constexpr int kC = tc::kC;
     if (MODE == 0) {
         uint4* dst = reinterpret_cast<uint4*>((__nv_bfloat16*)out_v + img * LL * kC) + pp;
@@ -363,11 +408,7 @@ __device__ __forceinline__ void conv_store(const float* v, const float* sbias, v
             dst[(size_t)c * LL] = make_float4(v[4 * c] + sbias[4 * c], v[4 * c + 1] + sbias[4 * c + 1],
                                               v[4 * c + 2] + sbias[4 * c + 2], v[4 * c + 3] + sbias[4 * c + 3]);
     } else {
-        const uint4* mk = reinterpret_cast<const uint4*>(mask + img * LL * kC) + pp;
         float4* dst = reinterpret_cast<float4*>((float*)out_v + img * LL * kC) + pp;
-        uint4 m4[kC / 8];   // all loads before the first store, which they could not pass
-#pragma unroll
-        for (int c = 0; c < kC / 8; ++c) m4[c] = __ldcg(mk + (size_t)c * LL);
 #pragma unroll
         for (int c = 0; c < kC / 8; ++c) {
             const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&m4[c]);
@@ -394,6 +435,35 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t ad, uint64_t bd, 
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
             "l"(ad), "l"(bd), "r"(tc::idesc<MODE, N>()), "r"(acc)
             : "memory");
+}
+
+// The same, always accumulating, with the instruction descriptor as a value and the operand
+// descriptors in halves (only the low one, with the start address, changes), so that little but the
+// MMA itself is issued: one of N = 144 takes 74 cycles, and with the descriptors computed per MMA
+// in one lane's branch the issue took 130.
+template <int MODE>
+__device__ __forceinline__ void tc_mma_n(uint32_t tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi, uint32_t idesc) {
+    if (MODE == 2)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, 1, 0;\n\t"
+            "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+            "tcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %5, p;\n\t}" ::"r"(tmem),
+            "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, 1, 0;\n\t"
+            "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}" ::"r"(tmem),
+            "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc)
+            : "memory");
+}
+
+// one lane of a warp that is together, known as such to the compiler (unlike lane == 0)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
 }
 
 // Per tile: stage the window, issue the MMAs, wait for their commit, run the epilogue; two
@@ -507,7 +577,9 @@ k_gen_conv_tc(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_b
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         const int pos = q0 + warp * 32 + lane, py = pos / P, px = pos - py * P;
         if (py >= 1 && py <= L && px >= 1 && px <= L) {
-            conv_store<MODE>(v, sbias, out_v, mask, (size_t)img, (size_t)(py - 1) * L + (px - 1), (size_t)L * L);
+            uint4 m4[kC / 8];
+            load_mask<MODE>(m4, mask, (size_t)img, (size_t)(py - 1) * L + (px - 1), (size_t)L * L);
+            conv_store<MODE>(v, sbias, out_v, m4, (size_t)img, (size_t)(py - 1) * L + (px - 1), (size_t)L * L);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     };
@@ -551,424 +623,304 @@ k_gen_conv_tc(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_b
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }
 
-// Bulk-copy-fed variant for L = 128 (the configured size): a tile is one image row (128 positions =
-// the 128 TMEM lanes). Its window is the three wrapped rows y-1, y, y+1, each staged as kCh
-// blocks (one per 16-byte channel chunk) of 130 slots (x = -1 .. 128). A row of a chunk plane is
-// 2048 contiguous bytes, so each block is one cp.async.bulk into slots 1 .. 128, completing on one
-// mbarrier: 3 kCh copies per tile. (As tensor-map boxes of 130 positions x 16 bytes the same
-// windows moved 16 bytes at a time: a hidden forward layer of 16 x 128^2 took 24.6 us and the TF32
-// data gradient 84 us.) The threads then copy x = 127 and x = 0 into slots 0 and 129 (periodic
-// in x), fence them to the async proxy, and thread 0 issues the 9 taps x kCh/2 MMAs, each tap a
-// descriptor offset (row block, and x shift of one slot). The next tile's copies are issued as
-// soon as the MMAs have committed, so they land while the epilogue drains the accumulator.
-namespace tma {
-constexpr int kSlots = 130;                   // x = -1 .. 128
-constexpr int kBlk = 2176;                    // bytes per (row, chunk) block: 130 x 16 B, 128-B aligned
-// MMA N for co output channels: M = 128 takes N in multiples of 16
-__host__ __device__ constexpr int nmma(int co) { return (co + 15) / 16 * 16; }
-template <int MODE, int KCH, int CO>
-__host__ __device__ constexpr int btap() { return (nmma(CO) / 8) * KCH * tc::kCore; }   // B bytes per tap
-template <int MODE, int ICH = tc::chunks<MODE>(), int KCH = ICH, int CO = tc::kC, int R = 1>
-__host__ __device__ constexpr int smem_bytes() { return 9 * btap<MODE, KCH, CO>() + (R + 2) * KCH * kBlk + 1024; }
-}  // namespace tma
-
-// Every convolution of the generator at L = 128 with bulk-copied windows. ICH input chunks
-// (16 bytes of channels each) come in by bulk copies; the K of one tap is KCH chunks (KCH - ICH zero
-// blocks when a layer's inputs do not fill an MMA's K: the first layer's 8 BF16 channels are
-// one chunk of the two of K = 16); N = CO output channels rounded up to 16.
+// Every convolution of the generator at L = 128 (the configured size), warp-specialised, one CTA
+// per SM. The CTAs take equal runs of consecutive rows of the batch; an input row (128 positions =
+// the 128 TMEM lanes) is copied once and used once: for each x shift one MMA multiplies it by the
+// weights of the three vertical taps side by side, N = 3 x 48 columns, into the accumulators of
+// the output rows r-1, r, r+1, which are neighbours in a ring of kAcc accumulators in tensor
+// memory (two MMAs where the three wrap around the ring's end). An output row is finished when the
+// row below it has been multiplied. The order of the taps in a sum is that of the other forms.
+// A row buffer holds KCH blocks (one per 16-byte channel chunk) of 130 slots (x = -1 .. 128); a
+// row of a chunk plane is 2048 contiguous bytes, one cp.async.bulk. (A bulk copy takes about 100
+// cycles to issue, whatever its size, so the periodic neighbours x = 127 and x = 0 are copied
+// within shared memory: as two more bulk copies per chunk they bounded the kernel.)
+//   warps 0-7: epilogue, two groups of four: group g takes the tiles k = g mod 2, its warp w the
+//              TMEM lanes 32 (w & 3) ..; the data gradient's mask is loaded before the wait for
+//              the accumulator, so it arrives during the MMAs;
+//   warp 8:    producer: after empty[slot], the byte count of raw[slot] and the row's copies;
+//   warp 10:   after raw[slot], slots 0 and 129 of the blocks, then full[slot];
+//   warp 9:    after full of the next row and tempty of the accumulator it begins, 3 x KCH/2
+//              MMAs, committed to empty of the row and tfull of the finished accumulator. The
+//              warp stays together (uniform descriptors), lane 0 issues.
+// Every MMA accumulates: the epilogue clears an accumulator that it has read.
+// Every wait is bounded and ends when another role gave up (a shared abort word); before the
+// tensor memory is freed the last copies have landed and a last commit has been waited for.
+// What bounds it: an MMA of M = 128 and K = 32 bytes reads A and B from shared memory, 45 cycles for
+// N = 48 and 74 for N = 144, so one per tap (27 in BF16, 54 in TF32 per row) costs nearly twice
+// what 9 or 18 wide ones do; beside that the start of a CTA (about 5 us) and, for the data
+// gradient, memory. 16 x 128^2: hidden forward layer 15.7 us, data gradient 21.7 us, first layer
+// 11.8 us, last 13.5 us; single-role CTAs with windows of four rows and one MMA per tap took
+// 18.5, 55, 12 and 17 us. 50 MB and 126 MB at the copy rate are 7.4 and 18.5 us.
 //   MODE 0: bias + ReLU, BF16 out (48 channels);  MODE 1: bias, FP32 out (48 channels);
 //   MODE 2: TF32 data gradient, times (activation > 0), FP32 out;
 //   MODE 3: bias, FP32 out of CO = 4 channels [pixel][4] (the generator's last layer).
-// A tile is R consecutive output rows of one image: its window holds R + 2 input rows, the
-// MMAs of output row j read window rows j .. j+2 into accumulator j (R x the TMEM columns),
-// and one commit and one epilogue pass cover the R rows, so the per-tile latency of the copy,
-// the commit and the epilogue is paid once for R rows.
+// ICH input chunks (16 bytes of channels each) come in by bulk copies; the K of one tap is KCH
+// chunks (KCH - ICH zero blocks when a layer's inputs do not fill an MMA's K: the first layer's
+// 8 BF16 channels are one chunk of the two of K = 16); N = CO output channels rounded up to 16.
 // With wimg the weights arrive by one bulk copy of their tensor-core image (k_gen_update) instead
 // of being rearranged by the threads.
-template <int MODE, int ICH, int KCH, int CO, int R>
-__global__ void __launch_bounds__(128, 2)
-k_gen_conv_tma(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_bfloat16* __restrict__ w,
+namespace row {
+constexpr int kSlots = 130;                   // x = -1 .. 128
+constexpr int kBlk = 2176;                    // bytes per (row, chunk) block: 130 x 16 B, 128-B aligned
+constexpr int kAcc = 10;                      // accumulators: 480 of 512 TMEM columns
+constexpr int kEpi = 8;                       // epilogue warps
+constexpr int kThreads = (kEpi + 3) * 32;
+// MMA N for co output channels: M = 128 takes N in multiples of 16
+__host__ __device__ constexpr int nmma(int co) { return (co + 15) / 16 * 16; }
+template <int CO>
+__host__ __device__ constexpr int cols() { return kAcc * nmma(CO) <= 256 ? 256 : 512; }   // TMEM columns allocated
+template <int KCH, int CO>
+__host__ __device__ constexpr int btap() { return (nmma(CO) / 8) * KCH * tc::kCore; }   // B bytes per tap
+// place of tap 3 (dy + 1) + dx + 1 among the weights: by dx, then dy descending, so that the three
+// taps of a dx are the columns of the output rows r-1, r, r+1
+__host__ __device__ constexpr int place(int tap) { return tap % 3 * 3 + 2 - tap / 3; }
+// row buffers: what fits beside the weights, eight at most (the data gradient: five)
+template <int KCH, int CO>
+__host__ __device__ constexpr int ring() {
+    const int fit = (tc::kSmemMax - 1024 - 9 * btap<KCH, CO>()) / (KCH * kBlk);
+    return fit < 8 ? fit : 8;
+}
+template <int KCH, int CO>
+__host__ __device__ constexpr int smem_bytes() { return 9 * btap<KCH, CO>() + ring<KCH, CO>() * KCH * kBlk + 1024; }
+}  // namespace row
+
+template <int MODE, int ICH, int KCH, int CO>
+__global__ void __launch_bounds__(row::kThreads, 1)
+k_gen_conv_row(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_bfloat16* __restrict__ w,
                const uint8_t* __restrict__ wimg, const float* __restrict__ bias,
-               const __nv_bfloat16* __restrict__ mask, void* __restrict__ out_v, int ntiles,
-               int* __restrict__ flag) {
+               const __nv_bfloat16* __restrict__ mask, void* __restrict__ out_v, int nrows, int* __restrict__ flag) {
     seq_begin();
     using namespace tc;
     using TA = typename Traits<MODE>::TA;
     constexpr int kEpc = Traits<MODE>::kEpc;
-    constexpr int NN = tma::nmma(CO);
+    constexpr int NN = row::nmma(CO);
     constexpr int CI = ICH * kEpc;                           // real input channels
-    constexpr int kBT = tma::btap<MODE, KCH, CO>();
-    constexpr int kCols = NN <= 32 ? 32 : 64;                // TMEM columns of one accumulator
+    constexpr int kBT = row::btap<KCH, CO>();
+    constexpr int kS = row::ring<KCH, CO>();
     constexpr int kL = kM;                                   // lattice edge of this kernel
-    constexpr int kTpi = kL / R;                             // tiles per image
-    constexpr uint32_t kRowB = kL * 16u, kTx = (R + 2u) * ICH * kRowB;   // bytes per chunk row and per window
-    static_assert(KCH % 2 == 0 && KCH >= ICH && NN <= 64 && (MODE != 3 || CO == 4) && (MODE == 3 || CO == kC) &&
-                  (R == 1 || R == 2 || R == 4) && kL % R == 0, "convolution shape");
+    constexpr uint32_t kRowB = kL * 16u;                     // bytes per row of a chunk plane
+    constexpr uint32_t kTx = ICH * kRowB;                    // bytes copied per row buffer
+    constexpr uint32_t kBuf = (uint32_t)KCH * row::kBlk;     // row buffer stride
+    static_assert(KCH % 2 == 0 && KCH >= ICH && ICH <= 16 && row::kAcc * NN <= 512 && (MODE != 3 || CO == 4) &&
+                  (MODE == 3 || CO == kC) && kS >= 4, "convolution shape");
     extern __shared__ uint8_t tsm_raw[];
-    __shared__ __align__(8) unsigned long long mbar;       // MMA commit
-    __shared__ __align__(8) unsigned long long tbar;       // window copies
-    __shared__ __align__(8) unsigned long long wbar;       // weight image copy
+    __shared__ __align__(8) unsigned long long raw[kS], full[kS], empty[kS], tfull[row::kAcc], tempty[row::kAcc], wbar, done;
     __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_word;
     __shared__ __align__(16) float sbias[NN];
     uint8_t* sB = (uint8_t*)(((uintptr_t)tsm_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* sA = sB + 9 * kBT;                             // 1024-aligned + 9 kBT (multiple of 128)
+    uint8_t* sA = sB + 9 * kBT;                              // 1024-aligned + 9 kBT (multiple of 128)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
     const uint32_t aBase = gen_smem_u32(sA), bBase = gen_smem_u32(sB);
-    const uint32_t mb = gen_smem_u32(&mbar), tb = gen_smem_u32(&tbar), wbr = gen_smem_u32(&wbar);
     const bool use_img = wimg != nullptr;
-    // warp 0: the window of tile t (image t / kTpi, rows R (t % kTpi) ..): R + 2 rows x ICH chunk
-    // blocks, one copy per lane at a time
-    auto issue_window = [&](int t) {
-        const int img = t / kTpi, y = (t - img * kTpi) * R;
-        if (lane == 0)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tb), "r"(kTx) : "memory");
-        __syncwarp();
-        const char* src = reinterpret_cast<const char*>(in) + (size_t)img * ICH * kL * kRowB;
-        for (int i = lane; i < (R + 2) * ICH; i += 32) {
-            const int r = i / ICH, c = i - r * ICH;
-            int yy = y + r - 1;
-            yy += (yy < 0) ? kL : ((yy >= kL) ? -kL : 0);
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    aBase + (uint32_t)((r * KCH + c) * tma::kBlk + 16)),
-                "l"(src + ((size_t)c * kL + yy) * kRowB), "r"(kRowB), "r"(tb)
-                : "memory");
-        }
-    };
-    const int first = blockIdx.x, stride = gridDim.x;
-    const int n = (ntiles > first) ? (ntiles - first + stride - 1) / stride : 0;
+    // rows [r0, r1) of the batch, in segments of one image each
+    const int r0 = (int)((long long)nrows * blockIdx.x / gridDim.x);
+    const int r1 = (int)((long long)nrows * (blockIdx.x + 1) / gridDim.x);
+
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tb) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbr) : "memory");
+        for (int s = 0; s < kS; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&raw[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&full[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&empty[s])) : "memory");
+        }
+        for (int a = 0; a < row::kAcc; ++a) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&tfull[a])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(gen_smem_u32(&tempty[a])) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&wbar)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&done)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (use_img && n > 0) {
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(wbr), "r"(9u * kBT) : "memory");
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(bBase),
-                "l"(reinterpret_cast<uint64_t>(wimg)), "r"(9u * kBT), "r"(wbr)
-                : "memory");
+        abort_word = 0;
+        if (use_img) {
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gen_smem_u32(&wbar)), "r"(9u * kBT)
+                         : "memory");
+            gen_bulk(bBase, wimg, 9u * kBT, gen_smem_u32(&wbar));
         }
     }
     if (warp == 0) {
-        __syncwarp();   // the barriers are initialised
-        if (n > 0) issue_window(first);   // the first window lands while the weights are staged
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gen_smem_u32(&tmem_slot)),
+                     "r"(row::cols<CO>())
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if constexpr (KCH > ICH) {   // K-padding blocks: zero once, never written by TMA
-        constexpr int kZ = KCH - ICH, kU = tma::kBlk / 16;
-        for (int i = tid; i < (R + 2) * kZ * kU; i += blockDim.x) {
-            const int zb = i / kU, r = zb / kZ, c = ICH + (zb - r * kZ);
-            *(uint4*)(sA + (r * KCH + c) * tma::kBlk + (i - zb * kU) * 16) = make_uint4(0, 0, 0, 0);
+    if constexpr (KCH > ICH) {   // K-padding blocks: zero once, never copied over
+        constexpr int kZ = KCH - ICH, kU = row::kBlk / 16;
+        for (int i = tid; i < kS * kZ * kU; i += row::kThreads) {
+            const int zb = i / kU, s = zb / kZ, c = ICH + (zb - s * kZ);
+            *(uint4*)(sA + s * kBuf + c * row::kBlk + (i - zb * kU) * 16) = make_uint4(0, 0, 0, 0);
         }
     }
-    if (use_img) {
-        // weights by the bulk copy above
-    } else if constexpr (ICH == KCH && CI == kC && CO == kC) {
-        stage_weights<MODE>(sB, w, tid, blockDim.x);   // 48 -> 48: 16-byte loads
-    } else {
-        // w[tap][k][n] (CI x CO) -> B_tap[n][k] over the padded NN x KCH*epc, zeros outside
-        constexpr int KK = KCH * kEpc;
-#pragma unroll 8
-        for (int i = tid; i < 9 * NN * KK; i += blockDim.x) {
-            const int tap = i / (NN * KK), r = i - tap * NN * KK, nn = r / KK, k = r - nn * KK;
-            const float v = (nn < CO && k < CI) ? __bfloat162float(__ldcg(w + (tap * CI + k) * CO + nn)) : 0.0f;
-            *(TA*)(sB + tap * kBT + ((nn >> 3) * KCH + k / kEpc) * kCore + (nn & 7) * 16 + (k % kEpc) * (int)sizeof(TA)) =
-                (TA)v;
+    if (!use_img) {
+        if constexpr (ICH == KCH && CI == kC && CO == kC) {
+            stage_weights<MODE, true>(sB, w, tid, row::kThreads);   // 48 -> 48: 16-byte loads
+        } else {
+            // w[tap][k][n] (CI x CO) -> B_tap[n][k] over the padded NN x KCH*epc, zeros outside
+            constexpr int KK = KCH * kEpc;
+#pragma unroll 4
+            for (int i = tid; i < 9 * NN * KK; i += row::kThreads) {
+                const int tap = i / (NN * KK), r = i - tap * NN * KK, nn = r / KK, k = r - nn * KK;
+                const float v = (nn < CO && k < CI) ? __bfloat162float(__ldcg(w + (tap * CI + k) * CO + nn)) : 0.0f;
+                *(TA*)(sB + row::place(tap) * kBT + ((nn >> 3) * KCH + k / kEpc) * kCore + (nn & 7) * 16 +
+                       (k % kEpc) * (int)sizeof(TA)) = (TA)v;
+            }
         }
     }
     if (tid < NN) sbias[tid] = (MODE == 2 || tid >= CO) ? 0.0f : __ldcg(bias + tid);
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gen_smem_u32(&tmem_slot)),
-                     "r"(R * kCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    uint32_t mphase = 0, tphase = 0;
-    auto bounded_wait = [&](uint32_t bar, uint32_t& ph, int code) -> bool {
-        bool done = false;
-        for (unsigned it = 0; it < kWaitLimit && !done; ++it) done = gen_mbar_try_wait(bar, ph);
-        if (__syncthreads_or(!done)) {
-            if (tid == 0) atomicExch(flag, code);
-            return false;
-        }
-        ph ^= 1u;
-        return true;
-    };
-
-    bool failed = false, window_pending = n > 0, weights_pending = use_img && n > 0;
-    if (weights_pending) {
-        uint32_t wph = 0;
-        if (!bounded_wait(wbr, wph, 6)) failed = true;
-        else weights_pending = false;
+    if (warp < 4) {   // every accumulator starts at zero
+        for (int c = 0; c < row::kAcc * NN; c += 16) tmem_zero16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
-    for (int k = 0; k < n && !failed; ++k) {
-        const int t = first + k * stride;
-        if (!bounded_wait(tb, tphase, 5)) {
-            failed = true;
-            break;
-        }
-        window_pending = false;
-        // periodic x: slot 0 <- x = 127 (slot 128), slot 129 <- x = 0 (slot 1), in the loaded blocks
-        if (tid < (R + 2) * ICH * 2) {
-            const int e = tid >> 1, r = e / ICH, c = e - r * ICH;
-            uint8_t* blk = sA + (r * KCH + c) * tma::kBlk;
-            const int to = (tid & 1) ? (tma::kSlots - 1) : 0, from = (tid & 1) ? 1 : kL;
-            *(uint4*)(blk + to * 16) = *(const uint4*)(blk + from * 16);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    if (warp < row::kEpi) {
+        const int grp = warp >> 2;
+        for (int r = r0 + grp; r < r1; r += 2) {
+            const int k = r - r0, acc = k % row::kAcc;
+            const int img = r / kL;
+            const size_t LL = (size_t)kL * kL, pp = (size_t)(r - img * kL) * kL + (size_t)((warp & 3) * 32 + lane);
+            uint4 m4[kC / 8];
+            load_mask<MODE>(m4, mask, (size_t)img, pp, LL);
+            const bool ok = gen_wait(gen_smem_u32(&tfull[acc]), (uint32_t)(k / row::kAcc) & 1u, &abort_word, flag, 4);
+            if (!__all_sync(0xFFFFFFFFu, ok)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < R; ++j) {
-#pragma unroll 1
-                for (int tap = 0; tap < 9; ++tap) {
-                    const int ty = tap / 3, tx = tap - 3 * ty;
-#pragma unroll
-                    for (int ks = 0; ks < KCH / 2; ++ks) {
-                        const uint64_t ad = umma_desc(aBase + (uint32_t)(((j + ty) * KCH + 2 * ks) * tma::kBlk + tx * 16),
-                                                      (uint32_t)tma::kBlk, 128);
-                        const uint64_t bd = umma_desc(bBase + tap * kBT + 2 * ks * kCore, kCore, KCH * kCore);
-                        tc_mma<MODE, NN>(tmem + (uint32_t)(j * kCols), ad, bd, (tap | ks) ? 1u : 0u);
-                    }
-                }
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mb)
-                         : "memory");
-        }
-        if (!bounded_wait(mb, mphase, 4)) {
-            failed = true;
-            break;
-        }
-        // the MMAs have read the window: the next tile's copies overlap this epilogue
-        if (k + 1 < n) {
-            if (warp == 0) issue_window(t + stride);
-            window_pending = true;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int img = t / kTpi, y0 = (t - img * kTpi) * R;
-#pragma unroll 1
-        for (int jr = 0; jr < R; ++jr) {
             float v[NN];
-            const uint32_t taddr = tmem + (uint32_t)(jr * kCols) + ((uint32_t)(warp * 32) << 16);
+            const uint32_t taddr = tmem + (uint32_t)(acc * NN) + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
             for (int j = 0; j < NN / 16; ++j) tmem_ld16(taddr + 16 * j, v + 16 * j);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const size_t pp = (size_t)(y0 + jr) * kL + (size_t)(warp * 32 + lane);
+#pragma unroll
+            for (int j = 0; j < NN / 16; ++j) tmem_zero16(taddr + 16 * j);   // the next tile is added to zero
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)   // the accumulator may be used again
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&tempty[acc])) : "memory");
             if constexpr (MODE == 3) {
-                float4* dst = reinterpret_cast<float4*>(out_v) + (size_t)img * kL * kL + pp;
+                float4* dst = reinterpret_cast<float4*>(out_v) + (size_t)img * LL + pp;
                 *dst = make_float4(v[0] + sbias[0], v[1] + sbias[1], v[2] + sbias[2], v[3] + sbias[3]);
             } else {
-                conv_store<MODE>(v, sbias, out_v, mask, (size_t)img, pp, (size_t)kL * kL);
+                conv_store<MODE>(v, sbias, out_v, m4, (size_t)img, pp, LL);
             }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    }
-    if (failed) {   // bounded waits for what may still be in flight before the TMEM is freed
-        bool done = false;
-        for (unsigned it = 0; it < kWaitLimit && !done; ++it) done = gen_mbar_try_wait(mb, mphase);
-    }
-    if (window_pending) {
-        bool done = false;
-        for (unsigned it = 0; it < kWaitLimit && !done; ++it) done = gen_mbar_try_wait(tb, tphase);
-    }
-    if (weights_pending) {
-        bool done = false;
-        for (unsigned it = 0; it < kWaitLimit && !done; ++it) done = gen_mbar_try_wait(wbr, 0);
-    }
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(R * kCols) : "memory");
-}
-
-// TMA-fed, warp-specialised forward convolution for L = 128 (BF16 modes), opt-in: one CTA per
-// SM, a ring of kWsStages windows and two TMEM accumulators, so the copies of later tiles, the
-// MMAs of tile k and the epilogue of tile k-1 overlap. Measured on GB300 (16 x 128^2, chunk-
-// planar activations) a warm-start pass takes 0.379 ms with it against 0.358 ms with two
-// single-role TMA CTAs per SM, which overlap one another's phases.
-//   warps 0-3: epilogue (warp w drains TMEM lanes 32w ..), then arrive on tempty[acc];
-//   warp 4:    producer (lane 0): after empty[stage], expect_tx on full[stage] and the
-//              window's 3 x kCh blocks, each one box of 130 slots (x = -1 .. 128, the two
-//              edge slots zero-filled) into a 128-byte aligned block;
-//   warp 5:    MMA issue: after full[stage] the 32 lanes copy the wrapped edge columns
-//              (x = 127 into slot 0, x = 0 into slot 129) and fence them to the async proxy;
-//              after tempty[acc] lane 0 issues the 27 MMAs and commits them to empty[stage]
-//              and tfull[acc]; the warp owns the TMEM allocation.
-// Every wait is bounded; a role that gives up sets the error word and stops, and the others
-// then time out on the barriers it no longer signals.
-constexpr int kWsStages = 4;
-constexpr int kTwsThreads = 192;
-template <int MODE>
-__host__ __device__ constexpr int tmaws_smem_bytes() {
-    return 9 * tc::btap<MODE>() + kWsStages * 3 * tc::chunks<MODE>() * tma::kBlk + 1024;
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(kTwsThreads, 1)
-k_gen_conv_tmaws(const __grid_constant__ CUtensorMap tmap, const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias, void* __restrict__ out_v,
-                 int ntiles, int* __restrict__ flag) {
-    static_assert(MODE == 0 || MODE == 1, "BF16 modes only");
-    using namespace tc;
-    constexpr int kCh = chunks<MODE>();
-    constexpr int kBT = btap<MODE>();
-    constexpr int kL = kM;
-    constexpr int kS = kWsStages;
-    constexpr uint32_t kWin = 3u * kCh * tma::kBlk;                // bytes per ring stage
-    constexpr uint32_t kTx = 3u * kCh * tma::kSlots * 16u;         // bytes per window
-    extern __shared__ uint8_t tsm_raw[];
-    __shared__ __align__(8) unsigned long long bars[2 * kS + 4];   // full[S], empty[S], tfull[2], tempty[2]
-    __shared__ uint32_t tmem_slot;
-    __shared__ __align__(16) float sbias[kC];
-    uint8_t* sB = (uint8_t*)(((uintptr_t)tsm_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* sA = sB + 9 * kBT;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-    if (warp == 5) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gen_smem_u32(&tmem_slot)),
-                     "r"(2 * kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 0) {
-        for (int b = 0; b < 2 * kS + 4; ++b) {
-            const unsigned cnt = (b >= 2 * kS + 2) ? 128u : 1u;
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gen_smem_u32(&bars[b])), "r"(cnt) : "memory");
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_slot;
-    const uint32_t aBase = gen_smem_u32(sA), bBase = gen_smem_u32(sB);
-    const uint32_t full0 = gen_smem_u32(&bars[0]), empty0 = gen_smem_u32(&bars[kS]);
-    const uint32_t tfull0 = gen_smem_u32(&bars[2 * kS]), tempty0 = gen_smem_u32(&bars[2 * kS + 2]);
-    const int first = blockIdx.x, stride = gridDim.x;
-    const int n = (ntiles > first) ? (ntiles - first + stride - 1) / stride : 0;
-    auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
-        for (unsigned it = 0; it < kWaitLimit; ++it)
-            if (gen_mbar_try_wait(bar, parity)) return true;
-        atomicExch(flag, 6);
-        return false;
-    };
-    auto tma_box = [&](uint32_t dst, int c, int y, int img, uint32_t bar) {   // x = -1 .. 128
-        asm volatile(
-            "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
-            "%6}], [%7];" ::"r"(dst),
-            "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(0), "r"(-1), "r"(y), "r"(c), "r"(img), "r"(bar)
-            : "memory");
-    };
-    // producer: the window of the CTA's tile k into stage k % S
-    auto issue = [&](int k) {
-        const int t = first + k * stride, img = t / kL, y = t - img * kL, st = k % kS;
-        const uint32_t bar = full0 + 8 * st;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTx) : "memory");
-#pragma unroll 1
-        for (int r = 0; r < 3; ++r) {
-            int yy = y + r - 1;
-            yy += (yy < 0) ? kL : ((yy >= kL) ? -kL : 0);
-#pragma unroll 1
-            for (int c = 0; c < kCh; ++c) {
-                tma_box(aBase + (uint32_t)st * kWin + (uint32_t)((r * kCh + c) * tma::kBlk), c, yy, img, bar);
+    } else if (warp == row::kEpi) {
+        int q = 0;   // rows copied
+        bool ok = true;
+        for (int r = r0; r < r1 && ok;) {
+            const int img = r / kL, y0 = r - img * kL, len = min(r1 - r, kL - y0);
+            const char* src = reinterpret_cast<const char*>(in) + (size_t)img * ICH * kL * kRowB;
+            for (int i = 0; i < len + 2; ++i, ++q) {
+                const int s = q % kS;
+                if (q >= kS) {
+                    ok = gen_wait(gen_smem_u32(&empty[s]), (uint32_t)(q / kS - 1) & 1u, &abort_word, flag, 5);
+                    if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
+                const int yy = (y0 + i - 1) & (kL - 1);
+                const uint32_t bar = gen_smem_u32(&raw[s]), buf = aBase + (uint32_t)s * kBuf;
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTx) : "memory");
+                __syncwarp();
+                for (int c = lane; c < ICH; c += 32)
+                    gen_bulk(buf + (uint32_t)(c * row::kBlk + 16), src + ((size_t)c * kL + yy) * kRowB, kRowB, bar);
             }
+            r += len;
         }
-    };
-    // the first stages are in flight while the weights are staged
-    if (warp == 4 && lane == 0)
-        for (int k = 0; k < n && k < kS; ++k) issue(k);
-    stage_weights<MODE>(sB, w, tid, blockDim.x);
-    if (tid < kC) sbias[tid] = bias[tid];
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-
-    if (warp == 4) {
-        // ---- producer ----
-        if (lane == 0) {
-            int issued = (n < kS) ? n : kS;
-            for (int k = kS; k < n; ++k) {
-                if (!wait(empty0 + 8 * (k % kS), ((k / kS) - 1) & 1)) break;   // MMAs of tile k - S done
-                issue(k);
-                issued = k + 1;
+        // the last fill of every slot lands before the CTA's shared memory can be released
+        if (lane == 0)
+            for (int j = max(0, q - kS); j < q; ++j)
+                for (unsigned it = 0; it < (kWaitLimit >> 4); ++it)
+                    if (gen_mbar_try_wait(gen_smem_u32(&raw[j % kS]), (uint32_t)(j / kS) & 1u)) break;
+    } else if (warp == row::kEpi + 1) {
+        const bool lead = elect_one();
+        const uint64_t a00 = umma_desc(aBase, (uint32_t)row::kBlk, 128), b00 = umma_desc(bBase, kCore, KCH * kCore);
+        const uint32_t alo = (uint32_t)a00, ahi = (uint32_t)(a00 >> 32), blo = (uint32_t)b00, bhi = (uint32_t)(b00 >> 32);
+        int q = 0, k0 = 0;   // input rows used; tiles of the segments before
+        bool ok = !use_img || gen_wait(gen_smem_u32(&wbar), 0, &abort_word, flag, 6);
+        for (int r = r0; r < r1 && ok;) {
+            const int len = min(r1 - r, kL - r % kL);
+            for (int i = 0; i < len + 2; ++i, ++q) {
+                const int s = q % kS;
+                // output rows j0 .. j1 of the segment take this input row
+                const int j0 = max(0, i - 2), j1 = min(len - 1, i), k = k0 + i;
+                ok = gen_wait(gen_smem_u32(&full[s]), (uint32_t)(q / kS) & 1u, &abort_word, flag, 5);
+                if (ok && i < len && k >= row::kAcc)
+                    ok = gen_wait(gen_smem_u32(&tempty[k % row::kAcc]), (uint32_t)(k / row::kAcc - 1) & 1u, &abort_word,
+                                  flag, 4);
+                if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int c = j1 - j0 + 1, c0 = (k0 + j0) % row::kAcc, n1 = min(c, row::kAcc - c0), n2 = c - n1;
+                // the first row's place among the three taps, and that of the first after the ring's end
+                const uint32_t as = alo + (((uint32_t)s * kBuf) >> 4), bs = blo + (uint32_t)(((2 - i + j0) * kBT) >> 4);
+                const uint32_t bs2 = bs + (uint32_t)((n1 * kBT) >> 4), d = tmem + (uint32_t)(c0 * NN);
+                const uint32_t i1 = idesc_n<MODE>((uint32_t)(n1 * NN)), i2 = idesc_n<MODE>((uint32_t)(n2 * NN));
+                if (lead) {
+#pragma unroll
+                    for (int m = 0; m < 3 * (KCH / 2); ++m) {
+                        const uint32_t ao = (uint32_t)((2 * (m % (KCH / 2)) * row::kBlk + m / (KCH / 2) * 16) >> 4);
+                        const uint32_t bo = (uint32_t)((3 * (m / (KCH / 2)) * kBT + 2 * (m % (KCH / 2)) * kCore) >> 4);
+                        tc_mma_n<MODE>(d, as + ao, ahi, bs + bo, bhi, i1);
+                    }
+                    if (n2) {   // the rest, at the ring's start
+#pragma unroll
+                        for (int m = 0; m < 3 * (KCH / 2); ++m) {
+                            const uint32_t ao = (uint32_t)((2 * (m % (KCH / 2)) * row::kBlk + m / (KCH / 2) * 16) >> 4);
+                            const uint32_t bo = (uint32_t)((3 * (m / (KCH / 2)) * kBT + 2 * (m % (KCH / 2)) * kCore) >> 4);
+                            tc_mma_n<MODE>(tmem, as + ao, ahi, bs2 + bo, bhi, i2);
+                        }
+                    }
+                    gen_commit(gen_smem_u32(&empty[s]));
+                    if (i >= 2) gen_commit(gen_smem_u32(&tfull[(k0 + i - 2) % row::kAcc]));
+                }
+                __syncwarp();
             }
-            // nothing of ours may land after the CTA ends: the last use of every stage completes
-            for (int j = (issued > kS ? issued - kS : 0); j < issued; ++j) wait(full0 + 8 * (j % kS), (j / kS) & 1);
+            k0 += len;
+            r += len;
+        }
+        // every MMA has completed before the tensor memory is freed (all waits above are bounded)
+        if (lead) {
+            gen_commit(gen_smem_u32(&done));
+            bool drained = false;
+            for (unsigned it = 0; it < kWaitLimit && !drained; ++it) drained = gen_mbar_try_wait(gen_smem_u32(&done), 0);
+            if (!drained) atomicExch(flag, 4);
+            if (use_img)   // the weight copy too, should the wait for it have given up
+                for (unsigned it = 0; it < (kWaitLimit >> 4); ++it)
+                    if (gen_mbar_try_wait(gen_smem_u32(&wbar), 0)) break;
         }
         __syncwarp();
-    } else if (warp == 5) {
-        // ---- edge columns and MMA issue ----
-        int k = 0;
-        for (; k < n; ++k) {
-            const int st = k % kS, ac = k & 1;
-            if (!__all_sync(0xffffffffu, wait(full0 + 8 * st, (k / kS) & 1))) break;
-            // periodic x: slot 0 <- x = 127 (slot 128), slot 129 <- x = 0 (slot 1); 3 kCh blocks
-            for (int e = lane; e < 3 * kCh * 2; e += 32) {
-                uint8_t* blk = sA + st * kWin + (e >> 1) * tma::kBlk;
-                const int to = (e & 1) ? (tma::kSlots - 1) : 0, from = (e & 1) ? 1 : kL;
+    } else {   // the periodic neighbours of the copied rows
+        int n = 0;   // rows of this CTA, with the two beside each segment
+        for (int r = r0; r < r1; n += 2) {
+            const int len = min(r1 - r, kL - r % kL);
+            n += len;
+            r += len;
+        }
+        for (int q = 0; q < n; ++q) {
+            const int s = q % kS;
+            const bool ok = gen_wait(gen_smem_u32(&raw[s]), (uint32_t)(q / kS) & 1u, &abort_word, flag, 5);
+            if (!__all_sync(0xFFFFFFFFu, ok)) break;
+            if (lane < 2 * ICH) {   // slot 0 <- x = 127 (slot 128), slot 129 <- x = 0 (slot 1)
+                uint8_t* blk = sA + (uint32_t)s * kBuf + (lane >> 1) * row::kBlk;
+                const int to = (lane & 1) ? (row::kSlots - 1) : 0, from = (lane & 1) ? 1 : kL;
                 *(uint4*)(blk + to * 16) = *(const uint4*)(blk + from * 16);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            bool go = true;
-            if (lane == 0) {
-                if (k >= 2 && !wait(tempty0 + 8 * ac, ((k >> 1) - 1) & 1)) go = false;
-            }
-            if (!__shfl_sync(0xffffffffu, go, 0)) break;
-            if (lane == 0) {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a0 = aBase + (uint32_t)st * kWin, d = tmem + (uint32_t)(ac * kTmemCols);
-#pragma unroll 1
-                for (int tap = 0; tap < 9; ++tap) {
-                    const int ty = tap / 3, tx = tap - 3 * ty;
-#pragma unroll
-                    for (int ks = 0; ks < kCh / 2; ++ks) {
-                        const uint64_t ad = umma_desc(a0 + (uint32_t)((ty * kCh + 2 * ks) * tma::kBlk + tx * 16),
-                                                      (uint32_t)tma::kBlk, 128);
-                        const uint64_t bd = umma_desc(bBase + tap * kBT + 2 * ks * kCore, kCore, kCh * kCore);
-                        tc_mma<MODE>(d, ad, bd, (tap | ks) ? 1u : 0u);
-                    }
-                }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 empty0 + 8 * st)
-                             : "memory");
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 tfull0 + 8 * ac)
-                             : "memory");
-            }
-            __syncwarp();
-        }
-        // the TMEM is freed only after the last committed MMAs have landed
-        if (lane == 0 && k > 0) wait(tfull0 + 8 * ((k - 1) & 1), ((k - 1) >> 1) & 1);
-        __syncwarp();
-    } else {
-        // ---- epilogue (warps 0-3) ----
-        for (int k = 0; k < n; ++k) {
-            const int ac = k & 1;
-            if (!wait(tfull0 + 8 * ac, (k >> 1) & 1)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int t = first + k * stride, img = t / kL, y = t - img * kL;
-            float v[kC];
-            const uint32_t taddr = tmem + (uint32_t)(ac * kTmemCols) + ((uint32_t)(warp * 32) << 16);
-            tmem_ld16(taddr + 0, v);
-            tmem_ld16(taddr + 16, v + 16);
-            tmem_ld16(taddr + 32, v + 32);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tempty0 + 8 * ac) : "memory");
-            conv_store<MODE>(v, sbias, out_v, nullptr, (size_t)img, (size_t)y * kL + (size_t)(warp * 32 + lane), (size_t)kL * kL);
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&full[s])) : "memory");
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 5)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kTmemCols) : "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(row::cols<CO>())
+                     : "memory");
 }
 
 // Warp-specialised variant of the BF16 modes (forward and probe), opt-in: one CTA per SM with a
@@ -1160,76 +1112,62 @@ k_gen_conv_ws(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restr
 // in[p + tap, ci] * dout[p, co], the positions p as the contraction (kind::f16, FP32
 // accumulators in tensor memory). The layer input is BF16 already; the FP32 output gradient
 // is split into BF16 hi + lo (lo = the remainder rounded again, 16 significant bits in all)
-// and both halves are multiplied into the same accumulator, which is more accurate than TF32.
-// A K-block is W = min(L, 64) consecutive positions of one image row. Both operands are
-// MN-major: a slot holds 8 channels (16 bytes) per position, the positions 16 bytes apart, so
-// the window of a tap shifted by dx positions is the same slot started dx * 16 bytes later
-// and the layer input is staged once per K-block (rows y-1, y, y+1 and columns x0-1 .. x0+W,
-// periodic), not once per tap. A row block holds 8 slots (6 of data, 2 of zeros) = 64 rows,
-// so one M = 128 MMA covers two vertical taps: for each dx, tile P starts at row block 0 (its
-// rows 0-63 are tap (-1, dx), rows 64-127 tap (0, dx)) and tile Q at row block 1 (rows 64-127
-// tap (+1, dx); its first half repeats P's second and is not read). B is the output gradient
-// (6 slots, N = 48). Six accumulators of 48 columns.
-// Warp-specialised over a ring of kStages slots (mbarriers loaded / full / empty per slot):
-//   warp 0:          producer: after `empty` (the slot's previous MMAs completed), lane 0 sets
-//                    the byte count of `loaded` (expect_tx) and 30 lanes issue bulk copies of
-//                    the K-block's input rows (one lane per row and channel group, in runs
-//                    split at the periodic x edge) and raw FP32 gradient rows (one lane each);
-//   warp 1, lane 0:  MMA issuer: after `full`, 6 tiles x W/16 steps x (hi, lo) MMAs, committed
-//                    to `empty`;
-//   warps 2-15:      after `loaded`, convert the raw gradient to the hi / lo operands in the
-//                    slot and arrive on `full` (one arrival per warp).
-// Every wait is bounded and also ends when another role gave up (a shared abort word); the
-// producer lets its last copies land and the epilogue waits for the last commit before the
-// tensor memory is freed. Each CTA covers a strided set of K-blocks over the batch; its
-// partial dW (read back with tcgen05.ld) goes to `part` and k_gen_sum_parts adds the partials
-// in a fixed order.
+// and both halves are multiplied, which is more accurate than TF32.
+// A K-block is W consecutive positions of one image row, a whole row up to L = 128. Both operands
+// are MN-major: a slot holds 8 channels (16 bytes) per position, the positions 16 bytes apart, so
+// the window of a tap shifted by dx positions is the same slot started dx * 16 bytes later. A is
+// the output gradient: rows 0-47 hi, rows 64-111 lo (slots 6, 7, 14 and 15 stay zero), so one MMA
+// multiplies both halves. B is the input: the 6 slots of each of the rows y-1, y, y+1, neighbours
+// in a ring of rows, are N = 144 columns (row, input channel); two MMAs where they wrap around
+// the ring's end. Three accumulators, one per dx; the epilogue adds the lo lanes to the hi lanes.
+// A CTA's K-blocks are consecutive in y, so each block brings one new row of input.
+// Roles, over a ring of kRows input rows (copied / ready / free per row) and of kStages gradient
+// operands (gfull / gfree):
+//   warp 0:      producer: after `free`, the byte count of `copied` and 6 bulk copies;
+//   warp 2:      after `copied`, where a row is its own neighbour (W = L) the slots of columns -1
+//                and W (else the producer copies them), then `ready`;
+//   warps 4-15:  read the raw gradient, a row ahead, from global memory into registers, write its
+//                hi / lo operands and arrive on gfull; they also add it up: the bias gradient, in
+//                FP32, without another pass over it;
+//   warp 1:      after `ready` and gfull, 3 x W/16 MMAs, committed to gfree and to `free` of the row
+//                that is not used again. The warp stays together, lane 0 issues.
+// Every wait is bounded and also ends when another role gave up (a shared abort word); the last
+// copies land and a last commit is waited for before the tensor memory is freed. Each CTA's partial
+// sums (read back with tcgen05.ld) go to `part` and k_gen_sum_parts adds the partials in a fixed
+// order.
+// What bounds it: the issue of the bulk copies, about 100 cycles each whatever their size, and the
+// reads of the operands from shared memory (68 x 128 bytes per MMA of 72 cycles). In blocks of 64
+// positions with three rows of input and the raw gradient copied for each (30 copies) it took 63 us
+// for 16 x 128^2 (75 MB: 11 us at the copy rate), of which the copies' issue 2 us per block; now
+// 29 us, with the bias gradient (13 us per layer as launches of its own): 21 us of K-blocks, 5 us
+// to write the partials.
 // ------------------------------------------------------------------------------------------
 namespace wg {
-constexpr int kWMax = 64;                                 // positions per K-block at most
+constexpr int kWMax = 128;                                // positions per K-block at most
 constexpr int kSlotA = (kWMax + 2) * 16;                  // bytes per input slot (with the halo)
-constexpr int kSlot = kWMax * 16;                         // bytes per gradient slot (raw or BF16)
-constexpr int kBytesA = 3 * 8 * kSlotA;                   // 25344: 3 row blocks x 8 slots
-constexpr int kBytesR = tc::kC / 4 * kSlot;               // 12288: raw FP32 gradient, 12 slots
-constexpr int kBytesB = tc::kC / 8 * kSlot;               // 6144: BF16 gradient, 6 slots (hi or lo)
-constexpr int kStages = 4;
-constexpr int kStage = kBytesA + kBytesR + 2 * kBytesB;   // 49920: one ring slot
+constexpr int kSlot = kWMax * 16;                         // bytes per gradient slot
+constexpr int kRowB = tc::kC / 8 * kSlotA;                // 12480: 6 slots of an input row
+constexpr int kRows = 9;                                  // ring of input rows
+constexpr int kBytesA = (kRows * kRowB + 127) / 128 * 128;
+constexpr int kStage = 16 * kSlot;                        // 32768: BF16 gradient, hi and lo, 8 slots each
+constexpr int kStages = 3;
 constexpr int kThreads = 512;
-constexpr int kConvWarps = kThreads / 32 - 2;
-constexpr int kCols = 512;                                // six accumulators at 64-column steps
-constexpr size_t kSmem = (size_t)kStages * kStage + 1024;
-// BF16 A and B, both MN-major (instruction-descriptor bits 15 and 16), N = 48, M = 128
-constexpr uint32_t kIdesc = tc::idesc<0, tc::kC>() | (1u << 15) | (1u << 16);
+constexpr int kConv = 384;                                // converting threads, warps 4-15
+constexpr int kN = 3 * tc::kC;                            // 144 columns: (row, input channel)
+constexpr int kAccCols = 160;                             // step of the accumulators
+constexpr int kCols = 512;                                // columns allocated (a power of two)
+constexpr size_t kSmem = (size_t)kBytesA + kStages * kStage + 1024;
+constexpr int kPart = 9 * tc::kC * tc::kC + tc::kC;       // floats per partial: weights, then biases
+static_assert((3 * kN * tc::kC + 8 * kConv) * 4 <= kBytesA + kStages * kStage, "epilogue scratch in the rings");
+// BF16 A and B, both MN-major (instruction-descriptor bits 15 and 16), N columns, M = 128
+__device__ __forceinline__ uint32_t idesc(int n) { return tc::idesc_n<0>((uint32_t)n) | (1u << 15) | (1u << 16); }
 // K-block length for an L x L image (0: the tensor-core form does not apply)
 __host__ __device__ constexpr int block_len(int L) {
-    return (L % 16 != 0) ? 0 : (L <= kWMax ? L : (L % kWMax == 0 ? kWMax : 0));
-}
-__device__ __forceinline__ void mma(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-        "l"(ad), "l"(bd), "r"(kIdesc), "r"(acc)
-        : "memory");
-}
-__device__ __forceinline__ void bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
+    return (L % 16 != 0) ? 0 : (L <= 64 || L == kWMax ? L : (L % 64 == 0 ? 64 : 0));
 }
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
-}
-// bounded wait for phase `parity` of `bar`; gives up (abort word and error flag set) after
-// `limit` polls or as soon as another role has given up
-__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort, int* flag) {
-    for (unsigned it = 0; it < tc::kWaitLimit; ++it) {
-        if (gen_mbar_try_wait(bar, parity)) return true;
-        if (*abort) return false;
-    }
-    *abort = 1;
-    atomicExch(flag, 4);
-    return false;
 }
 }  // namespace wg
 
@@ -1240,24 +1178,27 @@ k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ d
     seq_begin();
     using namespace wg;
     constexpr int kC = tc::kC, W = 16 * KS;
+    constexpr int kJobs = kC / 8 * W;                       // (channel group, position) of a K-block
+    constexpr int kPer = (kJobs + kConv - 1) / kConv;       // of these per converting thread, kStep apart
+    constexpr int kStep = kJobs / kPer;                     // = converting threads in use
+    static_assert(kJobs % kPer == 0 && kStep % 32 == 0 && W % (W / kPer) == 0, "whole warps");
     extern __shared__ uint8_t wsm_raw[];
-    __shared__ __align__(8) unsigned long long loaded[kStages], full[kStages], empty[kStages];
+    __shared__ __align__(8) unsigned long long copied[kRows], ready[kRows], rfree[kRows], gfull[kStages], gfree[kStages], done;
     __shared__ uint32_t tmem_slot;
-    __shared__ int last_mma;
     __shared__ volatile int abort_word;
     uint8_t* smem = (uint8_t*)(((uintptr_t)wsm_raw + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const size_t LL = (size_t)L * L;
-    const int bpr = L / W;                                  // K-blocks per image row
-    const uint32_t sbase = gen_smem_u32(smem);
-    const int first = blockIdx.x, stride = gridDim.x;
-    const int n = (nkb > first) ? (nkb - first + stride - 1) / stride : 0;
+    const int bpr = L / W;                                  // strips of W columns
+    const uint32_t sbase = gen_smem_u32(smem), gbase = sbase + (uint32_t)kBytesA;
+    // K-blocks [b0, b1) of the batch, ordered by image, strip, row: segments of one strip each
+    const int b0 = (int)((long long)nkb * blockIdx.x / gridDim.x), b1 = (int)((long long)nkb * (blockIdx.x + 1) / gridDim.x);
 
-    // the zero slots 6 and 7 of each row block, in every ring slot (never copied over)
-    for (int i = tid; i < kStages * 3 * 2 * (kSlotA / 16); i += kThreads) {
-        const int c = i % (kSlotA / 16), s = i / (kSlotA / 16);
-        const int st = s / 6, slot = (s % 6) / 2 * 8 + 6 + s % 2;
-        *reinterpret_cast<uint4*>(smem + st * kStage + slot * kSlotA + c * 16) = make_uint4(0, 0, 0, 0);
+    // the zero slots 6, 7, 14 and 15 of the gradient, in every stage (never written again)
+    for (int i = tid; i < kStages * 4 * (kSlot / 16); i += kThreads) {
+        const int c = i % (kSlot / 16), s = i / (kSlot / 16);
+        const int st = s / 4, slot = (s % 4) / 2 * 8 + 6 + s % 2;
+        *reinterpret_cast<uint4*>(smem + kBytesA + st * kStage + slot * kSlot + c * 16) = make_uint4(0, 0, 0, 0);
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gen_smem_u32(&tmem_slot)),
@@ -1266,14 +1207,17 @@ k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ d
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&loaded[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gen_smem_u32(&full[s])), "r"(kConvWarps)
-                         : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&empty[s])) : "memory");
+        for (int s = 0; s < kRows; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&copied[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&ready[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&rfree[s])) : "memory");
         }
+        for (int s = 0; s < kStages; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gen_smem_u32(&gfull[s])), "r"(kStep / 32) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&gfree[s])) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&done)) : "memory");
         abort_word = 0;
-        last_mma = -1;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // the zeroed slots are read by the tensor cores (async proxy)
@@ -1282,144 +1226,219 @@ k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ d
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    auto par = [](int j) { return (uint32_t)(j / kStages) & 1u; };
+    if (warp < 4) {   // the accumulators start at zero
+        for (int c = 0; c < 3 * kAccCols; c += 16) tmem_zero16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    if (warp == 0) {   // producer: lane 0 waits and sets the byte count, lanes 0-29 copy
-        constexpr uint32_t kTx = 3u * (kC / 8) * (W + 2) * 16 + (kC / 4) * W * 16;
-        int hi_fill = -1;
-        for (int j = 0; j < n; ++j) {
-            const int s = j % kStages;
-            if (j >= kStages) {
-                const bool ok = lane == 0 ? wait(gen_smem_u32(&empty[s]), par(j - kStages), &abort_word, flag) : true;
-                if (!__shfl_sync(0xFFFFFFFFu, ok, 0)) break;
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            }
-            const int kb = first + j * stride;
-            const int img = kb / (L * bpr), rem = kb - img * (L * bpr);
-            const int y = rem / bpr, x0 = (rem - y * bpr) * W;
-            const uint32_t bar = gen_smem_u32(&loaded[s]);
-            const uint32_t sA = sbase + (uint32_t)(s * kStage), sR = sA + (uint32_t)kBytesA;
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTx) : "memory");
-            __syncwarp();
-            if (lane < 3 * (kC / 8)) {   // input rows y-1, y, y+1 of channel group h
-                const int R = lane / (kC / 8), h = lane - R * (kC / 8);
-                const int yy = (y + R - 1 + L) % L;
-                const __nv_bfloat16* row = in + (((size_t)img * (kC / 8) + h) * LL + (size_t)yy * L) * 8;
-                const uint32_t dst = sA + (uint32_t)((R * 8 + h) * kSlotA);
-                int c = 0;
-                while (c < W + 2) {   // runs of columns x0-1 .. x0+W, split at the periodic edge
-                    const int x = (x0 - 1 + c + L) % L;
-                    const int run = min(W + 2 - c, L - x);
-                    bulk(dst + (uint32_t)(c * 16), row + (size_t)x * 8, (uint32_t)run * 16, bar);
-                    c += run;
+    const int ct = tid - (kThreads - kConv);                // converting thread
+    float bsum[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    bool ok = true;
+    if (warp == 0) {
+        int q = 0;   // rows copied
+        for (int b = b0; b < b1 && ok;) {
+            const int st = b / L, y0 = b - st * L, len = min(b1 - b, L - y0), img = st / bpr, x0 = (st - img * bpr) * W;
+            // columns x0-1 .. x0+W: what lies inside the row, then a neighbour across the periodic edge
+            const bool left = x0 == 0, right = x0 + W == L, own = bpr == 1;
+            const int xa = left ? 0 : x0 - 1, xb = right ? L : x0 + W + 1;
+            const uint32_t tx = (uint32_t)(kC / 8) * 16u * (uint32_t)(xb - xa + (own ? 0 : (int)left + (int)right));
+            for (int i = 0; i < len + 2; ++i, ++q) {
+                const int s = q % kRows;
+                if (q >= kRows) {
+                    ok = gen_wait(gen_smem_u32(&rfree[s]), (uint32_t)(q / kRows - 1) & 1u, &abort_word, flag, 4);
+                    if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 }
-            } else if (lane < 3 * (kC / 8) + kC / 4) {   // gradient slot g (4 channels)
-                const int g = lane - 3 * (kC / 8);
-                bulk(sR + (uint32_t)(g * kSlot), dout + (((size_t)img * (kC / 4) + g) * LL + (size_t)y * L + x0) * 4,
-                     (uint32_t)W * 16, bar);
+                int yy = y0 + i - 1;
+                yy += yy < 0 ? L : (yy >= L ? -L : 0);
+                const uint32_t bar = gen_smem_u32(&copied[s]);
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tx) : "memory");
+                __syncwarp();
+                if (lane < kC / 8) {
+                    const __nv_bfloat16* row = in + (((size_t)img * (kC / 8) + lane) * LL + (size_t)yy * L) * 8;
+                    const uint32_t dst = sbase + (uint32_t)(s * kRowB + lane * kSlotA);
+                    gen_bulk(dst + (left ? 16u : 0u), row + (size_t)xa * 8, (uint32_t)(xb - xa) * 16, bar);
+                    if (!own && left) gen_bulk(dst, row + (size_t)(L - 1) * 8, 16u, bar);
+                    if (!own && right) gen_bulk(dst + (W + 1) * 16u, row, 16u, bar);
+                }
+                __syncwarp();
             }
-            hi_fill = j;
+            b += len;
         }
-        // the last fill of every slot lands before the CTA's shared memory can be released
+        // the last copy into every row buffer lands before the CTA's shared memory can be released
         if (lane == 0)
-            for (int j = max(0, hi_fill - kStages + 1); j <= hi_fill; ++j)
+            for (int j = max(0, q - kRows); j < q; ++j)
                 for (unsigned it = 0; it < (tc::kWaitLimit >> 4); ++it)
-                    if (gen_mbar_try_wait(gen_smem_u32(&loaded[j % kStages]), par(j))) break;
+                    if (gen_mbar_try_wait(gen_smem_u32(&copied[j % kRows]), (uint32_t)(j / kRows) & 1u)) break;
     } else if (warp == 1) {
-        if (lane == 0) {   // MMA issuer
-            for (int k = 0; k < n; ++k) {
-                const int s = k % kStages;
-                if (!wait(gen_smem_u32(&loaded[s]), par(k), &abort_word, flag) ||
-                    !wait(gen_smem_u32(&full[s]), par(k), &abort_word, flag))
-                    break;
+        const bool lead = elect_one();
+        const uint64_t a00 = umma_desc(gbase, 128, kSlot), b00 = umma_desc(sbase, 128, kSlotA);
+        const uint32_t alo = (uint32_t)a00, ahi = (uint32_t)(a00 >> 32), blo = (uint32_t)b00, bhi = (uint32_t)(b00 >> 32);
+        int q0 = 0, k = 0;   // first row of the segment in the order of copies; K-blocks issued
+        for (int b = b0; b < b1 && ok;) {
+            const int len = min(b1 - b, L - b % L);
+            for (int j = 0; j < len; ++j, ++k) {
+                const int g = k % kStages, s = (q0 + j) % kRows;
+                for (int a = j ? q0 + j + 2 : q0; a <= q0 + j + 2 && ok; ++a)
+                    ok = gen_wait(gen_smem_u32(&ready[a % kRows]), (uint32_t)(a / kRows) & 1u, &abort_word, flag, 4);
+                ok = ok && gen_wait(gen_smem_u32(&gfull[g]), (uint32_t)(k / kStages) & 1u, &abort_word, flag, 4);
+                if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 // MN-major, no swizzle: LBO = 128 (8-position K groups), SBO = one slot (8-channel
                 // MN groups); the start address field (bits 0-13, address >> 4) is offset per MMA
-                const uint32_t sA = sbase + (uint32_t)(s * kStage);
-                const uint64_t a0 = umma_desc(sA, 128, kSlotA);
-                const uint64_t b0 = umma_desc(sA + (uint32_t)(kBytesA + kBytesR), 128, kSlot);
+                const uint32_t as = alo + ((uint32_t)(g * kStage) >> 4), bs = blo + ((uint32_t)(s * kRowB) >> 4);
+                const int n1 = min(3, kRows - s) * kC, n2 = kN - n1;   // columns up to the ring's end, and after it
+                const uint32_t i1 = idesc(n1), i2 = idesc(n2), d2 = tmem + (uint32_t)n1;
+                if (lead) {
 #pragma unroll
-                for (int t = 0; t < 6; ++t) {
-                    const int dxi = t >> 1, pq = t & 1;
+                    for (int m = 0; m < 3 * KS; ++m)
+                        tc_mma_n<0>(tmem + (uint32_t)(m / KS * kAccCols), as + (uint32_t)((m % KS * 256) >> 4), ahi,
+                                    bs + (uint32_t)(m / KS + 16 * (m % KS)), bhi, i1);
+                    if (n2) {   // the rest, at the ring's start
 #pragma unroll
-                    for (int ks = 0; ks < KS; ++ks) {
-                        const uint64_t ad = a0 + (uint64_t)((pq * 8 * kSlotA + (dxi + 16 * ks) * 16) >> 4);
-                        mma(tmem + (uint32_t)(t * 64), ad, b0 + (uint64_t)((ks * 256) >> 4), (k | ks) ? 1u : 0u);
-                        mma(tmem + (uint32_t)(t * 64), ad, b0 + (uint64_t)((kBytesB + ks * 256) >> 4), 1u);
+                        for (int m = 0; m < 3 * KS; ++m)
+                            tc_mma_n<0>(d2 + (uint32_t)(m / KS * kAccCols), as + (uint32_t)((m % KS * 256) >> 4), ahi,
+                                        blo + (uint32_t)(m / KS + 16 * (m % KS)), bhi, i2);
+                    }
+                    gen_commit(gen_smem_u32(&gfree[g]));
+                    gen_commit(gen_smem_u32(&rfree[s]));
+                    if (j == len - 1) {   // the segment's last two rows
+                        gen_commit(gen_smem_u32(&rfree[(q0 + len) % kRows]));
+                        gen_commit(gen_smem_u32(&rfree[(q0 + len + 1) % kRows]));
                     }
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 gen_smem_u32(&empty[s]))
-                             : "memory");
-                last_mma = k;
+                __syncwarp();
+            }
+            q0 += len + 2;
+            b += len;
+        }
+        // every MMA has completed before the accumulators are read or freed
+        if (lead) {
+            gen_commit(gen_smem_u32(&done));
+            bool drained = false;
+            for (unsigned it = 0; it < tc::kWaitLimit && !drained; ++it) drained = gen_mbar_try_wait(gen_smem_u32(&done), 0);
+            if (!drained) {
+                atomicExch(flag, 4);
+                ok = false;
             }
         }
-    } else {   // converters
-        const int ct = tid - 64;
-        for (int j = 0; j < n; ++j) {
-            const int s = j % kStages;
-            if (!wait(gen_smem_u32(&loaded[s]), par(j), &abort_word, flag)) break;
-            const uint8_t* sR = smem + s * kStage + kBytesA;
-            uint8_t* sB = smem + s * kStage + kBytesA + kBytesR;
-            for (int job = ct; job < (kC / 8) * W; job += kConvWarps * 32) {
-                const int h = job / W, c = job - h * W;
-                const float4 a = *reinterpret_cast<const float4*>(sR + 2 * h * kSlot + c * 16);
-                const float4 b = *reinterpret_cast<const float4*>(sR + (2 * h + 1) * kSlot + c * 16);
-                const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                uint32_t hi[4], lo[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    hi[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
-                    lo[e] = pack_bf16(f[2 * e] - __uint_as_float(hi[e] << 16),
-                                      f[2 * e + 1] - __uint_as_float(hi[e] & 0xFFFF0000u));
-                }
-                *reinterpret_cast<uint4*>(sB + h * kSlot + c * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(sB + kBytesB + h * kSlot + c * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        __syncwarp();
+    } else if (warp == 2) {
+        int n = 0;   // rows of this CTA, with the two beside each segment
+        for (int b = b0; b < b1; n += 2) {
+            const int len = min(b1 - b, L - b % L);
+            n += len;
+            b += len;
+        }
+        for (int q = 0; q < n; ++q) {
+            const int s = q % kRows;
+            ok = gen_wait(gen_smem_u32(&copied[s]), (uint32_t)(q / kRows) & 1u, &abort_word, flag, 4);
+            if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
+            if (bpr == 1 && lane < 2 * (kC / 8)) {   // slot 0 <- column W-1 (slot W), slot W+1 <- column 0
+                uint8_t* blk = smem + s * kRowB + (lane >> 1) * kSlotA;
+                const int to = (lane & 1) ? W + 1 : 0, from = (lane & 1) ? 1 : W;
+                *(uint4*)(blk + to * 16) = *(const uint4*)(blk + from * 16);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&full[s])) : "memory");
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&ready[s])) : "memory");
+        }
+    } else if (ct >= 0 && ct < kStep) {
+        // converters: channel group h at the positions c + i W / kPer of every K-block
+        constexpr int kWs = W / kPer;
+        const int h = ct / kWs, c = ct - h * kWs, n = b1 - b0;
+        float4 nx[kPer][2];   // the next K-block's gradient
+        auto fetch = [&](int b) {
+            const int st = b / L, y = b - st * L, img = st / bpr, x0 = (st - img * bpr) * W;
+            const float4* p = reinterpret_cast<const float4*>(dout) + ((size_t)img * (kC / 4) + 2 * h) * LL + (size_t)y * L + x0 + c;
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) {
+                nx[i][0] = __ldcg(p + i * kWs);
+                nx[i][1] = __ldcg(p + LL + i * kWs);
+            }
+        };
+        if (n > 0) fetch(b0);
+        for (int k = 0; k < n; ++k) {
+            const int g = k % kStages;
+            float f[kPer][8];
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) {
+                const float4 a = nx[i][0], b = nx[i][1];
+                f[i][0] = a.x, f[i][1] = a.y, f[i][2] = a.z, f[i][3] = a.w;
+                f[i][4] = b.x, f[i][5] = b.y, f[i][6] = b.z, f[i][7] = b.w;
+            }
+            if (k + 1 < n) fetch(b0 + k + 1);
+            if (k >= kStages) {
+                ok = gen_wait(gen_smem_u32(&gfree[g]), (uint32_t)(k / kStages - 1) & 1u, &abort_word, flag, 4);
+                if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
+            }
+            uint8_t* sG = smem + kBytesA + g * kStage;
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    hi[e] = pack_bf16(f[i][2 * e], f[i][2 * e + 1]);
+                    lo[e] = pack_bf16(f[i][2 * e] - __uint_as_float(hi[e] << 16),
+                                      f[i][2 * e + 1] - __uint_as_float(hi[e] & 0xFFFF0000u));
+                }
+                *reinterpret_cast<uint4*>(sG + h * kSlot + (c + i * kWs) * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(sG + (8 + h) * kSlot + (c + i * kWs) * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&gfull[g])) : "memory");
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) bsum[e] += f[i][e];
         }
     }
-    __syncthreads();
-    // all issued MMAs (they complete in order) before the accumulators are read or freed
-    bool ok = true;
-    if (tid == 0) {
-        const int lm = last_mma;
-        if (lm >= 0) {
-            bool done = false;
-            for (unsigned it = 0; it < tc::kWaitLimit && !done; ++it)
-                done = gen_mbar_try_wait(gen_smem_u32(&empty[lm % kStages]), par(lm));
-            if (!done) atomicExch(flag, 4);
-            ok = done && lm == n - 1 && !abort_word;
-        } else {
-            ok = n == 0 && !abort_word;
-        }
-    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     if (!__syncthreads_or(!ok)) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // epilogue: job = (tile, lane quarter); a warp reads its own quarter (warp % 4)
-        for (int job = warp; job < 24; job += kThreads / 32) {
-            const int t = job >> 2, q = job & 3, dxi = t >> 1, pq = t & 1;
-            if (pq == 1 && q < 2) continue;                 // tile Q's first half repeats tile P's
-            const int row = q * 32 + lane, ci = row & 63, dy = pq + (row >> 6) - 1;
-            float v[kC];
-            if (n > 0) {
-                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(t * 64);
-                tmem_ld16(taddr + 0, v);
-                tmem_ld16(taddr + 16, v + 16);
-                tmem_ld16(taddr + 32, v + 32);
+        // epilogue: a warp reads its own lane quarter q = warp % 4 in chunks of 16 columns; the lo
+        // quarters (2, 3) leave theirs in the ring's memory, the hi quarters add them and store
+        const int q = warp & 3, co = (q & 1) * 32 + lane;
+        float* slo = reinterpret_cast<float*>(smem);                  // [432 columns][48]
+        float* sbs = slo + 3 * kN * kC;                               // [8][converting thread]
+        float* dst = part + (size_t)blockIdx.x * kPart;
+        if (ct >= 0 && ct < kStep)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sbs[e * kStep + ct] = bsum[e];
+        float v[16];
+        const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
+        if (q >= 2)
+            for (int c = warp >> 2; c < 27; c += 4) {
+                tmem_ld16(tq + (uint32_t)(c / 9 * kAccCols + c % 9 * 16), v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            } else {
+                if (co < kC)
 #pragma unroll
-                for (int c = 0; c < kC; ++c) v[c] = 0.0f;
+                    for (int e = 0; e < 16; ++e) slo[(c * 16 + e) * kC + co] = v[e];
             }
-            if (ci < kC) {
-                const int r = ((dy + 1) * 3 + dxi) * kC + ci;
-                float4* dst = reinterpret_cast<float4*>(part + ((size_t)blockIdx.x * 9 * kC + r) * kC);
+        __syncthreads();
+        if (q < 2) {
+            for (int c = warp >> 2; c < 27; c += 4) {
+                const int dxi = c / 9, R = c % 9 / 3, ci0 = c % 3 * 16;
+                tmem_ld16(tq + (uint32_t)(dxi * kAccCols + c % 9 * 16), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (co < kC)
 #pragma unroll
-                for (int c = 0; c < kC / 4; ++c) dst[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                    for (int e = 0; e < 16; ++e)
+                        dst[((R * 3 + dxi) * kC + ci0 + e) * kC + co] = v[e] + slo[(c * 16 + e) * kC + co];
+            }
+        } else {   // biases: 8 warps x 6 channels, the positions in a fixed order
+            const int i = (warp >> 2) * 2 + (q & 1);
+            for (int ch = i * (kC / 8); ch < (i + 1) * (kC / 8); ++ch) {
+                float s = 0.0f;
+                for (int c = lane; c < W / kPer; c += 32) s += sbs[(ch & 7) * kStep + (ch >> 3) * (W / kPer) + c];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+                if (lane == 0) dst[9 * kC * kC + ch] = s;
             }
         }
     } else if (tid == 0) {
@@ -1630,24 +1649,39 @@ k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__
         }
 }
 
-// out[i] = the sum of nparts partials in order, the loads of 16 of them in flight at a time (one
-// at a time, each waited for the last: 13 us for 152 partials of 20736 weights, now 9.6 us).
-__global__ void __launch_bounds__(64)
-k_gen_sum_parts(const float* __restrict__ part, int nparts, int n, float* __restrict__ out) {
+// The sum of nparts partials of `stride` floats: the first nw of them to gw, the rest to gb. A block
+// takes 16 groups of four outputs, 8 threads each the partials t, t + 8, ... of a group, added in
+// a fixed order at the end. One thread per output had too few loads in flight: 9.6 us for 152
+// partials of 20736 weights, now 6.5 us.
+__global__ void __launch_bounds__(128)
+k_gen_sum_parts(const float* __restrict__ part, int nparts, int stride, float* __restrict__ gw, int nw, int n,
+                float* __restrict__ gb) {
     seq_begin();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float s = 0.0f;
-    int p = 0;
-    for (; p + 16 <= nparts; p += 16) {
-        float v[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = __ldcg(part + (size_t)(p + k) * n + i);
-#pragma unroll
-        for (int k = 0; k < 16; ++k) s += v[k];
+    __shared__ float4 red[8][16];
+    const int o = threadIdx.x & 15, t = threadIdx.x >> 4, i = (blockIdx.x * 16 + o) * 4;
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (i < n) {
+#pragma unroll 10
+        for (int p = t; p < nparts; p += 8) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(part + (size_t)p * stride + i));
+            s.x += v.x;
+            s.y += v.y;
+            s.z += v.z;
+            s.w += v.w;
+        }
     }
-    for (; p < nparts; ++p) s += __ldcg(part + (size_t)p * n + i);
-    out[i] = s;
+    red[t][o] = s;
+    __syncthreads();
+    if (threadIdx.x >= 16 || i >= n) return;
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+        const float4 v = red[k][o];
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
+    }
+    *reinterpret_cast<float4*>(i < nw ? gw + i : gb + (i - nw)) = s;
 }
 
 // Sum of many partials for few outputs: block i adds part[0..nparts)[i], thread t the parts
@@ -1716,7 +1750,7 @@ k_gen_bgrad_part(const float* __restrict__ dout, int LL, int cout, int nseg, flo
 // Adam steps, BF16 copies and operand images were 46 launches of about 3 us): thread i of layer
 // blockIdx.y steps weight i, then the biases (adam != 0), and writes wb[tap][ci][co], the flipped
 // transpose wt[8-tap][co][ci], and where the layer has them its images in the B-operand layout
-// k_gen_conv_tma uses in shared memory: per tap, NN/8 x KCH core matrices of 8 rows (n) x 16 bytes
+// k_gen_conv_row uses in shared memory: per tap, NN/8 x KCH core matrices of 8 rows (n) x 16 bytes
 // (8 BF16 or 4 TF32 consecutive k); entries past cin and cout stay zero from the allocation.
 struct UpdateArgs {
     GenLayer layer[kGenLayers];
@@ -1749,10 +1783,10 @@ __global__ void __launch_bounds__(128) k_gen_update(const __grid_constant__ Upda
     y.wb[i] = v;
     y.wt[((8 - tap) * cout + co) * cin + ci] = v;
     const int kch = y.kch, nn = (cout + 15) / 16 * 16;
-    *reinterpret_cast<__nv_bfloat16*>(y.wimg + tap * (nn / 8) * kch * 128 + ((co >> 3) * kch + ci / 8) * 128 + (co & 7) * 16 +
+    *reinterpret_cast<__nv_bfloat16*>(y.wimg + row::place(tap) * (nn / 8) * kch * 128 + ((co >> 3) * kch + ci / 8) * 128 + (co & 7) * 16 +
                                       (ci % 8) * 2) = v;
     if (y.wtimg)   // hidden layers: wt's k is co, its n is ci
-        *reinterpret_cast<float*>(y.wtimg + (8 - tap) * (kGenC / 8) * (kGenC / 4) * 128 +
+        *reinterpret_cast<float*>(y.wtimg + row::place(8 - tap) * (kGenC / 8) * (kGenC / 4) * 128 +
                                   ((ci >> 3) * (kGenC / 4) + co / 4) * 128 + (ci & 7) * 16 + (co % 4) * 4) =
             __bfloat162float(v);
 }
@@ -1943,94 +1977,29 @@ int conv_launch(nmmc_gen* g, const TIN* in, const __nv_bfloat16* w, const float*
 
 // Hidden-layer convolution on the tensor cores: persistent CTAs, as many per SM as the shared
 // memory allows (two for the BF16 modes at L = 128, one for the TF32 data gradient).
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled() {
-    static const EncodeTiledFn fn = []() -> EncodeTiledFn {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            return nullptr;
-        return (EncodeTiledFn)p;
-    }();
-    return fn;
-}
 
-// Tensor map of chunk-planar activations [nimg][ICH][L][L][epc] (ICH chunks of epc channels)
-// for the TMA-fed convolutions (L = 128): dimensions (element of a chunk, x, y, chunk, image),
-// so that one box [epc, 130, 1, 1, 1] at x = -1 is one (row, chunk) block of a window, 2080
-// contiguous bytes of which the two edge positions fall outside the row and are zero-filled.
-template <int MODE, int ICH = tc::chunks<MODE>()>
-int window_map(const typename tc::Traits<MODE>::TA* in, int L, int nimg, CUtensorMap* map) {
-    const EncodeTiledFn enc = encode_tiled();
-    if (!enc) return set_error(NMMC_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-    constexpr int kEpc = tc::Traits<MODE>::kEpc, kCh = ICH;
-    const cuuint64_t l = (cuuint64_t)L;
-    const cuuint64_t dims[5] = {(cuuint64_t)kEpc, l, l, (cuuint64_t)kCh, (cuuint64_t)nimg};
-    const cuuint64_t strides[4] = {16, 16ull * l, 16ull * l * l, 16ull * kCh * l * l};
-    const cuuint32_t box[5] = {(cuuint32_t)kEpc, (cuuint32_t)tma::kSlots, 1, 1, 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    const CUresult r = enc(map, MODE == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5,
-                           (void*)in, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return set_error(NMMC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-    return NMMC_OK;
-}
-
-// single-role kernel (every mode and layer shape) in tiles of NMMC_GEN_OPT_TILE_ROWS output rows
-// (default 2); the TF32 data gradient's window and weights leave room for one CTA per SM.
-template <int MODE, int ICH, int KCH, int CO, int R>
-int conv_tma_launch_r(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w, const uint8_t* wimg,
-                      const float* bias, const __nv_bfloat16* mask, void* out, int nimg) {
-    const int smem = tma::smem_bytes<MODE, ICH, KCH, CO, R>();
-    if (int rc = ensure_smem(g, (const void*)k_gen_conv_tma<MODE, ICH, KCH, CO, R>, smem, true)) return rc;
-    const int per_sm = std::max(1, std::min(2, g->smem_per_sm / (smem + 2048)));
-    const int ntiles = nimg * g->L / R;
-    const int grid = std::min(ntiles, per_sm * g->sm_count);
-    launch_seq(g->stream, k_gen_conv_tma<MODE, ICH, KCH, CO, R>, dim3(grid), 128, smem, in, w, wimg, bias, mask, out, ntiles,
-                                                                          g->d_flag);
-    return cuda_check(cudaGetLastError(), "k_gen_conv_tma");
-}
-
-// wimg: the layer's weight image (nullptr: the threads rearrange w)
+// L = 128: the row-ring kernel (every mode and layer shape), one CTA per SM. wimg: the layer's
+// weight image (nullptr: the threads rearrange w).
 template <int MODE, int ICH = tc::chunks<MODE>(), int KCH = ICH, int CO = tc::kC>
-int conv_tma_launch(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w, const float* bias,
+int conv_row_launch(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w, const float* bias,
                     const __nv_bfloat16* mask, void* out, int nimg, const uint8_t* wimg = nullptr) {
-    if (!g->use_wimg) wimg = nullptr;
-    if (g->tile_rows == 2) return conv_tma_launch_r<MODE, ICH, KCH, CO, 2>(g, in, w, wimg, bias, mask, out, nimg);
-    return conv_tma_launch_r<MODE, ICH, KCH, CO, 1>(g, in, w, wimg, bias, mask, out, nimg);
+    constexpr int smem = row::smem_bytes<KCH, CO>();
+    if (int rc = ensure_smem(g, (const void*)k_gen_conv_row<MODE, ICH, KCH, CO>, smem, true)) return rc;
+    const int nrows = nimg * g->L;
+    launch_seq(g->stream, k_gen_conv_row<MODE, ICH, KCH, CO>, dim3(std::min(nrows, g->sm_count)), row::kThreads, smem, in, w,
+               g->use_wimg ? wimg : nullptr, bias, mask, out, nrows, g->d_flag);
+    return cuda_check(cudaGetLastError(), "k_gen_conv_row");
 }
 
 // The first (8 -> 48, ReLU) and last (48 -> 4, linear) layers on the tensor cores when L = 128
-// and the TMA path is on; false when they run on the FMA pipes.
-bool edge_layers_on_tc(const nmmc_gen* g) { return g->use_tc && g->use_tma && g->L == tc::kM; }
-
-// warp-specialised TMA kernel (BF16 modes), one CTA per SM
-template <int MODE>
-int conv_tmaws_launch(nmmc_gen* g, const __nv_bfloat16* in, const __nv_bfloat16* w, const float* bias, void* out,
-                      int nimg) {
-    alignas(64) CUtensorMap map;
-    if (int rc = window_map<MODE>(in, g->L, nimg, &map)) return rc;
-    const int smem = tmaws_smem_bytes<MODE>();
-    if (int rc = ensure_smem(g, (const void*)k_gen_conv_tmaws<MODE>, smem, true)) return rc;
-    const int ntiles = nimg * g->L;
-    const int grid = std::min(ntiles, g->sm_count);
-    k_gen_conv_tmaws<MODE><<<grid, kTwsThreads, smem, g->stream>>>(map, w, bias, out, ntiles, g->d_flag);
-    return cuda_check(cudaGetLastError(), "k_gen_conv_tmaws");
-}
+// and the row-ring kernels are on; false when they run on the FMA pipes.
+bool edge_layers_on_tc(const nmmc_gen* g) { return g->use_tc && g->use_rows && g->L == tc::kM; }
 
 template <int MODE>
 int conv_tc_launch(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w, const float* bias,
                    const __nv_bfloat16* mask, void* out, int nimg, const uint8_t* wimg = nullptr) {
-    if (g->use_tma && g->L == tc::kM && !(MODE != 2 && g->use_ws)) {
-        if constexpr (MODE != 2)
-            if (g->use_tma == 2) return conv_tmaws_launch<MODE>(g, in, w, bias, out, nimg);
-        return conv_tma_launch<MODE>(g, in, w, bias, mask, out, nimg, wimg);
-    }
+    if (g->use_rows && g->L == tc::kM && !(MODE != 2 && g->use_ws))
+        return conv_row_launch<MODE>(g, in, w, bias, mask, out, nimg, wimg);
     if constexpr (MODE != 2) {   // BF16 modes: the warp-specialised kernel when two windows fit
         const int ws = ws_smem_bytes<MODE>(g->L);
         if (g->use_ws && ws <= tc::kSmemMax) {
@@ -2068,19 +2037,38 @@ int check_flag(nmmc_gen* g) {
     return set_error(NMMC_ERR_TIMEOUT, "a tensor-core convolution gave up waiting for its MMAs (code %d)", f);
 }
 
-// Hidden-layer weight gradient on the tensor cores (k_gen_wgrad_tc): as many CTAs as SMs (one
+// Bias gradient gb[co] = sum over the batch's pixels of dout[p, co] (wpart as scratch).
+int bgrad_launch(nmmc_gen* g, const float* dout, int nimg, int cout, float* gb) {
+    const int LL = g->L * g->L, nseg = (LL + kBgradRun - 1) / kBgradRun;
+    if (cout % 4 != 0 || cout > 256) return set_error(NMMC_ERR_ARG, "bias gradient: channels not a multiple of 4");
+    if ((size_t)nimg * nseg * cout > g->wpart_cap) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
+    launch_seq(g->stream, k_gen_bgrad_part, dim3(nseg, cout / 4, nimg), 256, 0, dout, LL, cout, nseg, g->wpart);
+    launch_seq(g->stream, k_gen_sum_parts_wide, dim3(cout), 128, 0, g->wpart, nimg * nseg, cout, gb);
+    return cuda_check(cudaGetLastError(), "k_gen_bgrad_part");
+}
+
+// gw (and gb, where the partials carry biases) from the partials in wpart
+void sum_parts(nmmc_gen* g, int nparts, int stride, float* gw, int nw, float* gb) {
+    const int n = gb ? stride : nw;   // multiples of four
+    launch_seq(g->stream, k_gen_sum_parts, dim3((n / 4 + 15) / 16), 128, 0, g->wpart, nparts, stride, gw, nw, n, gb);
+}
+
+// Hidden-layer weight and bias gradient on the tensor cores (k_gen_wgrad_tc): as many CTAs as SMs (one
 // per SM), as the partial scratch holds and as there are K-blocks.
-int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, int nimg) {
-    const size_t n = (size_t)9 * tc::kC * tc::kC;
+int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, float* gb, int nimg) {
+    const int nw = 9 * tc::kC * tc::kC;
     const int W = wg::block_len(g->L);
     const int nkb = (int)((size_t)nimg * g->L * (g->L / W));
-    const int nparts = (int)std::min<size_t>({(size_t)nkb, (size_t)std::max(1, g->sm_count), g->wpart_cap / n});
+    const int nparts = (int)std::min<size_t>({(size_t)nkb, (size_t)std::max(1, g->sm_count), g->wpart_cap / wg::kPart});
     if (nparts < 1) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
-    const void* fn = W == 64 ? (const void*)k_gen_wgrad_tc<4>
+    const void* fn = W == 128 ? (const void*)k_gen_wgrad_tc<8>
+                   : W == 64 ? (const void*)k_gen_wgrad_tc<4>
                    : W == 48 ? (const void*)k_gen_wgrad_tc<3>
                    : W == 32 ? (const void*)k_gen_wgrad_tc<2> : (const void*)k_gen_wgrad_tc<1>;
     if (int rc = ensure_smem(g, fn, (int)wg::kSmem, true)) return rc;
-    if (W == 64)
+    if (W == 128)
+        launch_seq(g->stream, k_gen_wgrad_tc<8>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
+    else if (W == 64)
         launch_seq(g->stream, k_gen_wgrad_tc<4>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
     else if (W == 48)
         launch_seq(g->stream, k_gen_wgrad_tc<3>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
@@ -2088,14 +2076,15 @@ int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, flo
         launch_seq(g->stream, k_gen_wgrad_tc<2>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
     else
         launch_seq(g->stream, k_gen_wgrad_tc<1>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
-    launch_seq(g->stream, k_gen_sum_parts, dim3((int)((n + 63) / 64)), 64, 0, g->wpart, nparts, (int)n, gw);
+    sum_parts(g, nparts, wg::kPart, gw, nw, gb);
     return cuda_check(cudaGetLastError(), "k_gen_wgrad_tc");
 }
 
+// Weight gradient of a layer, and its bias gradient where gb is not null.
 template <int CIN, int COUT>
-int wgrad_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, int nimg) {
+int wgrad_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, float* gb, int nimg) {
     if (CIN == tc::kC && COUT == tc::kC && g->use_tc && wg::block_len(g->L) > 0)
-        return wgrad_tc_launch(g, in, dout, gw, nimg);
+        return wgrad_tc_launch(g, in, dout, gw, gb, nimg);
     const int tiles = (g->L / kTile) * (g->L / kTile);
     const int per = 4;
     const int groups = (nimg + per - 1) / per;
@@ -2111,18 +2100,9 @@ int wgrad_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float*
         if (int rc = ensure_smem(g, (const void*)k_gen_wgrad_edge<CIN, COUT>, (int)E::smem, false)) return rc;
         launch_seq(g->stream, k_gen_wgrad_edge<CIN, COUT>, dim3(nparts), E::kThreads, E::smem, in, dout, g->wpart, g->L, per, nimg);
     }
-    launch_seq(g->stream, k_gen_sum_parts, dim3((int)((n + 63) / 64)), 64, 0, g->wpart, nparts, (int)n, gw);
-    return cuda_check(cudaGetLastError(), "k_gen_wgrad");
-}
-
-// Bias gradient gb[co] = sum over the batch's pixels of dout[p, co] (wpart as scratch).
-int bgrad_launch(nmmc_gen* g, const float* dout, int nimg, int cout, float* gb) {
-    const int LL = g->L * g->L, nseg = (LL + kBgradRun - 1) / kBgradRun;
-    if (cout % 4 != 0 || cout > 256) return set_error(NMMC_ERR_ARG, "bias gradient: channels not a multiple of 4");
-    if ((size_t)nimg * nseg * cout > g->wpart_cap) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
-    launch_seq(g->stream, k_gen_bgrad_part, dim3(nseg, cout / 4, nimg), 256, 0, dout, LL, cout, nseg, g->wpart);
-    launch_seq(g->stream, k_gen_sum_parts_wide, dim3(cout), 128, 0, g->wpart, nimg * nseg, cout, gb);
-    return cuda_check(cudaGetLastError(), "k_gen_bgrad_part");
+    sum_parts(g, nparts, (int)n, gw, (int)n, nullptr);
+    if (int rc = cuda_check(cudaGetLastError(), "k_gen_wgrad")) return rc;
+    return gb ? bgrad_launch(g, dout, nimg, COUT, gb) : NMMC_OK;
 }
 
 // The weights' compute forms, after one Adam step where `step` says so.
@@ -2160,7 +2140,7 @@ int ensure_batch(nmmc_gen* g, int b) {
     NMMC_CUDA(cudaMalloc(&g->g1, np * kGenC * sizeof(float)));
     NMMC_CUDA(cudaMalloc(&g->gv, np * kGenCout * sizeof(float)));
     const int tiles = (g->L / kTile) * (g->L / kTile);
-    g->wpart_cap = (size_t)tiles * ((b + 3) / 4) * 9 * kGenC * kGenC;
+    g->wpart_cap = (size_t)tiles * ((b + 3) / 4) * wg::kPart;
     NMMC_CUDA(cudaMalloc(&g->wpart, g->wpart_cap * sizeof(float)));
     NMMC_CUDA(cudaMalloc(&g->d_idx, sizeof(int) * b));
     NMMC_CUDA(cudaMalloc(&g->d_sig, sizeof(float) * b));
@@ -2174,7 +2154,7 @@ int forward(nmmc_gen* g, int nb) {
     int rc;
     GenLayer* y = g->layer;
     rc = edge_layers_on_tc(g)
-             ? conv_tma_launch<0, 1, 2, kGenC>(g, g->act[0], y[0].wb, y[0].b, nullptr, g->act[1], nb, y[0].wimg)
+             ? conv_row_launch<0, 1, 2, kGenC>(g, g->act[0], y[0].wb, y[0].b, nullptr, g->act[1], nb, y[0].wimg)
              : conv_launch<kGenCin0, kGenC, __nv_bfloat16, 0>(g, g->act[0], y[0].wb, y[0].b, nullptr, 0, g->act[1], nb);
     if (rc) return rc;
     for (int l = 1; l < kGenLayers - 1; ++l) {
@@ -2185,7 +2165,7 @@ int forward(nmmc_gen* g, int nb) {
     }
     const GenLayer& yl = y[kGenLayers - 1];
     if (edge_layers_on_tc(g))
-        return conv_tma_launch<3, 6, 6, kGenCout>(g, g->act[kGenLayers - 1], yl.wb, yl.b, nullptr, g->vout, nb,
+        return conv_row_launch<3, 6, 6, kGenCout>(g, g->act[kGenLayers - 1], yl.wb, yl.b, nullptr, g->vout, nb,
                                                   yl.wimg);
     return conv_launch<kGenC, kGenCout, __nv_bfloat16, 1>(g, g->act[kGenLayers - 1], yl.wb, yl.b, nullptr, 0, g->vout, nb);
 }
@@ -2196,15 +2176,13 @@ int backward(nmmc_gen* g, int nb) {
     GenLayer* y = g->layer;
     const int last = kGenLayers - 1;
     // last layer: weights and bias, then data gradient into g0 (masked by act[last] > 0)
-    if ((rc = wgrad_launch<kGenC, kGenCout>(g, g->act[last], g->gv, y[last].gw, nb))) return rc;
-    if ((rc = bgrad_launch(g, g->gv, nb, kGenCout, y[last].gb))) return rc;
+    if ((rc = wgrad_launch<kGenC, kGenCout>(g, g->act[last], g->gv, y[last].gw, y[last].gb, nb))) return rc;
     if ((rc = conv_launch<kGenCout, kGenC, float, 2>(g, g->gv, y[last].wt, nullptr, g->act[last], kGenC, g->g0, nb)))
         return rc;
     float* cur = g->g0;
     float* nxt = g->g1;
     for (int l = last - 1; l >= 1; --l) {
-        if ((rc = wgrad_launch<kGenC, kGenC>(g, g->act[l], cur, y[l].gw, nb))) return rc;
-        if ((rc = bgrad_launch(g, cur, nb, kGenC, y[l].gb))) return rc;
+        if ((rc = wgrad_launch<kGenC, kGenC>(g, g->act[l], cur, y[l].gw, y[l].gb, nb))) return rc;
         rc = g->use_tc ? conv_tc_launch<2>(g, cur, y[l].wt, nullptr, g->act[l], nxt, nb, y[l].wtimg)
                        : conv_launch<kGenC, kGenC, float, 2>(g, cur, y[l].wt, nullptr, g->act[l], kGenC, nxt, nb);
         if (rc) return rc;
@@ -2212,8 +2190,7 @@ int backward(nmmc_gen* g, int nb) {
         cur = nxt;
         nxt = t;
     }
-    if ((rc = wgrad_launch<kGenCin0, kGenC>(g, g->act[0], cur, y[0].gw, nb))) return rc;
-    if ((rc = bgrad_launch(g, cur, nb, kGenC, y[0].gb))) return rc;
+    if ((rc = wgrad_launch<kGenCin0, kGenC>(g, g->act[0], cur, y[0].gw, y[0].gb, nb))) return rc;
     return cuda_check(cudaGetLastError(), "backward");
 }
 
@@ -2555,10 +2532,10 @@ int nmmc_gen_probe_conv(nmmc_gen* g, int layer, int nimg, const float* in, float
     const bool tc_edge = tensor && edge_layers_on_tc(g);
     if (rc) {
     } else if (layer == 0) {
-        rc = tc_edge ? conv_tma_launch<1, 1, 2, kGenC>(g, d_in, y.wb, y.b, nullptr, d_out, nimg, y.wimg)
+        rc = tc_edge ? conv_row_launch<1, 1, 2, kGenC>(g, d_in, y.wb, y.b, nullptr, d_out, nimg, y.wimg)
                      : conv_launch<kGenCin0, kGenC, __nv_bfloat16, 1>(g, d_in, y.wb, y.b, nullptr, 0, d_out, nimg);
     } else if (layer == kGenLayers - 1) {
-        rc = tc_edge ? conv_tma_launch<3, 6, 6, kGenCout>(g, d_in, y.wb, y.b, nullptr, d_out, nimg, y.wimg)
+        rc = tc_edge ? conv_row_launch<3, 6, 6, kGenCout>(g, d_in, y.wb, y.b, nullptr, d_out, nimg, y.wimg)
                      : conv_launch<kGenC, kGenCout, __nv_bfloat16, 1>(g, d_in, y.wb, y.b, nullptr, 0, d_out, nimg);
     } else {
         rc = tensor ? conv_tc_launch<1>(g, d_in, y.wb, y.b, nullptr, d_out, nimg, y.wimg)
@@ -2601,7 +2578,7 @@ int nmmc_gen_probe_wgrad(nmmc_gen* g, int nimg, const float* in, const float* do
     if (!rc) rc = cuda_check(cudaMemcpy(d_g, hg.data(), ne * sizeof(float), cudaMemcpyHostToDevice), "probe H2D");
     const int keep = g->use_tc;
     g->use_tc = tensor ? 1 : 0;
-    if (!rc) rc = wgrad_launch<kGenC, kGenC>(g, d_in, d_g, d_w, nimg);
+    if (!rc) rc = wgrad_launch<kGenC, kGenC>(g, d_in, d_g, d_w, nullptr, nimg);
     g->use_tc = keep;
     if (!rc) rc = cuda_check(cudaStreamSynchronize(g->stream), "probe wgrad");
     if (!rc) rc = check_flag(g);
@@ -2616,7 +2593,7 @@ int nmmc_gen_set_option(nmmc_gen* g, int key, int64_t v) {
         NMMC_CUDA(cudaStreamSynchronize(g->stream));
         g->use_tc = v ? 1 : 0;
         g->use_ws = (v == 2) ? 1 : 0;
-        g->use_tma = (v == 3) ? 0 : ((v == 4) ? 2 : 1);
+        g->use_rows = v != 3;   // 4: the same kernels as 1
         return NMMC_OK;
     }
     if (key == NMMC_GEN_OPT_SCHEDULE) {
@@ -2632,9 +2609,7 @@ int nmmc_gen_set_option(nmmc_gen* g, int key, int64_t v) {
     }
     if (key == NMMC_GEN_OPT_TILE_ROWS) {
         if (v != 1 && v != 2) return set_error(NMMC_ERR_ARG, "tile rows must be 1 or 2");
-        NMMC_CUDA(cudaStreamSynchronize(g->stream));
-        g->tile_rows = (int)v;
-        return NMMC_OK;
+        return NMMC_OK;   // the L = 128 kernels take one row per tile in either case
     }
     return set_error(NMMC_ERR_ARG, "unknown generator option %d", key);
 }

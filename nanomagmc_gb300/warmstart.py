@@ -51,13 +51,13 @@ class Generator:
         return out
 
     def tensor_cores(self, mode):
-        """Hidden convolutions: 1 / True tensor cores (default; TMA-staged windows at L = 128),
-        2 warp-specialised forward with cp.async staging, 3 cp.async staging at every L,
-        4 warp-specialised forward with TMA staging (L = 128), 0 / False FP32 FMA pipes."""
+        """Hidden convolutions: 1 / True tensor cores (default; input rows through a ring of bulk
+        copies at L = 128), 2 warp-specialised forward with cp.async staging, 3 cp.async staging at
+        every L, 4 the same as 1, 0 / False FP32 FMA pipes."""
         L.check(self.lib.nmmc_gen_set_option(self.h, L.GEN_OPT_TENSOR_CORES, int(mode)))
 
     def tile_rows(self, rows):
-        """Output rows per tile of the TMA-staged forward convolutions at L = 128 (1 or 2)."""
+        """1 or 2, accepted for existing callers (one output row per tile in either case)."""
         L.check(self.lib.nmmc_gen_set_option(self.h, L.GEN_OPT_TILE_ROWS, int(rows)))
 
     def schedule(self, kind):
@@ -65,7 +65,7 @@ class Generator:
         L.check(self.lib.nmmc_gen_set_option(self.h, L.GEN_OPT_SCHEDULE, int(kind)))
 
     def weight_image(self, on):
-        """TMA-staged forward convolutions: weights by one bulk copy of their operand image."""
+        """Convolutions at L = 128: weights by one bulk copy of their operand image."""
         L.check(self.lib.nmmc_gen_set_option(self.h, L.GEN_OPT_WEIGHT_IMAGE, int(bool(on))))
 
     def __del__(self):
