@@ -51,7 +51,7 @@ struct StencilArgs {
     int C;                   // CTAs per chain
     int NU, R, U;            // slab units of the lattice, rows per unit, largest slab
     int qpr, ipr;            // quads and thread items per row (rounded up)
-    FastDiv div_ipr, div_pairs, div_rows, div_cols, div_planes;   // items, rows per unit; load columns, rows per plane
+    FastDiv div_ipr, div_pairs, div_rows, div_cols;   // items, pairs, rows per unit; load columns
     const double* Hd;
     double* obs;
     double* q;               // nullptr: not wanted
@@ -111,48 +111,49 @@ __global__ void __launch_bounds__(kStThreads, 1) k_resident_stencil(const DevMod
     const size_t P = (size_t)m.nhalf_pad;
     float* const gsp = g.spins + (size_t)chain * 6 * P;
 
-    for (int i = tid; i < (kQuadBytes + 2 * colb) / 16; i += blockDim.x)
+    // a periodic lattice of whole quads overwrites every site of the slab and its copies
+    const bool whole = (hx & 3) == 0;
+    for (int i = tid; i < (whole && per ? kQuadBytes : kQuadBytes + 2 * colb) / 16; i += blockDim.x)
         reinterpret_cast<float4*>(st_sm)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    // units u0 - 1 .. u0 + nu: the slab and its two copies, several loads in flight per thread
-    const bool whole = (hx & 3) == 0;
+    // units u0 - 1 .. u0 + nu: the slab and its two copies. The rows of a plane are contiguous over
+    // the units, so a place in the slab is decoded once for the six planes (three components of
+    // two colours), whose loads are in flight together. With three divisions per site and plane
+    // 8 chains of 30^3 took 8 us to load; with this, the same for the stores and the sums at the end,
+    // a call of 10 sweeps with observables went from 70 to 59 us.
     const int ncol = whole ? qpr : hx + 1;   // float4 columns, or sites and the padding repeat
     {
-        const int nrow = (nu + 2) * R, total = 6 * nrow * ncol;
-        constexpr int B = 6;
-        for (int i0 = tid; i0 < total; i0 += B * blockDim.x) {
-            float4 v[B];
-            char* dst[B];
-#pragma unroll
-            for (int b = 0; b < B; ++b) {
-                const int i = i0 + b * blockDim.x;
-                dst[b] = nullptr;
-                if (i >= total) continue;
-                const int pr = fdiv(i, g.div_cols), h = i - pr * ncol;
-                const int pu = fdiv(pr, g.div_rows), y = pr - pu * R;   // (plane, unit), row
-                const int pl = nu == g.U ? fdiv(pu, g.div_planes) : pu / (nu + 2);   // 3 colour + component
-                const int ul = pu - pl * (nu + 2);
-                int u = u0 - 1 + ul;
-                if (u < 0 || u >= NU) {
-                    if (!per) continue;
-                    u = u < 0 ? u + NU : u - NU;
-                }
-                const int k = pl >= 3 ? 1 : 0;
-                const float* src = gsp + pl * P + (size_t)(u * R + y) * hx;
-                char* d = base + k * colb + (ul * R + y) * rowb + (pl - 3 * k) * 16;
-                if (whole) {
-                    v[b] = __ldg(reinterpret_cast<const float4*>(src) + h);
-                    dst[b] = d + h * kQuadBytes;
-                } else if (h < hx || per) {
-                    v[b].x = __ldg(src + (h < hx ? h : 0));
-                    dst[b] = d + (h >> 2) * kQuadBytes + 4 * (h & 3);
-                }
+        const int total = (nu + 2) * R * ncol, all = NU * R, first = (u0 - 1) * R;
+#pragma unroll 2
+        for (int i = tid; i < total; i += blockDim.x) {
+            const int r = fdiv(i, g.div_cols), h = i - r * ncol;
+            int gr = first + r;   // row of the lattice
+            if (gr < 0 || gr >= all) {
+                if (!per) continue;
+                gr += gr < 0 ? all : -all;
             }
+            if (whole) {
+                const float4* src = reinterpret_cast<const float4*>(gsp + (size_t)gr * hx) + h;
+                float4* dst = reinterpret_cast<float4*>(base + r * rowb + h * kQuadBytes);
+                float4 v[6];
 #pragma unroll
-            for (int b = 0; b < B; ++b) {
-                if (!dst[b]) continue;
-                if (whole) *reinterpret_cast<float4*>(dst[b]) = v[b];
-                else *reinterpret_cast<float*>(dst[b]) = v[b].x;
+                for (int pl = 0; pl < 6; ++pl) v[pl] = __ldg(src + pl * (P / 4));
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    dst[c] = v[c];
+                    dst[colb / 16 + c] = v[3 + c];
+                }
+            } else if (h < hx || per) {
+                const float* src = gsp + (size_t)gr * hx + (h < hx ? h : 0);
+                char* dst = base + r * rowb + (h >> 2) * kQuadBytes + 4 * (h & 3);
+                float v[6];
+#pragma unroll
+                for (int pl = 0; pl < 6; ++pl) v[pl] = __ldg(src + pl * P);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    *reinterpret_cast<float*>(dst + 16 * c) = v[c];
+                    *reinterpret_cast<float*>(dst + colb + 16 * c) = v[3 + c];
+                }
             }
         }
     }
@@ -506,26 +507,39 @@ __global__ void __launch_bounds__(kStThreads, 1) k_resident_stencil(const DevMod
             if (lane == 0) wred[warp][k] = v;
         }
         __syncthreads();
-        // a lane per plane: its angles over the warps, the slice's charge in 3-D
-        if (warp == 0) {
+        // FP64 sums over the warps, side by side (an FP64 addition takes about 40 cycles here, so one
+        // warp adding up 24 warps' totals and angles took 5 us): a tree per total in the warps
+        // 0-9, the angles in the warp after them (the last one, where there are fewer)
+        auto put = [&](int k, double v) {
+            if (rank == 0) cred[0][k] = v;
+            else peer_st(peer_addr(&cred[rank][k], 0), v);
+        };
+        for (int k = warp; k < kNP - 1; k += nw) {
+            double v = lane < nw ? (double)wred[lane][k] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) put(k, v);
+        }
+        if (warp == (nw > kNP - 1 ? kNP - 1 : nw - 1)) {
             double qsum = 0.0;
-            for (int gr = lane; gr < ngroup; gr += 32) {
-                double t = 0.0;
-                for (int w = 0; w < nw; ++w) t += (double)qpart[gr * nw + w];
-                qsum += t;
-                if (DIM == 3 && g.q) g.q[(size_t)ci * g.nslices + u0 + gr] = t / (2 * M_PI);
+            if (DIM == 2) {
+                qsum = lane < nw ? (double)qpart[lane] : 0.0;
+            } else {   // a lane per plane: the slice's charge
+                for (int gr = lane; gr < ngroup; gr += 32) {
+                    double t0 = 0.0, t1 = 0.0;
+                    for (int w = 0; w + 1 < nw; w += 2) {
+                        t0 += (double)qpart[gr * nw + w];
+                        t1 += (double)qpart[gr * nw + w + 1];
+                    }
+                    if (nw & 1) t0 += (double)qpart[gr * nw + nw - 1];
+                    t0 += t1;
+                    qsum += t0;
+                    if (g.q) g.q[(size_t)ci * g.nslices + u0 + gr] = t0 / (2 * M_PI);
+                }
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) qsum += __shfl_down_sync(0xffffffffu, qsum, o);
-            qsum = __shfl_sync(0xffffffffu, qsum, 0);
-            double v = 0.0;
-            if (lane < kNP - 1)
-                for (int w = 0; w < nw; ++w) v += (double)wred[w][lane];
-            if (lane == kNP - 1) v = qsum;
-            if (lane < kNP) {
-                if (rank == 0) cred[0][lane] = v;
-                else peer_st(peer_addr(&cred[rank][lane], 0), v);
-            }
+            if (lane == 0) put(kNP - 1, qsum);
         }
         if (C > 1) {
             cluster_arrive();
@@ -545,18 +559,23 @@ __global__ void __launch_bounds__(kStThreads, 1) k_resident_stencil(const DevMod
     }
     // the slab back to HBM, without its copies
     {
-        const int n4 = whole ? qpr : hx, nrow = nu * R, total = 6 * nrow * n4;
-#pragma unroll 4
+        const int total = nu * R * ncol;   // the places of the load (a padding repeat is left out)
+#pragma unroll 2
         for (int i = tid; i < total; i += blockDim.x) {
-            const int pr = i / n4, h = i - pr * n4;
-            const int pl = pr / nrow, r = pr - pl * nrow;
-            const int k = pl >= 3 ? 1 : 0;
-            float* dst = gsp + pl * P + (size_t)(u0 * R + r) * hx;
-            const char* src = base + k * colb + unitb + r * rowb + (pl - 3 * k) * 16;
-            if (whole)
-                reinterpret_cast<float4*>(dst)[h] = *reinterpret_cast<const float4*>(src + h * kQuadBytes);
-            else
-                dst[h] = *reinterpret_cast<const float*>(src + site_at(h));
+            const int r = fdiv(i, g.div_cols), h = i - r * ncol;
+            float* dst = gsp + (size_t)(u0 * R + r) * hx;
+            const char* src = base + unitb + r * rowb;
+            if (whole) {
+                const float4* q = reinterpret_cast<const float4*>(src + h * kQuadBytes);
+#pragma unroll
+                for (int pl = 0; pl < 6; ++pl)
+                    reinterpret_cast<float4*>(dst + pl * P)[h] = q[(pl >= 3 ? colb / 16 : 0) + pl % 3];
+            } else if (h < hx) {
+                const char* q = src + site_at(h);
+#pragma unroll
+                for (int pl = 0; pl < 6; ++pl)
+                    dst[pl * P + h] = *reinterpret_cast<const float*>(q + (pl >= 3 ? colb : 0) + 16 * (pl % 3));
+            }
         }
     }
     if (rank == 0 && tid == 0) g.sweep[chain] = sw0 + (unsigned long long)g.nsweeps;
@@ -734,7 +753,6 @@ int launch_stencil_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool 
     g.div_pairs = fast_div((c.m.hx + 1) / 2);
     g.div_rows = fast_div(g.R);
     g.div_cols = fast_div(c.m.hx % 4 ? c.m.hx + 1 : g.qpr);
-    g.div_planes = fast_div(g.U + 2);
     g.Hd = c.d_Hd;
     g.obs = c.d_obs;
     g.q = c.d_q;
