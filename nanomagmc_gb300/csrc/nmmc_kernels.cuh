@@ -258,14 +258,14 @@ __device__ __forceinline__ void sphere_proposal(uint32_t r0, uint32_t r1, float&
     float sp, cp;
     __sincosf(phi, &sp, &cp);
     const float w = fmaf(-tz, tz, 1.0f);
-    const float rxy = w * rsqrtf(w);
+    const float rxy = w * rsqrt_norm(w);
     tx = rxy * cp;
     ty = rxy * sp;
 }
 
 // Proposal and Metropolis test for a site whose local field is (hx, hy, hz): returns true
 // and the new spin when accepted (Old/lib/state.cpp:182-200).
-__device__ __forceinline__ float accept_log(uint32_t r) { return __logf(nmmc_u01f(r)); }
+__device__ __forceinline__ float accept_log(uint32_t r) { return log2_norm(nmmc_u01f(r)) * kLn2; }
 
 // Metropolis test of a drawn proposal t with log-uniform lu = accept_log(r.z).
 __device__ __forceinline__ bool heis_accept(float hx, float hy, float hz, float sx, float sy, float sz,

@@ -236,13 +236,29 @@ k_resident(const DevModel m, const ResidentArgs a, const FusedMeasure fm) {
             sp[t] = a.bh[ch];
             ssw[t] = a.sweep[ch];
         }
-        for (int t = threadIdx.x; t < n; t += blockDim.x) {
-            const uint32_t off = a.goff[s0 + t];
-            if (ISING) {
-                sx[t] = (float)((const int8_t*)a.spins)[off];
-            } else {
-                const float* f = (const float*)a.spins;
-                s4[t] = make_float4(f[off], f[off + P], f[off + 2 * P], 0.0f);
+        // four sites at a time, so that their offsets and then their spins are in flight together (here
+        // and when the spins go back)
+        constexpr int kBatch = 4;
+        for (int t0 = threadIdx.x; t0 < n; t0 += kBatch * blockDim.x) {
+            uint32_t off[kBatch];
+            float4 v[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) off[k] = __ldg(a.goff + s0 + min(t0 + k * (int)blockDim.x, n - 1));
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) {
+                if (ISING) {
+                    v[k].x = (float)((const int8_t*)a.spins)[off[k]];
+                } else {
+                    const float* f = (const float*)a.spins + off[k];
+                    v[k] = make_float4(f[0], f[P], f[2 * P], 0.0f);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) {
+                const int t = t0 + k * blockDim.x;
+                if (t >= n) continue;
+                if (ISING) sx[t] = v[k].x;
+                else s4[t] = v[k];
             }
         }
         if (threadIdx.x == 0) {
@@ -352,17 +368,27 @@ k_resident(const DevModel m, const ResidentArgs a, const FusedMeasure fm) {
                                     fm.acc + (size_t)ch * NMMC_ACC_N, fm.accumulate);
             }
         }
-        for (int t = threadIdx.x; t < n; t += blockDim.x) {
-            if (sch[rec[t].w >> kBoxBits] < 0) continue;
-            const uint32_t off = a.goff[s0 + t];
-            if (ISING) {
-                ((int8_t*)a.spins)[off] = (int8_t)sx[t];
-            } else {
-                float* f = (float*)a.spins;
-                const float4 v = s4[t];
-                f[off] = v.x;
-                f[off + P] = v.y;
-                f[off + 2 * P] = v.z;
+        for (int t0 = threadIdx.x; t0 < n; t0 += kBatch * blockDim.x) {
+            uint32_t off[kBatch], w[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) {
+                const int t = min(t0 + k * (int)blockDim.x, n - 1);
+                off[k] = __ldg(a.goff + s0 + t);
+                w[k] = __ldg(&rec[t].w);
+            }
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) {
+                const int t = t0 + k * blockDim.x;
+                if (t >= n || sch[w[k] >> kBoxBits] < 0) continue;
+                if (ISING) {
+                    ((int8_t*)a.spins)[off[k]] = (int8_t)sx[t];
+                } else {
+                    float* f = (float*)a.spins + off[k];
+                    const float4 v = s4[t];
+                    f[0] = v.x;
+                    f[P] = v.y;
+                    f[2 * P] = v.z;
+                }
             }
         }
         for (int t = threadIdx.x; t < nslot; t += blockDim.x)

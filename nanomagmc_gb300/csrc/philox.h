@@ -56,7 +56,7 @@ __device__ __forceinline__ float nmmc_u12f(uint32_t r) { return __uint_as_float(
 // it is built from bits: (1 + k 2^-23) - (1 - 2^-24) is exact (Sterbenz) and equals the same value.
 NMMC_HD float nmmc_u01f(uint32_t r) {
 #if defined(__CUDA_ARCH__)
-    return __uint_as_float(0x3f800000u | (r >> 9)) - 0.99999994f;
+    return nmmc_u12f(r) - 0.99999994f;
 #else
     return ((float)(r >> 9) + 0.5f) * (1.0f / 8388608.0f);
 #endif
