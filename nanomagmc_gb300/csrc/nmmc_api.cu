@@ -196,10 +196,10 @@ int sweep_measure_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, 
             return accumulate ? launch_add_av(c) : NMMC_OK;
         }
         if ((rc = run_sweeps(c, d_chains, h_chains, n, nsweeps, res, false, 0, allow_timing))) return rc;
-        c.class_fresh = c.m.general != 0;
+        c.planes_fresh = !res;
     }
     rc = launch_measure(c, d_chains, n, accumulate);
-    c.class_fresh = false;
+    c.planes_fresh = false;
     if (rc) return rc;
     return accumulate ? launch_add_av(c) : NMMC_OK;
 }
@@ -394,6 +394,7 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
     c->inter = *inter;
     const bool weib = shape_is_weibull(opt->shape_code);
     c->masked = weib || (edge & 1);
+    c->box_full = !weib;
     for (int i = 0; i < nchains; ++i) {
         c->T.push_back(chains[i].T);
         c->H.push_back(chains[i].H);

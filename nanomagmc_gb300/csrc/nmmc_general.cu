@@ -696,7 +696,7 @@ int launch_energy_general(Ctx& c, const int* d_chains, int n, int rows, int nblk
                           double* partial) {
     if (!c.measure_fp64 && use_class(c) && c.d_class) {
         // a sample step's sweeps have left the listed chains' class planes current
-        if (!c.class_fresh)
+        if (!c.planes_fresh)
             if (int rc = class_copy(c, d_chains, n, true)) return rc;
         auto kern = c.dim == 3 ? (c.periodic ? k_class_energy<3, true> : k_class_energy<3, false>)
                                : (c.periodic ? k_class_energy<2, true> : k_class_energy<2, false>);

@@ -117,6 +117,7 @@ struct Ctx {
     int dim = 2, edge = 0, nchains = 0, nslices = 1;
     long long box_sites = 0;
     bool ising = false, periodic = false, masked = false;
+    bool box_full = true;               // every site of the box is filled (masked then: an odd edge)
     char shape = 's';
     double k_b = 1.0;
     uint64_t seed = 0;
@@ -167,7 +168,8 @@ struct Ctx {
     // general tables, unmasked Heisenberg: the class planes (nmmc_general.cu)
     float4* d_class = nullptr;
     bool class_no_memory = false;
-    bool class_fresh = false;           // within one sample step: the planes hold what its sweeps left
+    bool planes_fresh = false;           // within one sample step: the compact or class planes hold
+                                        // what its sweeps left
     float4* d_bh = nullptr;             // per chain (beta, H0, H1, H2) in FP32
     uint32_t* d_itab = nullptr;         // Ising word kernels: per chain 128 acceptance limits (nmmc_ising.cu)
     double* d_Hd = nullptr;             // per chain H in FP64 (3 doubles) for the energy

@@ -1405,6 +1405,71 @@ __device__ __forceinline__ void site_terms(const DevModel& m, const int x, const
     }
 }
 
+// The same in FP32 for Heisenberg spins, with the energy's field by the DMI's structure (DK, as the
+// sweeps: +-axis pairs share their sums and differences).
+template <int DIM, int DK>
+__device__ __forceinline__ void heis_site_terms(const DevModel& m, const int x, const int y, const int z, const float s0,
+                                                const float s1, const float s2, const float* n0, const float* n1,
+                                                const float* n2, const bool* qv, float* acc) {
+    float f0 = 0.0f, f1 = 0.0f, f2 = 0.0f;
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) {
+        const int kp = 2 * a, km = 2 * a + 1;
+        if (DK <= kDmiGeneral) {
+#pragma unroll
+            for (int k = kp; k <= km; ++k) {
+                f0 = fmaf(m.J[k], n0[k], f0);
+                f1 = fmaf(m.J[k], n1[k], f1);
+                f2 = fmaf(m.J[k], n2[k], f2);
+                if (DK == kDmiGeneral) {   // De x s_j
+                    f0 = fmaf(m.De[k][1], n2[k], fmaf(-m.De[k][2], n1[k], f0));
+                    f1 = fmaf(m.De[k][2], n0[k], fmaf(-m.De[k][0], n2[k], f1));
+                    f2 = fmaf(m.De[k][0], n1[k], fmaf(-m.De[k][1], n0[k], f2));
+                }
+            }
+        } else {
+            const float d0 = n0[kp] - n0[km], d1 = n1[kp] - n1[km], d2 = n2[kp] - n2[km];
+            f0 = fmaf(m.J[kp], n0[kp] + n0[km], f0);
+            f1 = fmaf(m.J[kp], n1[kp] + n1[km], f1);
+            f2 = fmaf(m.J[kp], n2[kp] + n2[km], f2);
+            if (DK == kDmiPairs) {
+                f0 = fmaf(m.De[kp][1], d2, fmaf(-m.De[kp][2], d1, f0));
+                f1 = fmaf(m.De[kp][2], d0, fmaf(-m.De[kp][0], d2, f1));
+                f2 = fmaf(m.De[kp][0], d1, fmaf(-m.De[kp][1], d0, f2));
+            } else {   // De(+a) = D_a e_a
+                const float D = m.De[kp][a];
+                if (a == 0) {
+                    f1 = fmaf(-D, d2, f1);
+                    f2 = fmaf(D, d1, f2);
+                } else if (a == 1) {
+                    f0 = fmaf(D, d2, f0);
+                    f2 = fmaf(-D, d0, f2);
+                } else {
+                    f0 = fmaf(-D, d1, f0);
+                    f1 = fmaf(D, d0, f1);
+                }
+            }
+        }
+    }
+    acc[0] = fmaf(s0, f0, fmaf(s1, f1, fmaf(s2, f2, acc[0])));
+    acc[1] += s0;
+    acc[2] += s1;
+    acc[3] += s2;
+    if (((x + y + z) & 1) == 0) {   // subM(0)
+        acc[4] += s0;
+        acc[5] += s1;
+        acc[6] += s2;
+    }
+    const int z4 = z & 3, posdiff = y - x + (m.edge & ~3);   // sub4M; C truncating remainders
+    if ((z4 & 1) == 0 && ((x + y) & 3) == z4 && posdiff % 4 == z4) {
+        acc[7] += s0;
+        acc[8] += s1;
+        acc[9] += s2;
+    }
+    if (qv[1] && qv[2]) acc[10] += solid_angle_f(s0, s1, s2, n0[1], n1[1], n2[1], n0[2], n1[2], n2[2]);
+    if (qv[0] && qv[3]) acc[10] += solid_angle_f(s0, s1, s2, n0[0], n1[0], n2[0], n0[3], n1[3], n2[3]);
+}
+
 template <int DIM, bool ISING, bool MASKED, typename RT>
 __global__ void __launch_bounds__(256)
 k_measure(const DevModel m, const void* __restrict__ spins_v, const uint8_t* __restrict__ mask,
@@ -1494,6 +1559,55 @@ k_measure(const DevModel m, const void* __restrict__ spins_v, const uint8_t* __r
         }
     }
     block_partials<RT>(acc, partial + ((size_t)ci * gridDim.x + b) * kNP);
+}
+
+// k_measure for unmasked Heisenberg lattices in FP32 whose rows are no multiple of four sites of a
+// colour (the others: k_measure_q4). A thread's neighbours all lie in the other colour's planes,
+// at offsets of one 32-bit place; the row is found by a multiplication (fdiv), the energy by the
+// DMI's structure. What bounds it: instructions. 32 open cubes of edge 33 took 43 us with every
+// neighbour's colour, place and wrap worked out by itself in 64 bits, now 20 us.
+template <int DIM, int DK>
+__global__ void __launch_bounds__(256, 4)
+k_measure_box(const DevModel m, const float* spins, const int* __restrict__ chains, int rows, int nblk_slice, FastDiv div_edge,
+              double* __restrict__ partial) {
+    seq_begin();
+    const int ci = blockIdx.y, chain = chains[ci], b = blockIdx.x;
+    const int z = b / nblk_slice, y0 = (b - z * nblk_slice) * rows, y1 = min(y0 + rows, m.ly);
+    const int nsite = (y1 - y0) * m.edge, e = m.edge, hx = m.hx;
+    const int plane = m.ly * hx;
+    const size_t P = (size_t)m.nhalf_pad;
+    const float* const base = spins + (size_t)chain * 6 * P;
+    const bool per = m.periodic, pq = per && m.periodic_q;
+    float acc[kNP];
+#pragma unroll
+    for (int k = 0; k < kNP; ++k) acc[k] = 0.0f;
+    for (int t = threadIdx.x; t < nsite; t += 256) {
+        const int yy = fdiv(t, div_edge), x = t - yy * e, y = y0 + yy;
+        const int colour = (x + y + z) & 1, row = (z * m.ly + y) * hx, at = row + (x >> 1);
+        const float* const own = base + (colour ? 3 * P : 0);
+        const float* const oth = base + (colour ? 0 : 3 * P);
+        const bool in[6] = {x + 1 < e, x > 0, y + 1 < e, y > 0, z + 1 < m.lz, z > 0};
+        const int nb[6] = {in[0] ? row + ((x + 1) >> 1) : row,
+                           in[1] ? row + ((x - 1) >> 1) : row + ((e - 1) >> 1),
+                           in[2] ? at + hx : at - (m.ly - 1) * hx,
+                           in[3] ? at - hx : at + (m.ly - 1) * hx,
+                           in[4] ? at + plane : at - (m.lz - 1) * plane,
+                           in[5] ? at - plane : at + (m.lz - 1) * plane};
+        float n0[2 * DIM], n1[2 * DIM], n2[2 * DIM];
+        bool qv[4];
+#pragma unroll
+        for (int k = 0; k < 2 * DIM; ++k) {
+            const bool ok = per || in[k];
+            const float* p = oth + nb[k];
+            n0[k] = ok ? p[0] : 0.0f;
+            n1[k] = ok ? p[P] : 0.0f;
+            n2[k] = ok ? p[2 * P] : 0.0f;
+            if (k < 4) qv[k] = in[k] || pq;
+        }
+        const float* p = own + at;
+        heis_site_terms<DIM, DK>(m, x, y, z, p[0], p[P], p[2 * P], n0, n1, n2, qv, acc);
+    }
+    block_partials<float>(acc, partial + ((size_t)ci * gridDim.x + b) * kNP);
 }
 
 // Heisenberg observables over quads of same-colour sites (unmasked lattices, rows holding a
@@ -1996,11 +2110,12 @@ k_measure_finalize_fused(const int* __restrict__ chains, const double* __restric
 // order) over the compact planes, gathered from the box layout just before, with neighbours
 // from the compact table. The same per-site terms of the same values in the same order as
 // k_measure, so the same sums; the dense planes spare the box layout's part-empty sectors.
-template <int DIM, bool PACKED>
+template <int DIM, bool PACKED, int DK>
 __global__ void __launch_bounds__(256)
 k_measure_compact(const DevModel m, const float4* __restrict__ cs, const int4* __restrict__ tab,
                   const int* __restrict__ fill_zoff, const int* __restrict__ chains, int nblk_slice,
                   double* __restrict__ partial) {
+    seq_begin();
     const int ci = blockIdx.y;
     const int chain = chains[ci];
     const int b = blockIdx.x;
@@ -2024,8 +2139,8 @@ k_measure_compact(const DevModel m, const float4* __restrict__ cs, const int4* _
         compact_entry<PACKED>(tab, seg, NH, j, nbi, box);
         const float4* own = cs + (size_t)seg * NH;
         const float4* oth = cs + (size_t)(chain * 2 + (colour ^ 1)) * NH;
-        const int x = (int)(box % (uint32_t)m.edge), y = (int)((box / (uint32_t)m.edge) % (uint32_t)m.edge);
-        const int zz = (DIM == 3) ? (int)(box / ((uint32_t)m.edge * (uint32_t)m.edge)) : 0;
+        const uint32_t line = box / (uint32_t)m.edge, zu = DIM == 3 ? line / (uint32_t)m.edge : 0u;
+        const int x = (int)(box - line * (uint32_t)m.edge), y = (int)(line - zu * (uint32_t)m.edge), zz = (int)zu;
         const float4 sv = own[j];
         const float s0 = sv.x, s1 = sv.y, s2 = sv.z;
         float n0[2 * DIM], n1[2 * DIM], n2[2 * DIM];
@@ -2034,7 +2149,7 @@ k_measure_compact(const DevModel m, const float4* __restrict__ cs, const int4* _
         for (int k = 0; k < 2 * DIM; ++k) {
             const int q = nbi[k];
             const bool exists = q >= 0;
-            const float4 v = exists ? __ldg(oth + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 v = exists ? oth[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             n0[k] = v.x;
             n1[k] = v.y;
             n2[k] = v.z;
@@ -2044,7 +2159,7 @@ k_measure_compact(const DevModel m, const float4* __restrict__ cs, const int4* _
                 qv[k] = exists && (inside || (m.periodic && m.periodic_q));
             }
         }
-        site_terms<DIM, false, float>(m, x, y, zz, s0, s1, s2, n0, n1, n2, qv, acc);
+        heis_site_terms<DIM, DK>(m, x, y, zz, s0, s1, s2, n0, n1, n2, qv, acc);
     }
     block_partials<float>(acc, partial + ((size_t)ci * gridDim.x + b) * kNP);
 }
@@ -2090,7 +2205,14 @@ static void measure_q4_launch(Ctx& c, dim3 grid, const float* sp, const int* d_c
 // Masked lattices are measured over their lists of filled sites (blocks = parts of z-slices),
 // except with a general interaction table, whose energy kernel adds into the partial sums of
 // the row-split blocks.
-static bool measure_by_list(const Ctx& c) { return c.masked && !c.m.general && c.d_fill; }
+// FP32 observables of Heisenberg boxes with every site filled (odd edges, which are masked for the
+// sweeps, too) by place: the lists of filled sites would only add a gather (32 open cubes of edge
+// 33: 43 us by list, 20 by place). Rows of whole quads have kernels of their own, below.
+static bool measure_by_box(const Ctx& c) {
+    return !c.ising && !c.measure_fp64 && c.box_full && !(c.periodic && (c.edge & 1)) && ((c.m.hx % 4) != 0 || c.masked || c.half_kernel == 1) &&
+           (4096 / c.edge + 1) * c.edge < 65536;   // fdiv's range
+}
+static bool measure_by_list(const Ctx& c) { return c.masked && !c.m.general && c.d_fill && !measure_by_box(c); }
 
 // FP32 observables of masked Heisenberg lattices whose compact form is built: the list split
 // over the compact planes (gathered from the box layout first).
@@ -2099,14 +2221,19 @@ static bool measure_by_compact(const Ctx& c) {
 }
 
 static int measure_compact_launch(Ctx& c, const int* d_chains, int n, int nblk, int nblk_slice, double* partial) {
-    int rc = compact_copy(c, d_chains, n, true);
-    if (rc) return rc;
+    // a sample step's sweeps have left the listed chains' planes current
+    if (!c.planes_fresh)
+        if (int rc = compact_copy(c, d_chains, n, true)) return rc;
     dim3 grid(nblk, n);
-#define NMMC_MC(D, PK) k_measure_compact<D, PK><<<grid, 256, 0, c.stream>>>(c.m, c.d_cspins, c.d_ctab, \
-                                                                             c.d_fill_zoff, d_chains, nblk_slice, partial)
-    if (c.dim == 3) { if (c.ctab_packed) NMMC_MC(3, true); else NMMC_MC(3, false); }
-    else { if (c.ctab_packed) NMMC_MC(2, true); else NMMC_MC(2, false); }
+    using Fn = void (*)(const DevModel, const float4*, const int4*, const int*, const int*, int, double*);
+#define NMMC_MC(D, PK)                                                                                            \
+    (c.m.dmi_kind == kDmiNone      ? (Fn)k_measure_compact<D, PK, kDmiNone>                                      \
+     : c.m.dmi_kind == kDmiGeneral ? (Fn)k_measure_compact<D, PK, kDmiGeneral>                                   \
+     : c.m.dmi_kind == kDmiPairs   ? (Fn)k_measure_compact<D, PK, kDmiPairs> : (Fn)k_measure_compact<D, PK, kDmiAxial>)
+    Fn fn = c.dim == 3 ? (c.ctab_packed ? NMMC_MC(3, true) : NMMC_MC(3, false))
+                       : (c.ctab_packed ? NMMC_MC(2, true) : NMMC_MC(2, false));
 #undef NMMC_MC
+    launch_seq(c, fn, grid, 256, 0, c.m, c.d_cspins, c.d_ctab, c.d_fill_zoff, d_chains, nblk_slice, partial);
     return NMMC_OK;
 }
 
@@ -2183,6 +2310,17 @@ static int measure_with(Ctx& c, const int* d_chains, int n, double* partial, dou
         dim3 grid(nblk, n);
         const float* sp = (const float*)c.d_spins;
         measure_q4_launch(c, grid, sp, d_chains, rows, nblk_slice, partial);
+    } else if (measure_by_box(c)) {
+        using Fn = void (*)(const DevModel, const float*, const int*, int, int, FastDiv, double*);
+        Fn fn = nullptr;
+        switch (c.m.dmi_kind) {
+            case kDmiNone: fn = c.dim == 3 ? (Fn)k_measure_box<3, kDmiNone> : (Fn)k_measure_box<2, kDmiNone>; break;
+            case kDmiGeneral: fn = c.dim == 3 ? (Fn)k_measure_box<3, kDmiGeneral> : (Fn)k_measure_box<2, kDmiGeneral>; break;
+            case kDmiPairs: fn = c.dim == 3 ? (Fn)k_measure_box<3, kDmiPairs> : (Fn)k_measure_box<2, kDmiPairs>; break;
+            default: fn = c.dim == 3 ? (Fn)k_measure_box<3, kDmiAxial> : (Fn)k_measure_box<2, kDmiAxial>; break;
+        }
+        launch_seq(c, fn, dim3(nblk, n), 256, 0, c.m, (const float*)c.d_spins, d_chains, rows, nblk_slice, fast_div(c.edge),
+                   partial);
     } else if (ising_words_ok(c) && c.half_kernel != 1) {   // integer sums: exact in both modes
         launch_measure_ising(c, dim3(nblk, n), d_chains, rows, nblk_slice, partial);
     } else if (c.ising) {

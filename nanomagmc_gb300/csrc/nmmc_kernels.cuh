@@ -64,6 +64,11 @@ __device__ __forceinline__ float log2_norm(float x) {
     return r;
 }
 
+// n / d for n, d < 65536 by one multiplication (mul = ceil(2^32 / d); d = 1 has mul = 0).
+struct FastDiv { uint32_t mul; int d; };
+__device__ __forceinline__ int fdiv(int n, const FastDiv& f) { return f.mul ? (int)__umulhi((uint32_t)n, f.mul) : n; }
+inline FastDiv fast_div(int d) { return FastDiv{d <= 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d), d}; }
+
 // Compact index, in the other colour's plane, of the neighbour of (x,y,z) in direction k
 // (+x,-x,+y,-y,+z,-z), or -1 when the neighbour falls off an open boundary.
 template <bool PERIODIC>

@@ -38,10 +38,6 @@ constexpr int kStThreads = 768;     // 80 registers: 24 warps per SM in one, two
 constexpr int kStMaxCluster = 16;
 constexpr int kQuadBytes = 48;
 
-// n / d for n, d < 65536 by one multiplication (mul = ceil(2^32 / d); d = 1 has mul = 0).
-struct FastDiv { uint32_t mul; int d; };
-__device__ __forceinline__ int fdiv(int n, const FastDiv& f) { return f.mul ? (int)__umulhi((uint32_t)n, f.mul) : n; }
-
 struct StencilArgs {
     float* spins;
     const float4* bh;
@@ -608,8 +604,6 @@ StencilFn stencil_kernel(const Ctx& c, int np, bool measure) {
     if (c.dim == 3) return measure ? stencil_kernel_np<3, true>(dk, np) : stencil_kernel_np<3, false>(dk, np);
     return measure ? stencil_kernel_np<2, true>(dk, np) : stencil_kernel_np<2, false>(dk, np);
 }
-
-FastDiv fast_div(int d) { return FastDiv{d <= 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d), d}; }
 
 int units_of(const Ctx& c) { return c.dim == 3 ? c.m.lz : c.m.ly; }
 int rows_of(const Ctx& c) { return c.dim == 3 ? c.m.ly : 1; }
