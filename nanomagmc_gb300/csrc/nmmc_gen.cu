@@ -1566,6 +1566,7 @@ k_gen_wgrad(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout
 // take every kGroups-th row of the tile, a thread one tap x 8 input channels x TC output channels
 // with 16-byte loads and packed multiply-adds. Rows of a pixel are padded by 4 floats so that the
 // staging's stores and the loads spread over the banks. 16 x 128^2: 136 -> 62 us and 54 -> 48 us.
+constexpr int kEdgePer = 4;   // images of a CTA (2: 51 and 63 us instead of 48 and 61)
 template <int CIN, int COUT>
 struct EdgeGrad {
     static constexpr int TC = COUT < 8 ? COUT : 8;                 // output channels of a thread
@@ -1675,63 +1676,61 @@ k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__
         }
 }
 
-// The sum of nparts partials of `stride` floats: the first nw of them to gw, the rest to gb. A block
-// takes 16 groups of four outputs, 8 threads each the partials t, t + 8, ... of a group, added in
-// a fixed order at the end. One thread per output had too few loads in flight: 9.6 us for 152
-// partials of 20736 weights, now 6.5 us.
-__global__ void __launch_bounds__(128)
-k_gen_sum_parts(const float* __restrict__ part, int nparts, int stride, float* __restrict__ gw, int nw, int n,
-                float* __restrict__ gb) {
+// Sums of partials, one job per blockIdx.y: nparts partials of `stride` floats, of which the first nw
+// sum to gw and the rest (up to n) to gb; all multiples of four. A block takes 16 groups of four
+// outputs, 8 threads each the partials t, t + 8, ... of a group, added in a fixed order at the end.
+// One thread per output had too few loads in flight (9.6 us for 152 partials of 20736 weights, this
+// 6.5), and a launch per layer too few blocks: a backward pass's sums are one launch, eight
+// layers of 16 x 128^2 in 23 us instead of 58.
+struct SumJob {
+    const float* part;
+    float *gw, *gb;
+    int nparts, stride, nw, n;
+};
+constexpr int kSumJobs = kGenLayers + 2;   // and the first and last layers' bias gradients
+struct SumArgs {
+    SumJob job[kSumJobs];
+    int n = 0;         // jobs
+    size_t used = 0;   // floats of the scratch that they hold
+};
+__global__ void __launch_bounds__(128) k_gen_sum_parts(const __grid_constant__ SumArgs a) {
     seq_begin();
     __shared__ float4 red[8][16];
+    const SumJob& s = a.job[blockIdx.y];
+    if ((int)blockIdx.x * 64 >= s.n) return;
     const int o = threadIdx.x & 15, t = threadIdx.x >> 4, i = (blockIdx.x * 16 + o) * 4;
-    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (i < n) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (i < s.n) {
+        const float* p0 = s.part + i;
+        const size_t stride = (size_t)s.stride;
+        const int nparts = s.nparts;
 #pragma unroll 10
         for (int p = t; p < nparts; p += 8) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(part + (size_t)p * stride + i));
-            s.x += v.x;
-            s.y += v.y;
-            s.z += v.z;
-            s.w += v.w;
+            const float4 w = __ldcg(reinterpret_cast<const float4*>(p0 + p * stride));
+            v.x += w.x;
+            v.y += w.y;
+            v.z += w.z;
+            v.w += w.w;
         }
     }
-    red[t][o] = s;
+    red[t][o] = v;
     __syncthreads();
-    if (threadIdx.x >= 16 || i >= n) return;
+    if (threadIdx.x >= 16 || i >= s.n) return;
 #pragma unroll
     for (int k = 1; k < 8; ++k) {
-        const float4 v = red[k][o];
-        s.x += v.x;
-        s.y += v.y;
-        s.z += v.z;
-        s.w += v.w;
+        const float4 w = red[k][o];
+        v.x += w.x;
+        v.y += w.y;
+        v.z += w.z;
+        v.w += w.w;
     }
-    *reinterpret_cast<float4*>(i < nw ? gw + i : gb + (i - nw)) = s;
-}
-
-// Sum of many partials for few outputs: block i adds part[0..nparts)[i], thread t the parts
-// t, t + 128, ..., then a fixed-order tree (the same result on every run).
-__global__ void __launch_bounds__(128)
-k_gen_sum_parts_wide(const float* __restrict__ part, int nparts, int n, float* __restrict__ out) {
-    seq_begin();
-    __shared__ float red[128];
-    const int i = blockIdx.x, t = threadIdx.x;
-    float s = 0.0f;
-    for (int p = t; p < nparts; p += 128) s += __ldcg(part + (size_t)p * n + i);
-    red[t] = s;
-    __syncthreads();
-    for (int h = 64; h > 0; h >>= 1) {
-        if (t < h) red[t] += red[t + h];
-        __syncthreads();
-    }
-    if (t == 0) out[i] = red[0];
+    *reinterpret_cast<float4*>(i < s.nw ? s.gw + i : s.gb + (i - s.nw)) = v;
 }
 
 // Bias gradient, first stage: a block sums kBgradRun consecutive pixels of one 4-channel plane of
 // one image of the planar FP32 dout (contiguous 16-byte loads, eight in flight per thread) into
 // part[image * segments + segment][co]; lanes and warps are added in a fixed order, the partials
-// by k_gen_sum_parts_wide. 31 -> 10.4 us for 16 x 128^2 x 48 (50 MB): a division per pixel and 21
+// by k_gen_sum_parts. 31 -> 10.4 us for 16 x 128^2 x 48 (50 MB): a division per pixel and 21
 // lanes per channel group before.
 constexpr int kBgradRun = 2048;
 __global__ void __launch_bounds__(256)
@@ -2064,72 +2063,102 @@ int check_flag(nmmc_gen* g) {
     return set_error(NMMC_ERR_TIMEOUT, "a tensor-core convolution gave up waiting for its MMAs (code %d)", f);
 }
 
-// Bias gradient gb[co] = sum over the batch's pixels of dout[p, co] (wpart as scratch).
-int bgrad_launch(nmmc_gen* g, const float* dout, int nimg, int cout, float* gb) {
-    const int LL = g->L * g->L, nseg = (LL + kBgradRun - 1) / kBgradRun;
-    if (cout % 4 != 0 || cout > 256) return set_error(NMMC_ERR_ARG, "bias gradient: channels not a multiple of 4");
-    if ((size_t)nimg * nseg * cout > g->wpart_cap) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
-    launch_seq(g->stream, k_gen_bgrad_part, dim3(nseg, cout / 4, nimg), 256, 0, dout, LL, cout, nseg, g->wpart);
-    launch_seq(g->stream, k_gen_sum_parts_wide, dim3(cout), 128, 0, g->wpart, nimg * nseg, cout, gb);
-    return cuda_check(cudaGetLastError(), "k_gen_bgrad_part");
+// The sums asked for so far, one launch.
+int launch_sums(nmmc_gen* g, SumArgs& a) {
+    int most = 0;
+    for (int k = 0; k < a.n; ++k) most = std::max(most, a.job[k].n);
+    if (a.n) launch_seq(g->stream, k_gen_sum_parts, dim3((most + 63) / 64, a.n), 128, 0, a);
+    a.n = 0;
+    a.used = 0;
+    return cuda_check(cudaGetLastError(), "k_gen_sum_parts");
 }
 
-// gw (and gb, where the partials carry biases) from the partials in wpart
-void sum_parts(nmmc_gen* g, int nparts, int stride, float* gw, int nw, float* gb) {
-    const int n = gb ? stride : nw;   // multiples of four
-    launch_seq(g->stream, k_gen_sum_parts, dim3((n / 4 + 15) / 16), 128, 0, g->wpart, nparts, stride, gw, nw, n, gb);
+// Room for nparts partials of `stride` floats in the scratch, for the sums of job `add`ed next; sums
+// that hold too much of it are launched first. nullptr: too small.
+float* sum_room(nmmc_gen* g, SumArgs& a, size_t nparts, size_t stride) {
+    const size_t need = (nparts * stride + 3) / 4 * 4;
+    if (a.n == kSumJobs || a.used + need > g->wpart_cap)
+        if (launch_sums(g, a)) return nullptr;
+    if (need > g->wpart_cap) return nullptr;
+    a.job[a.n].part = g->wpart + a.used;
+    a.job[a.n].nparts = (int)nparts;
+    a.job[a.n].stride = (int)stride;
+    a.used += need;
+    return g->wpart + a.used - need;
+}
+void sum_add(SumArgs& a, float* gw, int nw, float* gb) {
+    SumJob& j = a.job[a.n++];
+    j.gw = gw;
+    j.gb = gb;
+    j.nw = nw;
+    j.n = gb ? j.stride : nw;
+}
+
+// Bias gradient gb[co] = sum over the batch's pixels of dout[p, co].
+int bgrad_launch(nmmc_gen* g, const float* dout, int nimg, int cout, float* gb, SumArgs& sums) {
+    const int LL = g->L * g->L, nseg = (LL + kBgradRun - 1) / kBgradRun;
+    if (cout % 4 != 0 || cout > 256) return set_error(NMMC_ERR_ARG, "bias gradient: channels not a multiple of 4");
+    float* part = sum_room(g, sums, (size_t)nimg * nseg, cout);
+    if (!part) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
+    launch_seq(g->stream, k_gen_bgrad_part, dim3(nseg, cout / 4, nimg), 256, 0, dout, LL, cout, nseg, part);
+    sum_add(sums, gb, cout, nullptr);
+    return cuda_check(cudaGetLastError(), "k_gen_bgrad_part");
 }
 
 // Hidden-layer weight and bias gradient on the tensor cores (k_gen_wgrad_tc): as many CTAs as SMs (one
 // per SM), as the partial scratch holds and as there are K-blocks.
-int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, float* gb, int nimg) {
+int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, float* gb, int nimg,
+                    SumArgs& sums) {
     const int nw = 9 * tc::kC * tc::kC;
     const int W = wg::block_len(g->L);
     const int nkb = (int)((size_t)nimg * g->L * (g->L / W));
     const int nparts = (int)std::min<size_t>({(size_t)nkb, (size_t)std::max(1, g->sm_count), g->wpart_cap / wg::kPart});
-    if (nparts < 1) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
+    float* part = nparts < 1 ? nullptr : sum_room(g, sums, nparts, wg::kPart);
+    if (!part) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
     const void* fn = W == 128 ? (const void*)k_gen_wgrad_tc<8>
                    : W == 64 ? (const void*)k_gen_wgrad_tc<4>
                    : W == 48 ? (const void*)k_gen_wgrad_tc<3>
                    : W == 32 ? (const void*)k_gen_wgrad_tc<2> : (const void*)k_gen_wgrad_tc<1>;
     if (int rc = ensure_smem(g, fn, (int)wg::kSmem, true)) return rc;
     if (W == 128)
-        launch_seq(g->stream, k_gen_wgrad_tc<8>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
+        launch_seq(g->stream, k_gen_wgrad_tc<8>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
     else if (W == 64)
-        launch_seq(g->stream, k_gen_wgrad_tc<4>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
+        launch_seq(g->stream, k_gen_wgrad_tc<4>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
     else if (W == 48)
-        launch_seq(g->stream, k_gen_wgrad_tc<3>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
+        launch_seq(g->stream, k_gen_wgrad_tc<3>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
     else if (W == 32)
-        launch_seq(g->stream, k_gen_wgrad_tc<2>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
+        launch_seq(g->stream, k_gen_wgrad_tc<2>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
     else
-        launch_seq(g->stream, k_gen_wgrad_tc<1>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, g->wpart, g->L, nkb, g->d_flag);
-    sum_parts(g, nparts, wg::kPart, gw, nw, gb);
+        launch_seq(g->stream, k_gen_wgrad_tc<1>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
+    sum_add(sums, gw, nw, gb);
     return cuda_check(cudaGetLastError(), "k_gen_wgrad_tc");
 }
 
 // Weight gradient of a layer, and its bias gradient where gb is not null.
 template <int CIN, int COUT>
-int wgrad_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, float* gb, int nimg) {
+int wgrad_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, float* gb, int nimg,
+                 SumArgs& sums) {
     if (CIN == tc::kC && COUT == tc::kC && g->use_tc && wg::block_len(g->L) > 0)
-        return wgrad_tc_launch(g, in, dout, gw, gb, nimg);
+        return wgrad_tc_launch(g, in, dout, gw, gb, nimg, sums);
     const int tiles = (g->L / kTile) * (g->L / kTile);
-    const int per = 4;
+    const int per = CIN == kGenC && COUT == kGenC ? 4 : kEdgePer;   // images of a CTA
     const int groups = (nimg + per - 1) / per;
     const int nparts = tiles * groups;
     const size_t n = (size_t)9 * CIN * COUT;
-    if ((size_t)nparts * n > g->wpart_cap) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
+    float* part = sum_room(g, sums, nparts, n);
+    if (!part) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
     if constexpr (CIN == kGenC && COUT == kGenC) {
         const size_t smem = (size_t)((kTile + 2) * (kTile + 2) * CIN + kTile * kTile * COUT) * sizeof(float);
         if (int rc = ensure_smem(g, (const void*)k_gen_wgrad<CIN, COUT>, (int)smem, false)) return rc;
-        launch_seq(g->stream, k_gen_wgrad<CIN, COUT>, dim3(nparts), 432, smem, in, dout, g->wpart, g->L, per, nimg);
+        launch_seq(g->stream, k_gen_wgrad<CIN, COUT>, dim3(nparts), 432, smem, in, dout, part, g->L, per, nimg);
     } else {
         using E = EdgeGrad<CIN, COUT>;
         if (int rc = ensure_smem(g, (const void*)k_gen_wgrad_edge<CIN, COUT>, (int)E::smem, false)) return rc;
-        launch_seq(g->stream, k_gen_wgrad_edge<CIN, COUT>, dim3(nparts), E::kThreads, E::smem, in, dout, g->wpart, g->L, per, nimg);
+        launch_seq(g->stream, k_gen_wgrad_edge<CIN, COUT>, dim3(nparts), E::kThreads, E::smem, in, dout, part, g->L, per, nimg);
     }
-    sum_parts(g, nparts, (int)n, gw, (int)n, nullptr);
+    sum_add(sums, gw, (int)n, nullptr);
     if (int rc = cuda_check(cudaGetLastError(), "k_gen_wgrad")) return rc;
-    return gb ? bgrad_launch(g, dout, nimg, COUT, gb) : NMMC_OK;
+    return gb ? bgrad_launch(g, dout, nimg, COUT, gb, sums) : NMMC_OK;
 }
 
 // The weights' compute forms, after one Adam step where `step` says so.
@@ -2167,7 +2196,12 @@ int ensure_batch(nmmc_gen* g, int b) {
     NMMC_CUDA(cudaMalloc(&g->g1, np * kGenC * sizeof(float)));
     NMMC_CUDA(cudaMalloc(&g->gv, np * kGenCout * sizeof(float)));
     const int tiles = (g->L / kTile) * (g->L / kTile);
-    g->wpart_cap = (size_t)tiles * ((b + 3) / 4) * wg::kPart;
+    // the partials of one layer on the FMA pipes, or of a whole backward pass on the tensor cores
+    const size_t tc_parts = std::min<size_t>((size_t)b * g->L * std::max(1, g->L / 128), std::max(1, g->sm_count));
+    g->wpart_cap = std::max((size_t)tiles * ((b + 3) / 4) * wg::kPart,
+                            (kGenLayers - 2) * tc_parts * wg::kPart +
+                                (size_t)tiles * ((b + kEdgePer - 1) / kEdgePer) * 9 * kGenC * (kGenCin0 + kGenCout) +
+                                (size_t)b * ((g->L * g->L + kBgradRun - 1) / kBgradRun) * (kGenC + kGenCout));
     NMMC_CUDA(cudaMalloc(&g->wpart, g->wpart_cap * sizeof(float)));
     NMMC_CUDA(cudaMalloc(&g->d_idx, sizeof(int) * b));
     NMMC_CUDA(cudaMalloc(&g->d_sig, sizeof(float) * b));
@@ -2202,14 +2236,15 @@ int backward(nmmc_gen* g, int nb) {
     int rc;
     GenLayer* y = g->layer;
     const int last = kGenLayers - 1;
+    SumArgs sums;
     // last layer: weights and bias, then data gradient into g0 (masked by act[last] > 0)
-    if ((rc = wgrad_launch<kGenC, kGenCout>(g, g->act[last], g->gv, y[last].gw, y[last].gb, nb))) return rc;
+    if ((rc = wgrad_launch<kGenC, kGenCout>(g, g->act[last], g->gv, y[last].gw, y[last].gb, nb, sums))) return rc;
     if ((rc = conv_launch<kGenCout, kGenC, float, 2>(g, g->gv, y[last].wt, nullptr, g->act[last], kGenC, g->g0, nb)))
         return rc;
     float* cur = g->g0;
     float* nxt = g->g1;
     for (int l = last - 1; l >= 1; --l) {
-        if ((rc = wgrad_launch<kGenC, kGenC>(g, g->act[l], cur, y[l].gw, y[l].gb, nb))) return rc;
+        if ((rc = wgrad_launch<kGenC, kGenC>(g, g->act[l], cur, y[l].gw, y[l].gb, nb, sums))) return rc;
         rc = g->use_tc ? conv_tc_launch<2>(g, cur, y[l].wt, nullptr, g->act[l], nxt, nb, y[l].wtimg)
                        : conv_launch<kGenC, kGenC, float, 2>(g, cur, y[l].wt, nullptr, g->act[l], kGenC, nxt, nb);
         if (rc) return rc;
@@ -2217,8 +2252,8 @@ int backward(nmmc_gen* g, int nb) {
         cur = nxt;
         nxt = t;
     }
-    if ((rc = wgrad_launch<kGenCin0, kGenC>(g, g->act[0], cur, y[0].gw, y[0].gb, nb))) return rc;
-    return cuda_check(cudaGetLastError(), "backward");
+    if ((rc = wgrad_launch<kGenCin0, kGenC>(g, g->act[0], cur, y[0].gw, y[0].gb, nb, sums))) return rc;
+    return launch_sums(g, sums);
 }
 
 void free_gen(nmmc_gen* g) {
@@ -2605,7 +2640,9 @@ int nmmc_gen_probe_wgrad(nmmc_gen* g, int nimg, const float* in, const float* do
     if (!rc) rc = cuda_check(cudaMemcpy(d_g, hg.data(), ne * sizeof(float), cudaMemcpyHostToDevice), "probe H2D");
     const int keep = g->use_tc;
     g->use_tc = tensor ? 1 : 0;
-    if (!rc) rc = wgrad_launch<kGenC, kGenC>(g, d_in, d_g, d_w, nullptr, nimg);
+    SumArgs sums;
+    if (!rc) rc = wgrad_launch<kGenC, kGenC>(g, d_in, d_g, d_w, nullptr, nimg, sums);
+    if (!rc) rc = launch_sums(g, sums);
     g->use_tc = keep;
     if (!rc) rc = cuda_check(cudaStreamSynchronize(g->stream), "probe wgrad");
     if (!rc) rc = check_flag(g);
