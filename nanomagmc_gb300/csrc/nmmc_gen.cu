@@ -344,6 +344,12 @@ __device__ __forceinline__ void gen_bulk(uint32_t dst, const void* src, uint32_t
                  : "memory");
 }
 
+__device__ __forceinline__ void gen_mbar_init(void* bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gen_smem_u32(bar)), "r"(count) : "memory");
+}
+// barrier 1 for `threads` of the block's threads
+__device__ __forceinline__ void gen_bar_sync(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+
 // an arrival on `bar` when the MMAs issued so far by this thread have completed
 __device__ __forceinline__ void gen_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -686,6 +692,7 @@ namespace row {
 constexpr int kSlots = 130;                   // x = -1 .. 128
 constexpr int kBlk = 2176;                    // bytes per (row, chunk) block: 130 x 16 B, 128-B aligned
 constexpr int kAcc = 10;                      // accumulators: 480 of 512 TMEM columns
+static_assert(kAcc < 15, "one lane per barrier");
 constexpr int kEpi = 8;                       // epilogue warps
 constexpr int kThreads = (kEpi + 3) * 32;
 // MMA N for co output channels: M = 128 takes N in multiples of 16
@@ -740,21 +747,26 @@ k_gen_conv_row(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_
     const int r0 = (int)((long long)nrows * blockIdx.x / gridDim.x);
     const int r1 = (int)((long long)nrows * (blockIdx.x + 1) / gridDim.x);
 
-    if (tid == 0) {
-        for (int s = 0; s < kS; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&raw[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&full[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&empty[s])) : "memory");
+    // the block comes together once, after the barriers; the producer then begins, while the others
+    // clear the accumulators
+    if (warp == row::kEpi) {
+        if (lane < kS) {
+            gen_mbar_init(&raw[lane], 1);
+            gen_mbar_init(&full[lane], 1);
+            gen_mbar_init(&empty[lane], 1);
         }
-        for (int a = 0; a < row::kAcc; ++a) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&tfull[a])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(gen_smem_u32(&tempty[a])) : "memory");
+        if (lane >= 16 && lane < 16 + row::kAcc) {
+            gen_mbar_init(&tfull[lane - 16], 1);
+            gen_mbar_init(&tempty[lane - 16], 4);
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&wbar)) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&done)) : "memory");
+        if (lane == 31) {
+            gen_mbar_init(&wbar, 1);
+            gen_mbar_init(&done, 1);
+            abort_word = 0;
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        abort_word = 0;
-        if (use_img) {
+        __syncwarp();
+        if (lane == 31 && use_img) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gen_smem_u32(&wbar)), "r"(9u * kBT)
                          : "memory");
             gen_bulk(bBase, wimg, 9u * kBT, gen_smem_u32(&wbar));
@@ -794,13 +806,16 @@ k_gen_conv_row(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    if (warp < 4) {   // every accumulator starts at zero
-        for (int c = 0; c < row::kAcc * NN; c += 16) tmem_zero16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    if (warp != row::kEpi) {
+        if (warp < 8) {   // every accumulator starts at zero
+            for (int c = warp >> 2; c < row::kAcc * NN / 16; c += 2)
+                tmem_zero16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(16 * c));
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        gen_bar_sync(row::kThreads - 32);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     if (warp < row::kEpi) {
         const int grp = warp >> 2;
@@ -1230,18 +1245,20 @@ k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ d
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 0) {
-        for (int s = 0; s < kRows; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&copied[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&ready[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&rfree[s])) : "memory");
+    if (warp == 1) {
+        if (lane < kRows) {
+            gen_mbar_init(&copied[lane], 1);
+            gen_mbar_init(&ready[lane], 1);
+            gen_mbar_init(&rfree[lane], 1);
         }
-        for (int s = 0; s < kStages; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gen_smem_u32(&gfull[s])), "r"(kStep / 32) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&gfree[s])) : "memory");
+        if (lane >= 16 && lane < 16 + kStages) {
+            gen_mbar_init(&gfull[lane - 16], kStep / 32);
+            gen_mbar_init(&gfree[lane - 16], 1);
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gen_smem_u32(&done)) : "memory");
-        abort_word = 0;
+        if (lane == 31) {
+            gen_mbar_init(&done, 1);
+            abort_word = 0;
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // the zeroed slots are read by the tensor cores (async proxy)
@@ -1250,13 +1267,17 @@ k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ d
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    if (warp < 4) {   // the accumulators start at zero
-        for (int c = 0; c < 3 * kAccCols; c += 16) tmem_zero16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    // the accumulators start at zero: four of the converting warps clear them before the MMA warp
+    // begins; the others go on
+    if (warp == 1 || warp >= 12) {
+        if (warp >= 12) {
+            for (int c = 0; c < 3 * kAccCols; c += 16) tmem_zero16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        gen_bar_sync(5 * 32);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     const int ct = tid - (kThreads - kConv);                // converting thread
     float bsum[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
