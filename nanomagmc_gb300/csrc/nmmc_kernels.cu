@@ -1470,7 +1470,7 @@ __device__ __forceinline__ void heis_site_terms(const DevModel& m, const int x, 
     if (qv[0] && qv[3]) acc[10] += solid_angle_f(s0, s1, s2, n0[0], n1[0], n2[0], n0[3], n1[3], n2[3]);
 }
 
-template <int DIM, bool ISING, bool MASKED, typename RT>
+template <int DIM, bool ISING, bool MASKED, typename RT, int DK = -1>
 __global__ void __launch_bounds__(256)
 k_measure(const DevModel m, const void* __restrict__ spins_v, const uint8_t* __restrict__ mask,
           const uint32_t* __restrict__ fill, const int* __restrict__ fill_zoff,
@@ -1530,7 +1530,8 @@ k_measure(const DevModel m, const void* __restrict__ spins_v, const uint8_t* __r
             else n0[k] = n1[k] = n2[k] = RT(0);
             if (k < 4) qv[k] = exists && (inside || (m.periodic && m.periodic_q));
         }
-        site_terms<DIM, ISING, RT>(m, x, y, z, s0, s1, s2, n0, n1, n2, qv, acc);
+        if constexpr (DK >= 0) heis_site_terms<DIM, DK>(m, x, y, z, s0, s1, s2, n0, n1, n2, qv, acc);
+        else site_terms<DIM, ISING, RT>(m, x, y, z, s0, s1, s2, n0, n1, n2, qv, acc);
     };
     if (MASKED && fill) {
         // part `chunk` of z-slice z's filled sites, both colours, from the chain's lists
@@ -2244,7 +2245,15 @@ static void measure_launch(Ctx& c, const int* d_chains, int n, int rows, int nbl
     if (fp64)
         k_measure<DIM, ISING, MASKED, double><<<grid, 256, 0, c.stream>>>(
             c.m, c.d_spins, c.d_mask, fill, c.d_fill_zoff, d_chains, rows, nblk_slice, partial);
-    else
+    else if constexpr (!ISING && MASKED) {   // the terms of k_measure_compact, the same sums
+        using Fn = void (*)(const DevModel, const void*, const uint8_t*, const uint32_t*, const int*, const int*, int, int, double*);
+        const int dk = c.m.dmi_kind;
+        Fn fn = dk == kDmiNone      ? (Fn)k_measure<DIM, false, true, float, kDmiNone>
+                : dk == kDmiGeneral ? (Fn)k_measure<DIM, false, true, float, kDmiGeneral>
+                : dk == kDmiPairs   ? (Fn)k_measure<DIM, false, true, float, kDmiPairs>
+                                    : (Fn)k_measure<DIM, false, true, float, kDmiAxial>;
+        fn<<<grid, 256, 0, c.stream>>>(c.m, c.d_spins, c.d_mask, fill, c.d_fill_zoff, d_chains, rows, nblk_slice, partial);
+    } else
         k_measure<DIM, ISING, MASKED, float><<<grid, 256, 0, c.stream>>>(
             c.m, c.d_spins, c.d_mask, fill, c.d_fill_zoff, d_chains, rows, nblk_slice, partial);
 }
