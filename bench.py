@@ -462,8 +462,8 @@ def run_gpu(args, cfg):
         kernel, note = ("k_resident (sweeps and observables in one launch; time includes both)",
                         "shared-memory resident: HBM is not the bound; algorithmic bytes for comparison")
     elif general:
-        kernel, note = ("k_colour_sweep<3,periodic,Heisenberg> (%d colour classes)" % colours,
-                        "multi-colour gather sweep of a general interaction table; per launch, updates of "
+        kernel, note = ("k_class_sweep<3,periodic> (%d colour classes)" % colours,
+                        "class-plane sweep of a general interaction table; per launch, updates of "
                         "one class x 12 B x (classes + 1)")
     elif cfg["shape"] == "x":
         kernel, note = (("k_heis_compact<3,axial DMI> (filled sites in compact planes)" if compact else
