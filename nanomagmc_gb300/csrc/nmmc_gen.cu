@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256)
 k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
            const __nv_bfloat16* __restrict__ mask, int mask_c, void* __restrict__ out, int L) {
     seq_begin();
-    extern __shared__ float gsm[];
+    extern __shared__ __align__(16) float gsm[];
     constexpr int HALF = (COUT + 1) / 2;          // output channels per thread
     constexpr int T2 = kTile + 2;
     float* wsm = gsm;                              // [9][CIN][COUT]
@@ -132,8 +132,9 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
     for (int i = threadIdx.x; i < 9 * CIN * COUT / 8; i += blockDim.x) {
         const uint4 q = __ldcg(reinterpret_cast<const uint4*>(w) + i);
         const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) wsm[8 * i + k] = __bfloat162float(e[k]);
+        float4* d = reinterpret_cast<float4*>(wsm + 8 * i);
+        d[0] = make_float4(__bfloat162float(e[0]), __bfloat162float(e[1]), __bfloat162float(e[2]), __bfloat162float(e[3]));
+        d[1] = make_float4(__bfloat162float(e[4]), __bfloat162float(e[5]), __bfloat162float(e[6]), __bfloat162float(e[7]));
     }
     const size_t LL = (size_t)L * L, ibase = (size_t)img * LL;
     constexpr int EPV = epc<TIN>(), V = CIN / EPV;   // elements per load, chunks per pixel
@@ -154,6 +155,16 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
     const int px = pair & 15, py = pair >> 4;      // rows py and py + 8
     const int co0 = half * HALF;
     static_assert(HALF % 2 == 0 && COUT == 2 * HALF, "channel pairs");
+    // the mask of both pixels arrives during the sums
+    constexpr bool kWide = EPI == 2 && HALF % 8 == 0;   // whole 16-byte chunks
+    uint4 m4[kWide ? 2 : 1][kWide ? HALF / 8 : 1];
+    if constexpr (kWide)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int c = 0; c < HALF / 8; ++c)
+                m4[r][c] = __ldcg(reinterpret_cast<const uint4*>(
+                    mask + pl_off<__nv_bfloat16>(mask_c, LL, img, (size_t)(ty0 + py + 8 * r) * L + tx0 + px, co0 + 8 * c)));
     f2 a0[HALF / 2], a1[HALF / 2];   // channel pairs: packed multiply-adds
 #pragma unroll
     for (int k = 0; k < HALF / 2; ++k) {
@@ -169,11 +180,22 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
             const float x1 = tsm[(ci * T2 + py + 8 + dy) * T2 + px + dx];
             const f2 p0 = pk(x0, x0), p1 = pk(x1, x1);
             const float* wr = wsm + (tap * CIN + ci) * COUT + co0;
+            if constexpr (HALF % 4 == 0) {   // two channel pairs per load
 #pragma unroll
-            for (int k = 0; k < HALF / 2; ++k) {
-                const f2 wv{*reinterpret_cast<const unsigned long long*>(wr + 2 * k)};
-                a0[k] = fma2(p0, wv, a0[k]);
-                a1[k] = fma2(p1, wv, a1[k]);
+                for (int k = 0; k < HALF / 2; k += 2) {
+                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(wr + 2 * k);
+                    a0[k] = fma2(p0, f2{q.x}, a0[k]);
+                    a1[k] = fma2(p1, f2{q.x}, a1[k]);
+                    a0[k + 1] = fma2(p0, f2{q.y}, a0[k + 1]);
+                    a1[k + 1] = fma2(p1, f2{q.y}, a1[k + 1]);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < HALF / 2; ++k) {
+                    const f2 wv{*reinterpret_cast<const unsigned long long*>(wr + 2 * k)};
+                    a0[k] = fma2(p0, wv, a0[k]);
+                    a1[k] = fma2(p1, wv, a1[k]);
+                }
             }
         }
     }
@@ -187,12 +209,10 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
             v[2 * k] = lo(r ? a1[k] : a0[k]);
             v[2 * k + 1] = hi(r ? a1[k] : a0[k]);
         }
-        if constexpr (EPI == 2 && HALF % 8 == 0) {   // whole 16-byte chunks
+        if constexpr (kWide) {
 #pragma unroll
             for (int c = 0; c < HALF / 8; ++c) {
-                const uint4 m4 = __ldcg(reinterpret_cast<const uint4*>(
-                    mask + pl_off<__nv_bfloat16>(mask_c, LL, img, pp, co0 + 8 * c)));
-                const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&m4);
+                const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&m4[r][c]);
                 float o[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) o[k] = __bfloat162float(mh[k]) > 0.0f ? v[8 * c + k] : 0.0f;
