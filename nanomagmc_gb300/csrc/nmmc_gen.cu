@@ -32,6 +32,12 @@ constexpr int kGenCout = 4;      // 3 spin components + 1 zero (vector loads)
 constexpr int kWimgBytes = 9 * (kGenC / 8) * (kGenC / 8) * 128;   // largest layer weight image (48 -> 48)
 constexpr int kTile = 16;        // pixel tile edge of the convolution kernels
 
+__device__ __forceinline__ __nv_bfloat16 ld_seq(const __nv_bfloat16* p) {
+    unsigned short v;
+    asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return __ushort_as_bfloat16(v);
+}
+
 // Activations and gradients are stored chunk-planar: C channels of element type T as
 // [image][C / epc][L*L pixels][epc], epc = 16 / sizeof(T) (8 BF16 or 4 FP32 channels per
 // 16-byte chunk), so that a chunk of consecutive pixels of a row is contiguous: one bulk copy
@@ -115,8 +121,8 @@ namespace nmmc {
 // ------------------------------------------------------------------------------------------
 template <int CIN, int COUT, typename TIN, int EPI>
 __global__ void __launch_bounds__(256)
-k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
-           const __nv_bfloat16* __restrict__ mask, int mask_c, void* __restrict__ out, int L) {
+k_gen_conv(const TIN* in, const __nv_bfloat16* w, const float* bias,
+           const __nv_bfloat16* mask, int mask_c, void* out, int L) {
     seq_begin();
     extern __shared__ __align__(16) float gsm[];
     constexpr int HALF = (COUT + 1) / 2;          // output channels per thread
@@ -130,7 +136,7 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
     static_assert((9 * CIN * COUT) % 8 == 0 && (CIN * sizeof(TIN)) % 16 == 0, "16-byte staging");
 #pragma unroll 4
     for (int i = threadIdx.x; i < 9 * CIN * COUT / 8; i += blockDim.x) {
-        const uint4 q = __ldcg(reinterpret_cast<const uint4*>(w) + i);
+        const uint4 q = ld_seq(reinterpret_cast<const uint4*>(w) + i);
         const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
         float4* d = reinterpret_cast<float4*>(wsm + 8 * i);
         d[0] = make_float4(__bfloat162float(e[0]), __bfloat162float(e[1]), __bfloat162float(e[2]), __bfloat162float(e[3]));
@@ -145,7 +151,7 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
         int gy = ty0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
         gy += (gy < 0) ? L : ((gy >= L) ? -L : 0);
         gx += (gx < 0) ? L : ((gx >= L) ? -L : 0);
-        const uint4 q = __ldcg(src + (size_t)v * LL + (size_t)gy * L + gx);
+        const uint4 q = ld_seq(src + (size_t)v * LL + (size_t)gy * L + gx);
         const TIN* e = reinterpret_cast<const TIN*>(&q);
 #pragma unroll
         for (int k = 0; k < EPV; ++k) tsm[((v * EPV + k) * T2 + yy) * T2 + xx] = (float)e[k];
@@ -163,12 +169,12 @@ k_gen_conv(const TIN* __restrict__ in, const __nv_bfloat16* __restrict__ w, cons
         for (int r = 0; r < 2; ++r)
 #pragma unroll
             for (int c = 0; c < HALF / 8; ++c)
-                m4[r][c] = __ldcg(reinterpret_cast<const uint4*>(
+                m4[r][c] = ld_seq(reinterpret_cast<const uint4*>(
                     mask + pl_off<__nv_bfloat16>(mask_c, LL, img, (size_t)(ty0 + py + 8 * r) * L + tx0 + px, co0 + 8 * c)));
     f2 a0[HALF / 2], a1[HALF / 2];   // channel pairs: packed multiply-adds
 #pragma unroll
     for (int k = 0; k < HALF / 2; ++k) {
-        a0[k] = bias ? pk(__ldcg(bias + co0 + 2 * k), __ldcg(bias + co0 + 2 * k + 1)) : f2{0ull};
+        a0[k] = bias ? pk(ld_seq(bias + co0 + 2 * k), ld_seq(bias + co0 + 2 * k + 1)) : f2{0ull};
         a1[k] = a0[k];
     }
 #pragma unroll 1
@@ -408,7 +414,7 @@ __device__ __forceinline__ void stage_weights(uint8_t* sB, const __nv_bfloat16* 
     constexpr int kC = tc::kC, kG = 9 * kC * kC / 8;
 #pragma unroll 7
     for (int g8 = tid; g8 < kG; g8 += nthr) {
-        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(w) + g8);
+        const uint4 v = ld_seq(reinterpret_cast<const uint4*>(w) + g8);
         const int i = g8 * 8;
         const int tap = i / (kC * kC), r = i - tap * kC * kC, k = r / kC, n = r - k * kC;
         uint8_t* base = sB + (ROWS ? tap % 3 * 3 + 2 - tap / 3 : tap) * kBT + ((n >> 3) * kCh + k / kEpc) * tc::kCore + (k % kEpc) * (int)sizeof(TA);
@@ -425,7 +431,7 @@ __device__ __forceinline__ void load_mask(uint4* m4, const __nv_bfloat16* __rest
     if (MODE == 2) {
         const uint4* mk = reinterpret_cast<const uint4*>(mask + img * LL * tc::kC) + pp;
 #pragma unroll
-        for (int c = 0; c < tc::kC / 8; ++c) m4[c] = __ldcg(mk + (size_t)c * LL);
+        for (int c = 0; c < tc::kC / 8; ++c) m4[c] = ld_seq(mk + (size_t)c * LL);
     }
 }
 
@@ -521,9 +527,9 @@ __device__ __forceinline__ bool elect_one() {
 // epilogue were both slower.)
 template <int MODE>
 __global__ void __launch_bounds__(128, 2)
-k_gen_conv_tc(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_bfloat16* __restrict__ w,
-              const float* __restrict__ bias, const __nv_bfloat16* __restrict__ mask, void* __restrict__ out_v,
-              int L, int tiles_per_img, int ntiles, int* __restrict__ flag) {
+k_gen_conv_tc(const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w,
+              const float* bias, const __nv_bfloat16* mask, void* out_v,
+              int L, int tiles_per_img, int ntiles, int* flag) {
     seq_begin();
     using namespace tc;
     using TA = typename Traits<MODE>::TA;
@@ -543,7 +549,7 @@ k_gen_conv_tc(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_b
 
     // weights w[tap][k][n] (k: input channel of this convolution) -> B_tap[n][k], K-major
     stage_weights<MODE>(sB, w, tid, blockDim.x);
-    if (tid < kC) sbias[tid] = (MODE == 2) ? 0.0f : __ldcg(bias + tid);
+    if (tid < kC) sbias[tid] = (MODE == 2) ? 0.0f : ld_seq(bias + tid);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gen_smem_u32(&tmem_slot)),
                      "r"(kTmemCols)
@@ -736,9 +742,9 @@ __host__ __device__ constexpr int smem_bytes() { return 9 * btap<KCH, CO>() + ri
 
 template <int MODE, int ICH, int KCH, int CO>
 __global__ void __launch_bounds__(row::kThreads, 1)
-k_gen_conv_row(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_bfloat16* __restrict__ w,
-               const uint8_t* __restrict__ wimg, const float* __restrict__ bias,
-               const __nv_bfloat16* __restrict__ mask, void* __restrict__ out_v, int nrows, int* __restrict__ flag) {
+k_gen_conv_row(const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w,
+               const uint8_t* wimg, const float* bias,
+               const __nv_bfloat16* mask, void* out_v, int nrows, int* flag) {
     seq_begin();
     using namespace tc;
     using TA = typename Traits<MODE>::TA;
@@ -814,13 +820,13 @@ k_gen_conv_row(const typename tc::Traits<MODE>::TA* __restrict__ in, const __nv_
 #pragma unroll 4
             for (int i = tid; i < 9 * NN * KK; i += row::kThreads) {
                 const int tap = i / (NN * KK), r = i - tap * NN * KK, nn = r / KK, k = r - nn * KK;
-                const float v = (nn < CO && k < CI) ? __bfloat162float(__ldcg(w + (tap * CI + k) * CO + nn)) : 0.0f;
+                const float v = (nn < CO && k < CI) ? __bfloat162float(ld_seq(w + (tap * CI + k) * CO + nn)) : 0.0f;
                 *(TA*)(sB + row::place(tap) * kBT + ((nn >> 3) * KCH + k / kEpc) * kCore + (nn & 7) * 16 +
                        (k % kEpc) * (int)sizeof(TA)) = (TA)v;
             }
         }
     }
-    if (tid < NN) sbias[tid] = (MODE == 2 || tid >= CO) ? 0.0f : __ldcg(bias + tid);
+    if (tid < NN) sbias[tid] = (MODE == 2 || tid >= CO) ? 0.0f : ld_seq(bias + tid);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -1232,8 +1238,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 
 template <int KS>   // MMA K-steps (16 positions) per K-block: W = 16 KS
 __global__ void __launch_bounds__(wg::kThreads, 1)
-k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout, float* __restrict__ part,
-               int L, int nkb, int* __restrict__ flag) {
+k_gen_wgrad_tc(const __nv_bfloat16* in, const float* dout, float* part,
+               int L, int nkb, int* flag) {
     seq_begin();
     using namespace wg;
     constexpr int kC = tc::kC, W = 16 * KS;
@@ -1424,8 +1430,8 @@ k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ d
             const float4* p = reinterpret_cast<const float4*>(dout) + ((size_t)img * (kC / 4) + 2 * h) * LL + (size_t)y * L + x0 + c;
 #pragma unroll
             for (int i = 0; i < kPer; ++i) {
-                nx[i][0] = __ldcg(p + i * kWs);
-                nx[i][1] = __ldcg(p + LL + i * kWs);
+                nx[i][0] = ld_seq(p + i * kWs);
+                nx[i][1] = ld_seq(p + LL + i * kWs);
             }
         };
         if (n > 0) fetch(b0);
@@ -1523,7 +1529,7 @@ k_gen_wgrad_tc(const __nv_bfloat16* __restrict__ in, const float* __restrict__ d
 // Thread layout: 9 taps x (CIN/6) ci groups x (COUT/8) co groups (6 x 8 accumulators each).
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(432)
-k_gen_wgrad(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout, float* __restrict__ part,
+k_gen_wgrad(const __nv_bfloat16* in, const float* dout, float* part,
             int L, int images_per_cta, int nimg) {
     seq_begin();
     extern __shared__ float gsm[];
@@ -1561,7 +1567,7 @@ k_gen_wgrad(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout
             int gy = ty0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
             gy += (gy < 0) ? L : ((gy >= L) ? -L : 0);
             gx += (gx < 0) ? L : ((gx >= L) ? -L : 0);
-            const uint4 q = __ldcg(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
+            const uint4 q = ld_seq(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
             const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
             float* d = tin + pix * CIN + c8 * 8;
 #pragma unroll
@@ -1571,7 +1577,7 @@ k_gen_wgrad(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout
         for (int i = threadIdx.x; i < kTile * kTile * (COUT / 4); i += blockDim.x) {
             const int c4 = i / (kTile * kTile), pix = i - c4 * kTile * kTile, yy = pix / kTile, xx = pix - yy * kTile;
             reinterpret_cast<float4*>(tdo + pix * COUT)[c4] =
-                __ldcg(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
+                ld_seq(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
         }
         __syncthreads();
         if (active) {
@@ -1624,7 +1630,7 @@ struct EdgeGrad {
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(EdgeGrad<CIN, COUT>::kThreads, 2)
-k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__ dout, float* __restrict__ part,
+k_gen_wgrad_edge(const __nv_bfloat16* in, const float* dout, float* part,
                  int L, int images_per_cta, int nimg) {
     seq_begin();
     using E = EdgeGrad<CIN, COUT>;
@@ -1660,7 +1666,7 @@ k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__
             int gy = ty0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
             gy += (gy < 0) ? L : ((gy >= L) ? -L : 0);
             gx += (gx < 0) ? L : ((gx >= L) ? -L : 0);
-            const uint4 q = __ldcg(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
+            const uint4 q = ld_seq(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
             float4* d = reinterpret_cast<float4*>(tin + pix * E::SI + E::at(c8 * 8));   // a BF16 is an FP32's top half
             d[0] = make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xFFFF0000u),
                                __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xFFFF0000u));
@@ -1671,7 +1677,7 @@ k_gen_wgrad_edge(const __nv_bfloat16* __restrict__ in, const float* __restrict__
         for (int i = t; i < kTile * kTile * (COUT / 4); i += E::kThreads) {
             const int c4 = i / (kTile * kTile), pix = i - c4 * kTile * kTile, yy = pix / kTile, xx = pix - yy * kTile;
             *reinterpret_cast<float4*>(tdo + pix * E::SO + E::at(c4 * 4)) =
-                __ldcg(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
+                ld_seq(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
         }
         __syncthreads();
         for (int py = grp; py < kTile; py += E::kGroups) {
@@ -1750,7 +1756,7 @@ __global__ void __launch_bounds__(128) k_gen_sum_parts(const __grid_constant__ S
         const int nparts = s.nparts;
 #pragma unroll 10
         for (int p = t; p < nparts; p += 8) {
-            const float4 w = __ldcg(reinterpret_cast<const float4*>(p0 + p * stride));
+            const float4 w = ld_seq(reinterpret_cast<const float4*>(p0 + p * stride));
             v.x += w.x;
             v.y += w.y;
             v.z += w.z;
@@ -1778,7 +1784,7 @@ __global__ void __launch_bounds__(128) k_gen_sum_parts(const __grid_constant__ S
 // lanes per channel group before.
 constexpr int kBgradRun = 2048;
 __global__ void __launch_bounds__(256)
-k_gen_bgrad_part(const float* __restrict__ dout, int LL, int cout, int nseg, float* __restrict__ part) {
+k_gen_bgrad_part(const float* dout, int LL, int cout, int nseg, float* part) {
     seq_begin();
     const int seg = blockIdx.x, g = blockIdx.y, img = blockIdx.z, G = cout / 4;
     const float4* src = reinterpret_cast<const float4*>(dout) + ((size_t)img * G + g) * LL;
@@ -1786,7 +1792,7 @@ k_gen_bgrad_part(const float* __restrict__ dout, int LL, int cout, int nseg, flo
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int p = p0 + threadIdx.x; p < p1; p += 256) {
-        const float4 v = __ldcg(src + p);
+        const float4 v = ld_seq(src + p);
         s.x += v.x;
         s.y += v.y;
         s.z += v.z;
@@ -1869,10 +1875,10 @@ __global__ void __launch_bounds__(128) k_gen_update(const __grid_constant__ Upda
 // a' = 1 - s_prev^2, a = 1 - s^2, alpha = a'/a, y = sqrt(a)(1-alpha)/(1-a') x
 // + sqrt(alpha)(1-a)/(1-a') y' + sqrt((1-a)(1-alpha)/(1-a')) g, then normalised.
 __global__ void k_gen_input(int mode, const __nv_bfloat16* __restrict__ snaps, const int* __restrict__ idx,
-                            const float* __restrict__ cur, const float* __restrict__ sig,
+                            const float* cur, const float* __restrict__ sig,
                             const float* __restrict__ cnd, int L, uint32_t k0, uint32_t k1,
-                            unsigned long long draw0, __nv_bfloat16* __restrict__ act0,
-                            float* __restrict__ target, float s_prev) {
+                            unsigned long long draw0, __nv_bfloat16* act0,
+                            float* target, float s_prev) {
     seq_begin();
     const int item = blockIdx.y;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1882,7 +1888,7 @@ __global__ void k_gen_input(int mode, const __nv_bfloat16* __restrict__ snaps, c
         const __nv_bfloat16* s = snaps + ((size_t)idx[item] * L * L + p) * 3;
         for (int c = 0; c < 3; ++c) x[c] = __bfloat162float(s[c]);
     } else {
-        const float4 e = __ldcg(reinterpret_cast<const float4*>(cur) + (size_t)item * L * L + p);
+        const float4 e = ld_seq(reinterpret_cast<const float4*>(cur) + (size_t)item * L * L + p);
         x[0] = e.x;
         x[1] = e.y;
         x[2] = e.z;
@@ -1942,14 +1948,14 @@ __global__ void k_gen_input(int mode, const __nv_bfloat16* __restrict__ snaps, c
 // Loss and its gradient through spin = v/|v|: loss += |s - x|^2 / npix_total;
 // dL/dv = (g - s (s.g)) / |v| with g = 2 (s - x) / npix_total.
 __global__ void __launch_bounds__(256)
-k_gen_head(const float* __restrict__ v, const float* __restrict__ target, int npix, float scale,
-           float* __restrict__ gv, double* __restrict__ loss) {
+k_gen_head(const float* v, const float* target, int npix, float scale,
+           float* gv, double* loss) {
     seq_begin();
     __shared__ float red[8];
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     float l = 0.0f;
     if (p < npix) {
-        const float4 a4 = __ldcg(reinterpret_cast<const float4*>(v) + p), x4 = __ldcg(reinterpret_cast<const float4*>(target) + p);
+        const float4 a4 = ld_seq(reinterpret_cast<const float4*>(v) + p), x4 = ld_seq(reinterpret_cast<const float4*>(target) + p);
         const float a[3] = {a4.x, a4.y, a4.z}, x[3] = {x4.x, x4.y, x4.z};
         const float n2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + 1e-12f;
         const float inv = rsqrtf(n2);
@@ -1976,11 +1982,11 @@ k_gen_head(const float* __restrict__ v, const float* __restrict__ target, int np
 }
 
 // Sampling: cur <- normalise(v) (the denoised estimate)
-__global__ void k_gen_normalise(const float* __restrict__ v, int npix, float* __restrict__ cur) {
+__global__ void k_gen_normalise(const float* v, int npix, float* cur) {
     seq_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npix) return;
-    const float4 a = __ldcg(reinterpret_cast<const float4*>(v) + p);
+    const float4 a = ld_seq(reinterpret_cast<const float4*>(v) + p);
     const float n2 = a.x * a.x + a.y * a.y + a.z * a.z;
     const float inv = n2 > 0.0f ? rsqrtf(n2) : 0.0f;
     reinterpret_cast<float4*>(cur)[p] = make_float4(a.x * inv, a.y * inv, a.z * inv, 0.0f);

@@ -136,8 +136,8 @@ __device__ __forceinline__ void general_field(const DevModel& m, const void* __r
 // One colour class of every listed chain (grid.y = list position).
 template <int DIM, bool PERIODIC, bool MASKED, bool ISING>
 __global__ void __launch_bounds__(256)
-k_colour_sweep(const DevModel m, void* __restrict__ spins_v, const uint8_t* __restrict__ mask,
-               const float4* __restrict__ bh, const unsigned long long* __restrict__ sweep,
+k_colour_sweep(const DevModel m, void* spins_v, const uint8_t* __restrict__ mask,
+               const float4* __restrict__ bh, const unsigned long long* sweep,
                const int* __restrict__ chains, int colour, unsigned off) {
     seq_begin();
     const int chain = chains[blockIdx.y];
@@ -311,8 +311,8 @@ __device__ __forceinline__ void class_field(const ClassTable& t, const ClassBase
 template <int DIM, bool PERIODIC>
 __global__ void __launch_bounds__(256, 4)
 k_class_sweep(const __grid_constant__ DevModel m, const ClassShape s, const __grid_constant__ ClassTable t,
-              const __grid_constant__ ClassBase base, float4* __restrict__ planes, const float4* __restrict__ bh,
-              const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour, unsigned off) {
+              const __grid_constant__ ClassBase base, float4* planes, const float4* __restrict__ bh,
+              const unsigned long long* sweep, const int* __restrict__ chains, int colour, unsigned off) {
     extern __shared__ int cl_slots[];
     const int cell = blockIdx.x * blockDim.x + threadIdx.x;
     int x, y, z;
@@ -337,7 +337,7 @@ k_class_sweep(const __grid_constant__ DevModel m, const ClassShape s, const __gr
 // Between the box layout and the class planes of the listed chains.
 template <int DIM>
 __global__ void __launch_bounds__(256)
-k_class_copy(const DevModel m, const ClassShape s, float4* __restrict__ planes, float* __restrict__ spins,
+k_class_copy(const DevModel m, const ClassShape s, float4* planes, float* spins,
              const int* __restrict__ chains, int to_class) {
     seq_begin();
     const int chain = chains[blockIdx.y];
@@ -365,8 +365,8 @@ k_class_copy(const DevModel m, const ClassShape s, float4* __restrict__ planes, 
 template <int DIM, bool PERIODIC>
 __global__ void __launch_bounds__(256, 4)
 k_class_energy(const __grid_constant__ DevModel m, const ClassShape s, const __grid_constant__ ClassTable t,
-               const __grid_constant__ ClassBase base, const float4* __restrict__ planes, const int* __restrict__ chains,
-               int cls, int nblk, float scale, double* __restrict__ partial) {
+               const __grid_constant__ ClassBase base, const float4* planes, const int* __restrict__ chains,
+               int cls, int nblk, float scale, double* partial) {
     seq_begin();
     extern __shared__ int cl_slots[];
     __shared__ float red[8];

@@ -79,8 +79,8 @@ __global__ void __launch_bounds__(kItabMax) k_ising_table(const DevModel m, cons
 // One colour of every listed chain; a thread updates 4W consecutive sites of a row.
 template <int DIM, bool PERIODIC, int W>
 __global__ void __launch_bounds__(256)
-k_ising_words(const DevModel m, int8_t* __restrict__ spins, const float4* __restrict__ bh,
-              const unsigned long long* __restrict__ sweep, const int* __restrict__ chains,
+k_ising_words(const DevModel m, int8_t* spins, const float4* __restrict__ bh,
+              const unsigned long long* sweep, const int* __restrict__ chains,
               const uint32_t* __restrict__ tab, int colour, unsigned sweep_off) {
     seq_begin();
     constexpr int ND = 2 * DIM;

@@ -18,9 +18,9 @@ namespace nmmc {
 // ------------------------------------------------------------------------------------------
 template <int DIM, bool PERIODIC, bool MASKED, int DK>
 __global__ void __launch_bounds__(256)
-k_heis_half(const DevModel m, float* __restrict__ spins, const uint32_t* __restrict__ fill,
+k_heis_half(const DevModel m, float* spins, const uint32_t* __restrict__ fill,
             const int* __restrict__ fill_n, const float4* __restrict__ bh,
-            const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour,
+            const unsigned long long* sweep, const int* __restrict__ chains, int colour,
             unsigned sweep_off) {
     seq_begin();
     const int chain = chains[blockIdx.y];
@@ -65,9 +65,9 @@ k_heis_half(const DevModel m, float* __restrict__ spins, const uint32_t* __restr
 
 template <int DIM, bool PERIODIC, bool MASKED>
 __global__ void __launch_bounds__(256)
-k_ising_half(const DevModel m, int8_t* __restrict__ spins, const uint32_t* __restrict__ fill,
+k_ising_half(const DevModel m, int8_t* spins, const uint32_t* __restrict__ fill,
              const int* __restrict__ fill_n, const float4* __restrict__ bh,
-             const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour,
+             const unsigned long long* sweep, const int* __restrict__ chains, int colour,
              unsigned sweep_off) {
     seq_begin();
     const int chain = chains[blockIdx.y];
@@ -131,9 +131,9 @@ __device__ __forceinline__ void compact_entry(const int4* __restrict__ tab, int 
 
 template <int DIM, int DK, bool PACKED>
 __global__ void __launch_bounds__(256)
-k_heis_compact(const DevModel m, float4* __restrict__ cs, const int4* __restrict__ tab,
+k_heis_compact(const DevModel m, float4* cs, const int4* __restrict__ tab,
                const int* __restrict__ fill_n, const float4* __restrict__ bh,
-               const unsigned long long* __restrict__ sweep, const int* __restrict__ chains, int colour,
+               const unsigned long long* sweep, const int* __restrict__ chains, int colour,
                unsigned sweep_off) {
     seq_begin();
     const int chain = chains[blockIdx.y];
@@ -167,7 +167,7 @@ k_heis_compact(const DevModel m, float4* __restrict__ cs, const int4* __restrict
 // (grid.y = 2 x chains: chain, colour). The compact planes hold one float4 (x, y, z, 0) per
 // filled site, so that a neighbour is one 16-byte load.
 __global__ void __launch_bounds__(256)
-k_compact_copy(float4* __restrict__ cs, float* __restrict__ spins, const uint32_t* __restrict__ fill,
+k_compact_copy(float4* cs, float* spins, const uint32_t* __restrict__ fill,
                const int* __restrict__ fill_n, const int* __restrict__ chains, int nhalf, size_t P,
                int to_compact) {
     seq_begin();
@@ -401,9 +401,9 @@ __device__ __forceinline__ void q4_quad(const DevModel& m, float* __restrict__ s
 // waiting on DRAM; the prefetch changes no value.
 template <int DIM, bool PERIODIC, int DK, int MINB, int MEAS = 0>
 __global__ void __launch_bounds__(256, MINB)
-k_heis_half_q4(const DevModel m, float* __restrict__ spins, const float4* __restrict__ bh,
-               const unsigned long long* __restrict__ sweep, const int* __restrict__ chains,
-               int colour, unsigned sweep_off, int qpt, double* __restrict__ mpart, float esign, int pf,
+k_heis_half_q4(const DevModel m, float* spins, const float4* __restrict__ bh,
+               const unsigned long long* sweep, const int* __restrict__ chains,
+               int colour, unsigned sweep_off, int qpt, double* mpart, float esign, int pf,
                int nchain_list) {
     seq_begin();
     const int chain = chains[blockIdx.y];
@@ -1570,7 +1570,7 @@ k_measure(const DevModel m, const void* __restrict__ spins_v, const uint8_t* __r
 template <int DIM, int DK>
 __global__ void __launch_bounds__(256, 4)
 k_measure_box(const DevModel m, const float* spins, const int* __restrict__ chains, int rows, int nblk_slice, FastDiv div_edge,
-              double* __restrict__ partial) {
+              double* partial) {
     seq_begin();
     const int ci = blockIdx.y, chain = chains[ci], b = blockIdx.x;
     const int z = b / nblk_slice, y0 = (b - z * nblk_slice) * rows, y1 = min(y0 + rows, m.ly);
@@ -1991,9 +1991,9 @@ k_charge_rows(const DevModel m, const float* __restrict__ spins, const int* __re
 constexpr int kFinWarps = 16;
 __global__ void __launch_bounds__(32 * kFinWarps)
 k_measure_finalize(const int* __restrict__ chains, int nblk, int nblk_slice,
-                                   int nslices, int ising, const double* __restrict__ partial,
-                                   const double* __restrict__ Hd, double* __restrict__ obs,
-                                   double* __restrict__ q, double* __restrict__ accum,
+                                   int nslices, int ising, const double* partial,
+                                   const double* __restrict__ Hd, double* obs,
+                                   double* q, double* accum,
                                    int accumulate) {
     seq_begin();
     __shared__ double tot[kNP - 1], qs[kFinWarps - (kNP - 1)];
@@ -2004,7 +2004,7 @@ k_measure_finalize(const int* __restrict__ chains, int nblk, int nblk_slice,
     if (warp < kNP - 1) {
         double v = 0;
 #pragma unroll 8
-        for (int b = lane; b < nblk; b += 32) v += __ldcg(pp + (size_t)b * kNP + warp);
+        for (int b = lane; b < nblk; b += 32) v += ld_seq(pp + (size_t)b * kNP + warp);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if (lane == 0) tot[warp] = v;
@@ -2016,7 +2016,7 @@ k_measure_finalize(const int* __restrict__ chains, int nblk, int nblk_slice,
             const double* pz = pp + (size_t)zs * nblk_slice * kNP + 10;
             double v = 0;
 #pragma unroll 8
-            for (int b = tree ? lane : 0; b < nblk_slice; b += tree ? 32 : 1) v += __ldcg(pz + (size_t)b * kNP);
+            for (int b = tree ? lane : 0; b < nblk_slice; b += tree ? 32 : 1) v += ld_seq(pz + (size_t)b * kNP);
             if (tree)
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -2045,10 +2045,10 @@ k_measure_finalize(const int* __restrict__ chains, int nblk, int nblk_slice,
 // k_measure_finalize). One block of 256 threads per chain: each thread sums a fixed stride of
 // rows in FP64, then a fixed-order tree across the block, then one warp finishes the chain.
 __global__ void __launch_bounds__(256)
-k_measure_finalize_fused(const int* __restrict__ chains, const double* __restrict__ qpart, int nblk_q,
-                         int nblk_slice, int nslices, const double* __restrict__ rows, int nrows,
+k_measure_finalize_fused(const int* __restrict__ chains, const double* qpart, int nblk_q,
+                         int nblk_slice, int nslices, const double* rows, int nrows,
                          const double* __restrict__ Hd,
-                         double* __restrict__ obs, double* __restrict__ q, double* __restrict__ accum,
+                         double* obs, double* q, double* accum,
                          int accumulate) {
     seq_begin();
     const int ci = blockIdx.x;
@@ -2060,13 +2060,13 @@ k_measure_finalize_fused(const int* __restrict__ chains, const double* __restric
     for (int k = 0; k < 10; ++k) t[k] = 0.0;
     for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
         const double* bb = B + (size_t)r * 10;   // 2 e, M of colour 1, M of colour 0, sub4M
-        t[0] += __ldcg(bb);
+        t[0] += ld_seq(bb);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const double m1 = __ldcg(bb + 1 + c), m0 = __ldcg(bb + 4 + c);
+            const double m1 = ld_seq(bb + 1 + c), m0 = ld_seq(bb + 4 + c);
             t[1 + c] += m0 + m1;
             t[4 + c] += m0;
-            t[7 + c] += __ldcg(bb + 7 + c);
+            t[7 + c] += ld_seq(bb + 7 + c);
         }
     }
     __shared__ double red[10][256];
@@ -2094,7 +2094,7 @@ k_measure_finalize_fused(const int* __restrict__ chains, const double* __restric
     double qsum = 0;
     for (int zs = lane; zs < nslices; zs += 32) {
         double v = 0;
-        for (int b = 0; b < nblk_slice; ++b) v += __ldcg(pp + ((size_t)zs * nblk_slice + b) * kNP + 10);
+        for (int b = 0; b < nblk_slice; ++b) v += ld_seq(pp + ((size_t)zs * nblk_slice + b) * kNP + 10);
         v = v / (2 * M_PI);
         if (q) q[(size_t)ci * nslices + zs] = v;
         qsum += v;
@@ -2113,9 +2113,9 @@ k_measure_finalize_fused(const int* __restrict__ chains, const double* __restric
 // k_measure, so the same sums; the dense planes spare the box layout's part-empty sectors.
 template <int DIM, bool PACKED, int DK>
 __global__ void __launch_bounds__(256)
-k_measure_compact(const DevModel m, const float4* __restrict__ cs, const int4* __restrict__ tab,
+k_measure_compact(const DevModel m, const float4* cs, const int4* __restrict__ tab,
                   const int* __restrict__ fill_zoff, const int* __restrict__ chains, int nblk_slice,
-                  double* __restrict__ partial) {
+                  double* partial) {
     seq_begin();
     const int ci = blockIdx.y;
     const int chain = chains[ci];

@@ -13,11 +13,36 @@ constexpr float kLn2 = 0.693147180559945f;
 // soon as this one's are all running, then waits until the previous kernel is complete and its
 // writes are visible. Every thread of every block calls it before its first access to global
 // memory (a kernel that finished without waiting would let its successor overtake its
-// predecessor). Data that the previous kernel wrote is read with plain loads afterwards, not through
-// the read-only path.
+// predecessor). What sequenced kernels write is reached through plain pointers: a __restrict__
+// parameter is data that nothing else touches while the kernel runs, so its loads may take the
+// read-only path or move above the wait. __restrict__ stays on what the host uploads and on tables
+// that plainly launched kernels build.
 __device__ __forceinline__ void seq_begin() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Loads through L2 for data that a block reads once. They stay behind seq_begin, being volatile
+// (__ldcg need not).
+__device__ __forceinline__ float ld_seq(const float* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_seq(const double* p) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_seq(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_seq(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
 }
 
 // Packed pairs of FP32 values: one instruction for two IEEE operations (round to nearest).
