@@ -1835,8 +1835,10 @@ struct UpdateArgs {
 
 __device__ __forceinline__ float adam_step(const UpdateArgs& u, float* p, const float* g, float* m, float* v, int i) {
     const float gi = g[i];
-    const float mi = u.b1 * m[i] + (1.0f - u.b1) * gi;
-    const float vi = u.b2 * v[i] + (1.0f - u.b2) * gi * gi;
+    // fused as written: left to the compiler, the fused product depends on the code around it, and a
+    // weight's last bit decides now and then how its BF16 copy is rounded
+    const float mi = __fmaf_rn(1.0f - u.b1, gi, __fmul_rn(u.b1, m[i]));
+    const float vi = __fmaf_rn(__fmul_rn(1.0f - u.b2, gi), gi, __fmul_rn(u.b2, v[i]));
     m[i] = mi;
     v[i] = vi;
     p[i] -= u.lr * (mi / u.c1) / (sqrtf(vi / u.c2) + u.eps);
