@@ -292,10 +292,10 @@ template <int MODE>
 __host__ __device__ constexpr int btap() { return (kC / 8) * chunks<MODE>() * kCore; } // weight bytes per tap
 // instruction descriptor: D F32 (bits 4-5 = 1), A and B format (bits 7-9, 10-12), both
 // K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28
-template <int MODE, int N = kC>
+template <int MODE, int N = kC, int M = kM>
 __host__ __device__ constexpr uint32_t idesc() {
     return (1u << 4) | (Traits<MODE>::kFmt << 7) | (Traits<MODE>::kFmt << 10) | ((uint32_t)(N >> 3) << 17) |
-           ((uint32_t)(kM >> 4) << 24);
+           ((uint32_t)(M >> 4) << 24);
 }
 // the same for a number of columns n known at run time
 template <int MODE>
@@ -1177,58 +1177,63 @@ k_gen_conv_ws(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restr
 // in[p + tap, ci] * dout[p, co], the positions p as the contraction (kind::f16, FP32
 // accumulators in tensor memory). The layer input is BF16 already; the FP32 output gradient
 // is split into BF16 hi + lo (lo = the remainder rounded again, 16 significant bits in all)
-// and both halves are multiplied, which is more accurate than TF32.
-// A K-block is W consecutive positions of one image row, a whole row up to L = 128. Both operands
-// are MN-major: a slot holds 8 channels (16 bytes) per position, the positions 16 bytes apart, so
-// the window of a tap shifted by dx positions is the same slot started dx * 16 bytes later. A is
-// the output gradient: rows 0-47 hi, rows 64-111 lo (slots 6, 7, 14 and 15 stay zero), so one MMA
-// multiplies both halves. B is the input: the 6 slots of each of the rows y-1, y, y+1, neighbours
-// in a ring of rows, are N = 144 columns (row, input channel); two MMAs where they wrap around
-// the ring's end. Three accumulators, one per dx; the epilogue adds the lo lanes to the hi lanes.
-// A CTA's K-blocks are consecutive in y, so each block brings one new row of input.
-// Roles, over a ring of kRows input rows (copied / ready / free per row) and of kStages gradient
-// operands (gfull / gfree):
-//   warp 0:      producer: after `free`, the byte count of `copied` and 6 bulk copies;
-//   warp 2:      after `copied`, where a row is its own neighbour (W = L) the slots of columns -1
-//                and W (else the producer copies them), then `ready`;
-//   warps 4-15:  read the raw gradient, a row ahead, from global memory into registers, write its
-//                hi / lo operands and arrive on gfull; they also add it up: the bias gradient, in
-//                FP32, without another pass over it;
-//   warp 1:      after `ready` and gfull, 3 x W/16 MMAs, committed to gfree and to `free` of the row
-//                that is not used again. The warp stays together, lane 0 issues.
-// Every wait is bounded and also ends when another role gave up (a shared abort word); the last
-// copies land and a last commit is waited for before the tensor memory is freed. Each CTA's partial
-// sums (read back with tcgen05.ld) go to `part` and k_gen_sum_parts adds the partials in a fixed
-// order.
-// What bounds it: the issue of the bulk copies, about 100 cycles each whatever their size, and the
-// reads of the operands from shared memory (68 x 128 bytes per MMA of 72 cycles). In blocks of 64
-// positions with three rows of input and the raw gradient copied for each (30 copies) it took 63 us
-// for 16 x 128^2 (75 MB: 11 us at the copy rate), of which the copies' issue 2 us per block; now
-// 29 us, with the bias gradient (13 us per layer as launches of its own): 21 us of K-blocks, 5 us
-// to write the partials.
+// and both halves are multiplied into the same accumulator, which is more accurate than TF32.
+// The order of the additions is part of the result (an Adam step divides the gradient by its own
+// size and the weights are rounded to BF16, so that a last bit here is 1e-4 of the gradients a few
+// steps on) and does not depend on how the work is laid out: a K-block is W = min(L, 64)
+// consecutive positions of one image row, partial p takes the blocks p, p + nparts, ..., each in
+// steps of 16 positions, hi before lo; k_gen_sum_parts adds the partials from the first to the last.
+// Both operands are MN-major: a slot holds 8 channels (16 bytes) per position, the positions 16
+// bytes apart, so the window of a tap shifted by dx positions is the same slot started dx * 16
+// bytes later. A is the output gradient, hi or lo, 48 of M = 64 rows (the others read what follows
+// in the stage and are not looked at). B is the input: 6 slots of each of the rows y-1, y, y+1 are
+// N = 144 columns (row, input channel). Three accumulators, one per dx, by one CTA per partial or,
+// where there are few partials, by three.
+// Roles, over a ring of kStages stages (ready / gfull / free per stage):
+//   warps 1-3:   after `free`, copy the input rows with their periodic neighbours (cp.async, two
+//                blocks in flight), then `ready`;
+//   warps 4-15:  read the raw gradient, a block ahead, from global memory into registers, write its
+//                hi / lo operands and arrive on gfull;
+//   warp 0:      after `ready` and gfull, 2 W/16 MMAs per dx, committed to `free`. The warp stays
+//                together, one lane issues;
+//   warps 16-19: the bias gradient's first stage (bias_block), beside the MMAs; CTAs past the last
+//                partial do nothing else.
+// Every wait is bounded and also ends when another role gave up (a shared abort word); a last
+// commit is waited for before the tensor memory is read or freed.
+// What bounds it: reads from L2 (16 x 128^2: 78 MB of input, every row for three blocks, and the
+// gradient's 50 MB twice; without the input's copies 34 us, without the bias 37) beside the MMAs'
+// operand reads (208 x 32 bytes each, 24 per block). 16 x 128^2: 39 us with the bias gradient; with
+// 30 bulk copies per block and the bias in launches of its own it was 62 + 31 us. Whole rows in
+// order with hi and lo in separate accumulators took 28.5 us, but that is another sum.
 // ------------------------------------------------------------------------------------------
 namespace wg {
-constexpr int kWMax = 128;                                // positions per K-block at most
-constexpr int kSlotA = (kWMax + 2) * 16;                  // bytes per input slot (with the halo)
-constexpr int kSlot = kWMax * 16;                         // bytes per gradient slot
-constexpr int kRowB = tc::kC / 8 * kSlotA;                // 12480: 6 slots of an input row
-constexpr int kRows = 9;                                  // ring of input rows
-constexpr int kBytesA = (kRows * kRowB + 127) / 128 * 128;
-constexpr int kStage = 16 * kSlot;                        // 32768: BF16 gradient, hi and lo, 8 slots each
-constexpr int kStages = 3;
-constexpr int kThreads = 512;
+constexpr int kStages = 6;
+constexpr int kThreads = 640;
+constexpr int kLoad = 96;                                 // loading threads, warps 1-3
 constexpr int kConv = 384;                                // converting threads, warps 4-15
+constexpr int kBias = 128;                                // bias threads, warps 16-19
 constexpr int kN = 3 * tc::kC;                            // 144 columns: (row, input channel)
+constexpr int kM = 64;                                    // rows of A: 48 output channels, the rest not looked at
 constexpr int kAccCols = 160;                             // step of the accumulators
 constexpr int kCols = 512;                                // columns allocated (a power of two)
-constexpr size_t kSmem = (size_t)kBytesA + kStages * kStage + 1024;
-constexpr int kPart = 9 * tc::kC * tc::kC + tc::kC;       // floats per partial: weights, then biases
-static_assert((3 * kN * tc::kC + 8 * kConv) * 4 <= kBytesA + kStages * kStage, "epilogue scratch in the rings");
-// BF16 A and B, both MN-major (instruction-descriptor bits 15 and 16), N columns, M = 128
-__device__ __forceinline__ uint32_t idesc(int n) { return tc::idesc_n<0>((uint32_t)n) | (1u << 15) | (1u << 16); }
+constexpr int kPart = 9 * tc::kC * tc::kC;                // floats per partial
+__host__ __device__ constexpr int slot(int W) { return W * 16; }          // bytes per gradient slot
+__host__ __device__ constexpr int slot_in(int W) { return (W + 2) * 16; }   // bytes per input slot
+// a stage: hi and lo (6 slots each), then the input rows (18 slots)
+__host__ __device__ constexpr int stage(int W) { return (12 * slot(W) + 18 * slot_in(W) + 127) / 128 * 128; }
+constexpr size_t smem(int W) { return (size_t)kStages * stage(W) + 1024; }
+static_assert(14 * slot(64) <= stage(64) && 14 * slot(16) <= stage(16), "A of lo ends inside the stage");
+// BF16 A and B, both MN-major (instruction-descriptor bits 15 and 16), N = 144, M = 64
+constexpr uint32_t kIdesc = tc::idesc<0, kN, kM>() | (1u << 15) | (1u << 16);
 // K-block length for an L x L image (0: the tensor-core form does not apply)
-__host__ __device__ constexpr int block_len(int L) {
-    return (L % 16 != 0) ? 0 : (L <= 64 || L == kWMax ? L : (L % 64 == 0 ? 64 : 0));
+__host__ __device__ constexpr int block_len(int L) { return L % 16 != 0 ? 0 : (L <= 64 ? L : (L % 64 == 0 ? 64 : 0)); }
+__device__ __forceinline__ void mma(uint32_t tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}" ::"r"(tmem),
+        "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(kIdesc), "r"(acc)
+        : "memory");
 }
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -1236,35 +1241,74 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 }
 }  // namespace wg
 
+// Bias gradient, first stage: block b sums pixels [b * chunk, (b + 1) * chunk) of the planar FP32
+// gradient (G groups of 4 channels) into part[b][4 G], by `lanes` = 256 / G lanes a group: lane l
+// takes every lanes-th pixel from l on, then the lanes are added in order. bias_lane is one lane's
+// sum, bias_channel one channel's over the lanes.
+struct BiasArgs {
+    float* part;
+    int npix, chunk, nblk;
+};
+__device__ __forceinline__ float4 bias_lane(const float* dout, int G, int LL, int lanes, int g, int p, int p1) {
+    constexpr int kBatch = 8;   // loads in flight
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int img = p / LL;
+    int pp = p - img * LL;
+    const float4* src = reinterpret_cast<const float4*>(dout) + ((size_t)img * G + g) * LL + pp;
+    for (; p < p1; p += kBatch * lanes) {
+        float4 v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            v[k] = p + k * lanes < p1 ? ld_seq(src) : make_float4(0.f, 0.f, 0.f, 0.f);   // s + 0 is s
+            src += lanes;
+            pp += lanes;
+            if (pp >= LL) {   // the next image (an image holds at least as many pixels as there are lanes)
+                pp -= LL;
+                src += (size_t)(G - 1) * LL;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            s.x += v[k].x;
+            s.y += v[k].y;
+            s.z += v[k].z;
+            s.w += v[k].w;
+        }
+    }
+    return s;
+}
+__device__ __forceinline__ float bias_channel(const float4* red, int lanes, int c) {
+    const float* r = reinterpret_cast<const float*>(red + (c >> 2) * lanes) + (c & 3);
+    float v = 0.0f;
+    for (int k = 0; k < lanes; ++k) v += r[4 * k];
+    return v;
+}
+
 template <int KS>   // MMA K-steps (16 positions) per K-block: W = 16 KS
 __global__ void __launch_bounds__(wg::kThreads, 1)
-k_gen_wgrad_tc(const __nv_bfloat16* in, const float* dout, float* part,
-               int L, int nkb, int* flag) {
+k_gen_wgrad_tc(const __nv_bfloat16* in, const float* dout, float* part, int L, int nkb, int nparts, int split, BiasArgs bias,
+               int* flag) {
     seq_begin();
     using namespace wg;
-    constexpr int kC = tc::kC, W = 16 * KS;
-    constexpr int kJobs = kC / 8 * W;                       // (channel group, position) of a K-block
-    constexpr int kPer = (kJobs + kConv - 1) / kConv;       // of these per converting thread, kStep apart
-    constexpr int kStep = kJobs / kPer;                     // = converting threads in use
-    static_assert(kJobs % kPer == 0 && kStep % 32 == 0 && W % (W / kPer) == 0, "whole warps");
+    constexpr int kC = tc::kC, W = 16 * KS, kSlot = slot(W), kSlotIn = slot_in(W), kStage = stage(W);
+    constexpr int kIn = 12 * kSlot;                         // the input rows' place in a stage
+    constexpr int kJobs = kC / 8 * W;                       // (channel group, position) of a K-block, one per thread
+    static_assert(kJobs <= kConv && kJobs % 32 == 0, "whole converting warps");
     extern __shared__ uint8_t wsm_raw[];
-    __shared__ __align__(8) unsigned long long copied[kRows], ready[kRows], rfree[kRows], gfull[kStages], gfree[kStages], done;
+    __shared__ __align__(8) unsigned long long ready[kStages], gfull[kStages], sfree[kStages], done;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_word;
+    __shared__ float4 red[252];                             // 12 groups x 21 lanes
     uint8_t* smem = (uint8_t*)(((uintptr_t)wsm_raw + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const size_t LL = (size_t)L * L;
-    const int bpr = L / W;                                  // strips of W columns
-    const uint32_t sbase = gen_smem_u32(smem), gbase = sbase + (uint32_t)kBytesA;
-    // K-blocks [b0, b1) of the batch, ordered by image, strip, row: segments of one strip each
-    const int b0 = (int)((long long)nkb * blockIdx.x / gridDim.x), b1 = (int)((long long)nkb * (blockIdx.x + 1) / gridDim.x);
+    const int bpr = L / W;                                  // K-blocks per image row
+    const uint32_t sbase = gen_smem_u32(smem);
+    // this CTA's partial and accumulators dx0 .. dx0 + ndx - 1; its K-blocks first, first + nparts, ...
+    const int first = blockIdx.x / split, ndx = 3 / split, dx0 = (blockIdx.x - first * split) * ndx;
+    const bool mine = first < nparts;
+    const int n = mine ? (nkb - first + nparts - 1) / nparts : 0;
 
-    // the zero slots 6, 7, 14 and 15 of the gradient, in every stage (never written again)
-    for (int i = tid; i < kStages * 4 * (kSlot / 16); i += kThreads) {
-        const int c = i % (kSlot / 16), s = i / (kSlot / 16);
-        const int st = s / 4, slot = (s % 4) / 2 * 8 + 6 + s % 2;
-        *reinterpret_cast<uint4*>(smem + kBytesA + st * kStage + slot * kSlot + c * 16) = make_uint4(0, 0, 0, 0);
-    }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gen_smem_u32(&tmem_slot)),
                      "r"(kCols)
@@ -1272,14 +1316,10 @@ k_gen_wgrad_tc(const __nv_bfloat16* in, const float* dout, float* part,
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (warp == 1) {
-        if (lane < kRows) {
-            gen_mbar_init(&copied[lane], 1);
-            gen_mbar_init(&ready[lane], 1);
-            gen_mbar_init(&rfree[lane], 1);
-        }
-        if (lane >= 16 && lane < 16 + kStages) {
-            gen_mbar_init(&gfull[lane - 16], kStep / 32);
-            gen_mbar_init(&gfree[lane - 16], 1);
+        if (lane < kStages) {
+            gen_mbar_init(&ready[lane], kLoad / 32);
+            gen_mbar_init(&gfull[lane], kJobs / 32);
+            gen_mbar_init(&sfree[lane], 1);
         }
         if (lane == 31) {
             gen_mbar_init(&done, 1);
@@ -1287,110 +1327,49 @@ k_gen_wgrad_tc(const __nv_bfloat16* in, const float* dout, float* part,
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // the zeroed slots are read by the tensor cores (async proxy)
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    // the accumulators start at zero: four of the converting warps clear them before the MMA warp
-    // begins; the others go on
-    if (warp == 1 || warp >= 12) {
-        if (warp >= 12) {
-            for (int c = 0; c < 3 * kAccCols; c += 16) tmem_zero16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        gen_bar_sync(5 * 32);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    }
-
-    const int ct = tid - (kThreads - kConv);                // converting thread
-    float bsum[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    auto place = [&](int j, int& img, int& y, int& x0) {   // of this CTA's K-block j
+        const int kb = first + j * nparts, row = kb / bpr;
+        img = row / L;
+        y = row - img * L;
+        x0 = (kb - row * bpr) * W;
+    };
+    auto fresh = [&](int j) {   // stage of K-block j: its previous MMAs have completed
+        return j < kStages || gen_wait(gen_smem_u32(&sfree[j % kStages]), (uint32_t)(j / kStages - 1) & 1u, &abort_word, flag, 4);
+    };
     bool ok = true;
     if (warp == 0) {
-        int q = 0;   // rows copied
-        for (int b = b0; b < b1 && ok;) {
-            const int st = b / L, y0 = b - st * L, len = min(b1 - b, L - y0), img = st / bpr, x0 = (st - img * bpr) * W;
-            // columns x0-1 .. x0+W: what lies inside the row, then a neighbour across the periodic edge
-            const bool left = x0 == 0, right = x0 + W == L, own = bpr == 1;
-            const int xa = left ? 0 : x0 - 1, xb = right ? L : x0 + W + 1;
-            const uint32_t tx = (uint32_t)(kC / 8) * 16u * (uint32_t)(xb - xa + (own ? 0 : (int)left + (int)right));
-            for (int i = 0; i < len + 2; ++i, ++q) {
-                const int s = q % kRows;
-                if (q >= kRows) {
-                    ok = gen_wait(gen_smem_u32(&rfree[s]), (uint32_t)(q / kRows - 1) & 1u, &abort_word, flag, 4);
-                    if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                }
-                int yy = y0 + i - 1;
-                yy += yy < 0 ? L : (yy >= L ? -L : 0);
-                const uint32_t bar = gen_smem_u32(&copied[s]);
-                if (lane == 0)
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tx) : "memory");
-                __syncwarp();
-                if (lane < kC / 8) {
-                    const __nv_bfloat16* row = in + (((size_t)img * (kC / 8) + lane) * LL + (size_t)yy * L) * 8;
-                    const uint32_t dst = sbase + (uint32_t)(s * kRowB + lane * kSlotA);
-                    gen_bulk(dst + (left ? 16u : 0u), row + (size_t)xa * 8, (uint32_t)(xb - xa) * 16, bar);
-                    if (!own && left) gen_bulk(dst, row + (size_t)(L - 1) * 8, 16u, bar);
-                    if (!own && right) gen_bulk(dst + (W + 1) * 16u, row, 16u, bar);
-                }
-                __syncwarp();
-            }
-            b += len;
-        }
-        // the last copy into every row buffer lands before the CTA's shared memory can be released
-        if (lane == 0)
-            for (int j = max(0, q - kRows); j < q; ++j)
-                for (unsigned it = 0; it < (tc::kWaitLimit >> 4); ++it)
-                    if (gen_mbar_try_wait(gen_smem_u32(&copied[j % kRows]), (uint32_t)(j / kRows) & 1u)) break;
-    } else if (warp == 1) {
         const bool lead = elect_one();
-        const uint64_t a00 = umma_desc(gbase, 128, kSlot), b00 = umma_desc(sbase, 128, kSlotA);
+        // MN-major, no swizzle: LBO = 128 (8-position K groups), SBO = one slot (8-channel MN
+        // groups); the start address field (bits 0-13, address >> 4) is offset per MMA
+        const uint64_t a00 = umma_desc(sbase, 128, kSlot), b00 = umma_desc(sbase + (uint32_t)kIn, 128, kSlotIn);
         const uint32_t alo = (uint32_t)a00, ahi = (uint32_t)(a00 >> 32), blo = (uint32_t)b00, bhi = (uint32_t)(b00 >> 32);
-        int q0 = 0, k = 0;   // first row of the segment in the order of copies; K-blocks issued
-        for (int b = b0; b < b1 && ok;) {
-            const int len = min(b1 - b, L - b % L);
-            for (int j = 0; j < len; ++j, ++k) {
-                const int g = k % kStages, s = (q0 + j) % kRows;
-                for (int a = q0; j == 0 && a < q0 + 2 && ok; ++a)
-                    ok = gen_wait(gen_smem_u32(&ready[a % kRows]), (uint32_t)(a / kRows) & 1u, &abort_word, flag, 4);
-                const int a = q0 + j + 2;   // the newest row, and the gradient
-                ok = ok && gen_wait2(gen_smem_u32(&ready[a % kRows]), (uint32_t)(a / kRows) & 1u, gen_smem_u32(&gfull[g]),
-                                     (uint32_t)(k / kStages) & 1u, &abort_word, flag, 4);
-                if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // MN-major, no swizzle: LBO = 128 (8-position K groups), SBO = one slot (8-channel
-                // MN groups); the start address field (bits 0-13, address >> 4) is offset per MMA
-                const uint32_t as = alo + ((uint32_t)(g * kStage) >> 4), bs = blo + ((uint32_t)(s * kRowB) >> 4);
-                const int n1 = min(3, kRows - s) * kC, n2 = kN - n1;   // columns up to the ring's end, and after it
-                const uint32_t i1 = idesc(n1), i2 = idesc(n2), d2 = tmem + (uint32_t)n1;
-                if (lead) {
+        for (int k = 0; k < n; ++k) {
+            const int s = k % kStages;
+            const uint32_t par = (uint32_t)(k / kStages) & 1u;
+            ok = gen_wait2(gen_smem_u32(&ready[s]), par, gen_smem_u32(&gfull[s]), par, &abort_word, flag, 4);
+            if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t at = (uint32_t)(s * kStage) >> 4;
+            if (lead) {
+                for (int d = 0; d < ndx; ++d) {
+                    const uint32_t acc = tmem + (uint32_t)(d * kAccCols);
 #pragma unroll
-                    for (int m = 0; m < 3 * KS; ++m)
-                        tc_mma_n<0>(tmem + (uint32_t)(m / KS * kAccCols), as + (uint32_t)((m % KS * 256) >> 4), ahi,
-                                    bs + (uint32_t)(m / KS + 16 * (m % KS)), bhi, i1);
-                    if (n2) {   // the rest, at the ring's start
-#pragma unroll
-                        for (int m = 0; m < 3 * KS; ++m)
-                            tc_mma_n<0>(d2 + (uint32_t)(m / KS * kAccCols), as + (uint32_t)((m % KS * 256) >> 4), ahi,
-                                        blo + (uint32_t)(m / KS + 16 * (m % KS)), bhi, i2);
-                    }
-                    gen_commit(gen_smem_u32(&gfree[g]));
-                    gen_commit(gen_smem_u32(&rfree[s]));
-                    if (j == len - 1) {   // the segment's last two rows
-                        gen_commit(gen_smem_u32(&rfree[(q0 + len) % kRows]));
-                        gen_commit(gen_smem_u32(&rfree[(q0 + len + 1) % kRows]));
+                    for (int ks = 0; ks < KS; ++ks) {
+                        const uint32_t a = alo + at + (uint32_t)(16 * ks), b = blo + at + (uint32_t)(dx0 + d + 16 * ks);
+                        mma(acc, a, ahi, b, bhi, (k | ks) ? 1u : 0u);
+                        mma(acc, a + (uint32_t)((6 * kSlot) >> 4), ahi, b, bhi, 1u);
                     }
                 }
-                __syncwarp();
+                gen_commit(gen_smem_u32(&sfree[s]));
             }
-            q0 += len + 2;
-            b += len;
+            __syncwarp();
         }
         // every MMA has completed before the accumulators are read or freed
-        if (lead) {
+        if (lead && n > 0) {
             gen_commit(gen_smem_u32(&done));
             bool drained = false;
             for (unsigned it = 0; it < tc::kWaitLimit && !drained; ++it) drained = gen_mbar_try_wait(gen_smem_u32(&done), 0);
@@ -1400,122 +1379,106 @@ k_gen_wgrad_tc(const __nv_bfloat16* in, const float* dout, float* part,
             }
         }
         __syncwarp();
-    } else if (warp == 2) {
-        int n = 0;   // rows of this CTA, with the two beside each segment
-        for (int b = b0; b < b1; n += 2) {
-            const int len = min(b1 - b, L - b % L);
-            n += len;
-            b += len;
-        }
-        for (int q = 0; q < n; ++q) {
-            const int s = q % kRows;
-            ok = gen_wait(gen_smem_u32(&copied[s]), (uint32_t)(q / kRows) & 1u, &abort_word, flag, 4);
-            if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
-            if (bpr == 1 && lane < 2 * (kC / 8)) {   // slot 0 <- column W-1 (slot W), slot W+1 <- column 0
-                uint8_t* blk = smem + s * kRowB + (lane >> 1) * kSlotA;
-                const int to = (lane & 1) ? W + 1 : 0, from = (lane & 1) ? 1 : W;
-                *(uint4*)(blk + to * 16) = *(const uint4*)(blk + from * 16);
-            }
+    } else if (warp <= kLoad / 32) {
+        const int lt = tid - 32;
+        auto landed = [&](int j) {   // K-block j's copies of this warp are in shared memory
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&ready[s])) : "memory");
-        }
-    } else if (ct >= 0 && ct < kStep) {
-        // converters: channel group h at the positions c + i W / kPer of every K-block
-        constexpr int kWs = W / kPer;
-        const int h = ct / kWs, c = ct - h * kWs, n = b1 - b0;
-        float4 nx[kPer][2];   // the next K-block's gradient
-        auto fetch = [&](int b) {
-            const int st = b / L, y = b - st * L, img = st / bpr, x0 = (st - img * bpr) * W;
-            const float4* p = reinterpret_cast<const float4*>(dout) + ((size_t)img * (kC / 4) + 2 * h) * LL + (size_t)y * L + x0 + c;
-#pragma unroll
-            for (int i = 0; i < kPer; ++i) {
-                nx[i][0] = ld_seq(p + i * kWs);
-                nx[i][1] = ld_seq(p + LL + i * kWs);
-            }
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&ready[j % kStages])) : "memory");
         };
-        if (n > 0) fetch(b0);
-        for (int k = 0; k < n; ++k) {
-            const int g = k % kStages;
-            float f[kPer][8];
-#pragma unroll
-            for (int i = 0; i < kPer; ++i) {
-                const float4 a = nx[i][0], b = nx[i][1];
-                f[i][0] = a.x, f[i][1] = a.y, f[i][2] = a.z, f[i][3] = a.w;
-                f[i][4] = b.x, f[i][5] = b.y, f[i][6] = b.z, f[i][7] = b.w;
+        constexpr int kDepth = 2;   // blocks in flight
+        int j = 0;
+        for (; j < n; ++j) {
+            ok = fresh(j);
+            if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
+            int img, y, x0;
+            place(j, img, y, x0);
+            const uint4* src = reinterpret_cast<const uint4*>(in) + (size_t)img * (kC / 8) * LL;
+            const uint32_t dst = sbase + (uint32_t)((j % kStages) * kStage + kIn);
+            for (int i = lt; i < 18 * (W + 2); i += kLoad) {   // slot (row, channel group), column x0 - 1 + c
+                const int sl = i / (W + 2), c = i - sl * (W + 2), R = sl / 6, h = sl - 6 * R;
+                int yy = y + R - 1, x = x0 - 1 + c;
+                yy += yy < 0 ? L : (yy >= L ? -L : 0);
+                x += x < 0 ? L : (x >= L ? -L : 0);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(i * 16)),
+                             "l"(src + (size_t)h * LL + (size_t)yy * L + x)
+                             : "memory");
             }
-            if (k + 1 < n) fetch(b0 + k + 1);
-            if (k >= kStages) {
-                ok = gen_wait(gen_smem_u32(&gfree[g]), (uint32_t)(k / kStages - 1) & 1u, &abort_word, flag, 4);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (j >= kDepth) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kDepth) : "memory");
+                landed(j - kDepth);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (ok)
+            for (int q = max(0, n - kDepth); q < n; ++q) landed(q);
+    } else if (warp < 16) {
+        const int ct = tid - 128;
+        if (ct < kJobs) {   // channel group h at position c of every K-block
+            const int h = ct / W, c = ct - h * W;
+            float4 a, b;   // the next K-block's gradient
+            auto fetch = [&](int j) {
+                int img, y, x0;
+                place(j, img, y, x0);
+                const float4* p = reinterpret_cast<const float4*>(dout) + ((size_t)img * (kC / 4) + 2 * h) * LL + (size_t)y * L + x0 + c;
+                a = ld_seq(p);
+                b = ld_seq(p + LL);
+            };
+            if (n > 0) fetch(0);
+            for (int j = 0; j < n; ++j) {
+                const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                if (j + 1 < n) fetch(j + 1);
+                ok = fresh(j);
                 if (!(ok = __all_sync(0xFFFFFFFFu, ok))) break;
-            }
-            uint8_t* sG = smem + kBytesA + g * kStage;
-#pragma unroll
-            for (int i = 0; i < kPer; ++i) {
+                uint8_t* sG = smem + (j % kStages) * kStage + h * kSlot + c * 16;
                 uint32_t hi[4], lo[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    hi[e] = pack_bf16(f[i][2 * e], f[i][2 * e + 1]);
-                    lo[e] = pack_bf16(f[i][2 * e] - __uint_as_float(hi[e] << 16),
-                                      f[i][2 * e + 1] - __uint_as_float(hi[e] & 0xFFFF0000u));
+                    hi[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
+                    lo[e] = pack_bf16(f[2 * e] - __uint_as_float(hi[e] << 16), f[2 * e + 1] - __uint_as_float(hi[e] & 0xFFFF0000u));
                 }
-                *reinterpret_cast<uint4*>(sG + h * kSlot + (c + i * kWs) * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(sG + (8 + h) * kSlot + (c + i * kWs) * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                *reinterpret_cast<uint4*>(sG) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(sG + 6 * kSlot) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&gfull[j % kStages])) : "memory");
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gen_smem_u32(&gfull[g])) : "memory");
-#pragma unroll
-            for (int i = 0; i < kPer; ++i)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) bsum[e] += f[i][e];
+        }
+    } else if (bias.part) {
+        const int bt = tid - (kThreads - kBias);
+        for (int b = blockIdx.x; b < bias.nblk; b += gridDim.x) {
+            const int p0 = b * bias.chunk, p1 = min(p0 + bias.chunk, bias.npix);
+            for (int t = bt; t < 252; t += kBias) {
+                const int g = t / 21, pl = t - 21 * g;
+                red[t] = bias_lane(dout, kC / 4, (int)LL, 21, g, p0 + pl, p1);
+            }
+            gen_bar_sync(kBias);
+            if (bt < kC) bias.part[(size_t)b * kC + bt] = bias_channel(red, 21, bt);
+            gen_bar_sync(kBias);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (!__syncthreads_or(!ok)) {
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) atomicExch(flag, 4);
+    } else if (mine) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // epilogue: a warp reads its own lane quarter q = warp % 4 in chunks of 16 columns; the lo
-        // quarters (2, 3) leave theirs in the ring's memory, the hi quarters add them and store
-        const int q = warp & 3, co = (q & 1) * 32 + lane;
-        float* slo = reinterpret_cast<float*>(smem);                  // [432 columns][48]
-        float* sbs = slo + 3 * kN * kC;                               // [8][converting thread]
-        float* dst = part + (size_t)blockIdx.x * kPart;
-        if (ct >= 0 && ct < kStep)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sbs[e * kStep + ct] = bsum[e];
-        float v[16];
-        const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
-        if (q >= 2)
-            for (int c = warp >> 2; c < 27; c += 4) {
-                tmem_ld16(tq + (uint32_t)(c / 9 * kAccCols + c % 9 * 16), v);
+        // a warp reads its own lane quarter q = warp % 4 in chunks of 16 columns: the rows 16 q .. 16 q
+        // + 15 of M = 64 are the quarter's first 16 lanes
+        const int q = warp & 3, co = lane < 16 ? q * 16 + lane : kC;
+        float* dst = part + (size_t)first * kPart;
+        if (q < 3)
+            for (int c = warp >> 2; c < 9 * ndx; c += kThreads / 128) {
+                const int d = c / 9, R = c % 9 / 3, ci0 = c % 3 * 16;
+                float v[16];
+                tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(d * kAccCols + c % 9 * 16), v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (co < kC)
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) slo[(c * 16 + e) * kC + co] = v[e];
+                    for (int e = 0; e < 16; ++e) dst[((R * 3 + dx0 + d) * kC + ci0 + e) * kC + co] = v[e];
             }
-        __syncthreads();
-        if (q < 2) {
-            for (int c = warp >> 2; c < 27; c += 4) {
-                const int dxi = c / 9, R = c % 9 / 3, ci0 = c % 3 * 16;
-                tmem_ld16(tq + (uint32_t)(dxi * kAccCols + c % 9 * 16), v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (co < kC)
-#pragma unroll
-                    for (int e = 0; e < 16; ++e)
-                        dst[((R * 3 + dxi) * kC + ci0 + e) * kC + co] = v[e] + slo[(c * 16 + e) * kC + co];
-            }
-        } else {   // biases: 8 warps x 6 channels, the positions in a fixed order
-            const int i = (warp >> 2) * 2 + (q & 1);
-            for (int ch = i * (kC / 8); ch < (i + 1) * (kC / 8); ++ch) {
-                float s = 0.0f;
-                for (int c = lane; c < W / kPer; c += 32) s += sbs[(ch & 7) * kStep + (ch >> 3) * (W / kPer) + c];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-                if (lane == 0) dst[9 * kC * kC + ch] = s;
-            }
-        }
-    } else if (tid == 0) {
-        atomicExch(flag, 4);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -1608,136 +1571,134 @@ k_gen_wgrad(const __nv_bfloat16* in, const float* dout, float* part,
         }
 }
 
-// The same for the two edge layers (8 -> 48 and 48 -> 4), whose few channels left most threads of
-// that layout without work and one scalar load per multiply-add: kGroups groups of 54 threads
-// take every kGroups-th row of the tile, a thread one tap x 8 input channels x TC output channels
-// with 16-byte loads and packed multiply-adds. Rows of a pixel are padded by 4 floats so that the
-// staging's stores and the loads spread over the banks. 16 x 128^2: 136 -> 62 us and 54 -> 46 us.
-constexpr int kEdgePer = 4;   // images of a CTA (2: 51 and 63 us instead of 48 and 61)
-template <int CIN, int COUT>
+// The same for the two edge layers (8 -> 48 and 48 -> 4), whose few channels leave most threads of
+// that layout without work and one scalar load per multiply-add: 108 threads take one tap x TI
+// input x TO output channels each, with 16-byte loads and packed multiply-adds (two input channels
+// to an instruction), while the other 128 bring the next half tile into the second buffer. A sum
+// runs over the CTA's pixels in their order, as in k_gen_wgrad: the order is part of the result.
+// Rows of a pixel are padded by 4 floats so that the staging's stores spread over the banks.
+// What bounds it: 256 CTAs on 152 SMs leave two of them on most SMs, seven computing warps in all,
+// whose multiply-adds take 28 us. 16 x 128^2: 51 us (8 -> 48) and 36 us (48 -> 4) against 136 and
+// 54 in k_gen_wgrad's form; with 8 x 8 outputs to a thread 106 us.
+template <int CIN, int COUT, int TI, int TO>
 struct EdgeGrad {
-    static constexpr int TC = COUT < 8 ? COUT : 8;                 // output channels of a thread
-    static constexpr int CG = CIN / 8, OG = COUT / TC;             // channel groups
-    static constexpr int kThr = 9 * CG * OG, kGroups = 4, kThreads = kThr * kGroups;
+    static constexpr int CG = CIN / TI, OG = COUT / TO, kThr = 9 * CG * OG;
+    static constexpr int kCompute = 128, kThreads = 256, kHalf = kTile / 2;
     static constexpr int SI = CIN + (CIN > 8 ? 4 : 0), SO = COUT + (COUT > 8 ? 4 : 0);   // floats per pixel
-    // place of channel c of a pixel: from the 32nd on four floats later, so that the six groups of eight
-    // channels that a quarter warp reads lie in different banks (48 -> 4: 48.4 us with two in one, now 45.7)
-    __host__ __device__ static constexpr int at(int c) { return c + (c >= 32 ? 4 : 0); }
-    static constexpr int kTin = (kTile + 2) * (kTile + 2) * SI, kTdo = kTile * kTile * SO;
-    static constexpr int kRed = (kGroups - 1) * kThr * (8 * TC + 1);
-    static constexpr size_t smem = (kTin + kTdo > kRed ? kTin + kTdo : kRed) * sizeof(float);
+    static constexpr int kTin = (kHalf + 2) * (kTile + 2) * SI, kTdo = kHalf * kTile * SO;
+    static constexpr size_t smem = (size_t)2 * (kTin + kTdo) * sizeof(float);
+    static_assert(CIN % 8 == 0 && COUT % 4 == 0 && TI % 4 == 0 && TO % 4 == 0 && kThr <= kCompute, "16-byte accesses");
 };
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(EdgeGrad<CIN, COUT>::kThreads, 2)
-k_gen_wgrad_edge(const __nv_bfloat16* in, const float* dout, float* part,
-                 int L, int images_per_cta, int nimg) {
+template <int CIN, int COUT, int TI, int TO>
+__global__ void __launch_bounds__(256, 2)
+k_gen_wgrad_edge(const __nv_bfloat16* in, const float* dout, float* part, int L, int images_per_cta, int nimg) {
     seq_begin();
-    using E = EdgeGrad<CIN, COUT>;
-    static_assert(CIN % 8 == 0 && COUT % 4 == 0, "16-byte staging");
+    using E = EdgeGrad<CIN, COUT, TI, TO>;
     extern __shared__ __align__(16) float gsm[];
-    constexpr int T2 = kTile + 2, TC = E::TC;
-    float* tin = gsm;                // [T2*T2][SI]
-    float* tdo = gsm + E::kTin;      // [kTile*kTile][SO]
+    constexpr int T2 = kTile + 2, kRowsIn = E::kHalf + 2;
     const int tiles_x = L / kTile;
     const int tile = blockIdx.x % (tiles_x * tiles_x);
-    const int igrp = blockIdx.x / (tiles_x * tiles_x);
+    const int img0 = blockIdx.x / (tiles_x * tiles_x) * images_per_cta;
     const int ty0 = (tile / tiles_x) * kTile, tx0 = (tile % tiles_x) * kTile;
-    const int t = threadIdx.x, grp = t / E::kThr, tg = t - grp * E::kThr;
-    const int tap = tg / (E::CG * E::OG), rr = tg % (E::CG * E::OG), cg = rr / E::OG, og = rr % E::OG;
-    const int dy = tap / 3, dx = tap % 3;
-    f2 acc[8][TC / 2];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < TC / 2; ++j) acc[i][j] = f2{0ull};
+    const int steps = 2 * min(images_per_cta, nimg - img0);   // half tiles
     const size_t LL = (size_t)L * L;
-    for (int im = 0; im < images_per_cta; ++im) {
-        const int img = igrp * images_per_cta + im;
-        if (img >= nimg) break;
-        const size_t ibase = (size_t)img * LL;
+    // half tile `s` into its buffer, by threads t0, t0 + 1, ... (nthr of them)
+    auto stage = [&](int s, int t0, int nthr) {
+        const size_t ibase = (size_t)(img0 + (s >> 1)) * LL;
+        const int y0 = ty0 + (s & 1) * E::kHalf;
+        float* const tin = gsm + (s & 1) * (E::kTin + E::kTdo);   // [kRowsIn * T2][SI], then [kHalf * kTile][SO]
+        float* const tdo = tin + E::kTin;
         const uint4* isrc = reinterpret_cast<const uint4*>(in + ibase * CIN);
         const float4* gsrc = reinterpret_cast<const float4*>(dout + ibase * COUT);
-        __syncthreads();
-        // chunk planes of this image; pixel index fastest, so consecutive threads read consecutive pixels
+        // chunk planes of the image; pixel index fastest, so consecutive threads read consecutive pixels
+#pragma unroll 6
+        for (int i = t0; i < E::kHalf * kTile * (COUT / 4); i += nthr) {
+            const int c4 = i / (E::kHalf * kTile), pix = i - c4 * E::kHalf * kTile, yy = pix / kTile, xx = pix - yy * kTile;
+            *reinterpret_cast<float4*>(tdo + pix * E::SO + c4 * 4) = ld_seq(gsrc + (size_t)c4 * LL + (size_t)(y0 + yy) * L + tx0 + xx);
+        }
 #pragma unroll 4
-        for (int i = t; i < T2 * T2 * (CIN / 8); i += E::kThreads) {
-            const int c8 = i / (T2 * T2), pix = i - c8 * T2 * T2, yy = pix / T2, xx = pix - yy * T2;
-            int gy = ty0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
+        for (int i = t0; i < kRowsIn * T2 * (CIN / 8); i += nthr) {
+            const int c8 = i / (kRowsIn * T2), pix = i - c8 * kRowsIn * T2, yy = pix / T2, xx = pix - yy * T2;
+            int gy = y0 + yy - 1, gx = tx0 + xx - 1;   // in [-1, L]: one wrap
             gy += (gy < 0) ? L : ((gy >= L) ? -L : 0);
             gx += (gx < 0) ? L : ((gx >= L) ? -L : 0);
             const uint4 q = ld_seq(isrc + (size_t)c8 * LL + (size_t)gy * L + gx);
-            float4* d = reinterpret_cast<float4*>(tin + pix * E::SI + E::at(c8 * 8));   // a BF16 is an FP32's top half
+            float4* d = reinterpret_cast<float4*>(tin + pix * E::SI + c8 * 8);   // a BF16 is an FP32's top half
             d[0] = make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xFFFF0000u),
                                __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xFFFF0000u));
             d[1] = make_float4(__uint_as_float(q.z << 16), __uint_as_float(q.z & 0xFFFF0000u),
                                __uint_as_float(q.w << 16), __uint_as_float(q.w & 0xFFFF0000u));
         }
-#pragma unroll 4
-        for (int i = t; i < kTile * kTile * (COUT / 4); i += E::kThreads) {
-            const int c4 = i / (kTile * kTile), pix = i - c4 * kTile * kTile, yy = pix / kTile, xx = pix - yy * kTile;
-            *reinterpret_cast<float4*>(tdo + pix * E::SO + E::at(c4 * 4)) =
-                ld_seq(gsrc + (size_t)c4 * LL + (size_t)(ty0 + yy) * L + tx0 + xx);
+    };
+    const int t = threadIdx.x;
+    const int tap = t / (E::CG * E::OG), rr = t % (E::CG * E::OG), cg = rr / E::OG, og = rr % E::OG;
+    const int dy = tap / 3, dx = tap % 3;
+    f2 acc[TI / 2][TO];
+#pragma unroll
+    for (int i = 0; i < TI / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < TO; ++j) acc[i][j] = f2{0ull};
+    stage(0, t, E::kThreads);
+    __syncthreads();
+    for (int s = 0; s < steps; ++s) {
+        if (t >= E::kCompute) {
+            if (s + 1 < steps) stage(s + 1, t - E::kCompute, E::kThreads - E::kCompute);
+        } else if (t < E::kThr) {
+            const float* const tin = gsm + (s & 1) * (E::kTin + E::kTdo);
+            const float* const tdo = tin + E::kTin;
+            for (int py = 0; py < E::kHalf; ++py) {
+                const float* xi = tin + ((py + dy) * T2 + dx) * E::SI + cg * TI;
+                const float* go = tdo + py * kTile * E::SO + og * TO;
+#pragma unroll 8
+                for (int px = 0; px < kTile; ++px, xi += E::SI, go += E::SO) {
+                    f2 xv[TI / 2];
+#pragma unroll
+                    for (int i = 0; i < TI / 4; ++i) {
+                        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(xi + 4 * i);
+                        xv[2 * i].v = q.x;
+                        xv[2 * i + 1].v = q.y;
+                    }
+#pragma unroll
+                    for (int j = 0; j < TO / 4; ++j) {
+                        const float4 q = *reinterpret_cast<const float4*>(go + 4 * j);
+                        const f2 gv[4] = {pk(q.x, q.x), pk(q.y, q.y), pk(q.z, q.z), pk(q.w, q.w)};
+#pragma unroll
+                        for (int i = 0; i < TI / 2; ++i)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc[i][4 * j + e] = fma2(xv[i], gv[e], acc[i][4 * j + e]);
+                    }
+                }
+            }
         }
         __syncthreads();
-        for (int py = grp; py < kTile; py += E::kGroups) {
-            const float* xi = tin + ((py + dy) * T2 + dx) * E::SI + E::at(cg * 8);
-            const float* go = tdo + py * kTile * E::SO + E::at(og * TC);
-#pragma unroll 2
-            for (int px = 0; px < kTile; ++px, xi += E::SI, go += E::SO) {
-                const float4 x0 = *reinterpret_cast<const float4*>(xi), x1 = *reinterpret_cast<const float4*>(xi + 4);
-                const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-                f2 gv[TC / 2];
-#pragma unroll
-                for (int j = 0; j < TC / 4; ++j) {
-                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(go + 4 * j);
-                    gv[2 * j].v = q.x;
-                    gv[2 * j + 1].v = q.y;
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int j = 0; j < TC / 2; ++j) acc[i][j] = fma2(pk(xv[i], xv[i]), gv[j], acc[i][j]);
-            }
-        }
     }
-    // the groups' sums in order, through shared memory (the tiles are done with)
-    __syncthreads();
-    if (grp > 0) {
-        float* o = gsm + (size_t)((grp - 1) * E::kThr + tg) * (8 * TC + 1);   // odd stride: no bank conflicts
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < TC / 2; ++j) {
-                o[i * TC + 2 * j] = lo(acc[i][j]);
-                o[i * TC + 2 * j + 1] = hi(acc[i][j]);
-            }
-    }
-    __syncthreads();
-    if (grp > 0) return;
+    if (t >= E::kThr) return;
     float* dst = part + (size_t)blockIdx.x * 9 * CIN * COUT;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < TI; ++i)
 #pragma unroll
-        for (int j = 0; j < TC; ++j) {
-            float v = (j & 1) ? hi(acc[i][j >> 1]) : lo(acc[i][j >> 1]);
-            for (int q = 1; q < E::kGroups; ++q) v += gsm[(size_t)((q - 1) * E::kThr + tg) * (8 * TC + 1) + i * TC + j];
-            dst[(tap * CIN + cg * 8 + i) * COUT + og * TC + j] = v;
+        for (int j = 0; j < TO; j += 4) {
+            float o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = (i & 1) ? hi(acc[i >> 1][j + e]) : lo(acc[i >> 1][j + e]);
+            *reinterpret_cast<float4*>(dst + (tap * CIN + cg * TI + i) * COUT + og * TO + j) = make_float4(o[0], o[1], o[2], o[3]);
         }
 }
 
-// Sums of partials, one job per blockIdx.y: nparts partials of `stride` floats, of which the first nw
-// sum to gw and the rest (up to n) to gb; all multiples of four. A block takes 16 groups of four
-// outputs, 8 threads each the partials t, t + 8, ... of a group, added in a fixed order at the end.
-// One thread per output had too few loads in flight (9.6 us for 152 partials of 20736 weights, this
-// 6.5), and a launch per layer too few blocks: a backward pass's sums are one launch, eight
-// layers of 16 x 128^2 in 23 us instead of 58.
+// Sums of partials, one job per blockIdx.y, a backward pass's in one launch. Weights: a thread per
+// output adds the nparts partials from the first to the last. Biases (wide): a block per output,
+// thread t adds the partials t, t + 128, ..., then a tree. Both orders are part of the result.
+// What bounds it: the loads in flight, one chain of additions per output. The eight layers of 16 x
+// 128^2 (82 MB of partials) take 27.5 us with eight loads in flight per thread; with 4 29.7, with
+// 16 and 32 in predicated batches 51 and 90, two or four outputs per thread 34 and 45.
 struct SumJob {
     const float* part;
-    float *gw, *gb;
-    int nparts, stride, nw, n;
+    float* out;
+    int nparts, n;   // partials of n floats
+    int wide;
 };
-constexpr int kSumJobs = kGenLayers + 2;   // and the first and last layers' bias gradients
+constexpr int kSumJobs = 2 * kGenLayers;
 struct SumArgs {
     SumJob job[kSumJobs];
     int n = 0;         // jobs
@@ -1745,80 +1706,48 @@ struct SumArgs {
 };
 __global__ void __launch_bounds__(128) k_gen_sum_parts(const __grid_constant__ SumArgs a) {
     seq_begin();
-    __shared__ float4 red[8][16];
-    const SumJob& s = a.job[blockIdx.y];
-    if ((int)blockIdx.x * 64 >= s.n) return;
-    const int o = threadIdx.x & 15, t = threadIdx.x >> 4, i = (blockIdx.x * 16 + o) * 4;
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (i < s.n) {
-        const float* p0 = s.part + i;
-        const size_t stride = (size_t)s.stride;
-        const int nparts = s.nparts;
-#pragma unroll 10
-        for (int p = t; p < nparts; p += 8) {
-            const float4 w = ld_seq(reinterpret_cast<const float4*>(p0 + p * stride));
-            v.x += w.x;
-            v.y += w.y;
-            v.z += w.z;
-            v.w += w.w;
-        }
-    }
-    red[t][o] = v;
-    __syncthreads();
-    if (threadIdx.x >= 16 || i >= s.n) return;
+    const SumJob& j = a.job[blockIdx.y];
+    const int t = threadIdx.x, n = j.n, nparts = j.nparts;
+    if (!j.wide) {
+        const int i = blockIdx.x * 128 + t;
+        if (i >= n) return;
+        constexpr int kBatch = 8;
+        const float* p = j.part + i;
+        float s = 0.0f;
+        int k0 = 0;
+        for (; k0 + kBatch <= nparts; k0 += kBatch, p += (size_t)kBatch * n) {
+            float v[kBatch];
 #pragma unroll
-    for (int k = 1; k < 8; ++k) {
-        const float4 w = red[k][o];
-        v.x += w.x;
-        v.y += w.y;
-        v.z += w.z;
-        v.w += w.w;
+            for (int k = 0; k < kBatch; ++k) v[k] = ld_seq(p + (size_t)k * n);
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) s += v[k];
+        }
+        for (; k0 < nparts; ++k0, p += n) s += ld_seq(p);
+        j.out[i] = s;
+        return;
     }
-    *reinterpret_cast<float4*>(i < s.nw ? s.gw + i : s.gb + (i - s.nw)) = v;
+    __shared__ float red[128];
+    if ((int)blockIdx.x >= n) return;
+    float s = 0.0f;
+    for (int k = t; k < nparts; k += 128) s += ld_seq(j.part + (size_t)k * n + blockIdx.x);
+    red[t] = s;
+    __syncthreads();
+    for (int h = 64; h > 0; h >>= 1) {
+        if (t < h) red[t] += red[t + h];
+        __syncthreads();
+    }
+    if (t == 0) j.out[blockIdx.x] = red[0];
 }
 
-// Bias gradient, first stage: a block sums kBgradRun consecutive pixels of one 4-channel plane of
-// one image of the planar FP32 dout (contiguous 16-byte loads, eight in flight per thread) into
-// part[image * segments + segment][co]; lanes and warps are added in a fixed order, the partials
-// by k_gen_sum_parts. 31 -> 10.4 us for 16 x 128^2 x 48 (50 MB): a division per pixel and 21
-// lanes per channel group before.
-constexpr int kBgradRun = 2048;
-__global__ void __launch_bounds__(256)
-k_gen_bgrad_part(const float* dout, int LL, int cout, int nseg, float* part) {
+// First stage of a layer's bias gradient (the hidden layers' on the tensor cores: k_gen_wgrad_tc).
+__global__ void __launch_bounds__(256) k_gen_bgrad_part(const float* dout, int LL, int cout, BiasArgs b) {
     seq_begin();
-    const int seg = blockIdx.x, g = blockIdx.y, img = blockIdx.z, G = cout / 4;
-    const float4* src = reinterpret_cast<const float4*>(dout) + ((size_t)img * G + g) * LL;
-    const int p0 = seg * kBgradRun, p1 = min(p0 + kBgradRun, LL);
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int p = p0 + threadIdx.x; p < p1; p += 256) {
-        const float4 v = ld_seq(src + p);
-        s.x += v.x;
-        s.y += v.y;
-        s.z += v.z;
-        s.w += v.w;
-    }
-    __shared__ float red[8][4];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s.x += __shfl_down_sync(0xffffffffu, s.x, o);
-        s.y += __shfl_down_sync(0xffffffffu, s.y, o);
-        s.z += __shfl_down_sync(0xffffffffu, s.z, o);
-        s.w += __shfl_down_sync(0xffffffffu, s.w, o);
-    }
-    if (lane == 0) {
-        red[warp][0] = s.x;
-        red[warp][1] = s.y;
-        red[warp][2] = s.z;
-        red[warp][3] = s.w;
-    }
+    __shared__ float4 red[256];
+    const int G = cout / 4, lanes = 256 / G, t = threadIdx.x, g = t / lanes;
+    const int p0 = blockIdx.x * b.chunk, p1 = min(p0 + b.chunk, b.npix);
+    if (g < G) red[t] = bias_lane(dout, G, LL, lanes, g, p0 + t - g * lanes, p1);
     __syncthreads();
-    if (threadIdx.x < 4) {
-        float v = 0.0f;
-        for (int w = 0; w < 8; ++w) v += red[w][threadIdx.x];
-        part[((size_t)img * nseg + seg) * cout + 4 * g + threadIdx.x] = v;
-    }
+    if (t < cout) b.part[(size_t)blockIdx.x * cout + t] = bias_channel(red, lanes, t);
 }
 
 // Weight update and every form of the weights that a pass reads, one launch for all layers (the
@@ -2118,71 +2047,72 @@ int check_flag(nmmc_gen* g) {
 // The sums asked for so far, one launch.
 int launch_sums(nmmc_gen* g, SumArgs& a) {
     int most = 0;
-    for (int k = 0; k < a.n; ++k) most = std::max(most, a.job[k].n);
-    if (a.n) launch_seq(g->stream, k_gen_sum_parts, dim3((most + 63) / 64, a.n), 128, 0, a);
+    for (int k = 0; k < a.n; ++k) most = std::max(most, a.job[k].wide ? a.job[k].n : (a.job[k].n + 127) / 128);
+    if (a.n) launch_seq(g->stream, k_gen_sum_parts, dim3(most, a.n), 128, 0, a);
     a.n = 0;
     a.used = 0;
     return cuda_check(cudaGetLastError(), "k_gen_sum_parts");
 }
 
-// Room for nparts partials of `stride` floats in the scratch, for the sums of job `add`ed next; sums
-// that hold too much of it are launched first. nullptr: too small.
-float* sum_room(nmmc_gen* g, SumArgs& a, size_t nparts, size_t stride) {
-    const size_t need = (nparts * stride + 3) / 4 * 4;
-    if (a.n == kSumJobs || a.used + need > g->wpart_cap)
+// `floats` of the scratch for the partials of the next `jobs` sums; sums that hold too much of it are
+// launched first. nullptr: too small.
+float* sum_room(nmmc_gen* g, SumArgs& a, size_t floats, int jobs) {
+    const size_t need = (floats + 3) / 4 * 4;
+    if (a.n + jobs > kSumJobs || a.used + need > g->wpart_cap)
         if (launch_sums(g, a)) return nullptr;
     if (need > g->wpart_cap) return nullptr;
-    a.job[a.n].part = g->wpart + a.used;
-    a.job[a.n].nparts = (int)nparts;
-    a.job[a.n].stride = (int)stride;
     a.used += need;
     return g->wpart + a.used - need;
 }
-void sum_add(SumArgs& a, float* gw, int nw, float* gb) {
-    SumJob& j = a.job[a.n++];
-    j.gw = gw;
-    j.gb = gb;
-    j.nw = nw;
-    j.n = gb ? j.stride : nw;
+void sum_add(SumArgs& a, const float* part, int nparts, int n, float* out, int wide) {
+    a.job[a.n++] = SumJob{part, out, nparts, n, wide};
+}
+
+// Blocks of a bias gradient's first stage: about two per SM, chunks of a multiple of 64 pixels.
+BiasArgs bias_shape(const nmmc_gen* g, int nimg) {
+    const int npix = nimg * g->L * g->L, want = 2 * std::max(1, g->sm_count);
+    BiasArgs b{nullptr, npix, 0, 0};
+    b.chunk = std::max(64, ((npix + want - 1) / want + 63) / 64 * 64);
+    b.nblk = (npix + b.chunk - 1) / b.chunk;
+    return b;
 }
 
 // Bias gradient gb[co] = sum over the batch's pixels of dout[p, co].
 int bgrad_launch(nmmc_gen* g, const float* dout, int nimg, int cout, float* gb, SumArgs& sums) {
-    const int LL = g->L * g->L, nseg = (LL + kBgradRun - 1) / kBgradRun;
+    BiasArgs b = bias_shape(g, nimg);
     if (cout % 4 != 0 || cout > 256) return set_error(NMMC_ERR_ARG, "bias gradient: channels not a multiple of 4");
-    float* part = sum_room(g, sums, (size_t)nimg * nseg, cout);
-    if (!part) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
-    launch_seq(g->stream, k_gen_bgrad_part, dim3(nseg, cout / 4, nimg), 256, 0, dout, LL, cout, nseg, part);
-    sum_add(sums, gb, cout, nullptr);
+    b.part = sum_room(g, sums, (size_t)b.nblk * cout, 1);
+    if (!b.part) return set_error(NMMC_ERR_ARG, "bias-gradient scratch too small");
+    launch_seq(g->stream, k_gen_bgrad_part, dim3(b.nblk), 256, 0, dout, g->L * g->L, cout, b);
+    sum_add(sums, b.part, b.nblk, cout, gb, 1);
     return cuda_check(cudaGetLastError(), "k_gen_bgrad_part");
 }
 
-// Hidden-layer weight and bias gradient on the tensor cores (k_gen_wgrad_tc): as many CTAs as SMs (one
-// per SM), as the partial scratch holds and as there are K-blocks.
-int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, float* gb, int nimg,
-                    SumArgs& sums) {
-    const int nw = 9 * tc::kC * tc::kC;
-    const int W = wg::block_len(g->L);
+// Partials of a weight gradient on the FMA pipes: one per pixel tile and kPartImages images.
+constexpr int kPartImages = 4;
+size_t tile_parts(int L, int nimg) { return (size_t)(L / kTile) * (L / kTile) * ((nimg + kPartImages - 1) / kPartImages); }
+
+// Hidden-layer weight and bias gradient on the tensor cores (k_gen_wgrad_tc). The number of partials,
+// and with it the order of the sums, is that of SMs, K-blocks or the largest batch's pixel tiles,
+// whichever is the smallest; few partials are shared by three CTAs each.
+int wgrad_tc_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float* gw, float* gb, int nimg, SumArgs& sums) {
+    const int W = wg::block_len(g->L), sms = std::max(1, g->sm_count);
     const int nkb = (int)((size_t)nimg * g->L * (g->L / W));
-    const int nparts = (int)std::min<size_t>({(size_t)nkb, (size_t)std::max(1, g->sm_count), g->wpart_cap / wg::kPart});
-    float* part = nparts < 1 ? nullptr : sum_room(g, sums, nparts, wg::kPart);
+    const int nparts = (int)std::min<size_t>({(size_t)nkb, (size_t)sms, tile_parts(g->L, g->bcap)});
+    if (nparts < 1) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
+    BiasArgs bias = gb ? bias_shape(g, nimg) : BiasArgs{nullptr, 0, 0, 0};
+    const size_t nw = (size_t)nparts * wg::kPart;
+    float* part = sum_room(g, sums, nw + (size_t)bias.nblk * tc::kC, gb ? 2 : 1);
     if (!part) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
-    const void* fn = W == 128 ? (const void*)k_gen_wgrad_tc<8>
-                   : W == 64 ? (const void*)k_gen_wgrad_tc<4>
-                   : W == 48 ? (const void*)k_gen_wgrad_tc<3>
-                   : W == 32 ? (const void*)k_gen_wgrad_tc<2> : (const void*)k_gen_wgrad_tc<1>;
-    if (int rc = ensure_smem(g, fn, (int)wg::kSmem, true)) return rc;
-    if (W == 128)
-        launch_seq(g->stream, k_gen_wgrad_tc<8>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
-    else if (W == 64)
-        launch_seq(g->stream, k_gen_wgrad_tc<4>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
-    else if (W == 48)
-        launch_seq(g->stream, k_gen_wgrad_tc<3>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
-    else if (W == 32)
-        launch_seq(g->stream, k_gen_wgrad_tc<2>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
-    else
-        launch_seq(g->stream, k_gen_wgrad_tc<1>, dim3(nparts), wg::kThreads, wg::kSmem, in, dout, part, g->L, nkb, g->d_flag);
-    sum_add(sums, gw, nw, gb);
+    if (gb) bias.part = part + nw;
+    const int split = 3 * nparts <= sms ? 3 : 1;
+    const int grid = std::max(nparts * split, std::min(sms, bias.nblk));
+    auto fn = W == 64 ? k_gen_wgrad_tc<4> : W == 48 ? k_gen_wgrad_tc<3> : W == 32 ? k_gen_wgrad_tc<2> : k_gen_wgrad_tc<1>;
+    const int smem = (int)wg::smem(W);
+    if (int rc = ensure_smem(g, (const void*)fn, smem, true)) return rc;
+    launch_seq(g->stream, fn, dim3(grid), wg::kThreads, smem, in, dout, part, g->L, nkb, nparts, split, bias, g->d_flag);
+    sum_add(sums, part, nparts, wg::kPart, gw, 0);
+    if (gb) sum_add(sums, bias.part, bias.nblk, tc::kC, gb, 1);
     return cuda_check(cudaGetLastError(), "k_gen_wgrad_tc");
 }
 
@@ -2192,23 +2122,21 @@ int wgrad_launch(nmmc_gen* g, const __nv_bfloat16* in, const float* dout, float*
                  SumArgs& sums) {
     if (CIN == tc::kC && COUT == tc::kC && g->use_tc && wg::block_len(g->L) > 0)
         return wgrad_tc_launch(g, in, dout, gw, gb, nimg, sums);
-    const int tiles = (g->L / kTile) * (g->L / kTile);
-    const int per = CIN == kGenC && COUT == kGenC ? 4 : kEdgePer;   // images of a CTA
-    const int groups = (nimg + per - 1) / per;
-    const int nparts = tiles * groups;
-    const size_t n = (size_t)9 * CIN * COUT;
-    float* part = sum_room(g, sums, nparts, n);
+    const int nparts = (int)tile_parts(g->L, nimg), n = 9 * CIN * COUT;
+    float* part = sum_room(g, sums, (size_t)nparts * n, 1);
     if (!part) return set_error(NMMC_ERR_ARG, "weight-gradient scratch too small");
     if constexpr (CIN == kGenC && COUT == kGenC) {
         const size_t smem = (size_t)((kTile + 2) * (kTile + 2) * CIN + kTile * kTile * COUT) * sizeof(float);
         if (int rc = ensure_smem(g, (const void*)k_gen_wgrad<CIN, COUT>, (int)smem, false)) return rc;
-        launch_seq(g->stream, k_gen_wgrad<CIN, COUT>, dim3(nparts), 432, smem, in, dout, part, g->L, per, nimg);
+        launch_seq(g->stream, k_gen_wgrad<CIN, COUT>, dim3(nparts), 432, smem, in, dout, part, g->L, kPartImages, nimg);
     } else {
-        using E = EdgeGrad<CIN, COUT>;
-        if (int rc = ensure_smem(g, (const void*)k_gen_wgrad_edge<CIN, COUT>, (int)E::smem, false)) return rc;
-        launch_seq(g->stream, k_gen_wgrad_edge<CIN, COUT>, dim3(nparts), E::kThreads, E::smem, in, dout, part, g->L, per, nimg);
+        constexpr int TI = COUT < 8 ? 4 : 8, TO = 4;   // 108 threads
+        using E = EdgeGrad<CIN, COUT, TI, TO>;
+        auto fn = k_gen_wgrad_edge<CIN, COUT, TI, TO>;
+        if (int rc = ensure_smem(g, (const void*)fn, (int)E::smem, false)) return rc;
+        launch_seq(g->stream, fn, dim3(nparts), E::kThreads, E::smem, in, dout, part, g->L, kPartImages, nimg);
     }
-    sum_add(sums, gw, (int)n, nullptr);
+    sum_add(sums, part, nparts, n, gw, 0);
     if (int rc = cuda_check(cudaGetLastError(), "k_gen_wgrad")) return rc;
     return gb ? bgrad_launch(g, dout, nimg, COUT, gb, sums) : NMMC_OK;
 }
@@ -2247,13 +2175,11 @@ int ensure_batch(nmmc_gen* g, int b) {
     NMMC_CUDA(cudaMalloc(&g->g0, np * kGenC * sizeof(float)));
     NMMC_CUDA(cudaMalloc(&g->g1, np * kGenC * sizeof(float)));
     NMMC_CUDA(cudaMalloc(&g->gv, np * kGenCout * sizeof(float)));
-    const int tiles = (g->L / kTile) * (g->L / kTile);
-    // the partials of one layer on the FMA pipes, or of a whole backward pass on the tensor cores
-    const size_t tc_parts = std::min<size_t>((size_t)b * g->L * std::max(1, g->L / 128), std::max(1, g->sm_count));
-    g->wpart_cap = std::max((size_t)tiles * ((b + 3) / 4) * wg::kPart,
-                            (kGenLayers - 2) * tc_parts * wg::kPart +
-                                (size_t)tiles * ((b + kEdgePer - 1) / kEdgePer) * 9 * kGenC * (kGenCin0 + kGenCout) +
-                                (size_t)b * ((g->L * g->L + kBgradRun - 1) / kBgradRun) * (kGenC + kGenCout));
+    // the partials of one hidden layer on the FMA pipes, or of all on the tensor cores; beside them those
+    // of the edge layers and of the biases
+    const size_t parts = tile_parts(g->L, b), tc_parts = std::min<size_t>(parts, std::max(1, g->sm_count));
+    g->wpart_cap = std::max(parts, (kGenLayers - 2) * tc_parts) * wg::kPart + parts * 9 * kGenC * (kGenCin0 + kGenCout) +
+                   (size_t)bias_shape(g, b).nblk * kGenLayers * kGenC;
     NMMC_CUDA(cudaMalloc(&g->wpart, g->wpart_cap * sizeof(float)));
     NMMC_CUDA(cudaMalloc(&g->d_idx, sizeof(int) * b));
     NMMC_CUDA(cudaMalloc(&g->d_sig, sizeof(float) * b));
