@@ -450,8 +450,8 @@ int nmmc_gen_gated_warm_start(nmmc_gen* gen, nmmc_ctx* ctx, const int* chains, i
 /* NMMC_GEN_OPT_TILE_ROWS: 1 or 2 (default), accepted for existing callers: the convolutions at
  * L = 128 take one output row per tile in either case. */
 #define NMMC_GEN_OPT_TILE_ROWS 2
-/* NMMC_GEN_OPT_WEIGHT_IMAGE: 1 (default) the convolutions at L = 128 copy each layer's
- * weights into shared memory as one bulk copy of an image in the tensor-core operand layout
+/* NMMC_GEN_OPT_WEIGHT_IMAGE: 1 (default) the tensor-core convolutions copy each layer's
+ * weights into shared memory as one bulk copy of an image in the operand layout
  * (rebuilt whenever the weights change); 0 the threads rearrange the BF16 weights; the same
  * results. */
 #define NMMC_GEN_OPT_WEIGHT_IMAGE 3

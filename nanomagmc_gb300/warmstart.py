@@ -65,7 +65,7 @@ class Generator:
         L.check(self.lib.nmmc_gen_set_option(self.h, L.GEN_OPT_SCHEDULE, int(kind)))
 
     def weight_image(self, on):
-        """Convolutions at L = 128: weights by one bulk copy of their operand image."""
+        """Tensor-core convolutions: weights by one bulk copy of their operand image."""
         L.check(self.lib.nmmc_gen_set_option(self.h, L.GEN_OPT_WEIGHT_IMAGE, int(bool(on))))
 
     def __del__(self):
