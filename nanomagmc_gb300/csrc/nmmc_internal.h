@@ -81,9 +81,9 @@ struct ResidentTables {
     // sweeps of every site, so that the resident kernel's updates skip the generator.
     bool hbm_faster = false;      // the autotuner timed the HBM path faster: the automatic path takes it
     bool stencil = false;         // sweeps run on the stencil resident kernel (nmmc_stencil.cu)
-    // lattices too large for the record kernel: by the number of chains of a call, whether the
-    // stencil kernel takes it (else the HBM path)
-    std::map<int, bool> large_stencil;
+    // lattices too large for the record kernel: by class of batch size and option setting, whether the
+    // stencil kernel takes a call (else the HBM path)
+    std::map<long long, bool> large_stencil;
     bool predraw = false;         // the shape in use launches the drawn-ahead variant
     int* d_site_chain = nullptr;  // per site: its chain
     uint4* d_draws = nullptr;     // [sweep of the launch][site] Philox words

@@ -733,9 +733,9 @@ std::string config_key(const Ctx& c) {
     for (int v : c.num) mix((uint64_t)v);
     mix((uint64_t)c.m.dmi_kind);
     // table and kernel format (5: the path choice, stencil kernel included, is part of the entry;
-    // 6: 16 bytes of shared memory per Heisenberg site; 7: the stencil kernel on clusters, for the
-    // lattices it covers)
-    mix(c.ising || c.masked || c.m.general ? 6 : 7);
+    // 6: 16 bytes of shared memory per Heisenberg site; 8: the stencil kernel on clusters, for the
+    // lattices it covers, with batch sizes in classes)
+    mix(c.ising || c.masked || c.m.general ? 6 : 8);
     std::string g = c.gpu_name;
     for (char& ch : g)
         if (ch == ' ') ch = '_';
@@ -774,9 +774,14 @@ struct TuningSnapshot {
     DeviceScratch ds;
     void* spins = nullptr;
     unsigned long long* sweep = nullptr;
+    bool room(Ctx& c) {
+        const bool ok = ds.alloc(&spins, c.spins_bytes) == cudaSuccess &&
+                        ds.alloc(&sweep, sizeof(unsigned long long) * c.nchains) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }
     int take(Ctx& c) {
-        NMMC_CUDA(ds.alloc(&spins, c.spins_bytes));
-        NMMC_CUDA(ds.alloc(&sweep, sizeof(unsigned long long) * c.nchains));
+        if (!sweep && !room(c)) return set_error(NMMC_ERR_CUDA, "autotuning: no memory for a copy of the chains");
         NMMC_CUDA(cudaMemcpyAsync(spins, c.d_spins, c.spins_bytes, cudaMemcpyDeviceToDevice, c.stream));
         NMMC_CUDA(cudaMemcpyAsync(sweep, c.d_sweep, sizeof(unsigned long long) * c.nchains, cudaMemcpyDeviceToDevice,
                                   c.stream));
@@ -819,30 +824,53 @@ float best_of_three(Ctx& c, Step step) {
 }
 
 // Lattices too large for the record kernel, on the automatic path: the stencil kernel on
-// clusters against the HBM path, by the same timing, for each number of chains that is swept
-// together (8 chains of 30^3 take 4.5 us per sweep against 10.6 in launches, 16 of them 8.9
-// against 11.0) and kept in the same cache. The streaming path keeps lattices that fit no cluster
-// and batches that fill the GPU many times.
+// clusters against the HBM path, by the same timing (8 chains of 30^3 take 4.5 us per sweep
+// against 10.6 in launches, 16 of them 8.9 against 11.0). The streaming path keeps lattices that
+// fit no cluster and batches that fill the GPU many times. One choice serves a class of batch sizes,
+// four classes to a factor of two, so that a list that shrinks from call to call is timed a few
+// times and not at every size; each setting of the options that change the HBM path's side has
+// choices of its own, and only those of the default settings go to the cache.
+int batch_class(int n) {
+    int step = 1;
+    while (8 * step < n) step *= 2;   // n <= 8: each its own; above, the multiples of 1/8 to 1/4 of n
+    return (n + step - 1) / step * step;
+}
+
+long long large_key(const Ctx& c, int n) {
+    return (long long)batch_class(n) | (long long)(c.measure_fp64 ? 1 : 0) << 20 | (long long)c.charge_pass << 21 |
+           (long long)c.measure_sites << 22 | (long long)c.l2_prefetch << 26;
+}
+
 int tune_large(Ctx& c, const int* d_chains, int n) {
-    if (n <= 0 || c.res.large_stencil.count(n)) return NMMC_OK;
+    // the options that pick a streaming variant keep the streaming path (resident_chosen)
+    if (n <= 0 || c.half_kernel != 0 || c.wave) return NMMC_OK;
+    const long long at = large_key(c, n);
+    if (c.res.large_stencil.count(at)) return NMMC_OK;
     if (c.res_stencil == 1 || stencil_shape(c, n).C < 1) {
-        c.res.large_stencil[n] = false;
+        c.res.large_stencil[at] = false;
         return NMMC_OK;
     }
     if (c.res_stencil == 2) {
-        c.res.large_stencil[n] = true;
+        c.res.large_stencil[at] = true;
         return NMMC_OK;
     }
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NMMC_CUDA(cudaStreamIsCapturing(c.stream, &cs));
     if (cs != cudaStreamCaptureStatusNone) return NMMC_OK;   // nothing is timed in a capture: the HBM path
-    const std::string key = config_key(c) + "/" + std::to_string(n);
+    const Ctx fresh{};   // the default settings
+    const bool usual = !c.measure_fp64 && c.charge_pass == fresh.charge_pass && c.measure_sites == fresh.measure_sites &&
+                       c.l2_prefetch == fresh.l2_prefetch;
+    const std::string key = config_key(c) + "/" + std::to_string(batch_class(n));
     int cb = 0, ct = 0, cp = 0, ch = 0;
-    if (cache_lookup(key, cb, ct, cp, ch)) {
-        c.res.large_stencil[n] = ch == 2;
+    if (usual && cache_lookup(key, cb, ct, cp, ch)) {
+        c.res.large_stencil[at] = ch == 2;
         return NMMC_OK;
     }
     TuningSnapshot snap;
+    if (!snap.room(c)) {   // no memory to put the chains aside: the HBM path, which needs none
+        c.res.large_stencil[at] = false;
+        return NMMC_OK;
+    }
     int rc = snap.take(c);
     if (rc) return rc;
     const bool fused = !c.measure_fp64;
@@ -850,8 +878,8 @@ int tune_large(Ctx& c, const int* d_chains, int n) {
     const float ts = best_of_three(c, [&](int k) { return launch_stencil_sweeps(c, d_chains, n, k, fused, 0); });
     cudaGetLastError();
     if ((rc = snap.restore(c))) return rc;
-    c.res.large_stencil[n] = ts < th;
-    cache_store(key, 0, 0, 0, ts < th ? 2 : 1);
+    c.res.large_stencil[at] = ts < th;
+    if (usual) cache_store(key, 0, 0, 0, ts < th ? 2 : 1);
     return NMMC_OK;
 }
 
@@ -1028,7 +1056,7 @@ int resident_prepare(Ctx& c, const int* d_chains, int n) {
 // The stencil kernel takes a call on n chains.
 static bool takes_stencil(const Ctx& c, int n) {
     if (c.res.eligible) return c.res.stencil;
-    const auto it = c.res.large_stencil.find(n);
+    const auto it = c.res.large_stencil.find(large_key(c, n));
     return it != c.res.large_stencil.end() && it->second;
 }
 
