@@ -496,10 +496,13 @@ static bool use_class(const Ctx& c) {
            class_table(c, true, t);
 }
 
-// The class planes, allocated at the first sweep; without the memory the sweeps stay in the box.
+// The class planes, allocated at the first sweep; without the memory, and in a stream capture that
+// comes before it, the sweeps stay in the box.
 bool class_ready(Ctx& c) {
     if (!use_class(c)) return false;
     if (c.d_class) return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
     const ClassShape s = class_shape(c);
     if (cudaMalloc(&c.d_class, (size_t)c.nchains * s.chain * sizeof(float4)) != cudaSuccess ||
         cudaMemsetAsync(c.d_class, 0, (size_t)c.nchains * s.chain * sizeof(float4), c.stream) != cudaSuccess) {
