@@ -15,6 +15,7 @@ namespace nmmc {
 
 int cuda_check(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return NMMC_OK;
+    cudaGetLastError();   // reported here, not again by the next launch
     return set_error(NMMC_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
@@ -853,13 +854,13 @@ int nmmc_set_av_chains(nmmc_ctx* c, const int* chains, int n) {
         for (int k = 0; k < i; ++k)
             if (chains[k] == chains[i]) return set_error(NMMC_ERR_ARG, "chain %d listed twice", chains[i]);
     }
-    const bool same = (size_t)n == c->av_chains.size() && std::equal(chains, chains + n, c->av_chains.begin());
-    if (same && n) {   // the list is on the device: only the sums start again
+    if (n && (size_t)n == c->av_chains.size() && std::equal(chains, chains + n, c->av_chains.begin())) {
+        // the list is on the device: only the sums start again
         NMMC_CUDA(cudaMemsetAsync(c->d_av, 0, sizeof(double) * 3 * (size_t)c->box_sites * n, c->stream));
         return NMMC_OK;
     }
     NMMC_CUDA(cudaStreamSynchronize(c->stream));
-    c->av_chains.assign(chains, chains + n);
+    c->av_chains.clear();   // nothing is summed until the list and its sums are on the device
     if (!n) return NMMC_OK;
     if ((size_t)n > c->av_cap) {
         cudaFree(c->d_av);
@@ -872,7 +873,8 @@ int nmmc_set_av_chains(nmmc_ctx* c, const int* chains, int n) {
         c->av_cap = (size_t)n;
     }
     NMMC_CUDA(cudaMemcpy(c->d_av_list, chains, sizeof(int) * n, cudaMemcpyHostToDevice));
-    NMMC_CUDA(cudaMemset(c->d_av, 0, sizeof(double) * 3 * (size_t)c->box_sites * n));
+    NMMC_CUDA(cudaMemsetAsync(c->d_av, 0, sizeof(double) * 3 * (size_t)c->box_sites * n, c->stream));
+    c->av_chains.assign(chains, chains + n);
     return NMMC_OK;
 }
 
