@@ -819,8 +819,11 @@ int nmmc_reset_accumulators(nmmc_ctx* c) {
 int nmmc_get_spins(nmmc_ctx* c, int chain, double* xyz, size_t n_sites) {
     if (!c || !xyz || chain < 0 || chain >= c->nchains) return set_error(NMMC_ERR_ARG, "bad argument");
     if (n_sites != (size_t)c->box_sites) return set_error(NMMC_ERR_ARG, "expected %lld sites", c->box_sites);
-    if (!c->d_replay && cudaMalloc(&c->d_replay, sizeof(double) * 3 * (size_t)c->box_sites) != cudaSuccess) {
-        cudaGetLastError();   // no room for the FP64 box: the planes are rearranged on the host
+    // the FP64 box on the device stays with the context; a large one, or one without room, is
+    // rearranged on the host instead
+    const size_t box_bytes = sizeof(double) * 3 * (size_t)c->box_sites;
+    if (!c->d_replay && (box_bytes > (64u << 20) || cudaMalloc(&c->d_replay, box_bytes) != cudaSuccess)) {
+        cudaGetLastError();
         c->d_replay = nullptr;
         const size_t bytes = chain_elems(*c) * elem_bytes(*c);
         std::vector<char> buf(bytes);
@@ -830,8 +833,7 @@ int nmmc_get_spins(nmmc_ctx* c, int chain, double* xyz, size_t n_sites) {
         return NMMC_OK;
     }
     if (int rc = launch_to_fp64(*c, chain)) return rc;
-    NMMC_CUDA(cudaMemcpyAsync(xyz, c->d_replay, sizeof(double) * 3 * (size_t)c->box_sites, cudaMemcpyDeviceToHost,
-                              c->stream));
+    NMMC_CUDA(cudaMemcpyAsync(xyz, c->d_replay, box_bytes, cudaMemcpyDeviceToHost, c->stream));
     NMMC_CUDA(cudaStreamSynchronize(c->stream));
     return NMMC_OK;
 }
