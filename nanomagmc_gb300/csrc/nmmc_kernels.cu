@@ -1984,58 +1984,101 @@ k_charge_rows(const DevModel m, const float* __restrict__ spins, const int* __re
     meas_block_rows<1>(qv, out + 10);
 }
 
-// Per-chain finish of the measurement kernels: the sums of the blocks' partials, side by side (an
-// FP64 addition takes about 40 cycles here): warps 0-9 a total each, warps 10-15 the slices'
-// charges, a slice per lane or, where there are few slices, a warp per slice. By one warp it took
-// 10 to 14 us: 24 Ising chains of 64^3, 10 sweeps and observables, 314 us, now 285.
-constexpr int kFinWarps = 16;
-__global__ void __launch_bounds__(32 * kFinWarps)
-k_measure_finalize(const int* __restrict__ chains, int nblk, int nblk_slice,
-                                   int nslices, int ising, const double* partial,
-                                   const double* __restrict__ Hd, double* obs,
-                                   double* q, double* accum,
-                                   int accumulate) {
+// Per-chain finish of the measurement kernels: the sums of the blocks' partials. FP64 additions are
+// slow here (about 40 cycles, and two lanes a cycle and SM), so with few chains their chains of
+// additions go side by side (SIDE): warps 0-9 a total each, warps 10-15 the slices' charges, a slice per
+// lane or, where there are few slices, a warp per slice; by one warp it took 10 to 14 us (24 Ising
+// chains of 64^3, 10 sweeps and observables, 314 us, side by side 285). Once there are more chains than
+// blocks of 16 warps fit the GPU, a warp per chain does the same sums in the same order: 5769 chains of
+// 7^3 took 103 us side by side.
+constexpr int kFinWarps = 16, kFinQ = kFinWarps - (kNP - 1);
+
+// Lane 0's sum of the warp's values, those of the lanes from n on being 0: the tree over all lanes
+// without the levels that add nothing.
+__device__ __forceinline__ double fin_tree(double v, int n) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        if (o < n) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
+}
+
+template <bool SIDE>
+__global__ void __launch_bounds__(SIDE ? 32 * kFinWarps : 32)
+k_measure_finalize(const int* __restrict__ chains, int nblk, int nblk_slice, int nslices, int ising, const double* partial,
+                   const double* __restrict__ Hd, double* obs, double* q, double* accum, int accumulate) {
     seq_begin();
-    __shared__ double tot[kNP - 1], qs[kFinWarps - (kNP - 1)];
     const int ci = blockIdx.x;
     const int chain = chains[ci];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double* pp = partial + (size_t)ci * nblk * kNP;
-    if (warp < kNP - 1) {
-        double v = 0;
-#pragma unroll 8
-        for (int b = lane; b < nblk; b += 32) v += ld_seq(pp + (size_t)b * kNP + warp);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) tot[warp] = v;
-    } else {
-        const int w = warp - (kNP - 1), nw = kFinWarps - (kNP - 1);
-        const bool tree = nslices < 32;   // a warp per slice, else a lane
+    const bool tree = nslices < 32;   // a warp per slice, else a lane
+    // the charges of the slices w, w + kFinQ, ... (tree) or 32 w + lane, ...: their sum, in lane 0
+    auto charges = [&](int w) -> double {
         double qsum = 0;
-        for (int zs = tree ? w : w * 32 + lane; zs < nslices; zs += tree ? nw : 32 * nw) {
+        for (int zs = tree ? w : w * 32 + lane; zs < nslices; zs += tree ? kFinQ : 32 * kFinQ) {
             const double* pz = pp + (size_t)zs * nblk_slice * kNP + 10;
             double v = 0;
 #pragma unroll 8
             for (int b = tree ? lane : 0; b < nblk_slice; b += tree ? 32 : 1) v += ld_seq(pz + (size_t)b * kNP);
-            if (tree)
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (tree) v = fin_tree(v, nblk_slice);
             if (tree && lane) continue;
             v = ising ? 0.0 : v / (2 * M_PI);
             if (q) q[(size_t)ci * nslices + zs] = v;
             qsum += v;
         }
         __syncwarp();
+        return fin_tree(qsum, tree ? 1 : 32);
+    };
+    double mine = 0.0, qsum = 0.0;   // lane k: total k
+    if (SIDE) {
+        __shared__ double tot[kNP - 1], qs[kFinQ];
+        if (warp < kNP - 1) {
+            double v = 0;
+#pragma unroll 8
+            for (int b = lane; b < nblk; b += 32) v += ld_seq(pp + (size_t)b * kNP + warp);
+            v = fin_tree(v, nblk);
+            if (lane == 0) tot[warp] = v;
+        } else {
+            const int w = warp - (kNP - 1);
+            const double v = charges(w);
+            if (lane == 0) qs[w] = v;
+        }
+        __syncthreads();
+        if (warp) return;
+        mine = lane < kNP - 1 ? tot[lane] : 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) qsum += __shfl_down_sync(0xffffffffu, qsum, o);
-        if (lane == 0) qs[w] = qsum;
+        for (int w = 0; w < kFinQ; ++w) qsum += qs[w];
+    } else {
+        double t[kNP - 1];
+#pragma unroll
+        for (int k = 0; k < kNP - 1; ++k) t[k] = 0.0;
+        for (int b = lane; b < nblk; b += 32)
+#pragma unroll
+            for (int k = 0; k < kNP - 1; ++k) t[k] += ld_seq(pp + (size_t)b * kNP + k);
+#pragma unroll
+        for (int k = 0; k < kNP - 1; ++k) {
+            const double v = __shfl_sync(0xffffffffu, fin_tree(t[k], nblk), 0);
+            if (lane == k) mine = v;
+        }
+        if (tree && nblk_slice == 1) {   // a slice per lane; their sums as above
+            double v = 0.0, s = 0.0;
+            if (lane < nslices) {
+                v = ising ? 0.0 : ld_seq(pp + (size_t)lane * kNP + 10) / (2 * M_PI);
+                if (q) q[(size_t)ci * nslices + lane] = v;
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j += kFinQ) {
+                const double u = __shfl_sync(0xffffffffu, v, (lane + j) & 31);
+                if (lane < kFinQ && lane + j < nslices) s += u;
+            }
+#pragma unroll
+            for (int w = 0; w < kFinQ; ++w) qsum += __shfl_sync(0xffffffffu, s, w);
+        } else {
+#pragma unroll 1
+            for (int w = 0; w < kFinQ; ++w) qsum += __shfl_sync(0xffffffffu, charges(w), 0);
+        }
     }
-    __syncthreads();
-    if (warp) return;
-    double qsum = 0;
-#pragma unroll
-    for (int w = 0; w < kFinWarps - (kNP - 1); ++w) qsum += qs[w];
-    finalize_chain_warp(lane < kNP - 1 ? tot[lane] : 0.0, lane, Hd + 3 * (size_t)chain, qsum, obs + (size_t)ci * NMMC_OBS_N,
+    finalize_chain_warp(mine, lane, Hd + 3 * (size_t)chain, qsum, obs + (size_t)ci * NMMC_OBS_N,
                         accum + (size_t)chain * NMMC_ACC_N, accumulate);
 }
 
@@ -2347,8 +2390,9 @@ static int measure_with(Ctx& c, const int* d_chains, int n, double* partial, dou
         int rc = launch_energy_general(c, d_chains, n, rows, nblk_slice, nblk, partial);
         if (rc) return rc;
     }
-    launch_seq(c, k_measure_finalize, dim3(n), 32 * kFinWarps, 0, d_chains, nblk, nblk_slice, c.m.lz, c.ising ? 1 : 0, partial,
-                                               c.d_Hd, obs, q, c.d_acc, accumulate);
+    const bool side = n <= 4 * c.sm_count;   // four blocks of 16 warps per SM
+    launch_seq(c, side ? k_measure_finalize<true> : k_measure_finalize<false>, dim3(n), side ? 32 * kFinWarps : 32, 0, d_chains, nblk,
+               nblk_slice, c.m.lz, c.ising ? 1 : 0, partial, c.d_Hd, obs, q, c.d_acc, accumulate);
     return cuda_check(cudaGetLastError(), "measure launch");
 }
 
