@@ -205,6 +205,21 @@ int sweep_measure_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, 
     return accumulate ? launch_add_av(c) : NMMC_OK;
 }
 
+// The observables of `rows` chains (q: nullptr not wanted), once the stream has written them.
+static int read_results(Ctx& c, double* obs, double* q, size_t rows) {
+    const size_t no = sizeof(double) * NMMC_OBS_N * rows, nq = sizeof(double) * c.nslices * rows;
+    if (!c.out_host) {
+        NMMC_CUDA(cudaMemcpyAsync(obs, c.d_obs, no, cudaMemcpyDeviceToHost, c.stream));
+        if (q) NMMC_CUDA(cudaMemcpyAsync(q, c.d_q, nq, cudaMemcpyDeviceToHost, c.stream));
+    }
+    NMMC_CUDA(cudaStreamSynchronize(c.stream));
+    if (c.out_host) {
+        memcpy(obs, c.d_obs, no);
+        if (q) memcpy(q, c.d_q, nq);
+    }
+    return NMMC_OK;
+}
+
 static void destroy_ctx(Ctx* c) {
     if (!c) return;
     resident_free(*c);
@@ -237,7 +252,8 @@ static void destroy_ctx(Ctx* c) {
     cudaFree(c->d_gjed);
     cudaFree(c->d_partial);
     cudaFree(c->d_mrows);
-    cudaFreeHost(c->h_out);   // d_obs and d_q live there
+    if (c->out_host) cudaFreeHost(c->out);   // d_obs and d_q live there
+    else cudaFree(c->out);
     cudaFree(c->d_acc);
     cudaFree(c->d_replay);
     cudaFree(c->d_flag);
@@ -568,14 +584,17 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
     NMMC_TRY(cudaMalloc(&c->d_list, sizeof(int) * nchains));
     NMMC_TRY(cudaMalloc(&c->d_active, nchains));
     NMMC_TRY(cudaMalloc(&c->d_pos, sizeof(int) * nchains));
-    // the observables go straight to page-locked host memory: a few doubles per chain, written by
-    // the finishing kernel, cost less than the copy that would follow it. Room for several samples
-    // of nmmc_sample.
-    c->out_stride = (size_t)(NMMC_OBS_N + c->nslices) * nchains;
-    c->out_slots = std::max<size_t>(1, std::min<size_t>(64, (64u << 10) / (c->out_stride * sizeof(double))));
-    NMMC_TRY(cudaHostAlloc(&c->h_out, c->out_slots * c->out_stride * sizeof(double), cudaHostAllocDefault));
-    c->d_obs = c->h_out;
-    c->d_q = c->h_out + (size_t)NMMC_OBS_N * nchains;
+    // Up to 64 KB of observables go straight to page-locked host memory: written by the finishing
+    // kernel they cost less than the copy that would follow it (4 KB: 10 us against 14). Out of that
+    // memory the host then reads 14 GB/s, so more is left on the device and copied (1 MB: 21 us against
+    // 75). Room for several samples of nmmc_sample.
+    const size_t out_bytes = (size_t)(NMMC_OBS_N + c->nslices) * nchains * sizeof(double);
+    c->out_host = out_bytes <= (64u << 10);
+    c->out_slots = std::max<size_t>(1, std::min<size_t>(64, (c->out_host ? (64u << 10) : (4u << 20)) / out_bytes));
+    if (c->out_host) NMMC_TRY(cudaHostAlloc(&c->out, c->out_slots * out_bytes, cudaHostAllocDefault));
+    else NMMC_TRY(cudaMalloc(&c->out, c->out_slots * out_bytes));
+    c->d_obs = c->out;
+    c->d_q = c->out + c->out_slots * (size_t)NMMC_OBS_N * nchains;
     NMMC_TRY(cudaMalloc(&c->d_acc, sizeof(double) * NMMC_ACC_N * nchains));
     NMMC_TRY(cudaMemset(c->d_acc, 0, sizeof(double) * NMMC_ACC_N * nchains));
     NMMC_TRY(cudaMalloc(&c->d_flag, sizeof(int)));
@@ -739,10 +758,7 @@ int nmmc_measure(nmmc_ctx* c, const int* chains, int n, double* obs, double* q, 
     if ((rc = launch_measure(*c, d, n, accumulate))) return rc;
     if (accumulate && (rc = launch_add_av(*c))) return rc;
     if (!obs) return NMMC_OK;   // results stay on the device (accumulators), no synchronisation
-    NMMC_CUDA(cudaStreamSynchronize(c->stream));
-    memcpy(obs, c->d_obs, sizeof(double) * NMMC_OBS_N * n);
-    if (q) memcpy(q, c->d_q, sizeof(double) * c->nslices * n);
-    return NMMC_OK;
+    return read_results(*c, obs, q, n);
 }
 
 int nmmc_sweep_measure(nmmc_ctx* c, const int* chains, int n, int nsweeps, double* obs, double* q, int accumulate) {
@@ -757,10 +773,7 @@ int nmmc_sweep_measure(nmmc_ctx* c, const int* chains, int n, int nsweeps, doubl
     if ((rc = measure_prepare(*c, n))) return rc;
     if ((rc = sweep_measure_impl(*c, d, chains, n, nsweeps, accumulate, true))) return rc;
     if (!obs) return NMMC_OK;   // results stay on the device (accumulators), no synchronisation
-    NMMC_CUDA(cudaStreamSynchronize(c->stream));
-    memcpy(obs, c->d_obs, sizeof(double) * NMMC_OBS_N * n);
-    if (q) memcpy(q, c->d_q, sizeof(double) * c->nslices * n);
-    return NMMC_OK;
+    return read_results(*c, obs, q, n);
 }
 
 int nmmc_sample(nmmc_ctx* c, const int* chains, int n, int nsweeps, int nsamples, double* obs, double* q) {
@@ -772,27 +785,26 @@ int nmmc_sample(nmmc_ctx* c, const int* chains, int n, int nsweeps, int nsamples
     if (!chains) n = c->nchains;
     if (nsamples == 0 || n == 0) return NMMC_OK;
     if ((rc = measure_prepare(*c, n))) return rc;
-    // each sample's observables into their own slot of the page-locked results, the host reading
-    // them out once per out_slots samples
+    // each sample's observables behind those of the sample before, the host reading them once per
+    // out_slots samples
     double *const obs0 = c->d_obs, *const q0 = c->d_q;
     const size_t no = (size_t)NMMC_OBS_N * n, nq = (size_t)c->nslices * n;
     for (int done = 0; done < nsamples && !rc;) {
         const int k = (int)std::min<size_t>(c->out_slots, (size_t)(nsamples - done));
         for (int s = 0; s < k && !rc; ++s) {
-            c->d_obs = obs0 + s * c->out_stride;
-            c->d_q = q0 + s * c->out_stride;
+            c->d_obs = obs0 + s * no;
+            c->d_q = q0 + s * nq;
             rc = sweep_measure_impl(*c, d, chains, n, nsweeps, 1, false);
         }
-        const cudaError_t se = cudaStreamSynchronize(c->stream);
-        if (!rc) rc = cuda_check(se, "nmmc_sample");
-        for (int s = 0; s < k && !rc; ++s) {
-            memcpy(obs + no * (done + s), obs0 + s * c->out_stride, no * sizeof(double));
-            if (q) memcpy(q + nq * (done + s), q0 + s * c->out_stride, nq * sizeof(double));
+        c->d_obs = obs0;
+        c->d_q = q0;
+        if (rc) {
+            cudaStreamSynchronize(c->stream);
+            return rc;
         }
+        rc = read_results(*c, obs + no * done, q ? q + nq * done : nullptr, (size_t)k * n);
         done += k;
     }
-    c->d_obs = obs0;
-    c->d_q = q0;
     return rc;
 }
 

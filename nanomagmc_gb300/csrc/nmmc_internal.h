@@ -183,10 +183,11 @@ struct Ctx {
     size_t partial_cap = 0;             // doubles
     double* d_mrows = nullptr;          // block rows of the fused half-sweeps (nmmc_sweep_measure, HBM path)
     size_t mrows_cap = 0;               // doubles
-    // results of the current call, in page-locked host memory (h_out: out_slots slots of out_stride
-    // doubles, each nchains x NMMC_OBS_N, then nchains x nslices)
-    double* h_out = nullptr;
-    size_t out_stride = 0, out_slots = 1;
+    // results of the current call: out_slots x nchains x NMMC_OBS_N, then out_slots x nchains x
+    // nslices doubles, in page-locked host memory (out_host) or on the device
+    double* out = nullptr;
+    bool out_host = false;
+    size_t out_slots = 1;
     double* d_obs = nullptr;            // n x NMMC_OBS_N
     double* d_q = nullptr;              // n x nslices
     double* d_acc = nullptr;            // nchains x NMMC_ACC_N
