@@ -831,10 +831,11 @@ int nmmc_reset_accumulators(nmmc_ctx* c) {
 int nmmc_get_spins(nmmc_ctx* c, int chain, double* xyz, size_t n_sites) {
     if (!c || !xyz || chain < 0 || chain >= c->nchains) return set_error(NMMC_ERR_ARG, "bad argument");
     if (n_sites != (size_t)c->box_sites) return set_error(NMMC_ERR_ARG, "expected %lld sites", c->box_sites);
-    // the FP64 box on the device stays with the context; a large one, or one without room, is
-    // rearranged on the host instead
+    // the FP64 box on the device stays with the context; a large one, or one without room, and a small
+    // one are rearranged on the host instead (24^2: 15 us, by way of the device 18; 64^2 21 and 21, 30^3
+    // 55 and 33)
     const size_t box_bytes = sizeof(double) * 3 * (size_t)c->box_sites;
-    if (!c->d_replay && (box_bytes > (64u << 20) || cudaMalloc(&c->d_replay, box_bytes) != cudaSuccess)) {
+    if (!c->d_replay && (c->box_sites < 4096 || box_bytes > (64u << 20) || cudaMalloc(&c->d_replay, box_bytes) != cudaSuccess)) {
         cudaGetLastError();
         c->d_replay = nullptr;
         const size_t bytes = chain_elems(*c) * elem_bytes(*c);
