@@ -171,7 +171,9 @@ int sweep_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, int nswe
     if (rc) return rc;
     bool res = use_resident(c, d_chains, n, &rc);
     if (rc) return rc;
-    return run_sweeps(c, d_chains, h_chains, n, nsweeps, res, false, 0, allow_timing);
+    rc = run_sweeps(c, d_chains, h_chains, n, nsweeps, res, false, 0, allow_timing);
+    c.planes_fresh = false;
+    return rc;
 }
 
 // nsweeps sweeps, then the observables of the listed chains. On the resident path of a 2-D
@@ -196,8 +198,8 @@ int sweep_measure_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, 
             if ((rc = launch_measure_fused_tail(c, d_chains, n, accumulate))) return rc;
             return accumulate ? launch_add_av(c) : NMMC_OK;
         }
+        c.planes_fresh = false;   // set by the sweeps that leave them so
         if ((rc = run_sweeps(c, d_chains, h_chains, n, nsweeps, res, false, 0, allow_timing))) return rc;
-        c.planes_fresh = !res;
     }
     rc = launch_measure(c, d_chains, n, accumulate);
     c.planes_fresh = false;

@@ -540,6 +540,7 @@ static int class_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps) {
                                                 (unsigned)k);
     if (int rc = cuda_check(cudaGetLastError(), "k_class_sweep")) return rc;
     if (int rc = class_copy(c, d_chains, n, false)) return rc;
+    c.planes_fresh = true;
     return launch_advance(c, d_chains, n, nsweeps);
 }
 
@@ -567,7 +568,10 @@ static ColourFn pick_colour_pm(const Ctx& c) {
 }
 
 int launch_colour_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps) {
-    if (class_ready(c)) return class_sweeps(c, d_chains, n, nsweeps);
+    // A class launch saves a quarter (4 classes in 2-D) to two fifths (6 in 3-D) of a box launch, and the
+    // two copies cost as much as six of those quarters: 6944 chains of 24^2, one sweep, 157 us in class
+    // planes and 134 in the box, two sweeps 237 and 246; 36 of 48^3 (6 classes) one sweep 172 and 222.
+    if ((long long)nsweeps * c.m.col_q > 4 && class_ready(c)) return class_sweeps(c, d_chains, n, nsweeps);
     ColourFn f = (c.dim == 3) ? (c.periodic ? pick_colour_pm<3, true>(c) : pick_colour_pm<3, false>(c))
                               : (c.periodic ? pick_colour_pm<2, true>(c) : pick_colour_pm<2, false>(c));
     for (int s = 0; s < nsweeps; ++s)
@@ -697,12 +701,14 @@ static void energy_pm(Ctx& c, const int* d, int n, int rows, int nbs, int nbt, d
 
 int launch_energy_general(Ctx& c, const int* d_chains, int n, int rows, int nblk_slice, int nblk_total,
                           double* partial) {
-    if (!c.measure_fp64 && use_class(c) && c.d_class) {
+    // In class planes for 3-D tables and a million sites on (36 chains of 48^3: 177 us with the gather,
+    // 240 in the box); below, a launch per class costs more than it saves (21 of 24^3: 57 and 50 us), and in
+    // 2-D few records share a row (6944 of 24^2: 345 and 267 us, 1736 of 48^2 177 and 158).
+    if (!c.measure_fp64 && c.dim == 3 && (long long)n * c.box_sites >= 1000000 && use_class(c) && c.d_class) {
         // a sample step's sweeps have left the listed chains' class planes current
         if (!c.planes_fresh)
             if (int rc = class_copy(c, d_chains, n, true)) return rc;
-        auto kern = c.dim == 3 ? (c.periodic ? k_class_energy<3, true> : k_class_energy<3, false>)
-                               : (c.periodic ? k_class_energy<2, true> : k_class_energy<2, false>);
+        auto kern = c.periodic ? k_class_energy<3, true> : k_class_energy<3, false>;
         const ClassShape s = class_shape(c);
         ClassTable t;
         class_table(c, false, t);

@@ -1216,6 +1216,7 @@ int launch_global_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool f
             for (int colour = 0; colour < 2; ++colour) fc(c, d_chains, n, colour, (unsigned)s);
         if ((rc = cuda_check(cudaGetLastError(), "compact half-sweep launch"))) return rc;
         if ((rc = compact_copy(c, d_chains, n, false))) return rc;
+        c.planes_fresh = true;
         return launch_advance(c, d_chains, n, nsweeps);
     }
     HalfFn f = pick_half(c);

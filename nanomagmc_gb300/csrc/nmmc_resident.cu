@@ -788,6 +788,7 @@ struct TuningSnapshot {
         return upload_params(c);
     }
     int restore(Ctx& c) {
+        c.planes_fresh = false;
         NMMC_CUDA(cudaMemcpyAsync(c.d_spins, spins, c.spins_bytes, cudaMemcpyDeviceToDevice, c.stream));
         NMMC_CUDA(cudaMemcpyAsync(c.d_sweep, sweep, sizeof(unsigned long long) * c.nchains, cudaMemcpyDeviceToDevice,
                                   c.stream));
