@@ -53,7 +53,8 @@ int upload_params(Ctx& c) {
                               cudaMemcpyHostToDevice, c.stream));
     NMMC_CUDA(cudaEventRecord(c.ev_params, c.stream));
     c.params_dirty = false;
-    return launch_ising_table(c);
+    c.itab_stale = true;
+    return NMMC_OK;
 }
 
 // A list that names every chain in order is the all-chains call: no list upload, and the

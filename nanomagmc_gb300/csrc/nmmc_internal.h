@@ -172,6 +172,7 @@ struct Ctx {
                                         // what its sweeps left
     float4* d_bh = nullptr;             // per chain (beta, H0, H1, H2) in FP32
     uint32_t* d_itab = nullptr;         // Ising word kernels: per chain 128 acceptance limits (nmmc_ising.cu)
+    bool itab_stale = true;             // (beta, H) were uploaded since
     double* d_Hd = nullptr;             // per chain H in FP64 (3 doubles) for the energy
     unsigned long long* d_sweep = nullptr;  // per chain sweep counter
     int* d_all = nullptr;               // 0..nchains-1
@@ -314,7 +315,7 @@ int launch_advance(Ctx& c, const int* d_chains, int n, int nsweeps);
 // ---- Ising words (nmmc_ising.cu) ----
 bool ising_words_ok(const Ctx& c);             // the lattice is covered
 size_t ising_table_bytes(const Ctx& c);
-int launch_ising_table(Ctx& c);                // acceptance limits from the uploaded (beta, H)
+int launch_ising_table(Ctx& c);                // acceptance limits from the uploaded (beta, H), when stale
 void launch_ising_words(Ctx& c, const int* d_chains, int n, int colour, unsigned off);
 void launch_measure_ising(Ctx& c, dim3 grid, const int* d_chains, int rows, int nblk_slice, double* partial);
 

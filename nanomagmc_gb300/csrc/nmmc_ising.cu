@@ -266,9 +266,13 @@ bool ising_words_ok(const Ctx& c) { return c.ising && !c.masked && !c.m.general 
 size_t ising_table_bytes(const Ctx& c) { return ising_words_ok(c) ? (size_t)c.nchains * kItabMax * sizeof(uint32_t) : 0; }
 
 int launch_ising_table(Ctx& c) {
-    if (!c.d_itab) return NMMC_OK;
+    if (!c.d_itab || !c.itab_stale) return NMMC_OK;
     k_ising_table<<<c.nchains, kItabMax, 0, c.stream>>>(c.m, c.d_bh, c.d_itab);
-    return cuda_check(cudaGetLastError(), "k_ising_table");
+    if (int rc = cuda_check(cudaGetLastError(), "k_ising_table")) return rc;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    NMMC_CUDA(cudaStreamIsCapturing(c.stream, &cs));
+    c.itab_stale = cs != cudaStreamCaptureStatusNone;   // what a capture records has not run yet
+    return NMMC_OK;
 }
 
 template <int DIM, bool PERIODIC, int W>

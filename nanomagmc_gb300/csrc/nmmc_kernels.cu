@@ -1220,6 +1220,8 @@ int launch_global_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool f
         return launch_advance(c, d_chains, n, nsweeps);
     }
     HalfFn f = pick_half(c);
+    if (f == (HalfFn)launch_ising_words)
+        if (int rc = launch_ising_table(c)) return rc;
     HalfFn fm = nullptr;   // the last sweep's colour-1 half-sweep with the observables summed on the way
     if (fused && nsweeps > 0)
         fm = c.dim == 3 ? (c.periodic ? pick_heis_q4_meas<3, true>(c.m.dmi_kind) : pick_heis_q4_meas<3, false>(c.m.dmi_kind))
