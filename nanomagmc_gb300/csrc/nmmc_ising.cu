@@ -266,12 +266,16 @@ bool ising_words_ok(const Ctx& c) { return c.ising && !c.masked && !c.m.general 
 size_t ising_table_bytes(const Ctx& c) { return ising_words_ok(c) ? (size_t)c.nchains * kItabMax * sizeof(uint32_t) : 0; }
 
 int launch_ising_table(Ctx& c) {
-    if (!c.d_itab || !c.itab_stale) return NMMC_OK;
-    k_ising_table<<<c.nchains, kItabMax, 0, c.stream>>>(c.m, c.d_bh, c.d_itab);
-    if (int rc = cuda_check(cudaGetLastError(), "k_ising_table")) return rc;
+    if (!c.d_itab) return NMMC_OK;
+    // a capture records the launch in any case: its graph may be replayed after other points were
+    // uploaded, and has not run yet
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NMMC_CUDA(cudaStreamIsCapturing(c.stream, &cs));
-    c.itab_stale = cs != cudaStreamCaptureStatusNone;   // what a capture records has not run yet
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    if (!c.itab_stale && !capturing) return NMMC_OK;
+    k_ising_table<<<c.nchains, kItabMax, 0, c.stream>>>(c.m, c.d_bh, c.d_itab);
+    if (int rc = cuda_check(cudaGetLastError(), "k_ising_table")) return rc;
+    if (!capturing) c.itab_stale = false;
     return NMMC_OK;
 }
 
