@@ -17,9 +17,11 @@ constexpr float kLn2 = 0.693147180559945f;
 // parameter is data that nothing else touches while the kernel runs, so its loads may take the
 // read-only path or move above the wait. __restrict__ stays on what the host uploads and on tables
 // that plainly launched kernels build.
+__device__ __forceinline__ void seq_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void seq_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void seq_begin() {
-    asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    seq_next();
+    seq_wait();
 }
 
 // Plain loads that stay behind seq_begin even where their value is all that depends on them

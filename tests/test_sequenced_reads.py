@@ -31,7 +31,7 @@ def sequenced_kernels():
             while depth:
                 depth += {"{": 1, "}": -1}.get(src[i], 0)
                 i += 1
-            if "seq_begin()" in src[m.end():i]:
+            if re.search(r"seq_(begin|wait)\(\)", src[m.end():i]):
                 out.append((os.path.basename(path), m.group(1), m.group(2), src[m.end():i]))
     return out
 
@@ -57,5 +57,5 @@ def test_reads_of_a_predecessors_data(file, name, params, body):
     for arg in re.findall(r"__ldg\(\s*([^)]*)", body):
         assert re.match(r"&?(\w+)", arg).group(1) in STATIC[file], arg
     # the wait comes before anything is read: only declarations and index arithmetic ahead of it
-    ahead = body[:body.index("seq_begin()")]
+    ahead = body[:re.search(r"seq_(begin|wait)\(\)", body).start()]
     assert not re.search(r"\b(chains|spins|sweep|planes|bh|in|dout)\s*\[", ahead), ahead
