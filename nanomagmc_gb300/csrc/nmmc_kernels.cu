@@ -16,13 +16,16 @@ namespace nmmc {
 // ------------------------------------------------------------------------------------------
 // Half-sweep kernels
 // ------------------------------------------------------------------------------------------
+// One site per thread. The next launch's blocks move in as this one's end: from the start (seq_begin)
+// they kept blocks of this launch waiting for a place (5 sweeps of 14000 chains of 4^3: 180 us, now 140,
+// by plain launches 165; 11 of 30^3 63 and 54).
 template <int DIM, bool PERIODIC, bool MASKED, int DK>
 __global__ void __launch_bounds__(256)
 k_heis_half(const DevModel m, float* spins, const uint32_t* __restrict__ fill,
             const int* __restrict__ fill_n, const float4* __restrict__ bh,
             const unsigned long long* sweep, const int* __restrict__ chains, int colour,
             unsigned sweep_off) {
-    seq_begin();
+    seq_wait();
     const int chain = chains[blockIdx.y];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (MASKED) {   // thread j: the chain's j-th filled site of this colour
