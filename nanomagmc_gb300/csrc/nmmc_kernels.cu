@@ -1994,9 +1994,8 @@ k_charge_rows(const DevModel m, const float* __restrict__ spins, const int* __re
 // slow here (about 40 cycles, and two lanes a cycle and SM), so with few chains their chains of
 // additions go side by side (SIDE): warps 0-9 a total each, warps 10-15 the slices' charges, a slice per
 // lane or, where there are few slices, a warp per slice; by one warp it took 10 to 14 us (24 Ising
-// chains of 64^3, 10 sweeps and observables, 314 us, side by side 285). Once there are more chains than
-// blocks of 16 warps fit the GPU, a warp per chain does the same sums in the same order: 5769 chains of
-// 7^3 took 103 us side by side.
+// chains of 64^3, 10 sweeps and observables, 314 us, side by side 285). With many chains a warp per
+// chain does the same sums in the same order (5769 chains of 7^3: 103 us side by side, 35).
 constexpr int kFinWarps = 16, kFinQ = kFinWarps - (kNP - 1);
 
 // Lane 0's sum of the warp's values, those of the lanes from n on being 0: the tree over all lanes
@@ -2396,9 +2395,14 @@ static int measure_with(Ctx& c, const int* d_chains, int n, double* partial, dou
         int rc = launch_energy_general(c, d_chains, n, rows, nblk_slice, nblk, partial);
         if (rc) return rc;
     }
-    const bool side = n <= 4 * c.sm_count;   // four blocks of 16 warps per SM
-    launch_seq(c, side ? k_measure_finalize<true> : k_measure_finalize<false>, dim3(n), side ? 32 * kFinWarps : 32, 0, d_chains, nblk,
-               nblk_slice, c.m.lz, c.ising ? 1 : 0, partial, c.d_Hd, obs, q, c.d_acc, accumulate);
+    // Two blocks of 16 warps per SM at most. The one-warp blocks come by a plain launch: waiting beside the
+    // measurement they would keep its blocks from being spread evenly (842 chains of 6^3 64 us, now 49).
+    if (n <= 2 * c.sm_count)
+        launch_seq(c, k_measure_finalize<true>, dim3(n), 32 * kFinWarps, 0, d_chains, nblk, nblk_slice, c.m.lz, c.ising ? 1 : 0,
+                   partial, c.d_Hd, obs, q, c.d_acc, accumulate);
+    else
+        k_measure_finalize<false><<<n, 32, 0, c.stream>>>(d_chains, nblk, nblk_slice, c.m.lz, c.ising ? 1 : 0, partial, c.d_Hd,
+                                                          obs, q, c.d_acc, accumulate);
     return cuda_check(cudaGetLastError(), "measure launch");
 }
 
