@@ -242,8 +242,7 @@ static void destroy_ctx(Ctx* c) {
     cudaFree(c->d_active);
     cudaFree(c->d_pos);
     cudaFree(c->d_rm);
-    cudaFreeHost(c->h_bh);   // h_hd lives in the same block
-    cudaFreeHost(c->h_list);
+    cudaFreeHost(c->h_bh);   // h_hd, h_list and results in page-locked memory live in the same block
     if (c->ev_params) cudaEventDestroy(c->ev_params);
     if (c->ev_list) cudaEventDestroy(c->ev_list);
     cudaFree(c->d_av);
@@ -255,8 +254,7 @@ static void destroy_ctx(Ctx* c) {
     cudaFree(c->d_gjed);
     cudaFree(c->d_partial);
     cudaFree(c->d_mrows);
-    if (c->out_host) cudaFreeHost(c->out);   // d_obs and d_q live there
-    else cudaFree(c->out);
+    if (!c->out_host) cudaFree(c->out);   // d_obs and d_q live there
     cudaFree(c->d_acc);
     cudaFree(c->d_replay);
     cudaFree(c->d_flag);
@@ -594,7 +592,14 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
     const size_t out_bytes = (size_t)(NMMC_OBS_N + c->nslices) * nchains * sizeof(double);
     c->out_host = out_bytes <= (64u << 10);
     c->out_slots = std::max<size_t>(1, std::min<size_t>(64, (c->out_host ? (64u << 10) : (4u << 20)) / out_bytes));
-    if (c->out_host) NMMC_TRY(cudaHostAlloc(&c->out, c->out_slots * out_bytes, cudaHostAllocDefault));
+    // One page-locked block (an allocation takes 50 us): points, results, list of chains.
+    auto lines = [](size_t b) { return (b + 127) / 128 * 128; };
+    const size_t point_bytes = lines((sizeof(float4) + 3 * sizeof(double)) * nchains);
+    const size_t results = c->out_host ? lines(c->out_slots * out_bytes) : 0;
+    NMMC_TRY(cudaHostAlloc(&c->h_bh, point_bytes + results + sizeof(int) * nchains, cudaHostAllocDefault));
+    c->h_hd = reinterpret_cast<double*>(c->h_bh + nchains);
+    c->h_list = reinterpret_cast<int*>(reinterpret_cast<char*>(c->h_bh) + point_bytes + results);
+    if (c->out_host) c->out = reinterpret_cast<double*>(reinterpret_cast<char*>(c->h_bh) + point_bytes);
     else NMMC_TRY(cudaMalloc(&c->out, c->out_slots * out_bytes));
     c->d_obs = c->out;
     c->d_q = c->out + c->out_slots * (size_t)NMMC_OBS_N * nchains;
@@ -602,9 +607,6 @@ int nmmc_create(const nmmc_options* opt, const nmmc_interactions* inter, const n
     NMMC_TRY(cudaMemset(c->d_acc, 0, sizeof(double) * NMMC_ACC_N * nchains));
     NMMC_TRY(cudaMalloc(&c->d_flag, sizeof(int)));
     NMMC_TRY(cudaMemset(c->d_flag, 0, sizeof(int)));
-    NMMC_TRY(cudaHostAlloc(&c->h_bh, (sizeof(float4) + 3 * sizeof(double)) * nchains, cudaHostAllocDefault));
-    c->h_hd = reinterpret_cast<double*>(c->h_bh + nchains);
-    NMMC_TRY(cudaHostAlloc(&c->h_list, sizeof(int) * nchains, cudaHostAllocDefault));
     NMMC_TRY(cudaEventCreateWithFlags(&c->ev_params, cudaEventDisableTiming));
     NMMC_TRY(cudaEventCreateWithFlags(&c->ev_list, cudaEventDisableTiming));
     NMMC_TRY(cudaMalloc(&c->d_rm, sizeof(ReplayModel)));
