@@ -94,16 +94,16 @@ static int set_list(Ctx& c, const int* chains, int n, const int** d_out) {
     return NMMC_OK;
 }
 
-static bool use_resident(Ctx& c, const int* d_chains, int n, int* rc) {
+static bool use_resident(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure, int* rc) {
     *rc = NMMC_OK;
     if (c.sweep_path == 1) return false;
-    *rc = resident_prepare(c, d_chains, n);
+    *rc = resident_prepare(c, d_chains, n, nsweeps, measure);
     if (*rc) return false;
     if (c.sweep_path == 2 && !c.res.eligible) {
         *rc = set_error(NMMC_ERR_UNSUPPORTED, "lattice does not fit the shared-memory resident path");
         return false;
     }
-    return resident_chosen(c, n);
+    return resident_chosen(c);
 }
 
 long long count_sites(const Ctx& c, const int* h_chains, int n) {
@@ -170,7 +170,7 @@ int sweep_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, int nswe
     if (nsweeps <= 0 || n == 0) return NMMC_OK;
     int rc = upload_params(c);
     if (rc) return rc;
-    bool res = use_resident(c, d_chains, n, &rc);
+    bool res = use_resident(c, d_chains, n, nsweeps, false, &rc);
     if (rc) return rc;
     rc = run_sweeps(c, d_chains, h_chains, n, nsweeps, res, false, 0, allow_timing);
     c.planes_fresh = false;
@@ -186,9 +186,9 @@ int sweep_measure_impl(Ctx& c, const int* d_chains, const int* h_chains, int n, 
     int rc = upload_params(c);
     if (rc) return rc;
     if (nsweeps > 0) {
-        bool res = use_resident(c, d_chains, n, &rc);
+        bool res = use_resident(c, d_chains, n, nsweeps, true, &rc);
         if (rc) return rc;
-        if (res && resident_can_measure(c, n)) {
+        if (res && resident_can_measure(c)) {
             if ((rc = run_sweeps(c, d_chains, h_chains, n, nsweeps, true, true, accumulate, allow_timing))) return rc;
             return accumulate ? launch_add_av(c) : NMMC_OK;
         }

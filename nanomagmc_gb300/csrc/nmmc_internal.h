@@ -81,9 +81,10 @@ struct ResidentTables {
     // sweeps of every site, so that the resident kernel's updates skip the generator.
     bool hbm_faster = false;      // the autotuner timed the HBM path faster: the automatic path takes it
     bool stencil = false;         // sweeps run on the stencil resident kernel (nmmc_stencil.cu)
-    // lattices too large for the record kernel: by class of batch size and option setting, whether the
-    // stencil kernel takes a call (else the HBM path)
+    // lattices too large for the record kernel: by class of batch size, sweeps and option setting,
+    // whether the stencil kernel takes a call (else the HBM path); and that of the call at hand
     std::map<long long, bool> large_stencil;
+    bool large_now = false;
     bool predraw = false;         // the shape in use launches the drawn-ahead variant
     int* d_site_chain = nullptr;  // per site: its chain
     uint4* d_draws = nullptr;     // [sweep of the launch][site] Philox words
@@ -334,15 +335,15 @@ StencilShape stencil_shape(const Ctx& c, int n);   // of a call on n chains; C =
 int launch_stencil_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure, int accumulate);
 
 // ---- resident kernel (nmmc_resident.cu) ----
-int resident_prepare(Ctx& c, const int* d_chains, int n);   // for a call on these n chains
+int resident_prepare(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure);   // for this call
 // all: the list is every chain in order. measure: after the sweeps, compute the listed
 // chains' observables in the same launch (2-D lattices; see resident_can_measure).
 int launch_resident_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool all, bool measure,
                            int accumulate);
-bool resident_can_measure(const Ctx& c, int n);
+bool resident_can_measure(const Ctx& c);
 // The sweeps of this context run on the resident path (after resident_prepare): the option,
 // eligibility, and on the automatic path the autotuner's choice between the two paths.
-bool resident_chosen(const Ctx& c, int n);
+bool resident_chosen(const Ctx& c);
 void resident_free(Ctx& c);
 // Compact form of masked Heisenberg lattices on the HBM path: allocates and builds the tables
 // of every chain when the sweeps will use it (a no-op otherwise or when built); and rebuilds

@@ -734,7 +734,7 @@ std::string config_key(const Ctx& c) {
     mix((uint64_t)c.m.dmi_kind);
     // table and kernel format (5: the path choice, stencil kernel included, is part of the entry;
     // 6: 16 bytes of shared memory per Heisenberg site; 8: the stencil kernel on clusters, for the
-    // lattices it covers, with batch sizes in classes)
+    // lattices it covers, with classes of batch sizes and sweeps)
     mix(c.ising || c.masked || c.m.general ? 6 : 8);
     std::string g = c.gpu_name;
     for (char& ch : g)
@@ -827,61 +827,70 @@ float best_of_three(Ctx& c, Step step) {
 // Lattices too large for the record kernel, on the automatic path: the stencil kernel on
 // clusters against the HBM path, by the same timing (8 chains of 30^3 take 4.5 us per sweep
 // against 10.6 in launches, 16 of them 8.9 against 11.0). The streaming path keeps lattices that
-// fit no cluster and batches that fill the GPU many times. One choice serves a class of batch sizes,
-// four classes to a factor of two, so that a list that shrinks from call to call is timed a few
-// times and not at every size; each setting of the options that change the HBM path's side has
-// choices of its own, and only those of the default settings go to the cache.
+// fit no cluster and batches that fill the GPU many times, and calls of one or two sweeps on larger
+// batches (the stencil kernel loads and stores the lattices in every call: 237 of 30^3, one sweep, 154 us
+// against 110). One choice serves a class of batch sizes, four classes to a factor of two, so that a
+// list that shrinks from call to call is timed a few times and not at every size; a class of sweeps
+// per call, with and without observables; each setting of the options that change the HBM path's
+// side has choices of its own, and only those of the default settings go to the cache.
 int batch_class(int n) {
     int step = 1;
     while (8 * step < n) step *= 2;   // n <= 8: each its own; above, the multiples of 1/8 to 1/4 of n
     return (n + step - 1) / step * step;
 }
 
-long long large_key(const Ctx& c, int n) {
-    return (long long)batch_class(n) | (long long)(c.measure_fp64 ? 1 : 0) << 20 | (long long)c.charge_pass << 21 |
+int sweeps_class(int nsweeps) { return nsweeps <= 1 ? 1 : nsweeps <= 2 ? 2 : nsweeps <= 4 ? 4 : 8; }
+
+long long large_key(const Ctx& c, int n, int k, bool measure) {
+    return (long long)batch_class(n) | (long long)k << 33 | (long long)(measure ? 1 : 0) << 37 | (long long)(c.measure_fp64 ? 1 : 0) << 20 | (long long)c.charge_pass << 21 |
            (long long)c.measure_sites << 22 | (long long)c.l2_prefetch << 26;
 }
 
-int tune_large(Ctx& c, const int* d_chains, int n) {
-    // the options that pick a streaming variant keep the streaming path (resident_chosen)
+int tune_large(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure) {
+    c.res.large_now = false;
+    // the options that pick a streaming variant keep the streaming path
     if (n <= 0 || c.half_kernel != 0 || c.wave) return NMMC_OK;
-    const long long at = large_key(c, n);
-    if (c.res.large_stencil.count(at)) return NMMC_OK;
-    if (c.res_stencil == 1 || stencil_shape(c, n).C < 1) {
-        c.res.large_stencil[at] = false;
+    const int k = sweeps_class(nsweeps);
+    const long long at = large_key(c, n, k, measure);
+    auto chosen = [&](bool stencil) {
+        c.res.large_stencil[at] = c.res.large_now = stencil;
+        return NMMC_OK;
+    };
+    const auto known = c.res.large_stencil.find(at);
+    if (known != c.res.large_stencil.end()) {
+        c.res.large_now = known->second;
         return NMMC_OK;
     }
-    if (c.res_stencil == 2) {
-        c.res.large_stencil[at] = true;
-        return NMMC_OK;
-    }
+    if (c.res_stencil == 1 || stencil_shape(c, n).C < 1) return chosen(false);
+    if (c.res_stencil == 2) return chosen(true);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NMMC_CUDA(cudaStreamIsCapturing(c.stream, &cs));
     if (cs != cudaStreamCaptureStatusNone) return NMMC_OK;   // nothing is timed in a capture: the HBM path
     const Ctx fresh{};   // the default settings
     const bool usual = !c.measure_fp64 && c.charge_pass == fresh.charge_pass && c.measure_sites == fresh.measure_sites &&
                        c.l2_prefetch == fresh.l2_prefetch;
-    const std::string key = config_key(c) + "/" + std::to_string(batch_class(n));
+    const std::string key = config_key(c) + "/" + std::to_string(batch_class(n)) + "/" + std::to_string(k) + (measure ? "m" : "");
     int cb = 0, ct = 0, cp = 0, ch = 0;
-    if (usual && cache_lookup(key, cb, ct, cp, ch)) {
-        c.res.large_stencil[at] = ch == 2;
-        return NMMC_OK;
-    }
+    if (usual && cache_lookup(key, cb, ct, cp, ch)) return chosen(ch == 2);
     TuningSnapshot snap;
-    if (!snap.room(c)) {   // no memory to put the chains aside: the HBM path, which needs none
-        c.res.large_stencil[at] = false;
-        return NMMC_OK;
-    }
+    if (!snap.room(c)) return chosen(false);   // no memory to put the chains aside: the HBM path, which needs none
     int rc = snap.take(c);
     if (rc) return rc;
-    const bool fused = !c.measure_fp64;
-    const float th = best_of_three(c, [&](int k) { return hbm_tuning_step(c, d_chains, n, k, fused); });
-    const float ts = best_of_three(c, [&](int k) { return launch_stencil_sweeps(c, d_chains, n, k, fused, 0); });
+    const bool fused = measure && !c.measure_fp64;
+    // `total` sweeps in calls of k
+    auto calls = [&](int total, auto one) {
+        int r = NMMC_OK;
+        for (int done = 0; done < total && r == NMMC_OK; done += k) r = one(std::min(k, total));
+        return r;
+    };
+    const float th = best_of_three(c, [&](int t) { return calls(t, [&](int s) { return hbm_tuning_step(c, d_chains, n, s, fused); }); });
+    const float ts = best_of_three(c, [&](int t) {
+        return calls(t, [&](int s) { return launch_stencil_sweeps(c, d_chains, n, s, fused, 0); });
+    });
     cudaGetLastError();
     if ((rc = snap.restore(c))) return rc;
-    c.res.large_stencil[at] = ts < th;
     if (usual) cache_store(key, 0, 0, 0, ts < th ? 2 : 1);
-    return NMMC_OK;
+    return chosen(ts < th);
 }
 
 }  // namespace
@@ -893,7 +902,7 @@ int resident_launches(const Ctx& c, int nsweeps) {
 }
 
 // Decides eligibility and builds the tables (autotuned unless options fix the shape).
-int resident_prepare(Ctx& c, const int* d_chains, int n) {
+int resident_prepare(Ctx& c, const int* d_chains, int n, int nsweeps, bool measure) {
     if (c.res.built) return NMMC_OK;
     const size_t budget = smem_budget(c);
     const int cap_sites = (int)std::min<size_t>(65534, budget / site_bytes(c) - 1);
@@ -902,7 +911,7 @@ int resident_prepare(Ctx& c, const int* d_chains, int n) {
     // general interaction tables use the multi-colour gather sweep
     c.res.eligible = maxn > 0 && maxn <= cap_sites && !c.m.general;
     // the stencil kernel covers unmasked Heisenberg lattices that fit a cluster
-    if (!c.res.eligible) return c.sweep_path == 0 ? tune_large(c, d_chains, n) : NMMC_OK;
+    if (!c.res.eligible) return c.sweep_path == 0 ? tune_large(c, d_chains, n, nsweeps, measure) : NMMC_OK;
     const bool stencil_ok = c.res_stencil != 1 && stencil_shape(c, c.nchains).C > 0;
 
     std::vector<int> load(c.num.begin(), c.num.end());
@@ -1054,16 +1063,11 @@ int resident_prepare(Ctx& c, const int* d_chains, int n) {
     return rc;
 }
 
-// The stencil kernel takes a call on n chains.
-static bool takes_stencil(const Ctx& c, int n) {
-    if (c.res.eligible) return c.res.stencil;
-    const auto it = c.res.large_stencil.find(large_key(c, n));
-    return it != c.res.large_stencil.end() && it->second;
-}
+// The stencil kernel takes the call at hand (resident_prepare).
+static bool takes_stencil(const Ctx& c) { return c.res.eligible ? c.res.stencil : c.res.large_now; }
 
-bool resident_chosen(const Ctx& c, int n) {
-    if (!c.res.eligible)   // the options that pick a streaming variant keep the streaming path
-        return c.sweep_path == 0 && takes_stencil(c, n) && c.half_kernel == 0 && !c.wave;
+bool resident_chosen(const Ctx& c) {
+    if (!c.res.eligible) return c.sweep_path == 0 && takes_stencil(c);
     return !(c.sweep_path == 0 && c.res.hbm_faster);
 }
 
@@ -1075,8 +1079,8 @@ __global__ void k_mark_active(uint8_t* active, int* pos, const int* chains, int 
     }
 }
 
-bool resident_can_measure(const Ctx& c, int n) {
-    if (takes_stencil(c, n) && resident_chosen(c, n)) return !c.measure_fp64;
+bool resident_can_measure(const Ctx& c) {
+    if (takes_stencil(c) && resident_chosen(c)) return !c.measure_fp64;
     // one z-slice, FP32 observables, and whole warps for the per-slot reductions
     return c.res.built && c.res.eligible && c.dim == 2 && !c.measure_fp64 && c.res.threads >= 32 &&
            c.res.threads % 32 == 0;
@@ -1084,8 +1088,8 @@ bool resident_can_measure(const Ctx& c, int n) {
 
 int launch_resident_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool all, bool measure,
                            int accumulate) {
-    if (takes_stencil(c, n)) {   // whole chains from the list: no chain marks needed
-        if (measure && !resident_can_measure(c, n)) return set_error(NMMC_ERR_UNSUPPORTED, "fused measurement not available");
+    if (takes_stencil(c)) {   // whole chains from the list: no chain marks needed
+        if (measure && !resident_can_measure(c)) return set_error(NMMC_ERR_UNSUPPORTED, "fused measurement not available");
         return launch_stencil_sweeps(c, d_chains, n, nsweeps, measure, accumulate);
     }
     // Mark the chains of this call; the others keep their spins and counters. A direct call on
@@ -1103,7 +1107,7 @@ int launch_resident_sweeps(Ctx& c, const int* d_chains, int n, int nsweeps, bool
         c.active_all = false;
     }
     if (!measure) return do_launch(c, nsweeps, nullptr);
-    if (!resident_can_measure(c, n)) return set_error(NMMC_ERR_UNSUPPORTED, "fused measurement not available");
+    if (!resident_can_measure(c)) return set_error(NMMC_ERR_UNSUPPORTED, "fused measurement not available");
     FusedMeasure fm{c.d_obs, c.d_q, c.d_acc, c.d_Hd, direct_all ? nullptr : c.d_pos,
                     c.res.d_slot_red, c.res.d_slot_black, accumulate};
     return do_launch(c, nsweeps, &fm);
