@@ -197,8 +197,6 @@ template <int SPT> struct SiteVec { using T = float4; };
 template <> struct SiteVec<2> { using T = float2; };
 __device__ __forceinline__ float vel(const float4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); }
 __device__ __forceinline__ float vel(const float2& v, int k) { return k == 0 ? v.x : v.y; }
-__device__ __forceinline__ float4 make_vec(const float (&a)[4]) { return make_float4(a[0], a[1], a[2], a[3]); }
-__device__ __forceinline__ float2 make_vec(const float (&a)[2]) { return make_float2(a[0], a[1]); }
 
 // Block sums of NV per-thread FP32 values: FP32 warp sums, then FP64 across the block's warps
 // on the lanes that own each value (every thread of the block must call it, from the same

@@ -37,8 +37,9 @@ __device__ __forceinline__ F2x2 shifted_quad(const F2x2& same, float ex, bool xp
 }
 
 // Adds one axis' terms of the local field to h (and, with EF, of its DMI part to d) for a pair
-// of sites whose +axis and -axis neighbours are P and M: the operations of heis_field (and
-// heis_dmi_part) for that axis. For the +-pair kinds the sign `flip` (axis 0 only) swaps the
+// of sites whose +axis and -axis neighbours are P and M: the operations of heis_field for that
+// axis, in its order; d takes the DMI's of them alone. For the +-pair kinds the sign `flip` (axis 0
+// only) swaps the
 // two neighbours' roles: their sum is symmetric and their difference changes sign, so it is
 // folded into the DMI strength and the neighbours need not be sorted by direction.
 template <int DK, int A, bool EF>
