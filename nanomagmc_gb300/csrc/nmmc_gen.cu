@@ -57,7 +57,7 @@ struct GenLayer {
     float* b = nullptr;              // [cout]
     __nv_bfloat16* wb = nullptr;     // BF16 compute copy [9][cin][cout]
     __nv_bfloat16* wt = nullptr;     // BF16 flipped transpose [9][cout][cin] (data gradient)
-    uint8_t* wimg = nullptr;         // BF16 weights in the tensor-core B layout of k_gen_conv_row
+    uint8_t* wimg = nullptr;         // BF16 weights in the tensor-core B layout (tc::place)
                                      // (kWimgBytes), staged by one bulk copy per CTA
     uint8_t* wtimg = nullptr;        // hidden layers: wt as TF32 in that layout (2 kWimgBytes)
     int kch = 0;                     // 16-byte chunks of K per tap in wimg
@@ -102,7 +102,7 @@ struct nmmc_gen {
     int use_ws = 0;                  // warp-specialised tcgen05 kernel for the BF16 modes (opt-in)
     int use_rows = 1;                // L = 128: the row-ring kernels (0: cp.async staging)
     int schedule = 0;                // warm-start noise levels: 0 linear, 1 quadratic, 2 cosine
-    int use_wimg = 1;                // the row-ring kernels stage the weights by one bulk copy of
+    int use_wimg = 1;                // the tensor-core kernels stage the weights by one bulk copy of
                                      // their image (0: the threads rearrange the BF16 weights)
     int sm_count = 0;
     int smem_per_sm = 0;             // shared memory per SM of the generator's device
@@ -735,8 +735,8 @@ k_gen_conv_tc(const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w, c
 // What bounds it: an MMA of M = 128 and K = 32 bytes reads A and B from shared memory, 45 cycles for
 // N = 48 and 74 for N = 144, so one per tap (27 in BF16, 54 in TF32 per row) costs nearly twice
 // what 9 or 18 wide ones do; beside that the start of a CTA (about 5 us) and, for the data
-// gradient, memory. 16 x 128^2: hidden forward layer 15.7 us, data gradient 21.7 us, first layer
-// 11.8 us, last 13.5 us; single-role CTAs with windows of four rows and one MMA per tap took
+// gradient, memory. 16 x 128^2: hidden forward layer 14.2 us, data gradient 21.0 us, first layer
+// 10.2 us, last 12.7 us; single-role CTAs with windows of four rows and one MMA per tap took
 // 18.5, 55, 12 and 17 us. 50 MB and 126 MB at the copy rate are 7.4 and 18.5 us.
 //   MODE 0: bias + ReLU, BF16 out (48 channels);  MODE 1: bias, FP32 out (48 channels);
 //   MODE 2: TF32 data gradient, times (activation > 0), FP32 out;
@@ -1229,11 +1229,12 @@ k_gen_conv_ws(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restr
 //                partial do nothing else.
 // Every wait is bounded and also ends when another role gave up (a shared abort word); a last
 // commit is waited for before the tensor memory is read or freed.
-// What bounds it: reads from L2 (16 x 128^2: 78 MB of input, every row for three blocks, and the
-// gradient's 50 MB twice; without the input's copies 34 us, without the bias 37) beside the MMAs'
-// operand reads (208 x 32 bytes each, 24 per block). 16 x 128^2: 39 us with the bias gradient; with
-// 30 bulk copies per block and the bias in launches of its own it was 62 + 31 us. Whole rows in
-// order with hi and lo in separate accumulators took 28.5 us, but that is another sum.
+// What bounds it: the MMAs (tensor pipe 59 % active, 72 cycles each for N = 144 whatever the rows of
+// A hold), what a CTA takes to start and to store its partials, and the reads from L2 beside them
+// (16 x 128^2: 78 MB of input, every row for three blocks, and the gradient's 50 MB twice; without the
+// input's copies 34 us, without the bias 37). 39 us with the bias gradient; with 30 bulk copies per
+// block and the bias in launches of its own it was 62 + 31 us. Whole rows in order with hi and lo in
+// separate accumulators took 28.5 us, but that is another sum.
 // ------------------------------------------------------------------------------------------
 namespace wg {
 constexpr int kStages = 6;
@@ -1719,8 +1720,8 @@ k_gen_wgrad_edge(const __nv_bfloat16* in, const float* dout, float* part, int L,
 // output adds the nparts partials from the first to the last. Biases (wide): a block per output,
 // thread t adds the partials t, t + 128, ..., then a tree. Both orders are part of the result.
 // What bounds it: the loads in flight, one chain of additions per output. The eight layers of 16 x
-// 128^2 (82 MB of partials) take 27.5 us with eight loads in flight per thread; with 4 29.7, with
-// 16 and 32 in predicated batches 51 and 90, two or four outputs per thread 34 and 45.
+// 128^2 (82 MB of partials) take 24 us with eight loads in flight per thread; in one comparison 8 27.5,
+// 4 29.7, 16 and 32 in predicated batches 51 and 90, two or four outputs per thread 34 and 45.
 struct SumJob {
     const float* part;
     float* out;
@@ -2011,9 +2012,6 @@ int conv_launch(nmmc_gen* g, const TIN* in, const __nv_bfloat16* w, const float*
     return cuda_check(cudaGetLastError(), "k_gen_conv");
 }
 
-// Hidden-layer convolution on the tensor cores: persistent CTAs, as many per SM as the shared
-// memory allows (two for the BF16 modes at L = 128, one for the TF32 data gradient).
-
 // L = 128: the row-ring kernel (every mode and layer shape), one CTA per SM. wimg: the layer's
 // weight image (nullptr: the threads rearrange w).
 template <int MODE, int ICH = tc::chunks<MODE>(), int KCH = ICH, int CO = tc::kC>
@@ -2031,6 +2029,8 @@ int conv_row_launch(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const 
 // and the row-ring kernels are on; false when they run on the FMA pipes.
 bool edge_layers_on_tc(const nmmc_gen* g) { return g->use_tc && g->use_rows && g->L == tc::kM; }
 
+// Hidden-layer convolution on the tensor cores: the row-ring kernel at L = 128, else persistent CTAs,
+// as many per SM as the shared memory allows (at most two).
 template <int MODE>
 int conv_tc_launch(nmmc_gen* g, const typename tc::Traits<MODE>::TA* in, const __nv_bfloat16* w, const float* bias,
                    const __nv_bfloat16* mask, void* out, int nimg, const uint8_t* wimg = nullptr) {

@@ -39,9 +39,8 @@ __device__ __forceinline__ F2x2 shifted_quad(const F2x2& same, float ex, bool xp
 // Adds one axis' terms of the local field to h (and, with EF, of its DMI part to d) for a pair
 // of sites whose +axis and -axis neighbours are P and M: the operations of heis_field for that
 // axis, in its order; d takes the DMI's of them alone. For the +-pair kinds the sign `flip` (axis 0
-// only) swaps the
-// two neighbours' roles: their sum is symmetric and their difference changes sign, so it is
-// folded into the DMI strength and the neighbours need not be sorted by direction.
+// only) swaps the two neighbours' roles: their sum is symmetric and their difference changes sign,
+// so it is folded into the DMI strength and the neighbours need not be sorted by direction.
 template <int DK, int A, bool EF>
 __device__ __forceinline__ void axis_terms(const DevModel& m, const f2 (&P)[3], const f2 (&M)[3], float flip,
                                            f2 (&h)[3], f2 (&d)[3]) {

@@ -344,8 +344,8 @@ def evaluate_point(gen: Generator, T, B, D, nchains=16, tmax=4000, every=10, ref
 
 def speed(L_edge=128, batch=16, steps=20, passes=16):
     """Generator timings with the hidden convolutions on the FP32 FMA pipes and on the tensor
-    cores (warp-specialised forward kernel, cp.async-staged windows, and the default: TMA-staged
-    windows at L = 128): training step (forward, backward, no update) and warm-start pass, in ms
+    cores (warp-specialised forward kernel, cp.async-staged windows, and the default, also as
+    mode 4: input rows through a ring at L = 128): training step (forward, backward, no update) and warm-start pass, in ms
     (wall time of synchronised calls, after warm-up)."""
     import time
     gen = Generator(L_edge, capacity=batch, seed=5)
@@ -356,7 +356,7 @@ def speed(L_edge=128, batch=16, steps=20, passes=16):
     gen.add_snapshots(s, np.arange(batch), cond)
     idx, sig = np.arange(batch, dtype=np.int32), np.full(batch, 0.5, np.float32)
     out = {"L": L_edge, "batch": batch}
-    for tensor in (0, 2, 3, 4, 1):   # FMA, cp.async WS, cp.async, TMA WS, default
+    for tensor in (0, 2, 3, 4, 1):   # FMA, cp.async WS, cp.async, default under its other number, default
         gen.tensor_cores(tensor)
         for _ in range(3):
             gen.train_step(idx, sig, lr=0.0)
