@@ -711,7 +711,9 @@ int launch_energy_general(Ctx& c, const int* d_chains, int n, int rows, int nblk
     // In class planes for 3-D tables and a million sites on (36 chains of 48^3: 177 us with the gather,
     // 240 in the box); below, a launch per class costs more than it saves (21 of 24^3: 57 and 50 us), and in
     // 2-D few records share a row (6944 of 24^2: 345 and 267 us, 1736 of 48^2 177 and 158).
-    if (!c.measure_fp64 && c.dim == 3 && (long long)n * c.box_sites >= 1000000 && use_class(c) && c.d_class) {
+    // Not for a caller's own scratch (nmmc_measure_static): its launches may be replayed from a graph
+    // while the context sweeps in those planes.
+    if (!c.measure_fp64 && c.dim == 3 && (long long)n * c.box_sites >= 1000000 && partial == c.d_partial && use_class(c) && c.d_class) {
         // a sample step's sweeps have left the listed chains' class planes current
         if (!c.planes_fresh)
             if (int rc = class_copy(c, d_chains, n, true)) return rc;
