@@ -309,6 +309,14 @@ static void planes_to_box(const Ctx& c, const void* planes, double* xyz) {
             }
 }
 
+// Whether a chain may hold empty Ising sites (spin 0), which the word kernels cannot.
+static void mark_empty(Ctx& c, int chain, bool empty) {
+    if (!c.ising || c.masked) return;
+    c.ising_empty.resize(c.nchains, 0);
+    c.ising_empties += (int)empty - (int)c.ising_empty[chain];
+    c.ising_empty[chain] = empty;
+}
+
 static size_t chain_elems(const Ctx& c) { return (size_t)2 * (c.ising ? 1 : 3) * c.m.nhalf_pad; }
 static size_t elem_bytes(const Ctx& c) { return c.ising ? 1 : 4; }
 
@@ -737,6 +745,7 @@ int nmmc_fork(nmmc_ctx* c, int src, int dst) {
     c->T[dst] = c->T[src];
     c->H[dst] = c->H[src];
     c->params_dirty = true;
+    mark_empty(*c, dst, !c->ising_empty.empty() && c->ising_empty[src]);
     return NMMC_OK;
 }
 
@@ -864,6 +873,9 @@ int nmmc_set_spins(nmmc_ctx* c, int chain, const double* xyz, size_t n_sites) {
     box_to_planes(*c, xyz, c->masked ? &c->mask[(size_t)chain * c->box_sites] : nullptr, buf.data());
     NMMC_CUDA(cudaStreamSynchronize(c->stream));
     NMMC_CUDA(cudaMemcpy((char*)c->d_spins + chain * bytes, buf.data(), bytes, cudaMemcpyHostToDevice));
+    bool empty = false;
+    for (size_t i = 0; c->ising && i < n_sites && !empty; ++i) empty = !(xyz[3 * i] > 0 || xyz[3 * i] < 0);
+    mark_empty(*c, chain, empty);
     return NMMC_OK;
 }
 

@@ -174,6 +174,8 @@ struct Ctx {
     float4* d_bh = nullptr;             // per chain (beta, H0, H1, H2) in FP32
     uint32_t* d_itab = nullptr;         // Ising word kernels: per chain 128 acceptance limits (nmmc_ising.cu)
     bool itab_stale = true;             // (beta, H) were uploaded since
+    std::vector<uint8_t> ising_empty;   // per chain (empty: none): it was given sites without a spin
+    int ising_empties = 0;              // such chains: the context's words stay unused
     double* d_Hd = nullptr;             // per chain H in FP64 (3 doubles) for the energy
     unsigned long long* d_sweep = nullptr;  // per chain sweep counter
     int* d_all = nullptr;               // 0..nchains-1

@@ -260,8 +260,8 @@ k_measure_ising(const DevModel m, const int8_t* __restrict__ spins, const int* _
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
-// Unmasked checkerboard lattices whose rows hold whole words of a colour.
-bool ising_words_ok(const Ctx& c) { return c.ising && !c.masked && !c.m.general && c.m.hx % 4 == 0; }
+// Unmasked checkerboard lattices whose rows hold whole words of a colour, every site +1 or -1.
+bool ising_words_ok(const Ctx& c) { return c.ising && !c.masked && !c.m.general && c.m.hx % 4 == 0 && c.ising_empties == 0; }
 
 size_t ising_table_bytes(const Ctx& c) { return ising_words_ok(c) ? (size_t)c.nchains * kItabMax * sizeof(uint32_t) : 0; }
 
