@@ -1989,16 +1989,23 @@ __global__ void k_gen_to_chain(const DevModel m, float* __restrict__ spins, cons
 // ------------------------------------------------------------------------------------------
 namespace {
 
-// Raises a kernel's dynamic shared-memory limit on the generator's device (once per size);
+// Raises a kernel's dynamic shared-memory limit on the generator's device (once per kernel and generator);
 // max_shared also asks for the whole L1/shared array as shared memory.
 int ensure_smem(nmmc_gen* g, const void* fn, int bytes, bool max_shared) {
-    auto it = g->attr_smem.find(fn);
-    if (it != g->attr_smem.end() && it->second >= bytes) return NMMC_OK;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (bytes <= g->attr_smem[fn]) return NMMC_OK;
+    // The limit belongs to the kernel, not to the generator: every generator sets the device's, so that one of
+    // a smaller edge does not lower it for the others.
+    cudaFuncAttributes at{};
+    int dev = 0, most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&at, fn);
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    most -= (int)at.sharedSizeBytes;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(most, bytes));
     if (e == cudaSuccess && max_shared)
         e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return cuda_check(e, "cudaFuncSetAttribute(generator kernel)");
-    g->attr_smem[fn] = bytes;
+    g->attr_smem[fn] = most;
     return NMMC_OK;
 }
 
